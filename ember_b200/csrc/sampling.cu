@@ -12,7 +12,8 @@
 // Instead of sorting, the k-th largest value and the top-p cut are found by radix selection
 // over an order-preserving integer image of the floats (4 passes of 8 bits; counts for top-k,
 // probability mass in double for top-p).  Ties at a cut are resolved as the host does, by
-// index: the cut keeps the lowest indices among equal values.  (The reference's device sampler,
+// index: the cut keeps the lowest indices among equal values.  A small top-k does not need the
+// selection over the whole row: see gather_candidates.  (The reference's device sampler,
 // src/backend/cuda/k_sampling.cu:149-166, has the same outline; this one is written anew.)
 #include "common.cuh"
 
@@ -22,6 +23,10 @@ namespace ember {
 
 constexpr int SAMPLE_THREADS = 1024;
 constexpr int SAMPLE_LIST = 1024;      // a top-k up to this size is finished on a list in shared memory
+constexpr int GROUP_LANES = 4;         // neighbouring threads that share a maximum in gather_candidates
+// Above this the candidates would often outgrow the list: of k largest values about k^2 / (2 * 2,048) share a group of
+// threads with a larger one, 64 at 512.
+constexpr int CANDIDATE_K = 512;
 
 struct SampleParams {  // 32 bytes per row, mirrored by the Python side
     float temperature;
@@ -73,10 +78,17 @@ struct Shared {
     // the kept set of a small top-k, gathered in the first block (any order), then sorted by (value descending,
     // index ascending)
     int n_list;
+    float cut;                      // gather_candidates: raw logits below this are out
+    int cut_ok, saw_nan;
     float list_x[SAMPLE_LIST];
     int list_i[SAMPLE_LIST];
-    float sort_x[SAMPLE_LIST];
-    int sort_i[SAMPLE_LIST];
+    union {
+        struct {
+            float sort_x[SAMPLE_LIST];
+            int sort_i[SAMPLE_LIST];
+        };
+        float maxima[8 * SAMPLE_THREADS / GROUP_LANES];         // of the groups of threads of a cluster of eight
+    };
     double sort_e[SAMPLE_LIST];
 };
 
@@ -281,6 +293,194 @@ __device__ int nth_equal_index(const float* __restrict__ logits, float inv_t_div
     return found;
 }
 
+// One pass of the selection of the remaining_k-th largest: sh.count holds how many keys with the prefix fall in each of
+// 256 bins; the bin is the first one (above 0), walking down from bin 255, at which the running count reaches what is
+// still wanted, else bin 0.  Done by threads 0..255 (barrier 1): thread b holds the count of bins b..255 (a suffix sum
+// over eight warps).
+__device__ __forceinline__ void decide_bin(Shared& sh, int shift, unsigned prefix, unsigned mask) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const unsigned own = sh.count[tid];
+    unsigned suf = own;                                 // within the warp: bins tid .. warp end
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned v = __shfl_down_sync(0xffffffffu, suf, o);
+        if (lane + o < 32) suf += v;
+    }
+    if (lane == 0) sh.warp_counts[warp] = (int)suf;     // total of this warp's 32 bins
+    asm volatile("bar.sync 1, 256;" ::: "memory");
+    unsigned above = 0;                                 // bins of the warps above this one
+    for (int w = warp + 1; w < 8; w++) above += (unsigned)sh.warp_counts[w];
+    const unsigned long long rem = sh.remaining_k;
+    const unsigned long long s_b = (unsigned long long)suf + above;     // count of bins tid..255
+    const unsigned long long s_next = s_b - own;                        // count of bins tid+1..255
+    const bool here = tid > 0 && s_b >= rem && s_next < rem;
+    const unsigned any = __ballot_sync(0xffffffffu, here);
+    if (lane == 0) sh.red_i[warp] = (int)any;
+    asm volatile("bar.sync 1, 256;" ::: "memory");
+    bool found = false;
+    for (int w = 0; w < 8; w++) found |= sh.red_i[w] != 0;
+    if (here || (!found && tid == 0)) {
+        sh.remaining_k = rem - s_next;      // how many of this bin (with the prefix) are still wanted
+        sh.prefix = prefix | ((unsigned)tid << shift);
+        sh.select_mask = mask | (255u << shift);
+    }
+}
+
+// The draw from a kept set of n <= SAMPLE_LIST elements (list_x, list_i in any order, in this block's shared memory), as
+// the host does it, on the list sorted by (value descending, index ascending): cumulative mass for top-p, min-p, the draw.
+// ``arg``: the largest element's index, ``xmax`` its value.  One block; block barriers only.
+__device__ void draw_from_list(Shared& sh, int n, const SampleParams& p, float xmax, int arg, int* __restrict__ out) {
+    const int tid = threadIdx.x;
+    // position of every element in the sorted order: how many come before it
+    for (int j = tid; j < n; j += SAMPLE_THREADS) {
+        const float xj = sh.list_x[j];
+        const int ij = sh.list_i[j];
+        int before = 0;
+        for (int l = 0; l < n; l++) {
+            const float xl = sh.list_x[l];
+            before += (xl > xj || (xl == xj && sh.list_i[l] < ij)) ? 1 : 0;
+        }
+        sh.sort_x[before] = xj;
+        sh.sort_i[before] = ij;
+        sh.sort_e[before] = exp((double)xj - (double)xmax);
+    }
+    __syncthreads();
+    // top-p: the shortest prefix whose mass reaches top_p * Z (one thread walks the list: it is short)
+    if (tid == 0) {
+        int keep_n = n;
+        if (p.top_p < 1.0f) {
+            double Z = 0.0;
+            for (int j = 0; j < n; j++) Z += sh.sort_e[j];
+            const double want = (double)p.top_p * Z;
+            double cum = 0.0;
+            keep_n = 0;
+            while (keep_n < n) {
+                cum += sh.sort_e[keep_n++];
+                if (cum >= want) break;
+            }
+        }
+        sh.found = keep_n;
+    }
+    __syncthreads();
+    const int keep_n = sh.found;
+    const double floor_p = p.min_p > 0.0f ? (double)p.min_p : -1.0;
+    float best_s = -INFINITY;
+    int best_t = 0x7fffffff;
+    for (int j = tid; j < keep_n; j += SAMPLE_THREADS) {
+        const int i = sh.sort_i[j];
+        if (floor_p > 0.0 && i != arg && !(sh.sort_e[j] >= floor_p)) continue;
+        const float s_ = sh.sort_x[j] + gumbel_noise(p.seed, p.counter, (unsigned)i);
+        if (s_ > best_s || (s_ == best_s && i < best_t)) { best_s = s_; best_t = i; }
+    }
+    int tok;
+    cluster_max_arg<1>(best_s, best_t, &tok, sh);
+    if (tid == 0) *out = tok == 0x7fffffff ? arg : tok;
+}
+
+// f(logit, index) for every element of [lo, hi), this thread's share.  ``pieces``: lo and the row are aligned to 16 bytes.
+template <typename F>
+__device__ __forceinline__ void scan_part(const float* __restrict__ logits, int lo, int hi, bool pieces, F f) {
+    if (pieces) {
+#pragma unroll 2
+        for (int i = lo + 4 * (int)threadIdx.x; i < hi; i += 4 * SAMPLE_THREADS) {      // hi is a multiple of 4
+            const float4 v = *(const float4*)(logits + i);
+            f(v.x, i); f(v.y, i + 1); f(v.z, i + 2); f(v.w, i + 3);
+        }
+    } else {
+        for (int i = lo + (int)threadIdx.x; i < hi; i += SAMPLE_THREADS) f(logits[i], i);
+    }
+}
+
+// A small top-k in two scans of the raw logits instead of seven of the scaled ones (which spend their time on the
+// division and on the cluster's barriers, not on memory: 32 rows of 151,936 with top-k 20 took 102 us, now 44 with the
+// parameters' copy).
+//
+// Every group of four threads has the largest logit it saw; the k-th largest L of the cluster's 2,048 group maxima
+// cannot lie above the k-th largest logit, so the kept set is among the elements whose scaled value reaches L / T.
+// Division by T is monotone, and elements below L that round to the same quotient are within 2^-22 of it, so
+// the second scan takes raw logits from L - 2^-21 |L| on; about k^2 / 4096 elements more than k come along.  The
+// first block divides these, keeps the k first by (key, index) and returns true there with the kept set in its list;
+// the other blocks return true too and are done.  False (in every block): a NaN, a cut that is no normal number, or
+// a list that overflowed (many equal values); nothing but the candidates' own fields has been touched.
+template <int CL>
+__device__ bool gather_candidates(const float* __restrict__ logits, int V, const SampleParams& p, Shared& sh) {
+    static_assert(CL * SAMPLE_THREADS / GROUP_LANES == 2 * SAMPLE_THREADS, "two group maxima per thread of the first block");
+    const int tid = threadIdx.x, lane = tid & 31;
+    const unsigned rank = cl_rank();
+    Shared* first = cl_peer<CL>(&sh, 0);
+    const int per = ((V + CL - 1) / CL + 3) / 4 * 4;
+    const int lo = min(V, (int)rank * per), hi = min(V, lo + per);
+    const bool pieces = (V & 3) == 0 && ((uintptr_t)logits & 15) == 0;
+
+    float best = -INFINITY;
+    scan_part(logits, lo, hi, pieces, [&](float x, int) { best = fmaxf(best, x); });      // a NaN is passed over here, seen below
+#pragma unroll
+    for (int o = 1; o < GROUP_LANES; o <<= 1) best = fmaxf(best, __shfl_xor_sync(0xffffffffu, best, o));
+    cl_sync<CL>();                                       // the first block has started
+    if (lane % GROUP_LANES == 0) first->maxima[(rank * SAMPLE_THREADS + tid) / GROUP_LANES] = best;
+    if (rank == 0 && tid == 0) { sh.prefix = 0; sh.select_mask = 0; sh.remaining_k = (unsigned long long)p.top_k; sh.n_list = 0; sh.saw_nan = 0; }
+    cl_sync<CL>();
+    if (rank == 0) {
+        const unsigned key0 = float_key(sh.maxima[tid]), key1 = float_key(sh.maxima[tid + SAMPLE_THREADS]);
+        for (int shift = 24; shift >= 0; shift -= 8) {
+            if (tid < 256) sh.count[tid] = 0;
+            __syncthreads();
+            const unsigned prefix = sh.prefix, mask = sh.select_mask;
+            if ((key0 & mask) == prefix) atomicAdd(&sh.count[(key0 >> shift) & 255u], 1u);
+            if ((key1 & mask) == prefix) atomicAdd(&sh.count[(key1 >> shift) & 255u], 1u);
+            __syncthreads();
+            if (tid < 256) decide_bin(sh, shift, prefix, mask);
+            __syncthreads();
+        }
+        if (tid == 0) {
+            const unsigned key = sh.prefix;
+            const float L = __uint_as_float((key & 0x80000000u) ? (key & 0x7fffffffu) : ~key);
+            const float x = L / p.temperature;
+            const float low = 1.17549435e-38f, high = 3.0e38f;       // normal, and L's neighbourhood finite
+            sh.cut_ok = fabsf(L) >= low && fabsf(L) <= high && fabsf(x) >= low && fabsf(x) <= high;
+            sh.cut = L - fabsf(L) * 4.76837158e-7f;
+        }
+    }
+    cl_sync<CL>();
+    if (!first->cut_ok) {
+        cl_sync<CL>();                                   // everybody has read it
+        return false;
+    }
+    const float cut = first->cut;
+    scan_part(logits, lo, hi, pieces, [&](float x, int i) {
+        if (x < cut) return;
+        if (x != x) first->saw_nan = 1;
+        const int slot = atomicAdd(&first->n_list, 1);
+        if (slot < SAMPLE_LIST) { first->list_x[slot] = x / p.temperature; first->list_i[slot] = i; }
+    });
+    cl_sync<CL>();
+    const int n = first->n_list;
+    const bool ok = n <= SAMPLE_LIST && !first->saw_nan;
+    cl_sync<CL>();
+    if (!ok || rank != 0) return ok;
+    // one element per thread: kept if fewer than k come before it
+    const float xj = tid < n ? sh.list_x[tid] : 0.0f;
+    const int ij = tid < n ? sh.list_i[tid] : 0;
+    const unsigned kj = float_key(xj);
+    int before = 0;
+    if (tid < n) {
+        for (int l = 0; l < n; l++) {
+            const unsigned kl = float_key(sh.list_x[l]);
+            before += (kl > kj || (kl == kj && sh.list_i[l] < ij)) ? 1 : 0;
+        }
+    }
+    __syncthreads();
+    if (tid == 0) sh.n_list = 0;
+    __syncthreads();
+    if (tid < n && before < p.top_k) {
+        const int slot = atomicAdd(&sh.n_list, 1);
+        sh.list_x[slot] = xj;
+        sh.list_i[slot] = ij;
+    }
+    __syncthreads();
+    return true;
+}
+
 template <int CL>
 __global__ void __launch_bounds__(SAMPLE_THREADS)
 sample_kernel(const float* __restrict__ logits_all, int V, const SampleParams* __restrict__ params,
@@ -295,8 +495,19 @@ sample_kernel(const float* __restrict__ logits_all, int V, const SampleParams* _
     const int per = (V + CL - 1) / CL;
     const int lo = min(V, (int)rank * per), hi = min(V, lo + per);
 
-    // ---- greedy, and the maximum for everything else
     const bool greedy = p.temperature <= 1e-5f;
+    if constexpr (CL > 1) {
+        if (!greedy && p.top_k > 0 && p.top_k <= CANDIDATE_K && gather_candidates<CL>(logits, V, p, sh)) {
+            if (rank != 0) return;
+            const int n = sh.n_list;
+            int arg;
+            const float xmax = cluster_max_arg<1>(tid < n ? sh.list_x[tid] : -INFINITY, tid < n ? sh.list_i[tid] : 0x7fffffff, &arg, sh);
+            draw_from_list(sh, n, p, xmax, arg, out + row);
+            return;
+        }
+    }
+
+    // ---- greedy, and the maximum for everything else
     const float tdiv = greedy ? 1.0f : p.temperature;
     float best = -INFINITY;
     int best_i = 0x7fffffff;
@@ -328,37 +539,7 @@ sample_kernel(const float* __restrict__ logits_all, int V, const SampleParams* _
             }
             __syncthreads();
             cluster_merge_bins<CL, false>(sh);
-            if (rank == 0 && tid < 256) {
-                // the bin of the k-th largest: walking down from bin 255, the first bin (above 0) at which the
-                // running count reaches what is still wanted, else bin 0.  Done by 256 threads: thread b holds
-                // the count of bins b..255 (a suffix sum over eight warps).
-                const int lane = tid & 31, warp = tid >> 5;
-                const unsigned own = sh.count[tid];
-                unsigned suf = own;                                 // within the warp: bins tid .. warp end
-#pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const unsigned v = __shfl_down_sync(0xffffffffu, suf, o);
-                    if (lane + o < 32) suf += v;
-                }
-                if (lane == 0) sh.warp_counts[warp] = (int)suf;     // total of this warp's 32 bins
-                asm volatile("bar.sync 1, 256;" ::: "memory");
-                unsigned above = 0;                                 // bins of the warps above this one
-                for (int w = warp + 1; w < 8; w++) above += (unsigned)sh.warp_counts[w];
-                const unsigned long long rem = sh.remaining_k;
-                const unsigned long long s_b = (unsigned long long)suf + above;     // count of bins tid..255
-                const unsigned long long s_next = s_b - own;                        // count of bins tid+1..255
-                const bool here = tid > 0 && s_b >= rem && s_next < rem;
-                const unsigned any = __ballot_sync(0xffffffffu, here);
-                if (lane == 0) sh.red_i[warp] = (int)any;
-                asm volatile("bar.sync 1, 256;" ::: "memory");
-                bool found = false;
-                for (int w = 0; w < 8; w++) found |= sh.red_i[w] != 0;
-                if (here || (!found && tid == 0)) {
-                    sh.remaining_k = rem - s_next;      // how many of this bin (with the prefix) are still wanted
-                    sh.prefix = prefix | ((unsigned)tid << shift);
-                    sh.select_mask = mask | (255u << shift);
-                }
-            }
+            if (rank == 0 && tid < 256) decide_bin(sh, shift, prefix, mask);
             cluster_share_decision<CL>(sh);
             __syncthreads();
         }
@@ -384,51 +565,7 @@ sample_kernel(const float* __restrict__ logits_all, int V, const SampleParams* _
         }
         cl_sync<CL>();
         if (rank != 0) return;                       // the first block goes on alone (block barriers only)
-        const int n = min(sh.n_list, SAMPLE_LIST);
-        // position of every element in the sorted order: how many come before it
-        for (int j = tid; j < n; j += SAMPLE_THREADS) {
-            const float xj = sh.list_x[j];
-            const int ij = sh.list_i[j];
-            int before = 0;
-            for (int l = 0; l < n; l++) {
-                const float xl = sh.list_x[l];
-                before += (xl > xj || (xl == xj && sh.list_i[l] < ij)) ? 1 : 0;
-            }
-            sh.sort_x[before] = xj;
-            sh.sort_i[before] = ij;
-            sh.sort_e[before] = exp((double)xj - (double)xmax);
-        }
-        __syncthreads();
-        // top-p: the shortest prefix whose mass reaches top_p * Z (one thread walks the list: it is short)
-        if (tid == 0) {
-            int keep_n = n;
-            if (p.top_p < 1.0f) {
-                double Z = 0.0;
-                for (int j = 0; j < n; j++) Z += sh.sort_e[j];
-                const double want = (double)p.top_p * Z;
-                double cum = 0.0;
-                keep_n = 0;
-                while (keep_n < n) {
-                    cum += sh.sort_e[keep_n++];
-                    if (cum >= want) break;
-                }
-            }
-            sh.found = keep_n;
-        }
-        __syncthreads();
-        const int keep_n = sh.found;
-        const double floor_p = p.min_p > 0.0f ? (double)p.min_p : -1.0;
-        float best_s = -INFINITY;
-        int best_t = 0x7fffffff;
-        for (int j = tid; j < keep_n; j += SAMPLE_THREADS) {
-            const int i = sh.sort_i[j];
-            if (floor_p > 0.0 && i != arg && !(sh.sort_e[j] >= floor_p)) continue;
-            const float s_ = sh.sort_x[j] + gumbel_noise(p.seed, p.counter, (unsigned)i);
-            if (s_ > best_s || (s_ == best_s && i < best_t)) { best_s = s_; best_t = i; }
-        }
-        int tok;
-        cluster_max_arg<1>(best_s, best_t, &tok, sh);
-        if (tid == 0) out[row] = tok == 0x7fffffff ? arg : tok;
+        draw_from_list(sh, min(sh.n_list, SAMPLE_LIST), p, xmax, arg, out + row);
         return;
     }
 

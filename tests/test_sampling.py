@@ -77,3 +77,32 @@ def test_device_draws_stay_in_the_kept_set_and_follow_the_distribution():
     top = max(dist, key=dist.get)
     freq, pt = float((got == top).mean()), dist[top]
     assert abs(freq - pt) < 4 * np.sqrt(pt * (1 - pt) / draws)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("vocab", [8192, 8195, 30004, 151936])
+@pytest.mark.parametrize("kind", ["normal", "ties", "run", "zeros", "infinite"])
+def test_device_sampler_small_top_k(vocab, kind):
+    """Rows whose small top-k is found among the maxima of groups of threads: the edge of that rule, ties at the cut, equal
+    values that outgrow the list, the largest values side by side (a few groups hold them all), a cut at zero, infinities."""
+    import torch
+    from ember_b200.sampling import device
+    rng = np.random.default_rng(vocab)
+    ks = [1, 2, 20, 200, 511, 512, 513]
+    rows = len(ks)
+    logits = (rng.standard_normal((rows, vocab)) * 3).astype(np.float32)
+    if kind == "ties":
+        logits = np.round(logits)
+    elif kind == "run":
+        logits[:, 700:1500] += 40.0
+    elif kind == "zeros":
+        logits = np.where(logits > 8.0, logits, 0.0).astype(np.float32)
+    elif kind == "infinite":
+        logits[:, ::3] = -np.inf
+        logits[3, 1::3] = -np.inf
+        logits[3, 50:] = -np.inf
+    params = [SamplingParams(temperature=[0.6, 1.0, 1.3][r % 3], top_k=k, top_p=[1.0, 0.95][r % 2], min_p=[0.0, 0.02][r // 4], seed=11 + r)
+              for r, k in enumerate(ks)]
+    counters = [3 + 7 * r for r in range(rows)]
+    got = device.sample(torch.from_numpy(logits).cuda(), params, counters).cpu().tolist()
+    assert got == [sample_host(logits[r], params[r], counters[r]) for r in range(rows)]
