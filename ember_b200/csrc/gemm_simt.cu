@@ -3,8 +3,15 @@
 // This is the true 32-bit matrix product of the float32 path (no tensor cores, no TF32) and
 // the fall-back of the bfloat16 path for shapes the tensor-core kernel refuses.  Activations A
 // are float or bf16, weights W are float or bf16 independently (a weight stored in 32-bit
-// stays so), accumulation is fp32 with k ascending for every output, so a row's result does
-// not depend on what else is in the batch.
+// stays so).  Accumulation is fp32 in an order that only K fixes, so a row's result does not
+// depend on what else is in the batch:
+//
+//   * float x float with rows of whole 16-byte pieces (every product of the float32 path): K is
+//     cut into KPARTS parts, each summed with k ascending, and the parts are added in order.  The
+//     parts are what lets a product of few tokens keep the whole chip busy; two kernels share
+//     this order, one for few tokens (bound by the weights' way in) and one for many (bound by
+//     the FMA pipes).
+//   * anything else: k ascending over the whole row, the kernel for all sizes.
 //
 // Epilogues (the reference's are src/backend/cuda/k_gemm.cu:29-53):
 //   0 store in the activation dtype      1 store fp32
@@ -92,6 +99,285 @@ gemm_simt_kernel(const TA* __restrict__ A, int lda, const TW* __restrict__ W, in
     }
 }
 
+// ---------------------------------------------------------------------------------------------------------------
+// float x float, 16-byte pieces.  Part p of K is [p * len, min(K, (p + 1) * len)), len a multiple of PART_UNIT.
+constexpr int KPARTS = 8, PART_UNIT = 32;
+
+__device__ __forceinline__ int part_length(int K) { return ((K + KPARTS - 1) / KPARTS + PART_UNIT - 1) / PART_UNIT * PART_UNIT; }
+
+// 16 bytes from global to shared memory without a register; zeros when !valid (src is then not read).
+__device__ __forceinline__ void copy16(float* dst, const float* src, bool valid) {
+    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(valid ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void copies_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void copies_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+// The sums of columns n and n + 1 (n even) of row m -> the output.
+__device__ __forceinline__ void finish_pair(float c0, float c1, const float* __restrict__ bias, float* __restrict__ C, int ldc, int m,
+                                            int n, int N, int epi) {
+    const bool two = n + 1 < N;
+    if (bias) {
+        c0 += bias[n];
+        if (two) c1 += bias[n + 1];
+    }
+    if (epi == 3 || epi == 6 || epi == 7) {                       // N is even
+        const float a = epi == 6 ? fmaxf(c0, 0.0f)
+                      : (epi == 7 ? 0.5f * c0 * (1.0f + tanhf(0.7978845608028654f * fmaf(0.044715f * c0 * c0, c0, c0))) : c0 / (1.0f + expf(-c0)));
+        C[(size_t)m * ldc + (n >> 1)] = a * c1;
+        return;
+    }
+    float* p = C + (size_t)m * ldc + n;
+    if (epi == 8) {
+        c0 = 0.5f * c0 * (1.0f + erff(c0 * 0.7071067811865476f));
+        c1 = 0.5f * c1 * (1.0f + erff(c1 * 0.7071067811865476f));
+    } else if (epi == 9) {
+        c0 = fmaxf(c0, 0.0f); c0 *= c0;
+        c1 = fmaxf(c1, 0.0f); c1 *= c1;
+    } else if (epi == 2) {
+        c0 += p[0];
+        if (two) c1 += p[1];
+    }
+    p[0] = c0;
+    if (two) p[1] = c1;
+}
+
+// Few tokens (MT of them per block): bound by the weights' way in.  A thread sums one part of K for one weight row
+// and MT tokens; a warp holds NB weight rows x 32 / NB parts and feeds itself through a ring of cp.async stages of 32
+// elements of k (a whole 128-byte line of each row), so nothing but the final addition of the parts needs a block
+// barrier and 3 x 4.5 KB a warp are on their way.  Weights that no earlier kernel writes are asked for before the
+// wait for the kernel before.  Rows of 36 floats keep the 16-byte reads of a quarter warp in different banks.
+// Four tokens at the 0.6B widths (hidden 1,024), in a step: o and down 9.1 and 13.8 us, gate/up 4.7, the head's 622 MB 99 us
+// (6.3 TB/s); with the 64 x 64 tiles of the general kernel a whole such step took about 15 ms, now 2.3 ms.
+constexpr int FEW_K = 32, FEW_STAGES = 3, FEW_ROW = FEW_K + 4;
+
+template <int MT, int NB>
+constexpr size_t few_stage_floats() { return 32 * FEW_ROW + (32 / NB) * MT * FEW_K; }
+template <int MT, int NB>
+constexpr size_t few_smem() { return (NB * KPARTS / 32) * FEW_STAGES * few_stage_floats<MT, NB>() * sizeof(float); }
+
+template <int MT, int NB>
+__global__ void __launch_bounds__(NB * KPARTS)
+gemm_f32_few_kernel(const float* __restrict__ A, int lda, const float* __restrict__ W, int ldw, const float* __restrict__ bias,
+                    float* __restrict__ C, int ldc, int M, int N, int K, int epi) {
+    extern __shared__ __align__(16) float few_shared[];
+    constexpr int WP = 32 / NB;                                   // parts of a warp
+    pdl_launch_dependents();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int n0 = blockIdx.x * NB, m0 = blockIdx.y * MT;
+    const int len = part_length(K), steps = len / FEW_K;
+    float* stages = few_shared + warp * FEW_STAGES * few_stage_floats<MT, NB>();
+    const int piece = (lane & 7) * 4;                             // this lane's 16 bytes of a row of a stage
+
+    auto fetch_w = [&](int step) {
+        float* dst = stages + (step % FEW_STAGES) * few_stage_floats<MT, NB>();
+#pragma unroll
+        for (int r0 = 0; r0 < 32; r0 += 4) {
+            const int r = r0 + (lane >> 3), part = warp * WP + r / NB, n = n0 + r % NB;
+            const int k = part * len + step * FEW_K + piece;
+            const bool ok = n < N && k < K;
+            copy16(dst + r * FEW_ROW + piece, ok ? W + (size_t)n * ldw + k : W, ok);
+        }
+    };
+    auto fetch_a = [&](int step) {
+        float* dst = stages + (step % FEW_STAGES) * few_stage_floats<MT, NB>() + 32 * FEW_ROW;
+#pragma unroll
+        for (int r0 = 0; r0 < WP * MT; r0 += 4) {
+            const int r = r0 + (lane >> 3), part = warp * WP + r / MT, m = m0 + r % MT;
+            const int k = part * len + step * FEW_K + piece;
+            const bool ok = m < M && k < K;
+            if (r < WP * MT) copy16(dst + r * FEW_K + piece, ok ? A + (size_t)m * lda + k : A, ok);
+        }
+    };
+#pragma unroll
+    for (int s = 0; s < FEW_STAGES - 1; s++)
+        if (s < steps) fetch_w(s);
+    pdl_wait();
+#pragma unroll
+    for (int s = 0; s < FEW_STAGES - 1; s++) {
+        if (s < steps) fetch_a(s);
+        copies_commit();
+    }
+
+    float acc[MT];
+#pragma unroll
+    for (int m = 0; m < MT; m++) acc[m] = 0.0f;
+    for (int step = 0; step < steps; step++) {
+        if (step + FEW_STAGES - 1 < steps) {
+            fetch_w(step + FEW_STAGES - 1);
+            fetch_a(step + FEW_STAGES - 1);
+        }
+        copies_commit();
+        copies_wait<FEW_STAGES - 1>();
+        __syncwarp();                                             // every lane's copies of this stage are there
+        const float* ws = stages + (step % FEW_STAGES) * few_stage_floats<MT, NB>();
+        const float* as = ws + 32 * FEW_ROW + (lane / NB) * MT * FEW_K;
+        ws += lane * FEW_ROW;
+#pragma unroll
+        for (int k = 0; k < FEW_K; k += 4) {
+            const float4 w = *(const float4*)(ws + k);
+#pragma unroll
+            for (int m = 0; m < MT; m++) {
+                const float4 a = *(const float4*)(as + m * FEW_K + k);
+                acc[m] = fmaf(a.x, w.x, acc[m]);
+                acc[m] = fmaf(a.y, w.y, acc[m]);
+                acc[m] = fmaf(a.z, w.z, acc[m]);
+                acc[m] = fmaf(a.w, w.w, acc[m]);
+            }
+        }
+        __syncwarp();                                             // the stage may be written again
+    }
+
+    copies_wait<0>();
+    __syncthreads();
+    float* parts = few_shared;                                    // [KPARTS][MT][NB]
+    const int part = threadIdx.x / NB, nn = threadIdx.x % NB;
+#pragma unroll
+    for (int m = 0; m < MT; m++) parts[(part * MT + m) * NB + nn] = acc[m];
+    __syncthreads();
+    for (int i = threadIdx.x; i < MT * NB / 2; i += NB * KPARTS) {
+        const int m = i / (NB / 2), n = (i % (NB / 2)) * 2;
+        if (m0 + m >= M || n0 + n >= N) continue;
+        float c0 = parts[m * NB + n], c1 = parts[m * NB + n + 1];
+#pragma unroll
+        for (int q = 1; q < KPARTS; q++) {
+            c0 += parts[(q * MT + m) * NB + n];
+            c1 += parts[(q * MT + m) * NB + n + 1];
+        }
+        finish_pair(c0, c1, bias, C, ldc, m0 + m, n0 + n, N, epi);
+    }
+}
+
+// Many tokens: bound by the FMA pipes.  A block makes a 64 x 64 tile, its eight warps one part of K each: a warp
+// keeps the whole tile of its part in registers (16 x 8 sums a thread, 24 eight-byte reads of shared memory per 256
+// FMAs) and feeds itself through two cp.async stages of 16 elements of k, so again only the addition of the parts
+// needs block barriers.  Rows of 20 floats keep the eight rows that a warp reads at once in different banks.
+// 300 tokens x 6,144 columns x 1,024: 137 us, 28 TFLOP/s.
+constexpr int MANY_T = 64, MANY_K = 16, MANY_ROW = MANY_K + 4, MANY_OUT = MANY_T + 8;
+constexpr int MANY_STAGE = 2 * MANY_T * MANY_ROW;                 // floats: 64 rows of A, 64 of W
+constexpr size_t MANY_SMEM = (size_t)KPARTS * 2 * MANY_STAGE * sizeof(float);
+static_assert(MANY_SMEM >= (size_t)KPARTS * MANY_T * MANY_OUT * sizeof(float), "the parts' tiles take the stages' place");
+
+__global__ void __launch_bounds__(KPARTS * 32, 1)
+gemm_f32_many_kernel(const float* __restrict__ A, int lda, const float* __restrict__ W, int ldw, const float* __restrict__ bias,
+                     float* __restrict__ C, int ldc, int M, int N, int K, int epi) {
+    extern __shared__ __align__(16) float many_shared[];
+    pdl_launch_dependents();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, tx = lane & 7, ty = lane >> 3;
+    const int n0 = blockIdx.x * MANY_T, m0 = blockIdx.y * MANY_T;
+    const int len = part_length(K), steps = len / MANY_K, k_first = warp * len;
+    float* stages = many_shared + warp * 2 * MANY_STAGE;
+    const int piece = (lane & 3) * 4;
+
+    auto fetch = [&](int step, const float* X, int ldx, int x0, int rows, float* dst) {
+        const int k = k_first + step * MANY_K + piece;
+#pragma unroll
+        for (int r0 = 0; r0 < MANY_T; r0 += 8) {
+            const int r = r0 + (lane >> 2);
+            const bool ok = x0 + r < rows && k < K;
+            copy16(dst + r * MANY_ROW + piece, ok ? X + (size_t)(x0 + r) * ldx + k : X, ok);
+        }
+    };
+    auto fetch_w = [&](int step) { fetch(step, W, ldw, n0, N, stages + (step & 1) * MANY_STAGE + MANY_T * MANY_ROW); };
+    auto fetch_a = [&](int step) { fetch(step, A, lda, m0, M, stages + (step & 1) * MANY_STAGE); };
+    fetch_w(0);
+    pdl_wait();
+    fetch_a(0);
+    copies_commit();
+
+    float acc[16][8];
+#pragma unroll
+    for (int i = 0; i < 16; i++)
+#pragma unroll
+        for (int j = 0; j < 8; j++) acc[i][j] = 0.0f;
+    for (int step = 0; step < steps; step++) {
+        if (step + 1 < steps) {
+            fetch_w(step + 1);
+            fetch_a(step + 1);
+        }
+        copies_commit();
+        copies_wait<1>();
+        __syncwarp();
+        const float* as = stages + (step & 1) * MANY_STAGE + ty * MANY_ROW;
+        const float* ws = stages + (step & 1) * MANY_STAGE + (MANY_T + tx) * MANY_ROW;
+#pragma unroll 2
+        for (int k = 0; k < MANY_K; k += 2) {
+            float2 a[16], w[8];
+#pragma unroll
+            for (int i = 0; i < 16; i++) a[i] = *(const float2*)(as + i * 4 * MANY_ROW + k);
+#pragma unroll
+            for (int j = 0; j < 8; j++) w[j] = *(const float2*)(ws + j * 8 * MANY_ROW + k);
+#pragma unroll
+            for (int i = 0; i < 16; i++)
+#pragma unroll
+                for (int j = 0; j < 8; j++) acc[i][j] = fmaf(a[i].x, w[j].x, acc[i][j]);
+#pragma unroll
+            for (int i = 0; i < 16; i++)
+#pragma unroll
+                for (int j = 0; j < 8; j++) acc[i][j] = fmaf(a[i].y, w[j].y, acc[i][j]);
+        }
+        __syncwarp();
+    }
+
+    copies_wait<0>();
+    __syncthreads();
+    float* parts = many_shared;                                   // [KPARTS][64][MANY_OUT]
+#pragma unroll
+    for (int i = 0; i < 16; i++)
+#pragma unroll
+        for (int j = 0; j < 8; j++) parts[(warp * MANY_T + i * 4 + ty) * MANY_OUT + j * 8 + tx] = acc[i][j];
+    __syncthreads();
+    for (int i = threadIdx.x; i < MANY_T * MANY_T / 2; i += KPARTS * 32) {
+        const int m = i / (MANY_T / 2), n = (i % (MANY_T / 2)) * 2;
+        if (m0 + m >= M || n0 + n >= N) continue;
+        float2 c = *(const float2*)(parts + m * MANY_OUT + n);
+#pragma unroll
+        for (int q = 1; q < KPARTS; q++) {
+            const float2 d = *(const float2*)(parts + (q * MANY_T + m) * MANY_OUT + n);
+            c.x += d.x;
+            c.y += d.y;
+        }
+        finish_pair(c.x, c.y, bias, C, ldc, m0 + m, n0 + n, N, epi);
+    }
+}
+
+template <typename Kernel>
+int launch_f32(Kernel kernel, dim3 grid, int threads, size_t smem, cudaStream_t st, const float* A, int lda, const float* W, int ldw,
+               const float* bias, float* C, int ldc, int M, int N, int K, int epi) {
+    if (smem > 48 * 1024) {
+        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return fail("gemm: shared memory %zu: %s", smem, cudaGetErrorString(e));
+    }
+    launch_kernel(kernel, grid, threads, smem, st, A, lda, W, ldw, bias, C, ldc, M, N, K, epi);
+    return check_launch("gemm_f32");
+}
+
+// Up to this many tokens the weights' way in is what a product waits for, even when two blocks read them (17 to 32
+// tokens, the second from the L2): a 64-token tile would be more than half padding.
+constexpr int FEW_TOKENS = 32;
+
+template <int MT>
+int launch_few(const float* A, int lda, const float* W, int ldw, const float* bias, float* C, int ldc, int M, int N, int K, int epi,
+               cudaStream_t st) {
+    const unsigned y = (unsigned)((M + MT - 1) / MT);
+    // blocks of 16 weight rows once they fill the SMs twice, else of 8
+    if (N >= 16 * 296)
+        return launch_f32(gemm_f32_few_kernel<MT, 16>, dim3((N + 15) / 16, y), 16 * KPARTS, few_smem<MT, 16>(), st, A, lda, W, ldw, bias, C, ldc, M, N, K, epi);
+    return launch_f32(gemm_f32_few_kernel<MT, 8>, dim3((N + 7) / 8, y), 8 * KPARTS, few_smem<MT, 8>(), st, A, lda, W, ldw, bias, C, ldc, M, N, K, epi);
+}
+
+int launch_pieces(const float* A, int lda, const float* W, int ldw, const float* bias, float* C, int ldc, int M, int N, int K, int epi,
+                  cudaStream_t st) {
+    if (M <= 1) return launch_few<1>(A, lda, W, ldw, bias, C, ldc, M, N, K, epi, st);
+    if (M <= 2) return launch_few<2>(A, lda, W, ldw, bias, C, ldc, M, N, K, epi, st);
+    if (M <= 4) return launch_few<4>(A, lda, W, ldw, bias, C, ldc, M, N, K, epi, st);
+    if (M <= 8) return launch_few<8>(A, lda, W, ldw, bias, C, ldc, M, N, K, epi, st);
+    if (M <= FEW_TOKENS) return launch_few<16>(A, lda, W, ldw, bias, C, ldc, M, N, K, epi, st);
+    return launch_f32(gemm_f32_many_kernel, dim3((N + MANY_T - 1) / MANY_T, (M + MANY_T - 1) / MANY_T), KPARTS * 32, MANY_SMEM, st, A, lda, W, ldw,
+                      bias, C, ldc, M, N, K, epi);
+}
+
 template <typename TA, typename TW>
 int launch(const void* A, int lda, const void* W, int ldw, const float* bias, void* C, int ldc, int M, int N, int K,
            int epi, cudaStream_t st) {
@@ -126,6 +412,13 @@ EMBER_API int ember_gemm_simt(const void* A, int a_dtype, int lda, const void* W
     if (ldc < (gated ? N / 2 : N)) return fail("gemm: output stride %d too small for N=%d", ldc, N);
     if ((M + BM - 1) / BM > 65535) return fail("gemm: M=%d is too large for one launch", M);
     cudaStream_t st = (cudaStream_t)stream;
+    const bool pieces = a_dtype == EMBER_F32 && w_dtype == EMBER_F32 && K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 &&
+                        (((uintptr_t)A | (uintptr_t)W) & 15) == 0;
+    if (pieces) {
+        if (epilogue != 0 && epilogue != 1 && epilogue != 2 && epilogue != 3 && !(epilogue >= 6 && epilogue <= 9))
+            return fail("gemm: unknown epilogue %d", epilogue);
+        return launch_pieces((const float*)A, lda, (const float*)W, ldw, bias, (float*)C, ldc, M, N, K, epilogue, st);
+    }
     if (a_dtype == EMBER_F32 && w_dtype == EMBER_F32)
         return launch<float, float>(A, lda, W, ldw, bias, C, ldc, M, N, K, epilogue, st);
     if (a_dtype == EMBER_F32 && w_dtype == EMBER_BF16)

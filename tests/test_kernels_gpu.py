@@ -130,6 +130,38 @@ def test_gemm_simt_is_independent_of_the_batch():
     assert torch.equal(one[0], full[77])
 
 
+@pytest.mark.parametrize("N,K", [(1, 4), (30, 36), (66, 260), (1000, 1000), (4735, 64), (4740, 260)])
+@pytest.mark.parametrize("epilogue", [1, 2, 3])
+def test_gemm_f32_kernels_share_one_order(N, K, epilogue):
+    """float32 products of whole 16-byte pieces: every count of tokens (the edges of both kernels and of their tiles) gives a
+    row the same bits, within the bound of a sum of K products in eight parts of at most ceil(K / 8) + 32."""
+    from ember_b200 import ops
+    if epilogue == 3 and N % 2:
+        N += 1
+    torch.manual_seed(N + K)
+    a = torch.randn(131, K, device="cuda")
+    w = torch.randn(N, K, device="cuda")
+    bias = torch.randn(N, device="cuda")
+    n_out = N // 2 if epilogue == 3 else N
+    prev = torch.randn(132, n_out, device="cuda")
+    c = a.double() @ w.double().t() + bias.double()
+    sums = a.double().abs() @ w.double().abs().t() + bias.double().abs() + 1.0
+    first = None
+    for M in (131, 1, 2, 3, 4, 7, 8, 9, 16, 17, 32, 33, 64, 65, 128):
+        out = prev.clone()
+        ops.gemm_simt(a, w, out, M, epilogue, bias=bias)
+        assert torch.equal(out[M:], prev[M:])
+        if first is None:
+            first = out
+            if epilogue != 3:
+                want = c + (prev[:M].double() if epilogue == 2 else 0.0)
+                assert float(((out[:M].double() - want).abs() / (sums + want.abs())).max()) < (K / 8 + 48) * 2.0 ** -24
+            else:
+                g, u = c[:, 0::2], c[:, 1::2]
+                assert rel(out[:M].double(), g * torch.sigmoid(g) * u) < 2e-6
+        assert torch.equal(out[:M], first[:M]), M
+
+
 @pytest.mark.parametrize("H", [64, 96, 1000, 2048, 5120])
 @pytest.mark.parametrize("odt", [torch.float32, torch.bfloat16])
 def test_rmsnorm(H, odt):
