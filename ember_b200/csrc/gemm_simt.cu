@@ -7,8 +7,8 @@
 // depend on what else is in the batch:
 //
 //   * float x float with rows of whole 16-byte pieces (every product of the float32 path): K is
-//     cut into KPARTS parts, each summed with k ascending, and the parts are added in order.  The
-//     parts are what lets a product of few tokens keep the whole chip busy; two kernels share
+//     cut into KPARTS parts, a part's elements of even k and of odd k are summed apart with k
+//     ascending, and the sums are added in order.  The parts are what lets a product of few tokens keep the whole chip busy; two kernels share
 //     this order, one for few tokens (bound by the weights' way in) and one for many (bound by
 //     the FMA pipes).
 //   * anything else: k ascending over the whole row, the kernel for all sizes.
@@ -114,6 +114,16 @@ __device__ __forceinline__ void copies_commit() { asm volatile("cp.async.commit_
 template <int N>
 __device__ __forceinline__ void copies_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
+// Two fp32 multiply-adds in one instruction, on elements k and k + 1 of two rows as they lie in shared memory.
+__device__ __forceinline__ unsigned long long fma_pair(unsigned long long a, unsigned long long b, unsigned long long c) {
+    unsigned long long d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ float pair_sum(unsigned long long v) {
+    return __uint_as_float((unsigned)v) + __uint_as_float((unsigned)(v >> 32));
+}
+
 // The sums of columns n and n + 1 (n even) of row m -> the output.
 __device__ __forceinline__ void finish_pair(float c0, float c1, const float* __restrict__ bias, float* __restrict__ C, int ldc, int m,
                                             int n, int N, int epi) {
@@ -200,9 +210,9 @@ gemm_f32_few_kernel(const float* __restrict__ A, int lda, const float* __restric
         copies_commit();
     }
 
-    float acc[MT];
+    unsigned long long acc[MT];
 #pragma unroll
-    for (int m = 0; m < MT; m++) acc[m] = 0.0f;
+    for (int m = 0; m < MT; m++) acc[m] = 0;
     for (int step = 0; step < steps; step++) {
         if (step + FEW_STAGES - 1 < steps) {
             fetch_w(step + FEW_STAGES - 1);
@@ -216,14 +226,12 @@ gemm_f32_few_kernel(const float* __restrict__ A, int lda, const float* __restric
         ws += lane * FEW_ROW;
 #pragma unroll
         for (int k = 0; k < FEW_K; k += 4) {
-            const float4 w = *(const float4*)(ws + k);
+            const ulonglong2 w = *(const ulonglong2*)(ws + k);
 #pragma unroll
             for (int m = 0; m < MT; m++) {
-                const float4 a = *(const float4*)(as + m * FEW_K + k);
-                acc[m] = fmaf(a.x, w.x, acc[m]);
-                acc[m] = fmaf(a.y, w.y, acc[m]);
-                acc[m] = fmaf(a.z, w.z, acc[m]);
-                acc[m] = fmaf(a.w, w.w, acc[m]);
+                const ulonglong2 a = *(const ulonglong2*)(as + m * FEW_K + k);
+                acc[m] = fma_pair(a.x, w.x, acc[m]);
+                acc[m] = fma_pair(a.y, w.y, acc[m]);
             }
         }
         __syncwarp();                                             // the stage may be written again
@@ -234,7 +242,7 @@ gemm_f32_few_kernel(const float* __restrict__ A, int lda, const float* __restric
     float* parts = few_shared;                                    // [KPARTS][MT][NB]
     const int part = threadIdx.x / NB, nn = threadIdx.x % NB;
 #pragma unroll
-    for (int m = 0; m < MT; m++) parts[(part * MT + m) * NB + nn] = acc[m];
+    for (int m = 0; m < MT; m++) parts[(part * MT + m) * NB + nn] = pair_sum(acc[m]);
     __syncthreads();
     for (int i = threadIdx.x; i < MT * NB / 2; i += NB * KPARTS) {
         const int m = i / (NB / 2), n = (i % (NB / 2)) * 2;
@@ -249,15 +257,16 @@ gemm_f32_few_kernel(const float* __restrict__ A, int lda, const float* __restric
     }
 }
 
-// Many tokens: bound by the FMA pipes.  A block makes a 64 x 64 tile, its eight warps one part of K each: a warp
-// keeps the whole tile of its part in registers (16 x 8 sums a thread, 24 eight-byte reads of shared memory per 256
-// FMAs) and feeds itself through two cp.async stages of 16 elements of k, so again only the addition of the parts
-// needs block barriers.  Rows of 20 floats keep the eight rows that a warp reads at once in different banks.
-// 300 tokens x 6,144 columns x 1,024: 137 us, 28 TFLOP/s.
-constexpr int MANY_T = 64, MANY_K = 16, MANY_ROW = MANY_K + 4, MANY_OUT = MANY_T + 8;
-constexpr int MANY_STAGE = 2 * MANY_T * MANY_ROW;                 // floats: 64 rows of A, 64 of W
+// Many tokens: bound by the FMA pipes.  A block makes a tile of 32 tokens x 64 columns, its eight warps one part of K
+// each: a warp keeps the whole tile of its part in registers (8 x 8 pairs of sums a thread, sixteen 16-byte reads of
+// shared memory per 128 paired multiply-adds) and feeds itself through two cp.async stages of 16 elements of k, so again
+// only the addition of the parts needs block barriers.  Rows of 20 floats keep the eight rows that a warp reads at
+// once in different banks.  Sums of one element of k at a time and tiles of 64 x 64 took 137 us for 300 tokens x 6,144
+// columns x 1,024, this 132.
+constexpr int MANY_M = 32, MANY_N = 64, MANY_K = 16, MANY_ROW = MANY_K + 4, MANY_OUT = MANY_N + 8;
+constexpr int MANY_STAGE = (MANY_M + MANY_N) * MANY_ROW;          // floats
 constexpr size_t MANY_SMEM = (size_t)KPARTS * 2 * MANY_STAGE * sizeof(float);
-static_assert(MANY_SMEM >= (size_t)KPARTS * MANY_T * MANY_OUT * sizeof(float), "the parts' tiles take the stages' place");
+static_assert(MANY_SMEM >= (size_t)KPARTS * MANY_M * MANY_OUT * sizeof(float), "the parts' tiles take the stages' place");
 
 __global__ void __launch_bounds__(KPARTS * 32, 1)
 gemm_f32_many_kernel(const float* __restrict__ A, int lda, const float* __restrict__ W, int ldw, const float* __restrict__ bias,
@@ -265,32 +274,41 @@ gemm_f32_many_kernel(const float* __restrict__ A, int lda, const float* __restri
     extern __shared__ __align__(16) float many_shared[];
     pdl_launch_dependents();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, tx = lane & 7, ty = lane >> 3;
-    const int n0 = blockIdx.x * MANY_T, m0 = blockIdx.y * MANY_T;
+    const int n0 = blockIdx.x * MANY_N, m0 = blockIdx.y * MANY_M;
     const int len = part_length(K), steps = len / MANY_K, k_first = warp * len;
     float* stages = many_shared + warp * 2 * MANY_STAGE;
     const int piece = (lane & 3) * 4;
 
-    auto fetch = [&](int step, const float* X, int ldx, int x0, int rows, float* dst) {
+    auto fetch_w = [&](int step) {
+        float* dst = stages + (step & 1) * MANY_STAGE + MANY_M * MANY_ROW;
         const int k = k_first + step * MANY_K + piece;
 #pragma unroll
-        for (int r0 = 0; r0 < MANY_T; r0 += 8) {
+        for (int r0 = 0; r0 < MANY_N; r0 += 8) {
             const int r = r0 + (lane >> 2);
-            const bool ok = x0 + r < rows && k < K;
-            copy16(dst + r * MANY_ROW + piece, ok ? X + (size_t)(x0 + r) * ldx + k : X, ok);
+            const bool ok = n0 + r < N && k < K;
+            copy16(dst + r * MANY_ROW + piece, ok ? W + (size_t)(n0 + r) * ldw + k : W, ok);
         }
     };
-    auto fetch_w = [&](int step) { fetch(step, W, ldw, n0, N, stages + (step & 1) * MANY_STAGE + MANY_T * MANY_ROW); };
-    auto fetch_a = [&](int step) { fetch(step, A, lda, m0, M, stages + (step & 1) * MANY_STAGE); };
+    auto fetch_a = [&](int step) {
+        float* dst = stages + (step & 1) * MANY_STAGE;
+        const int k = k_first + step * MANY_K + piece;
+#pragma unroll
+        for (int r0 = 0; r0 < MANY_M; r0 += 8) {
+            const int r = r0 + (lane >> 2);
+            const bool ok = m0 + r < M && k < K;
+            copy16(dst + r * MANY_ROW + piece, ok ? A + (size_t)(m0 + r) * lda + k : A, ok);
+        }
+    };
     fetch_w(0);
     pdl_wait();
     fetch_a(0);
     copies_commit();
 
-    float acc[16][8];
+    unsigned long long acc[8][8];                                 // token i * 4 + ty, column j * 8 + tx
 #pragma unroll
-    for (int i = 0; i < 16; i++)
+    for (int i = 0; i < 8; i++)
 #pragma unroll
-        for (int j = 0; j < 8; j++) acc[i][j] = 0.0f;
+        for (int j = 0; j < 8; j++) acc[i][j] = 0;
     for (int step = 0; step < steps; step++) {
         if (step + 1 < steps) {
             fetch_w(step + 1);
@@ -300,41 +318,41 @@ gemm_f32_many_kernel(const float* __restrict__ A, int lda, const float* __restri
         copies_wait<1>();
         __syncwarp();
         const float* as = stages + (step & 1) * MANY_STAGE + ty * MANY_ROW;
-        const float* ws = stages + (step & 1) * MANY_STAGE + (MANY_T + tx) * MANY_ROW;
-#pragma unroll 2
-        for (int k = 0; k < MANY_K; k += 2) {
-            float2 a[16], w[8];
+        const float* ws = stages + (step & 1) * MANY_STAGE + (MANY_M + tx) * MANY_ROW;
 #pragma unroll
-            for (int i = 0; i < 16; i++) a[i] = *(const float2*)(as + i * 4 * MANY_ROW + k);
+        for (int k = 0; k < MANY_K; k += 4) {
+            ulonglong2 a[8], w[8];
 #pragma unroll
-            for (int j = 0; j < 8; j++) w[j] = *(const float2*)(ws + j * 8 * MANY_ROW + k);
+            for (int i = 0; i < 8; i++) a[i] = *(const ulonglong2*)(as + i * 4 * MANY_ROW + k);
 #pragma unroll
-            for (int i = 0; i < 16; i++)
+            for (int j = 0; j < 8; j++) w[j] = *(const ulonglong2*)(ws + j * 8 * MANY_ROW + k);
 #pragma unroll
-                for (int j = 0; j < 8; j++) acc[i][j] = fmaf(a[i].x, w[j].x, acc[i][j]);
+            for (int i = 0; i < 8; i++)
 #pragma unroll
-            for (int i = 0; i < 16; i++)
+                for (int j = 0; j < 8; j++) acc[i][j] = fma_pair(a[i].x, w[j].x, acc[i][j]);
 #pragma unroll
-                for (int j = 0; j < 8; j++) acc[i][j] = fmaf(a[i].y, w[j].y, acc[i][j]);
+            for (int i = 0; i < 8; i++)
+#pragma unroll
+                for (int j = 0; j < 8; j++) acc[i][j] = fma_pair(a[i].y, w[j].y, acc[i][j]);
         }
         __syncwarp();
     }
 
     copies_wait<0>();
     __syncthreads();
-    float* parts = many_shared;                                   // [KPARTS][64][MANY_OUT]
+    float* parts = many_shared;                                   // [KPARTS][MANY_M][MANY_OUT]
 #pragma unroll
-    for (int i = 0; i < 16; i++)
+    for (int i = 0; i < 8; i++)
 #pragma unroll
-        for (int j = 0; j < 8; j++) parts[(warp * MANY_T + i * 4 + ty) * MANY_OUT + j * 8 + tx] = acc[i][j];
+        for (int j = 0; j < 8; j++) parts[(warp * MANY_M + i * 4 + ty) * MANY_OUT + j * 8 + tx] = pair_sum(acc[i][j]);
     __syncthreads();
-    for (int i = threadIdx.x; i < MANY_T * MANY_T / 2; i += KPARTS * 32) {
-        const int m = i / (MANY_T / 2), n = (i % (MANY_T / 2)) * 2;
+    for (int i = threadIdx.x; i < MANY_M * MANY_N / 2; i += KPARTS * 32) {
+        const int m = i / (MANY_N / 2), n = (i % (MANY_N / 2)) * 2;
         if (m0 + m >= M || n0 + n >= N) continue;
         float2 c = *(const float2*)(parts + m * MANY_OUT + n);
 #pragma unroll
         for (int q = 1; q < KPARTS; q++) {
-            const float2 d = *(const float2*)(parts + (q * MANY_T + m) * MANY_OUT + n);
+            const float2 d = *(const float2*)(parts + (q * MANY_M + m) * MANY_OUT + n);
             c.x += d.x;
             c.y += d.y;
         }
@@ -374,8 +392,15 @@ int launch_pieces(const float* A, int lda, const float* W, int ldw, const float*
     if (M <= 4) return launch_few<4>(A, lda, W, ldw, bias, C, ldc, M, N, K, epi, st);
     if (M <= 8) return launch_few<8>(A, lda, W, ldw, bias, C, ldc, M, N, K, epi, st);
     if (M <= FEW_TOKENS) return launch_few<16>(A, lda, W, ldw, bias, C, ldc, M, N, K, epi, st);
-    return launch_f32(gemm_f32_many_kernel, dim3((N + MANY_T - 1) / MANY_T, (M + MANY_T - 1) / MANY_T), KPARTS * 32, MANY_SMEM, st, A, lda, W, ldw,
-                      bias, C, ldc, M, N, K, epi);
+    // a grid has at most 65,535 rows of blocks, half as many tokens here as the 64-row tiles of the general kernel take
+    constexpr int ROWS = 65535 * MANY_M;
+    for (long long m = 0; m < M; m += ROWS) {
+        const int rows = M - m < ROWS ? (int)(M - m) : ROWS;
+        const int rc = launch_f32(gemm_f32_many_kernel, dim3((N + MANY_N - 1) / MANY_N, (rows + MANY_M - 1) / MANY_M), KPARTS * 32, MANY_SMEM, st,
+                                  A + (size_t)m * lda, lda, W, ldw, bias, C + (size_t)m * ldc, ldc, rows, N, K, epi);
+        if (rc) return rc;
+    }
+    return 0;
 }
 
 template <typename TA, typename TW>
