@@ -11,6 +11,8 @@
 // key tiles) x one split of the key range.  Splits have a fixed length anchored at key 0 and
 // are merged in ascending order by attention_combine, so the result for a token does not
 // depend on what else is in the step.
+#include <type_traits>
+
 #include "common.cuh"
 
 EMBER_DEFINE_LAST_ERROR
@@ -168,6 +170,200 @@ attention_tile_kernel(AttnParams p) {
     }
 }
 
+template <typename T>
+__device__ __forceinline__ float4 load4(const T* p);
+template <>
+__device__ __forceinline__ float4 load4<float>(const float* p) { return *(const float4*)p; }
+template <>
+__device__ __forceinline__ float4 load4<__nv_bfloat16>(const __nv_bfloat16* p) {
+    const uint2 u = *(const uint2*)p;
+    const float2 a = __bfloat1622float2(*(const __nv_bfloat162*)&u.x), b = __bfloat1622float2(*(const __nv_bfloat162*)&u.y);
+    return make_float4(a.x, a.y, b.x, b.y);
+}
+template <typename T>
+__device__ __forceinline__ void store4(T* p, float4 v) {
+    p[0] = from_float<T>(v.x); p[1] = from_float<T>(v.y); p[2] = from_float<T>(v.z); p[3] = from_float<T>(v.w);
+}
+template <>
+__device__ __forceinline__ void store4<float>(float* p, float4 v) { *(float4*)p = v; }
+
+// The same for heads of whole groups of four elements (N4 of them a lane): every sum in the same order, so the same bits.
+// What bounded the kernel above was not arithmetic but the way there: an index division and a page lookup for every
+// element, loads that nothing overlapped, one key tile's latency after another.  Here a warp copies whole keys (four a
+// tile, 16 bytes a lane), the next tile's are on their way while a tile is computed, and a warp's four rows share the
+// reads of a key and of a value.  A layer of the 0.6B widths, float32, four decoded tokens behind 75 and 300 prompt
+// tokens of four requests: 42 and 64 us with the kernel above.
+template <typename T, int N4>
+__global__ void __launch_bounds__(ATT_WARPS * 32, 1)
+attention_tile4_kernel(AttnParams p) {
+    extern __shared__ __align__(16) float smem[];
+    pdl_launch_dependents();
+    pdl_wait();
+    constexpr int R = ATT_ROWS_PER_WARP, KEYS = ATT_KT / ATT_WARPS;
+    const int D = p.D, DP = D + 4, D4 = D / 4;
+    float* Ks = smem;                       // [KT][D+4]
+    float* Vs = Ks + ATT_KT * DP;           // [KT][D]
+    float* Qs = Vs + ATT_KT * D;            // [rows][D]
+
+    const int tile = blockIdx.x, kvh = blockIdx.y, split = blockIdx.z;
+    const int seq = p.tiles[tile * 4 + 0], row0 = p.tiles[tile * 4 + 1], nq = p.tiles[tile * 4 + 2],
+              pos0 = p.tiles[tile * 4 + 3];
+    const int G = p.n_heads / p.n_kv;
+    const int rows = nq * G;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const T* q = (const T*)p.q;
+    const T* kp = (const T*)p.k_pool;
+    const T* vp = (const T*)p.v_pool;
+    const int* bt = p.block_table + (size_t)seq * p.max_blocks;
+
+    int lo = p.window > 0 ? max(0, pos0 - p.window + 1) : 0;
+    int hi = pos0 + nq;  // exclusive
+    if (p.n_splits > 1) {
+        lo = max(lo, split * p.split_keys);
+        hi = min(hi, (split + 1) * p.split_keys);
+    }
+    const int start = lo - (lo % ATT_KT);
+
+    float4 kr[KEYS][N4], vr[KEYS][N4];      // this lane's pieces of the warp's keys of the next tile
+    auto fetch = [&](int k0) {
+#pragma unroll
+        for (int i = 0; i < KEYS; i++) {
+            const int key = k0 + warp + ATT_WARPS * i;
+            size_t off = 0;
+            bool ok = key >= lo && key < hi;
+            if (ok) {
+                const int blk = bt[key / p.page];
+                ok = blk >= 0 && blk < p.num_pages;
+                if (ok) off = (((size_t)blk * p.n_kv + kvh) * p.page + (key % p.page)) * D;
+                else if (lane == 0 && p.err) atomicOr(p.err, EMBER_ERR_PAGE_RANGE);
+            }
+#pragma unroll
+            for (int c = 0; c < N4; c++) {
+                const int d = (lane + 32 * c) * 4;
+                const bool here = ok && d < D;
+                kr[i][c] = here ? load4<T>(kp + off + d) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                vr[i][c] = here ? load4<T>(vp + off + d) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            }
+        }
+    };
+    if (start < hi) fetch(start);
+    // queries of this tile -> shared memory (row r = query r / G, head kvh * G + r % G)
+    for (int r = warp; r < rows; r += ATT_WARPS) {
+        const T* src = q + ((size_t)(row0 + r / G) * p.n_heads + kvh * G + r % G) * D;
+        for (int c = lane; c < D4; c += 32) *(float4*)(Qs + r * D + 4 * c) = load4<T>(src + 4 * c);
+    }
+    const int mine = rows > warp ? min(R, (rows - warp + ATT_WARPS - 1) / ATT_WARPS) : 0;        // rows of this warp
+
+    float m[R], l[R];
+    float4 acc[R][N4];
+#pragma unroll
+    for (int i = 0; i < R; i++) {
+        m[i] = -INFINITY;
+        l[i] = 0.0f;
+#pragma unroll
+        for (int c = 0; c < N4; c++) acc[i][c] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    }
+    // the first ROWS of the warp's rows against the tile in shared memory (rows past `mine` hold nothing that is kept)
+    auto take = [&](auto rows_c, int k0) {
+        constexpr int ROWS = decltype(rows_c)::value;
+        float s[ROWS];
+#pragma unroll
+        for (int i = 0; i < ROWS; i++) s[i] = 0.0f;
+#pragma unroll 4
+        for (int d = 0; d < D; d += 4) {
+            const float4 k = *(const float4*)(Ks + lane * DP + d);
+#pragma unroll
+            for (int i = 0; i < ROWS; i++) {
+                const float4 x = *(const float4*)(Qs + (warp + i * ATT_WARPS) * D + d);
+                s[i] = fmaf(x.x, k.x, s[i]); s[i] = fmaf(x.y, k.y, s[i]);
+                s[i] = fmaf(x.z, k.z, s[i]); s[i] = fmaf(x.w, k.w, s[i]);
+            }
+        }
+        float pj[ROWS];
+        bool live[ROWS], all = true;
+#pragma unroll
+        for (int i = 0; i < ROWS; i++) {
+            const int qpos = pos0 + (warp + i * ATT_WARPS) / G, key = k0 + lane;
+            const bool visible = key >= lo && key < hi && key <= qpos && (p.window <= 0 || key > qpos - p.window);
+            const float x = visible ? s[i] * p.scale : -INFINITY;
+            const float m_new = fmaxf(m[i], warp_max(x));
+            live[i] = m_new != -INFINITY;          // else nothing visible so far
+            all = all && live[i];
+            const float corr = live[i] ? expf(m[i] - m_new) : 1.0f;  // m = -inf -> 0
+            pj[i] = visible ? expf(x - m_new) : 0.0f;
+            l[i] = l[i] * corr + warp_sum(pj[i]);
+            m[i] = m_new;
+#pragma unroll
+            for (int c = 0; c < N4; c++) { acc[i][c].x *= corr; acc[i][c].y *= corr; acc[i][c].z *= corr; acc[i][c].w *= corr; }
+        }
+        auto add = [&](int j, int i, const float4 (&v)[N4]) {
+            const float w = __shfl_sync(0xffffffffu, pj[i], j);
+#pragma unroll
+            for (int c = 0; c < N4; c++) {
+                acc[i][c].x = fmaf(w, v[c].x, acc[i][c].x); acc[i][c].y = fmaf(w, v[c].y, acc[i][c].y);
+                acc[i][c].z = fmaf(w, v[c].z, acc[i][c].z); acc[i][c].w = fmaf(w, v[c].w, acc[i][c].w);
+            }
+        };
+#pragma unroll 8
+        for (int j = 0; j < ATT_KT; j++) {
+            float4 v[N4];
+#pragma unroll
+            for (int c = 0; c < N4; c++) {
+                const int d = (lane + 32 * c) * 4;
+                v[c] = d < D ? *(const float4*)(Vs + j * D + d) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            }
+            if (all) {
+#pragma unroll
+                for (int i = 0; i < ROWS; i++) add(j, i, v);
+            } else {
+#pragma unroll
+                for (int i = 0; i < ROWS; i++)
+                    if (live[i]) add(j, i, v);
+            }
+        }
+    };
+    for (int k0 = start; k0 < hi; k0 += ATT_KT) {
+        __syncthreads();  // previous tile fully consumed
+#pragma unroll
+        for (int i = 0; i < KEYS; i++)
+#pragma unroll
+            for (int c = 0; c < N4; c++) {
+                const int j = warp + ATT_WARPS * i, d = (lane + 32 * c) * 4;
+                if (d < D) {
+                    *(float4*)(Ks + j * DP + d) = kr[i][c];
+                    *(float4*)(Vs + j * D + d) = vr[i][c];
+                }
+            }
+        __syncthreads();
+        if (k0 + ATT_KT < hi) fetch(k0 + ATT_KT);
+        // (uniform per warp; a decoded token's warps have one row each, and pay for one)
+        if (mine == 1) take(std::integral_constant<int, 1>(), k0);
+        else if (mine > 1) take(std::integral_constant<int, R>(), k0);
+    }
+
+#pragma unroll
+    for (int i = 0; i < R; i++) {
+        const int r = warp + i * ATT_WARPS;
+        if (r >= rows) continue;
+        const int qi = r / G, g = r - qi * G;
+        const size_t th = (size_t)(row0 + qi) * p.n_heads + kvh * G + g;
+        const float inv = p.n_splits > 1 ? 1.0f : (l[i] > 0.0f ? 1.0f / l[i] : 0.0f);
+#pragma unroll
+        for (int c = 0; c < N4; c++) {
+            const int d = (lane + 32 * c) * 4;
+            if (d >= D) continue;
+            const float4 o = make_float4(acc[i][c].x * inv, acc[i][c].y * inv, acc[i][c].z * inv, acc[i][c].w * inv);
+            if (p.n_splits > 1) *(float4*)(p.part_o + (th * p.n_splits + split) * D + d) = o;
+            else store4<T>((T*)p.out + th * D + d, o);
+        }
+        if (p.n_splits > 1 && lane == 0) {
+            float* ml = p.part_ml + (th * p.n_splits + split) * 2;
+            ml[0] = m[i];
+            ml[1] = l[i];
+        }
+    }
+}
+
 // Merges the partial results of the splits of one (token, head) in ascending split order.
 template <typename T>
 __global__ void attention_combine_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml,
@@ -198,7 +394,10 @@ template <typename T>
 int launch_attention(const AttnParams& p, int n_tiles, int T_tokens, cudaStream_t st) {
     const int D = p.D;
     const int G = p.n_heads / p.n_kv;
-    const size_t smem = ((size_t)ATT_KT * (D + 1) + (size_t)ATT_KT * D + (size_t)ATT_MAX_ROWS * D) * sizeof(float);
+    // whole groups of four elements on boundaries of as many bytes: the kernel that copies them so
+    const uintptr_t bases = (uintptr_t)p.q | (uintptr_t)p.k_pool | (uintptr_t)p.v_pool | (uintptr_t)p.out;
+    const bool by4 = D % 4 == 0 && bases % (4 * sizeof(T)) == 0 && ((uintptr_t)p.part_o & 15) == 0;
+    const size_t smem = ((size_t)ATT_KT * (D + (by4 ? 4 : 1)) + (size_t)ATT_KT * D + (size_t)ATT_MAX_ROWS * D) * sizeof(float);
     dim3 grid(n_tiles, p.n_kv, p.n_splits);
     const int nc = (D + 31) / 32;
     auto run = [&](auto kernel) -> int {
@@ -210,7 +409,8 @@ int launch_attention(const AttnParams& p, int n_tiles, int T_tokens, cudaStream_
         return check_launch("attention");
     };
     int rc;
-    if (nc <= 1) rc = run(attention_tile_kernel<T, 1>);
+    if (by4) rc = nc <= 4 ? run(attention_tile4_kernel<T, 1>) : run(attention_tile4_kernel<T, 2>);
+    else if (nc <= 1) rc = run(attention_tile_kernel<T, 1>);
     else if (nc <= 2) rc = run(attention_tile_kernel<T, 2>);
     else if (nc <= 4) rc = run(attention_tile_kernel<T, 4>);
     else rc = run(attention_tile_kernel<T, 8>);
