@@ -883,6 +883,362 @@ __global__ void __launch_bounds__(32 * RG, CT == 1 ? 3 : 1) scan_chunks_kernel(S
     regs_store<RS, RG>(st, tile, S, D, V, col0, extra);
 }
 
+// ------------------------------------------------------------------ prompt portions: roles for the warps
+// A portion's tokens follow one another, so what counts is the time of one token.  Three things bounded it in the
+// kernel above: every four columns read all of a token's vectors from shared memory (half the time its bandwidth),
+// every warp stopped between chunks to prepare the next one's tokens, and every token's output waited for its own
+// shuffles.  Here a thread keeps RS rows of C columns, so a read serves C columns and rows go in pairs through the packed
+// fp32 instructions; four warps do nothing but prepare (loads of the chunk after the next, norms, decays, gates of
+// the next); and the outputs of eight tokens are summed over the row groups together.  Every sum is formed in the order
+// of the kernel above.  Delta rule, 16 heads of 128 x 128: one run of 1,500 tokens 735 us there, 392 here; 24 runs of 60
+// 366 there, 256 here (with two computing warps a block, or eight preparing ones, the one run gets no faster).
+constexpr int PORTION_WARPS = 4, PORTION_PREPARE = 4;      // computing and preparing warps of a block
+
+__device__ __forceinline__ unsigned long long pair_of(float lo, float hi) {
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(__float_as_uint(lo)), "r"(__float_as_uint(hi)));
+    return r;
+}
+__device__ __forceinline__ float pair_lo(unsigned long long v) { return __uint_as_float((unsigned)v); }
+__device__ __forceinline__ float pair_hi(unsigned long long v) { return __uint_as_float((unsigned)(v >> 32)); }
+__device__ __forceinline__ unsigned long long pair_mul(unsigned long long a, unsigned long long b) {
+    unsigned long long d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ unsigned long long pair_fma(unsigned long long a, unsigned long long b, unsigned long long c) {
+    unsigned long long d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+
+template <int N, int C>
+struct PortionRegs {                                // one token's vectors (pairs of rows), scalars and C column values
+    ulonglong2 v0[N], v1[N], v2[N];
+    float4 sc;
+    float val[C];
+};
+
+template <int MODE, int RS, int CT, int C>
+__global__ void __launch_bounds__(32 * (PORTION_WARPS + PORTION_PREPARE), 1) scan_portion_kernel(ScanArgs p) {
+    constexpr int RG = 8, NCW = PORTION_WARPS, NP = PORTION_PREPARE, THREADS = 32 * (NCW + NP), COLS = 4 * C * NCW;
+    extern __shared__ __align__(16) float smem[];
+    pdl_launch_dependents();
+    pdl_wait();
+    constexpr int NV = (MODE == 0 || MODE == 3 || MODE == 4) ? 3 : 2;
+    constexpr int VS = RG * (RS + 4);               // a vector in shared memory: row group r starts at r (RS + 4)
+    constexpr int TOK = NV * VS + 4 + COLS;         // vectors, four scalars, the block's column values
+    constexpr int TPW = CT / NP, EPL = RG * RS / 32;
+    static_assert(CT % NP == 0 && CT % 8 == 0, "whole tokens per preparing warp, whole batches of eight");
+    const int s = blockIdx.x, h = blockIdx.y, col0 = blockIdx.z * COLS;
+    const int D = p.D, V = p.V, H = p.H, grp = h / (H / p.G);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int first = p.query_start[s], end = p.query_start[s + 1];
+    if (first >= end) return;                       // an empty run leaves its state as it is
+
+    if (warp >= NCW) {
+        // ------------------------------------------------------------------------------- preparing warps
+        // Without branches on the token or the row (both are clamped; a row past D is stored as zero, a token past the
+        // end is never used), so that the chains of a warp's TPW x EPL elements run side by side.
+        const int pw = warp - NCW;
+        const float rate = (MODE == 1 || MODE == 3 || MODE == 4) ? 0.0f : expf(p.A_log[h]);
+        const float qscale = 1.0f / sqrtf((float)D);
+        // where this head's vectors start in a row of x
+        constexpr bool PROJ = MODE == 1 || MODE == 3 || MODE == 4;        // q (or r), k, v at given columns of one projection
+        const int off0 = MODE == 0 ? p.G * D + grp * D : (PROJ ? p.off_k + h * D : H * V + grp * D);               // k | k | B
+        const int off1 = MODE == 0 ? grp * D : (PROJ ? p.off_q + h * D : H * V + p.G * D + grp * D);               // q | q | C
+        const int off_col = MODE == 0 ? 2 * p.G * D + h * V : (PROJ ? p.off_v + h * V : h * V);                    // v | v | x
+        int row_of[EPL];
+        bool row_ok[EPL];
+        float bias[EPL], bonus[EPL];
+#pragma unroll
+        for (int m = 0; m < EPL; m++) {
+            row_ok[m] = lane + 32 * m < D;
+            row_of[m] = row_ok[m] ? lane + 32 * m : D - 1;
+            bias[m] = 0.0f; bonus[m] = 0.0f;
+            if (MODE == 0) bias[m] = p.dt_bias[p.a_head ? h : h * D + row_of[m]];
+            if (MODE == 4 || (MODE == 3 && p.dt_bias)) bias[m] = p.dt_bias[h * D + row_of[m]];
+            if (MODE == 4) bonus[m] = p.bonus[h * D + row_of[m]];
+        }
+        const float bias_h = MODE == 2 ? p.dt_bias[h] : 0.0f;
+        const int my_col = col0 + lane;
+        const bool col_ok = lane < COLS && my_col < V;
+        float f0[TPW][EPL], f1[TPW][EPL], f2[TPW][EPL], fc[TPW], fs[TPW], ft[TPW];
+        auto prefetch = [&](int t0) {
+#pragma unroll
+            for (int w = 0; w < TPW; w++) {
+                const int t = min(t0 + pw + NP * w, end - 1);
+                const float* row = p.x + (size_t)t * p.ld_x;
+#pragma unroll
+                for (int m = 0; m < EPL; m++) {
+                    f0[w][m] = row[off0 + row_of[m]];
+                    f1[w][m] = row[off1 + row_of[m]];
+                    if (NV == 3) f2[w][m] = p.a[(size_t)t * p.ld_a + ((MODE == 0 && p.a_head) ? h : h * D + row_of[m])];
+                }
+                fc[w] = col_ok ? row[off_col + my_col] : 1.0f;
+                if (MODE == 0 || MODE == 2) fs[w] = p.b[(size_t)t * p.ld_b + h];
+                if (MODE == 1) {
+                    const float* g = p.gates + ((size_t)t * H + h) * 4;
+                    fs[w] = g[0]; ft[w] = g[1];
+                }
+            }
+        };
+        auto prepare = [&](float* buf) {
+            float g[TPW][EPL], s0[TPW], s1[TPW], s01[TPW];
+#pragma unroll
+            for (int w = 0; w < TPW; w++) {
+                s0[w] = s1[w] = s01[w] = 0.0f;
+#pragma unroll
+                for (int m = 0; m < EPL; m++) {
+                    if (!row_ok[m]) f0[w][m] = f1[w][m] = 0.0f;
+                    g[w][m] = 0.0f;
+                    if (MODE == 3)      // alpha = sigmoid(z)^(1 / tau) = exp(logsigmoid(z) / tau)
+                        g[w][m] = expf(logsigmoidf_(f2[w][m] + bias[m]) * p.decay_power);
+                    if (MODE == 4) {
+                        g[w][m] = expf(-expf(f2[w][m] + bias[m]));
+                        s0[w] = fmaf(f1[w][m] * bonus[m], f0[w][m], s0[w]);          // r . (u k)
+                    }
+                    if (MODE == 0) {
+                        g[w][m] = expf(-rate * softplusf_(f2[w][m] + bias[m]));
+                        s0[w] = fmaf(f0[w][m], f0[w][m], s0[w]);
+                        s1[w] = fmaf(f1[w][m], f1[w][m], s1[w]);
+                        s01[w] = fmaf(f0[w][m], f1[w][m], s01[w]);
+                    }
+                    if (!row_ok[m]) g[w][m] = 0.0f;
+                }
+            }
+            if (MODE == 0 || MODE == 4) {
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+                    for (int w = 0; w < TPW; w++) {
+                        s0[w] += __shfl_xor_sync(0xffffffffu, s0[w], o);
+                        if (MODE == 0) {
+                            s1[w] += __shfl_xor_sync(0xffffffffu, s1[w], o);
+                            s01[w] += __shfl_xor_sync(0xffffffffu, s01[w], o);
+                        }
+                    }
+            }
+#pragma unroll
+            for (int w = 0; w < TPW; w++) {
+                float* tok = buf + (pw + NP * w) * TOK;
+#pragma unroll
+                for (int m = 0; m < EPL; m++) {
+                    const int i = lane + 32 * m, vi = i + (i / RS) * 4;
+                    tok[vi] = f0[w][m];
+                    tok[VS + vi] = (MODE == 1 || MODE == 3) ? f1[w][m] * qscale : f1[w][m];
+                    if (NV == 3) tok[2 * VS + vi] = g[w][m];
+                }
+                if (lane < COLS) tok[NV * VS + 4 + lane] = fc[w];
+                float4 sc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                if (MODE == 0) {
+                    sc.x = 1.0f / sqrtf(s0[w] + p.key_eps);            // 1 / |k|
+                    sc.y = qscale / sqrtf(s1[w] + p.key_eps);          // D^-1/2 / |q|
+                    sc.z = s01[w];                                     // k . q, before the norms
+                    sc.w = sigmoidf_(fs[w]);
+                } else if (MODE == 4) {
+                    sc.x = s0[w];
+                } else if (MODE == 1) {
+                    sc.x = fs[w]; sc.y = ft[w];
+                } else if (MODE == 2) {
+                    const float dt = softplusf_(fs[w] + bias_h);
+                    sc.x = expf(-rate * dt); sc.y = dt;
+                }
+                if (lane == 0) *reinterpret_cast<float4*>(tok + NV * VS) = sc;
+            }
+        };
+        prefetch(first);
+        prepare(smem);
+        prefetch(first + CT);
+        asm volatile("bar.sync 1, %0;" ::"n"(THREADS) : "memory");
+        int cur = 0;
+        for (int t0 = first; t0 < end; t0 += CT, cur ^= 1) {
+            if (t0 + CT < end) {
+                prepare(smem + (cur ^ 1) * CT * TOK);
+                prefetch(t0 + 2 * CT);
+            }
+            asm volatile("bar.sync 1, %0;" ::"n"(THREADS) : "memory");
+        }
+        return;
+    }
+
+    // ----------------------------------------------------------------------------------- computing warps
+    const int r = lane % RG, cw = warp * 4 * C + (lane / RG) * C, j = col0 + cw, base = r * (RS + 4);
+    const int n_cols = MODE == 1 ? V + 1 : V;       // (matrix memory: column V is n)
+    float* sbase = p.state + (size_t)p.slots[s] * p.state_stride;
+    float* S = sbase + (size_t)h * D * V;
+    float* extra = MODE == 1 ? sbase + (size_t)H * D * V + (size_t)h * D : nullptr;
+    unsigned long long st[C][RS / 2];
+    auto place = [&](int i, int c) -> float* {      // row i of column c of this thread, null if there is none
+        if (i >= D || j + c >= n_cols) return nullptr;
+        return MODE == 1 && j + c == V ? extra + i : S + (size_t)i * V + j + c;
+    };
+#pragma unroll
+    for (int ii = 0; ii < RS; ii += 2)
+#pragma unroll
+        for (int c = 0; c < C; c++) {
+            const float* lo = place(r * RS + ii, c);
+            const float* hi = place(r * RS + ii + 1, c);
+            st[c][ii / 2] = pair_of(lo ? *lo : 0.0f, hi ? *hi : 0.0f);
+        }
+    const float skip = MODE == 2 ? p.skip[h] : 0.0f;
+    asm volatile("bar.sync 1, %0;" ::"n"(THREADS) : "memory");
+    int cur = 0;
+    for (int t0 = first; t0 < end; t0 += CT, cur ^= 1) {
+        const int n = min(CT, end - t0);
+        const float* buf = smem + cur * CT * TOK;
+        // a token's operands are fetched into registers while the token before it is computed (two register sets),
+        // so that no multiply-add waits for shared memory
+        auto fetch = [&](int tt, PortionRegs<RS / 4, C>& x) {
+            const float* tok = buf + tt * TOK;
+            x.sc = *reinterpret_cast<const float4*>(tok + NV * VS);
+#pragma unroll
+            for (int c = 0; c < C; c++) x.val[c] = tok[NV * VS + 4 + cw + c];
+#pragma unroll
+            for (int i4 = 0; i4 < RS / 4; i4++) {
+                x.v0[i4] = reinterpret_cast<const ulonglong2*>(tok + base)[i4];
+                x.v1[i4] = reinterpret_cast<const ulonglong2*>(tok + VS + base)[i4];
+                if (NV == 3) x.v2[i4] = reinterpret_cast<const ulonglong2*>(tok + 2 * VS + base)[i4];
+            }
+        };
+        // One token: the state moves on; o[c] is this thread's share of the output's dot product, add[c] what `finish`
+        // wants beside its sum over the eight row groups.
+        auto step = [&](const PortionRegs<RS / 4, C>& x, float (&o)[C], float (&add)[C]) {
+            if (MODE == 0) {
+                unsigned long long ak[C][2], aq[C][2];
+#pragma unroll
+                for (int c = 0; c < C; c++) ak[c][0] = ak[c][1] = aq[c][0] = aq[c][1] = 0;
+#pragma unroll
+                for (int i4 = 0; i4 < RS / 4; i4++)
+#pragma unroll
+                    for (int c = 0; c < C; c++) {
+                        st[c][2 * i4] = pair_mul(st[c][2 * i4], x.v2[i4].x);
+                        st[c][2 * i4 + 1] = pair_mul(st[c][2 * i4 + 1], x.v2[i4].y);
+                        ak[c][0] = pair_fma(st[c][2 * i4], x.v0[i4].x, ak[c][0]);
+                        ak[c][1] = pair_fma(st[c][2 * i4 + 1], x.v0[i4].y, ak[c][1]);
+                    }
+                float sk[C];
+#pragma unroll
+                for (int c = 0; c < C; c++) sk[c] = (pair_lo(ak[c][0]) + pair_hi(ak[c][0])) + (pair_lo(ak[c][1]) + pair_hi(ak[c][1]));
+#pragma unroll
+                for (int off = 1; off < RG; off <<= 1)
+#pragma unroll
+                    for (int c = 0; c < C; c++) sk[c] += __shfl_xor_sync(0xffffffffu, sk[c], off);
+                // (while the shuffles are under way)
+#pragma unroll
+                for (int i4 = 0; i4 < RS / 4; i4++)
+#pragma unroll
+                    for (int c = 0; c < C; c++) {
+                        aq[c][0] = pair_fma(st[c][2 * i4], x.v1[i4].x, aq[c][0]);
+                        aq[c][1] = pair_fma(st[c][2 * i4 + 1], x.v1[i4].y, aq[c][1]);
+                    }
+#pragma unroll
+                for (int c = 0; c < C; c++) {
+                    o[c] = (pair_lo(aq[c][0]) + pair_hi(aq[c][0])) + (pair_lo(aq[c][1]) + pair_hi(aq[c][1]));
+                    const float uk = x.sc.w * (x.val[c] - sk[c] * x.sc.x) * x.sc.x;      // beta (v - S^T k) / |k|
+                    add[c] = uk;
+                    const unsigned long long u2 = pair_of(uk, uk);
+#pragma unroll
+                    for (int i4 = 0; i4 < RS / 4; i4++) {
+                        st[c][2 * i4] = pair_fma(x.v0[i4].x, u2, st[c][2 * i4]);
+                        st[c][2 * i4 + 1] = pair_fma(x.v0[i4].y, u2, st[c][2 * i4 + 1]);
+                    }
+                }
+            } else {
+                // S <- keep S + k v^T with a decay per row (3, 4) or per token (1, 2), read before (4) or behind
+#pragma unroll
+                for (int c = 0; c < C; c++) {
+                    const float put = (MODE == 1 || MODE == 2) ? x.sc.y * x.val[c] : x.val[c];              // put v | dt x
+                    const unsigned long long put2 = pair_of(put, put), keep2 = pair_of(x.sc.x, x.sc.x);
+                    unsigned long long a0 = 0, a1 = 0;
+#pragma unroll
+                    for (int i4 = 0; i4 < RS / 4; i4++) {
+                        const unsigned long long g0 = NV == 3 ? x.v2[i4].x : keep2, g1 = NV == 3 ? x.v2[i4].y : keep2;
+                        if (MODE == 4) {
+                            a0 = pair_fma(st[c][2 * i4], x.v1[i4].x, a0);
+                            a1 = pair_fma(st[c][2 * i4 + 1], x.v1[i4].y, a1);
+                        }
+                        st[c][2 * i4] = pair_fma(x.v0[i4].x, put2, pair_mul(g0, st[c][2 * i4]));
+                        st[c][2 * i4 + 1] = pair_fma(x.v0[i4].y, put2, pair_mul(g1, st[c][2 * i4 + 1]));
+                        if (MODE != 4) {
+                            a0 = pair_fma(st[c][2 * i4], x.v1[i4].x, a0);
+                            a1 = pair_fma(st[c][2 * i4 + 1], x.v1[i4].y, a1);
+                        }
+                    }
+                    o[c] = (pair_lo(a0) + pair_hi(a0)) + (pair_lo(a1) + pair_hi(a1));
+                    add[c] = x.val[c];
+                }
+            }
+        };
+        auto finish = [&](const float4& sc, float sum, float add) {
+            if (MODE == 0) return sc.y * fmaf(add, sc.z, sum);
+            if (MODE == 4) return fmaf(sc.x, add, sum);
+            if (MODE == 2) return fmaf(skip, add, sum);
+            return sum;
+        };
+        auto store = [&](int t, int col, float y) {
+            if (col < V) __stcs(p.out + (size_t)t * H * V + h * V + col, y);
+            else if (col < n_cols) p.gates[((size_t)t * H + h) * 4 + 3] = y;
+        };
+        PortionRegs<RS / 4, C> X[2];
+        fetch(0, X[0]);
+        int tt = 0;
+        for (; tt + 8 <= n; tt += 8) {
+            // eight tokens, whose outputs are summed over the row groups together: a lane gives away half of its
+            // tokens at each of the three exchanges and ends with the whole sums of token tt + r
+            float o[8][C], add[8][C], keep[C];
+            float4 sc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+            for (int u = 0; u < 8; u++) {
+                fetch(min(tt + u + 1, CT - 1), X[(u + 1) & 1]);
+                step(X[u & 1], o[u], add[u]);
+                if (r == u) {
+                    sc = X[u & 1].sc;
+#pragma unroll
+                    for (int c = 0; c < C; c++) keep[c] = add[u][c];
+                }
+            }
+#pragma unroll
+            for (int c = 0; c < C; c++) {
+                float a[4], b[2];
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    const float mine = (r & 1) ? o[2 * i + 1][c] : o[2 * i][c], other = (r & 1) ? o[2 * i][c] : o[2 * i + 1][c];
+                    a[i] = mine + __shfl_xor_sync(0xffffffffu, other, 1);
+                }
+#pragma unroll
+                for (int i = 0; i < 2; i++) {
+                    const float mine = (r & 2) ? a[2 * i + 1] : a[2 * i], other = (r & 2) ? a[2 * i] : a[2 * i + 1];
+                    b[i] = mine + __shfl_xor_sync(0xffffffffu, other, 2);
+                }
+                const float mine = (r & 4) ? b[1] : b[0], other = (r & 4) ? b[0] : b[1];
+                store(t0 + tt + r, j + c, finish(sc, mine + __shfl_xor_sync(0xffffffffu, other, 4), keep[c]));
+            }
+        }
+        for (; tt < n; tt++) {                      // X[0] holds token tt
+            float o[C], add[C];
+            fetch(min(tt + 1, CT - 1), X[1]);
+            step(X[0], o, add);
+#pragma unroll
+            for (int c = 0; c < C; c++) {
+                const float sum = rows_sum<RG>(o[c]);
+                if (r == c) store(t0 + tt, j + c, finish(X[0].sc, sum, add[c]));
+            }
+            X[0] = X[1];
+        }
+        asm volatile("bar.sync 1, %0;" ::"n"(THREADS) : "memory");
+    }
+#pragma unroll
+    for (int ii = 0; ii < RS; ii += 2)
+#pragma unroll
+        for (int c = 0; c < C; c++) {
+            float* lo = place(r * RS + ii, c);
+            float* hi = place(r * RS + ii + 1, c);
+            if (lo) *lo = pair_lo(st[c][ii / 2]);
+            if (hi) *hi = pair_hi(st[c][ii / 2]);
+        }
+}
+
 inline int rows_per_thread(int D) { return D <= 32 ? 4 : (D <= 64 ? 8 : (D <= 128 ? 16 : (D <= 256 ? 32 : 0))); }
 inline bool regs_kernels_on() {
     static int on = -1;
@@ -901,17 +1257,27 @@ inline int launch_scan_ct(const ScanArgs& p, int S, int n_cols, cudaStream_t st)
     launch_kernel(scan_chunks_kernel<MODE, RS, CT, RG>, dim3(S, p.H, (n_cols + RCOLS - 1) / RCOLS), 32 * RG, smem, st, p);
     return 0;
 }
-// `single`: every run of the step is one token (a decode step): chunks of one token, small blocks, several per SM
-// (the step is bound by the state's bytes).  Eight lanes a column in both cases: sixteen (half the rows a thread, one
-// more shuffle) were measured equal for prompt portions (6.49 against 6.34 ms for the eight scans of a 2,048-token
-// step at heads of 128), so the kernel keeps the parameter and the launcher one choice.
+template <int MODE, int RS, int CT, int C>
+inline int launch_portion(const ScanArgs& p, int S, int n_cols, cudaStream_t st) {
+    constexpr int NV = (MODE == 0 || MODE == 3 || MODE == 4) ? 3 : 2, COLS = 4 * C * PORTION_WARPS;
+    constexpr size_t smem = (size_t)2 * CT * (NV * 8 * (RS + 4) + 4 + COLS) * sizeof(float);
+    if (smem > 48 * 1024) {
+        cudaError_t e = cudaFuncSetAttribute(scan_portion_kernel<MODE, RS, CT, C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return fail("scan: %s", cudaGetErrorString(e));
+    }
+    launch_kernel(scan_portion_kernel<MODE, RS, CT, C>, dim3(S, p.H, (n_cols + COLS - 1) / COLS), 32 * (PORTION_WARPS + PORTION_PREPARE),
+                  smem, st, p);
+    return 0;
+}
+// `single`: as many runs as tokens (a decode step): chunks of one token, small blocks, several per SM (the step is
+// bound by the state's bytes).  Anything else goes to the kernel with roles.
 template <int MODE>
 inline int launch_scan(const ScanArgs& p, int S, int n_cols, bool single, cudaStream_t st) {
     switch (rows_per_thread(p.D)) {
-        case 4: return single ? launch_scan_ct<MODE, 4, 1, 8>(p, S, n_cols, st) : launch_scan_ct<MODE, 4, 16, 8>(p, S, n_cols, st);
-        case 8: return single ? launch_scan_ct<MODE, 8, 1, 8>(p, S, n_cols, st) : launch_scan_ct<MODE, 8, 16, 8>(p, S, n_cols, st);
-        case 16: return single ? launch_scan_ct<MODE, 16, 1, 8>(p, S, n_cols, st) : launch_scan_ct<MODE, 16, 16, 8>(p, S, n_cols, st);
-        default: return single ? launch_scan_ct<MODE, 32, 1, 8>(p, S, n_cols, st) : launch_scan_ct<MODE, 32, 8, 8>(p, S, n_cols, st);
+        case 4: return single ? launch_scan_ct<MODE, 4, 1, 8>(p, S, n_cols, st) : launch_portion<MODE, 4, 16, 2>(p, S, n_cols, st);
+        case 8: return single ? launch_scan_ct<MODE, 8, 1, 8>(p, S, n_cols, st) : launch_portion<MODE, 8, 16, 2>(p, S, n_cols, st);
+        case 16: return single ? launch_scan_ct<MODE, 16, 1, 8>(p, S, n_cols, st) : launch_portion<MODE, 16, 16, 2>(p, S, n_cols, st);
+        default: return single ? launch_scan_ct<MODE, 32, 1, 8>(p, S, n_cols, st) : launch_portion<MODE, 32, 8, 1>(p, S, n_cols, st);
     }
 }
 

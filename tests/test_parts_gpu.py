@@ -525,3 +525,48 @@ def test_attention_refuses_a_group_the_kernels_do_not_take():
     build_part("mixer", AttentionSpec(hidden_size=64, num_heads=32, num_kv_heads=1, head_dim=16))
     with pytest.raises(ConfigError, match="at most 32"):
         build_part("mixer", AttentionSpec(hidden_size=64, num_heads=66, num_kv_heads=2, head_dim=16))
+
+
+@pytest.mark.parametrize("mode", ["delta", "memory", "ssm", "gla", "wkv"])
+@pytest.mark.parametrize("dim,vdim", [(24, 20), (64, 33), (100, 48), (128, 128), (256, 16)])
+def test_scans_of_portions_equal_single_tokens(mode, dim, vdim):
+    """Runs of 0 to 35 tokens (the edges of a chunk of 8 or 16, and of two) in one step against the same tokens one at a
+    time: outputs and states.  Both kernels add in one order, so what is allowed is the rounding of a few operations."""
+    from ember_b200 import ops
+    torch.manual_seed(dim + vdim)
+    lens, H = [1, 16, 0, 17, 7, 8, 35, 2], 2
+    T, S = sum(lens), len(lens)
+    rand = lambda *shape: torch.randn(*shape, device="cuda")                      # noqa: E731
+    qk, v = H * dim, H * vdim
+    proj, z, beta = rand(T, 2 * qk + v), rand(T, qk), rand(T, H)
+    bias, per_head, per_head2 = rand(qk) - 1.0, rand(H) - 1.0, rand(H)
+    size = H * dim * vdim + H * dim + H
+    states = [rand(S + 1, size).abs() if mode == "memory" else rand(S + 1, size)]
+    states.append(states[0].clone())
+    outs = [torch.zeros(T, v, device="cuda") for _ in range(2)]
+    gate_rows = [torch.zeros(T, H, 4, device="cuda") for _ in range(2)]
+
+    def run(which, rows, qs, slots, t, s):
+        st, out, gates = states[which], outs[which][rows], gate_rows[which][rows]
+        qs, slots = (torch.tensor(x, dtype=torch.int32, device="cuda") for x in (qs, slots))
+        p, zz, b = proj[rows].contiguous(), z[rows].contiguous(), beta[rows].contiguous()
+        if mode == "delta":
+            ops.delta_scan(p, b, 0, zz, 0, bias, per_head, st, out, qs, slots, t, s, H, H, dim, vdim, 1e-6)
+        elif mode == "memory":
+            full = torch.cat([p, b, zz[:, :H]], 1).contiguous()
+            ops.memory_scan(full, 0, qk, 2 * qk, 2 * qk + v, 2 * qk + v + H, per_head, per_head2, 15.0, st, gates, out, qs, slots, t, s, H, dim, vdim)
+        elif mode == "ssm":
+            ops.ssm_scan(p[:, :v + 2 * dim].contiguous(), b, 0, per_head, per_head2, per_head, st, out, qs, slots, t, s, H, 1, dim, vdim)
+        elif mode == "gla":
+            ops.gla_scan(p, 0, qk, 2 * qk, zz, 0, bias, 0.0625, st, out, qs, slots, t, s, H, dim, vdim)
+        else:
+            ops.wkv_scan(p, p.shape[1], 0, qk, 2 * qk, zz, 0, bias, bias, st, out, qs, slots, t, s, H, dim, vdim)
+
+    starts = [sum(lens[:i]) for i in range(S + 1)]
+    run(0, slice(0, T), starts, list(range(S, 0, -1)), T, S)
+    for i, n in enumerate(lens):
+        for t in range(n):
+            run(1, slice(starts[i] + t, starts[i] + t + 1), [0, 1], [S - i], 1, 1)
+    assert torch.isfinite(outs[0]).all()
+    for a, b in ((outs[0], outs[1]), (states[0], states[1]), (gate_rows[0], gate_rows[1])):
+        assert float((a - b).norm()) <= 1e-6 * float(b.norm()) + 1e-30
