@@ -130,6 +130,68 @@ static void best_tile_and_parts(int M, int N, int num_k_blocks, int slots, int u
     }
 }
 
+// A cluster's partial sums in shared memory: every block receives its share of the token columns from all of them.
+static size_t cluster_recv_bytes(const GemmTcParams& p) {
+    if (p.cluster_splits <= 1 && p.epilogue != 4) return 0;
+    const int S = p.cluster_splits;
+    return (size_t)S * ((p.block_cols + S - 1) / S) * TILE_ROWS * sizeof(float);
+}
+
+// Stages and shared memory of a decode-sized product (swapped orientation).  About 96 KiB of stages and, from 17 tokens
+// on, no more than 110 KiB in all, so that two blocks fit on an SM: the next kernel's blocks become resident and
+// prefetch their weights while this kernel drains, the memory system sees more independent streams, and a cluster finds
+// its SMs.  More than 64 tokens, where that would leave two stages, take an SM whole if there are no more blocks than SMs.
+static size_t decode_smem(GemmTcParams& p, int num_sms) {
+    const int stage_bytes = TILE_ROWS * TILE_K * 2 + ((p.block_cols * TILE_K * 2 + 1023) & ~1023);
+    const size_t recv = cluster_recv_bytes(p);
+    const size_t whole = (size_t)(p.block_cols > 64 && p.total_tiles * p.cluster_splits <= num_sms ? 190 : 110) * 1024;
+    size_t budget = (size_t)96 * 1024;
+    if (p.block_cols > 16 && recv) budget = recv < whole ? whole - recv : 0;
+    int stages = (int)(budget / stage_bytes);
+    if (stages > MAX_STAGES) stages = MAX_STAGES;
+    if (stages < 2) stages = 2;
+    if (stages > p.k_blocks_per_split) stages = p.k_blocks_per_split < 2 ? 2 : p.k_blocks_per_split;
+    p.stages = stages;
+    return (size_t)stages * stage_bytes + 1024 /* alignment slack */ + 256 /* barriers */ + recv;
+}
+
+// The decode-sized kernel may use an SM's whole shared memory (set once per process).
+static bool raise_smem_limit() {
+    static const bool done = [] {
+        cudaError_t e = cudaFuncSetAttribute(gemm_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+        if (e != cudaSuccess) { cudaGetLastError(); return false; }
+        cudaFuncSetAttribute(gemm_tc_kernel<false>, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared);
+        cudaFuncSetAttribute(gemm_tc_kernel<true>, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared);
+        return true;
+    }();
+    return done;
+}
+
+// Parts of K, one block of a cluster each, for 17 to 128 tokens; 0: atomics are better.  Up to 64 tokens two blocks fit
+// on an SM, and the most parts win that keep the blocks within about 240 (256 for long K); beyond, a block has an SM to
+// itself, and clusters of eight find too few SMs side by side.  Three and seven parts are slow at every size.  us, by
+// atomics and the pass that rounds -> clusters [parts]:
+//   N x K            stored 4,096 x 2,048  added 2,048 x 2,048  added 2,048 x 6,144  gated 12,288 x 2,048  stored 6,144 x 4,096
+//   24 tokens          9.4 ->  6.3 [6]       5.7 -> 4.9 [8]       8.4 ->  8.5 [8]     14.5 -> 12.6 [2]      14.6 -> 11.1 [5]
+//   64 tokens         13.0 ->  7.6 [6]       7.9 -> 6.9 [8]      10.6 -> 10.5 [8]     18.2 -> 14.9 [2]      19.0 -> 12.9 [5]
+//   96 tokens         15.8 ->  8.5 [4]       9.9 -> 7.9 [6]      12.7 -> 11.5 [6]     20.7 -> 19.0 [2]      21.9 -> 16.4 [2]
+//   128 tokens        18.4 ->  9.6 [4]      11.5 -> 9.1 [6]      14.6 -> 13.4 [6]     24.7 <- 30.0 [2]      25.4 -> 19.6 [2]
+// (added 4,096 x 12,288 at 128 tokens: 27.7 <- 31.3 [4]; what atomics cost is their traffic, 0.06 us a token at N = 2,048,
+// 1.07 TB/s at the L2.)
+static int cluster_parts(const GemmTcParams& p, int tiles) {
+    static const int choices[] = {8, 6, 5, 4, 2};
+    const bool small = p.block_cols <= 64;
+    if (!small && p.epilogue == 2 && p.num_k_blocks >= 128) return 0;
+    for (int s : choices) {
+        const int most = small ? (p.num_k_blocks >= 128 ? 256 : 240) : (s == 8 ? 64 : (s == 5 ? 0 : 128));
+        const int per = (p.num_k_blocks + s - 1) / s;
+        if (tiles * s <= most && per >= 2 && (p.num_k_blocks + per - 1) / per == s) return s;
+    }
+    if (!small && p.block_cols <= 96 && tiles <= 120 && p.num_k_blocks >= 4) return 2;
+    return small && p.epilogue != 2 ? 1 : 0;
+}
+
 // The pair kernel: 256-token tiles on clusters of two blocks, as many pairs as the device co-schedules.
 static int launch_pair(const void* A, const void* W, GemmTcParams p, int block_cols, int max_pairs, cudaStream_t st) {
     p.block_cols = block_cols;
@@ -179,7 +241,6 @@ static int launch_persistent(const void* A, const void* W, GemmTcParams p, int b
     p.row_tiles = (p.M + TILE_ROWS - 1) / TILE_ROWS;
     p.total_tiles = p.row_tiles * ((p.N + block_cols - 1) / block_cols);
     p.cluster_splits = 1;
-    p.rows_per = TILE_ROWS;
     // a short prompt portion has fewer tiles than the device has SMs; the adding epilogue (its sums are added at the L2
     // anyway) then cuts K so that every SM gets a unit of at least 8 k-blocks (512 tokens, K = 6144: 34 -> 12 us)
     int k_splits = 1;
@@ -224,7 +285,7 @@ static int launch_grouped(const void* A, const void* W, GemmTcParams p, int num_
     p.swapped = 0;
     p.num_k_blocks = (p.K + TILE_K - 1) / TILE_K;
     p.k_blocks_per_split = p.num_k_blocks;
-    p.cluster_splits = 1; p.rows_per = TILE_ROWS; p.accum = nullptr; p.accum_ld = 0; p.row_tiles = 0; p.total_tiles = 0;
+    p.cluster_splits = 1; p.accum = nullptr; p.accum_ld = 0; p.row_tiles = 0; p.total_tiles = 0;
     // The tile width by the model of best_block_cols, with rows dealt evenly (half a row tile a group is lost to its end).
     const double row_tiles = (double)p.M / TILE_ROWS + 0.5 * (p.groups < p.M ? p.groups : p.M);
     int block_cols = 256;
@@ -341,7 +402,7 @@ EMBER_API int ember_gemm_tc(const void* A, const void* W, void* out, int ldc, in
                 const int bc_pair = best_block_cols(M, N, max_pairs, 2, &cost_pair);
                 if (split_mode == 4 || (M >= 2048 && cost_pair <= cost_single * 1.001)) {
                     p.epilogue = epilogue; p.out = out; p.ldc = ldc; p.err = err;
-                    p.accum = nullptr; p.accum_ld = 0; p.rows_per = TILE_ROWS; p.stages = 0;
+                    p.accum = nullptr; p.accum_ld = 0; p.stages = 0;
                     return launch_pair(A, W, p, bc_pair, max_pairs, st);
                 }
             }
@@ -357,19 +418,26 @@ EMBER_API int ember_gemm_tc(const void* A, const void* W, void* out, int ldc, in
     // With few output tiles the K range is split so that every SM streams weights.  Two ways to
     // sum the partial results (split_mode 0 picks one):
     //   cluster: the splits of a tile form a thread-block cluster and are summed in shared memory,
-    //            in block order (no scratch, no second kernel) -- best for up to 16 tokens;
+    //            in block order (no scratch, no second kernel) -- best from 17 tokens on, and for any
+    //            number under a storing epilogue;
     //   atomic:  fp32 atomic adds into the residual (add epilogue) or into zeroed scratch that a
-    //            small kernel converts and clears -- best for wider token tiles.
-    // The split count depends on N and K only.
+    //            small kernel converts and clears -- best for up to 16 tokens added into the residual
+    //            (1 / 8 tokens, N 2,048 x K 6,144: 6.2 / 7.0 us against 7.7 / 8.1).
+    // The split count depends on N and K only (and on the token tile's width from 17 tokens on).
     const int tiles = row_tiles * col_tiles;
     const bool store_epilogue = epilogue != 2;
-    const bool use_cluster = split_mode == 2 || split_mode >= 32 || (split_mode == 0 && p.block_cols <= 16 && store_epilogue);
+    p.epilogue = epilogue;
+    const bool wide = p.swapped && p.block_cols > 16;
+    const int parts = wide && (split_mode == 0 || split_mode == 2) && !sums ? cluster_parts(p, tiles) : 0;
+    const bool use_cluster = p.swapped && (split_mode == 2 || split_mode >= 32 || (split_mode == 0 && (wide ? parts > 0 : store_epilogue)));
     int splits = 1;
     if (p.swapped && use_cluster && split_mode >= 32) {
         splits = split_mode - 32;                      // tuning and tests: a cluster of this many blocks
         if (splits > 8) splits = 8;
         if (splits < 1) splits = 1;
         while (splits > 1 && p.num_k_blocks / splits < 2) splits--;
+    } else if (use_cluster && wide) {
+        splits = parts > 0 ? parts : 1;
     } else if (p.swapped && use_cluster) {
         // fill the SMs once: clusters of up to 8 blocks, at least 2 k-blocks each
         if (tiles < num_sms) {
@@ -382,12 +450,9 @@ EMBER_API int ember_gemm_tc(const void* A, const void* W, void* out, int ldc, in
         if (splits < 1) splits = 1;
         while (splits > 1 && p.num_k_blocks / splits < 2) splits--;
     } else if (p.swapped && p.block_cols > 16) {
-        // Token tiles of 17 to 128: two such blocks fit on an SM, the stream reaches the memory's rate once about
-        // that many blocks are in flight, and every further part of K costs atomics and a wider finalize pass.  So:
-        // as many parts as keep tiles x parts within two blocks an SM, at least four k-blocks each.  Measured at 64
-        // tokens (us; parts in brackets): 1.7B widths q/k/v 12.6 (8), O 7.7 (8), gate/up 18.1 (3), down 10.5 (16),
-        // head 137 (1); 8B widths 18.6 (6), 11.9 (8), 43.0 (1), 22.3 (8), 232 (1).  (Counting waves over the SMs
-        // alone gave the head 16 parts, 364 us, and the 8B gate/up 3 parts, 51 us.)
+        // Token tiles of 17 to 128 by atomics: two such blocks fit on an SM, the stream reaches the memory's rate once
+        // about that many blocks are in flight, and every further part of K costs atomics.  So: as many parts as keep
+        // tiles x parts within two blocks an SM, at least four k-blocks each.
         splits = 2 * num_sms / (tiles > 0 ? tiles : 1);
         if (splits > 16) splits = 16;
         if (splits > p.num_k_blocks / 4) splits = p.num_k_blocks / 4;
@@ -406,7 +471,6 @@ EMBER_API int ember_gemm_tc(const void* A, const void* W, void* out, int ldc, in
     p.epilogue = epilogue; p.out = out; p.ldc = ldc; p.err = err;
     p.accum = nullptr; p.accum_ld = 0;
     p.cluster_splits = use_cluster ? splits : 1;
-    p.rows_per = (use_cluster && splits > 1) ? 2 * ((TILE_ROWS / 2 + splits - 1) / splits) : TILE_ROWS;
     if (!use_cluster && splits > 1) {
         if (epilogue == 2) {
             p.accum = (float*)out;
@@ -426,17 +490,17 @@ EMBER_API int ember_gemm_tc(const void* A, const void* W, void* out, int ldc, in
     const int rows_bytes = TILE_ROWS * TILE_K * 2;
     const int cols_bytes = p.block_cols * TILE_K * 2;
     const int stage_bytes = rows_bytes + ((cols_bytes + 1023) & ~1023);
-    const size_t recv_bytes = p.cluster_splits > 1 ? (size_t)splits * p.rows_per * p.block_cols * sizeof(float) : 0;
-    // Decode-sized tiles keep their blocks small (about 96 KiB of stages) so that two or three fit on
-    // an SM: the next kernel's blocks become resident and prefetch their weights while this kernel
-    // drains, and the memory system sees more independent streams.  Prefill tiles take all they can.
-    const size_t budget = p.swapped ? (size_t)96 * 1024 : (size_t)200 * 1024 - recv_bytes;
-    int stages = (int)(budget / stage_bytes);
-    if (stages > MAX_STAGES) stages = MAX_STAGES;
-    if (stages < 2) stages = 2;
-    if (stages > p.k_blocks_per_split) stages = p.k_blocks_per_split < 2 ? 2 : p.k_blocks_per_split;
-    p.stages = stages;
-    const size_t smem = (size_t)stages * stage_bytes + 1024 /* alignment slack */ + 256 /* barriers */ + recv_bytes;
+    size_t smem;
+    if (p.swapped) {
+        smem = decode_smem(p, num_sms);
+    } else {                                                   // prefill tiles take all they can
+        int stages = (int)((size_t)200 * 1024 / stage_bytes);
+        if (stages > MAX_STAGES) stages = MAX_STAGES;
+        if (stages < 2) stages = 2;
+        if (stages > p.k_blocks_per_split) stages = p.k_blocks_per_split < 2 ? 2 : p.k_blocks_per_split;
+        p.stages = stages;
+        smem = (size_t)stages * stage_bytes + 1024 + 256;
+    }
 
     CUtensorMap map_rows, map_cols;
     const void* rows_ptr = p.swapped ? W : A;
@@ -446,15 +510,7 @@ EMBER_API int ember_gemm_tc(const void* A, const void* W, void* out, int ldc, in
         !tensor_map(cols_ptr, cols_extent, K, p.block_cols, &map_cols))
         return fail("gemm_tc: cuTensorMapEncodeTiled failed or is unavailable");
 
-    static bool attr_set = false;
-    if (!attr_set) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-        if (e != cudaSuccess) return fail("gemm_tc: cannot raise the shared-memory limit: %s", cudaGetErrorString(e));
-        cudaFuncSetAttribute(gemm_tc_kernel<false>, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared);
-        cudaFuncSetAttribute(gemm_tc_kernel<true>, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared);
-        attr_set = true;
-    }
+    if (!raise_smem_limit()) return fail("gemm_tc: cannot raise the shared-memory limit");
     dim3 grid(row_tiles, col_tiles, splits);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
@@ -495,22 +551,26 @@ EMBER_API int ember_gemm_tc(const void* A, const void* W, void* out, int ldc, in
 }
 
 // The fused projection of a layer's attention: [q | k | v] = A . W^T for M > 128 tokens (rotation from the angle
-// table cos_sin) or for at most 16 (rotation from the frequencies inv_freq; either may be null), and straight from the
+// table cos_sin) or for at most 128 (rotation from the frequencies inv_freq; either may be null), and straight from the
 // accumulator every query and key head gets its RMSNorm (weights may be null) and its rotation (cos_sin, the table
 // of ember_rope_table with cs_ld tokens a row, may be null), queries go to q_out, keys and values into their cache pages.  Heads are 128 wide.  1 if these sizes are taken.
 EMBER_API int ember_gemm_tc_qkv_supported(int M, int N, int K, int n_heads, int n_kv, int head_dim) {
-    return M > 0 && (M <= 16 || M > 128) && K > 0 && K % 8 == 0 && head_dim == 128 && n_heads > 0 && n_kv > 0 &&
+    return M > 0 && K > 0 && K % 8 == 0 && head_dim == 128 && n_heads > 0 && n_kv > 0 &&
            N == (n_heads + 2 * n_kv) * 128;
 }
 
-// The fused projection of a decode-sized step (at most 16 tokens): 128 weight rows (one head slot) x the tokens per
+// The fused projection of a decode-sized step (at most 128 tokens): 128 weight rows (one head slot) x the tokens per
 // tile, the K range split over a thread-block cluster whose blocks share the tokens out and finish whole heads.
 static int launch_heads_swapped(const void* A, const void* W, GemmTcParams p, int num_sms, cudaStream_t st) {
+    if (!raise_smem_limit()) return fail("gemm_tc: cannot raise the shared-memory limit");
     p.swapped = 1;
-    p.block_cols = 16;
+    p.block_cols = (p.M + 15) / 16 * 16;
     const int tiles = p.N / TILE_ROWS;
     int splits = 1;
-    if (tiles < num_sms) {
+    if (p.block_cols > 16) {
+        const int parts = cluster_parts(p, tiles);
+        splits = parts > 0 ? parts : 1;
+    } else if (tiles < num_sms) {
         splits = (num_sms + tiles - 1) / tiles;
         if (splits > 8) splits = 8;
         while (splits > 1 && p.num_k_blocks / splits < 2) splits--;
@@ -518,31 +578,16 @@ static int launch_heads_swapped(const void* A, const void* W, GemmTcParams p, in
     p.k_blocks_per_split = (p.num_k_blocks + splits - 1) / splits;
     splits = (p.num_k_blocks + p.k_blocks_per_split - 1) / p.k_blocks_per_split;
     p.cluster_splits = splits;
-    p.rows_per = TILE_ROWS;
     p.row_tiles = tiles;
     p.total_tiles = tiles;
-    p.tmem_cols = 32;
+    int tc = 32;
+    while (tc < p.block_cols) tc <<= 1;
+    p.tmem_cols = tc;
     p.accum = nullptr; p.accum_ld = 0;
-    const int per = (p.block_cols + splits - 1) / splits;
-    const size_t recv_bytes = ((size_t)splits * per + 1) * TILE_ROWS * sizeof(float) + 64;     // partial sums, one head, 4 sums
-    const int stage_bytes = TILE_ROWS * TILE_K * 2 + ((p.block_cols * TILE_K * 2 + 1023) & ~1023);
-    int stages = (int)(((size_t)96 * 1024) / stage_bytes);
-    if (stages > MAX_STAGES) stages = MAX_STAGES;
-    if (stages > p.k_blocks_per_split) stages = p.k_blocks_per_split < 2 ? 2 : p.k_blocks_per_split;
-    p.stages = stages;
-    const size_t smem = (size_t)stages * stage_bytes + 1024 + 256 + recv_bytes;
+    const size_t smem = decode_smem(p, num_sms);
     CUtensorMap map_rows, map_cols;
     if (!tensor_map(W, p.N, p.K, TILE_ROWS, &map_rows) || !tensor_map(A, p.M, p.K, p.block_cols, &map_cols))
         return fail("gemm_tc: cuTensorMapEncodeTiled failed or is unavailable");
-    static bool attr_set = false;
-    if (!attr_set) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-        if (e != cudaSuccess) return fail("gemm_tc: cannot raise the shared-memory limit: %s", cudaGetErrorString(e));
-        cudaFuncSetAttribute(gemm_tc_kernel<false>, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared);
-        cudaFuncSetAttribute(gemm_tc_kernel<true>, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared);
-        attr_set = true;
-    }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(tiles, 1, splits);
     cfg.blockDim = dim3(GEMM_THREADS);
@@ -580,17 +625,16 @@ EMBER_API int ember_gemm_tc_qkv(const void* A, const void* W, int M, int N, int 
     p.M = M; p.N = N; p.K = K;
     p.num_k_blocks = (K + TILE_K - 1) / TILE_K;
     p.epilogue = 4; p.out = nullptr; p.ldc = 0; p.err = err;
-    p.rows_per = TILE_ROWS;
     p.qkv.n_heads = n_heads; p.qkv.n_kv = n_kv; p.qkv.q_norm_w = q_norm_w; p.qkv.k_norm_w = k_norm_w; p.qkv.eps = eps;
     if (cos_sin && cs_ld < M) return fail("gemm_tc_qkv: the rotation table has %d columns for %d tokens", cs_ld, M);
-    if (M <= 16 ? (cos_sin && !inv_freq) : (inv_freq && !cos_sin))
-        return fail("gemm_tc_qkv: %d tokens rotate with %s", M, M <= 16 ? "the frequencies" : "the angle table");
+    if (M <= 128 ? (cos_sin && !inv_freq) : (inv_freq && !cos_sin))
+        return fail("gemm_tc_qkv: %d tokens rotate with %s", M, M <= 128 ? "the frequencies" : "the angle table");
     p.qkv.inv_freq = inv_freq;
     p.qkv.cos_sin = (const float4*)cos_sin; p.qkv.cs_ld = cs_ld; p.qkv.positions = positions; p.qkv.seq_of = seq_of;
     p.qkv.block_table = block_table; p.qkv.max_blocks = max_blocks; p.qkv.page = page; p.qkv.num_pages = num_pages;
     p.qkv.q_out = (__nv_bfloat16*)q_out; p.qkv.k_pool = (__nv_bfloat16*)k_pool; p.qkv.v_pool = (__nv_bfloat16*)v_pool;
     p.qkv.write_kv = write_kv;
-    if (M <= 16) return launch_heads_swapped(A, W, p, num_sms, st);
+    if (M <= 128) return launch_heads_swapped(A, W, p, num_sms, st);
     const int block_cols = (N % 256 == 0) ? 256 : 128;          // whole heads in a tile
     if (split_mode != 5) {
         const int max_pairs = pair_capacity(num_sms);

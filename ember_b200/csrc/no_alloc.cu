@@ -99,7 +99,7 @@ EMBER_API int ember_gemm_tc_noalloc(const void* A, const void* W, void* out, int
     p.epilogue = epilogue; p.out = out; p.ldc = ldc; p.err = err;
     p.accum = nullptr; p.accum_ld = 0;
     p.row_tiles = 0; p.total_tiles = 0;
-    p.cluster_splits = 1; p.rows_per = TILE_ROWS;      // this variant sums its K splits with atomics into the scratch
+    p.cluster_splits = 1;      // this variant sums its K splits with atomics into the scratch
     if (splits > 1) {
         if (epilogue == 2) {
             p.accum = (float*)out;

@@ -493,12 +493,12 @@ def gemm_tc_grouped(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, M: int,
 
 def gemm_tc_qkv_usable(x: torch.Tensor, w: torch.Tensor, bias, M: int, n_heads: int, n_kv: int, head_dim: int,
                        rotary: int) -> bool:
-    """Whether the fused projection takes this step: bf16, no bias, heads of 128 rotated whole (or not at all),
-    more than 128 tokens or at most 16 (the rule of ember_gemm_tc_qkv_supported)."""
+    """Whether the fused projection takes this step: bf16, no bias, heads of 128 rotated whole or not at all
+    (the rule of ember_gemm_tc_qkv_supported)."""
     if bias is not None or not gemm_tc_usable(x, w, bias, EPI_STORE):
         return False
     n, k = w.shape
-    return (0 < M <= 16 or M > 128) and head_dim == 128 and rotary in (0, 128) and n == (n_heads + 2 * n_kv) * 128
+    return M > 0 and head_dim == 128 and rotary in (0, 128) and n == (n_heads + 2 * n_kv) * 128
 
 
 # From how many tokens on a step's q/k/v product finishes the heads itself.  Measured at the 1.7B shape, product +
@@ -506,10 +506,11 @@ def gemm_tc_qkv_usable(x: torch.Tensor, w: torch.Tensor, bias, M: int, n_heads: 
 # 74.5 / 51.3 at 4,096 (below, the step is one or two tiles an SM and the longer epilogue has no next tile to
 # hide behind).
 QKV_FUSE_MIN_TOKENS = 512
-# Up to how many tokens a decode step's q/k/v product does (product + head kernel against the fused product, in a
-# graph: 8.4 / 6.2 us at 1 token, 9.1 / 7.6 at 8, 9.4 / 10.1 at 16: a block of the cluster finishes its share of
-# the tokens one after the other, and only the first two are prepared while the product runs).
-QKV_FUSE_MAX_DECODE_TOKENS = 8
+# Up to how many tokens the product in the orientation of few tokens does, and up to how many rows of weights it does so
+# beyond 64 tokens (more tiles than a cluster each finds SMs for).  Product + head kernel against the fused product, in a
+# graph, 16/8 heads, K = 2,048: 7.9 / 6.2 us at 8 tokens, 9.9 / 6.7 at 24, 13.1 / 10.3 at 64 (five parts), 17.8 / 16.5 at 128.
+QKV_FUSE_MAX_DECODE_TOKENS = 128
+QKV_FUSE_WIDE_ROWS = 8192
 
 
 def rope_table(positions: torch.Tensor, inv_freq: torch.Tensor, T: int, out: torch.Tensor, stream: Optional[int] = None) -> None:
@@ -535,7 +536,7 @@ def gemm_tc_qkv(a: torch.Tensor, w: torch.Tensor, M: int, n_heads: int, n_kv: in
     """[q | k | v] = a[:M] @ w.T on the tcgen05 tensor cores with the heads finished in the epilogue: RMSNorm and
     rotation of query and key heads in fp32 on the accumulator, queries to ``q_out``, keys and values into their
     cache pages.  More than 128 tokens rotate with ``cos_sin`` [32, tokens a row, 4] from ``rope_table``, at most
-    16 with the frequencies ``inv_freq`` [64] (both None: no rotation).  Heads are 128 wide."""
+    128 with the frequencies ``inv_freq`` [64] (both None: no rotation).  Heads are 128 wide."""
     _check(a, "a", torch.bfloat16)
     _check(w, "w", torch.bfloat16)
     _check(q_out, "q_out", torch.bfloat16)

@@ -137,14 +137,15 @@ class Attention(Mixer):
         att = ctx.buf("attention.out", (mt, s.q_dim), rt.dtype)
         table = ctx.block_table(cache.group)
         rotates = self.inv_freq is not None and self.rotary > 0
-        if (self.FUSE_QKV and (T >= ops.QKV_FUSE_MIN_TOKENS or T <= ops.QKV_FUSE_MAX_DECODE_TOKENS) and
+        few = T <= (ops.QKV_FUSE_MAX_DECODE_TOKENS if self.qkv.n <= ops.QKV_FUSE_WIDE_ROWS else 64)
+        if (self.FUSE_QKV and (T >= ops.QKV_FUSE_MIN_TOKENS or few) and
                 ops.gemm_tc_qkv_usable(x, self.qkv.weight, self.qkv.bias, T, s.num_heads, s.num_kv_heads, s.head_dim,
                                        self.rotary if rotates else 0)):
             # norm, rotation and the cache write happen in the product's epilogue: a prompt portion rotates with
-            # the step's angle table, a decode step of a few tokens computes its angles itself
-            cos_sin = self.position.cos_sin(ctx, rt) if rotates and T > 16 else None
+            # the step's angle table, a step of up to 128 tokens computes its angles itself
+            cos_sin = self.position.cos_sin(ctx, rt) if rotates and T > 128 else None
             ops.gemm_tc_qkv(x, self.qkv.weight, T, s.num_heads, s.num_kv_heads, self.q_norm_w, self.k_norm_w,
-                            s.qk_norm_eps, cos_sin, self.inv_freq if rotates and T <= 16 else None, ctx.positions,
+                            s.qk_norm_eps, cos_sin, self.inv_freq if rotates and T <= 128 else None, ctx.positions,
                             ctx.seq_of, table, cache.page_tokens, cache.k, cache.v, q, write_kv=owns_cache, err=ctx.err,
                             stream=ctx.stream)
         elif (self.SUMS_TO_HEADS and 16 < T <= 128 and self.qkv.bias is None and ops.gemm_tc_usable(x, self.qkv.weight, self.qkv.bias, ops.EPI_STORE)

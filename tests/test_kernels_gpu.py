@@ -569,6 +569,62 @@ def test_gemm_tc_qkv(heads, kv, page, M, norm, rotate):
     assert int(err.item()) == 2
 
 
+@pytest.mark.parametrize("heads,kv,M,K", [(16, 8, 17, 2048), (16, 8, 64, 2048), (3, 1, 65, 136), (4, 2, 100, 328), (16, 8, 128, 2048),
+                                          (40, 8, 33, 4096), (1, 1, 48, 64)])
+@pytest.mark.parametrize("norm,rotate", [(True, True), (False, True), (True, False)])
+def test_gemm_tc_qkv_few_tokens(heads, kv, M, K, norm, rotate):
+    """17 to 128 tokens: heads finished by the cluster's warps (one to sixteen tokens a block, the first two of a warp prepared
+    early) against the product's sums and the head kernel; both round the same fp32 heads once to bfloat16."""
+    from ember_b200 import ops
+    torch.manual_seed(heads * M)
+    dev, D, page = "cuda", 128, 16
+    N, pages = (heads + 2 * kv) * D, 8 * M
+    a, w = torch.randn(M, K, device=dev).bfloat16(), (torch.randn(N, K, device=dev) * 0.1).bfloat16()
+    qw, kw = (1 + 0.1 * torch.randn(D, device=dev), 1 + 0.1 * torch.randn(D, device=dev)) if norm else (None, None)
+    inv = 1.0 / (10000.0 ** (torch.arange(D // 2, device=dev).float() * 2 / D)) if rotate else None
+    pos = torch.randint(0, 8 * page, (M,), device=dev).int()
+    seq = torch.arange(M, device=dev).int()
+    table = torch.randperm(pages, device=dev).int().view(M, 8)
+    table[M - 1, int(pos[M - 1]) // page] = pages + 3                      # recorded, not written
+    got = []
+    for fused in (True, False):
+        kp = torch.zeros(pages, kv, page, D, device=dev, dtype=torch.bfloat16)
+        vp, q, err = torch.zeros_like(kp), torch.zeros(M, heads * D, device=dev, dtype=torch.bfloat16), torch.zeros(1, dtype=torch.int32, device=dev)
+        if fused:
+            ops.gemm_tc_qkv(a, w, M, heads, kv, qw, kw, 1e-5, None, inv, pos, seq, table, page, kp, vp, q, err=err)
+        else:
+            sums = ops.gemm_tc(a, w, None, M, ops.EPI_SUMS, err=err)
+            ops.qk_norm_rope_store_sums(sums, M, heads, kv, qw, kw, 1e-5, inv, pos, seq, table, page, kp, vp, q, err=err)
+        assert int(err.item()) == 2
+        got.append((q, kp, vp))
+    for x, y in zip(*got):
+        assert float((x.float() - y.float()).norm()) <= 2.0 ** -8 * float(y.float().norm())
+
+
+@pytest.mark.parametrize("M", [24, 64, 96, 128])
+@pytest.mark.parametrize("N,K", [(2048, 2048), (1001, 264), (4099, 1000), (128, 64), (20000, 200)])
+@pytest.mark.parametrize("epilogue", [0, 1, 2, 8, 9])
+def test_gemm_tc_cluster_sums_with_bias(M, N, K, epilogue):
+    """The sums of a cluster joined by a bias and an activation; rows of outputs that are no multiple of four."""
+    from ember_b200 import ops
+    torch.manual_seed(M + N)
+    a, w = torch.randn(M, K, device="cuda").bfloat16(), (torch.randn(N, K, device="cuda") * 0.1).bfloat16()
+    bias, prev = torch.randn(N, device="cuda"), torch.randn(M + 1, N, device="cuda")
+    x = a.double() @ w.double().t() + bias.double()
+    if epilogue == 8:
+        x = torch.nn.functional.gelu(x)
+    elif epilogue == 9:
+        x = torch.relu(x) ** 2
+    elif epilogue == 2:
+        x = x + prev[:M].double()
+    out = prev.clone() if epilogue in (1, 2) else torch.zeros(M + 1, N, device="cuda", dtype=torch.bfloat16)
+    last = out[M].clone()
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    ops.gemm_tc(a, w, out, M, epilogue, err=err, bias=bias)
+    assert int(err.item()) == 0 and torch.equal(out[M], last)
+    assert rel(out[:M].double(), x) < (1e-5 if epilogue in (1, 2) else 2.0 ** -8)
+
+
 @pytest.mark.parametrize("heads,kv,page,M,K", [(16, 8, 64, 64, 2048), (4, 2, 16, 17, 328), (3, 1, 32, 128, 136), (40, 8, 16, 100, 512),
                                                (32, 8, 64, 33, 4096)])
 @pytest.mark.parametrize("norm,rotate", [(True, True), (False, True), (True, False)])
