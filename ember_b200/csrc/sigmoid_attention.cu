@@ -7,7 +7,7 @@
 // pages: k_pool [pages, kv_heads, page, D], v_pool [pages, kv_heads, page, V].
 // attend: one block per (tile of consecutive queries of a run, heads of one key/value head): 16 (token, head) rows;
 // keys are walked in tiles of 32 in ascending order, so an output's sum has the same order however the tokens were
-// cut into steps.
+// cut into steps (the tensor-core form: within the parts that a tile's keys are cut into).
 #include "common.cuh"
 
 EMBER_DEFINE_LAST_ERROR
@@ -210,7 +210,13 @@ inline int heads_per_block(int group) {
 // rounded one) and the three products are added in the fp32 accumulator.  A block: 16 (token, head) rows, 64-key
 // tiles fetched with cp.async into two buffers; warp w takes keys 16 w .. 16 w + 15 of a tile for the scores and a
 // quarter of the value columns for the read-out; the weights pass through shared memory.
-constexpr int TC_KEYS = 64;
+//
+// A tile of 64 keys takes a block about 3 us whatever else runs, so a step of few blocks (a decoded token: one per
+// request and key/value head) is bound by its longest key range.  Such a step runs each tile on a cluster of up to eight
+// blocks (gridDim.z): block z takes the z-th part of the key tiles, the partial sums (nothing is normalised: they
+// just add) wait in each block's shared memory, and every block adds a share of the outputs over the cluster in key
+// order.  One request at 1,500 keys, 16/8 heads of 128: 72 -> 17 us.  Blocks start with the tiles of most keys.
+constexpr int TC_KEYS = 64, TC_SPLITS = 8;
 
 __device__ __forceinline__ void mma_bf16_16816(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
@@ -238,7 +244,7 @@ sigmoid_attention_tc_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bflo
     extern __shared__ __align__(16) unsigned char smem_raw[];
     pdl_launch_dependents();
     pdl_wait();
-    const int* tile = tiles + 4 * blockIdx.x;
+    const int* tile = tiles + 4 * (gridDim.x - 1 - blockIdx.x);        // later tiles of a run have more keys
     const int run = tile[0], row0 = tile[1], nq = tile[2], pos0 = tile[3];
     const int h0 = blockIdx.y * hpb, kv = h0 / (H / G);
     const int n_rows = nq * hpb;
@@ -299,12 +305,16 @@ sigmoid_attention_tc_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bflo
 #pragma unroll
     for (int nb = 0; nb < NBV; nb++) acc[nb][0] = acc[nb][1] = acc[nb][2] = acc[nb][3] = 0.0f;
 
-    fetch(0, 0);
+    // this block's key tiles
+    const int splits = (int)gridDim.z, key_tiles = (n_keys + TC_KEYS - 1) / TC_KEYS, per = (key_tiles + splits - 1) / splits;
+    const int k_first = min(key_tiles, (int)blockIdx.z * per) * TC_KEYS;
+    const int k_end = min(n_keys, min(key_tiles, ((int)blockIdx.z + 1) * per) * TC_KEYS);
+    if (k_first < k_end) fetch(k_first, 0);
     int buf = 0;
-    for (int k0 = 0; k0 < n_keys; k0 += TC_KEYS, buf ^= 1) {
+    for (int k0 = k_first; k0 < k_end; k0 += TC_KEYS, buf ^= 1) {
         asm volatile("cp.async.wait_group 0;\n" ::: "memory");
         __syncthreads();                                            // the tile is in; the other buffer and P are free
-        if (k0 + TC_KEYS < n_keys) fetch(k0 + TC_KEYS, buf ^ 1);
+        if (k0 + TC_KEYS < k_end) fetch(k0 + TC_KEYS, buf ^ 1);
         const __nv_bfloat16* Kt = Ks + (size_t)buf * TC_KEYS * DP;
         const __nv_bfloat16* Vt = Vs + (size_t)buf * TC_KEYS * VP;
         // scores of this warp's 16 keys, their weights in three pieces to shared memory
@@ -369,6 +379,39 @@ sigmoid_attention_tc_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bflo
             }
         }
     }
+    if (splits > 1) {
+        float* sums = reinterpret_cast<float*>(Vs);                 // [16][V] in the place of the value tiles
+        __syncthreads();
+#pragma unroll
+        for (int nb = 0; nb < NBV; nb++) {
+            if (nb < nbv) {
+                const int col = warp * vw + nb * 8 + 2 * c;
+                *reinterpret_cast<float2*>(sums + g * V + col) = make_float2(acc[nb][0], acc[nb][1]);
+                *reinterpret_cast<float2*>(sums + (g + 8) * V + col) = make_float2(acc[nb][2], acc[nb][3]);
+            }
+        }
+        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+        const float* part[TC_SPLITS];
+#pragma unroll
+        for (int z = 0; z < TC_SPLITS; z++)
+            if (z < splits) asm volatile("mapa.u64 %0, %1, %2;" : "=l"(part[z]) : "l"(sums), "r"(z));
+        const int pairs = n_rows * V / 2;                           // V is even
+        for (int e = (int)blockIdx.z * 128 + (int)threadIdx.x; e < pairs; e += splits * 128) {
+            float2 t = make_float2(0.0f, 0.0f);
+#pragma unroll
+            for (int z = 0; z < TC_SPLITS; z++)
+                if (z < splits) {
+                    const float2 u = reinterpret_cast<const float2*>(part[z])[e];
+                    t.x += u.x; t.y += u.y;
+                }
+            const int r = 2 * e / V, col = 2 * e - r * V;
+            *reinterpret_cast<uint32_t*>(out + ((size_t)(row0 + r / hpb) * H + h0 + r % hpb) * V + col) = pack_bf16(t.x, t.y);
+        }
+        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");      // nobody leaves while others read its sums
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+        return;
+    }
 #pragma unroll
     for (int nb = 0; nb < NBV; nb++) {
         if (nb < nbv) {
@@ -394,9 +437,23 @@ int launch_attend_tc(const void* q, const void* k_pool, const void* v_pool, void
                      const float* head_bias, int* err, cudaStream_t st) {
     const size_t smem = ((size_t)2 * TC_KEYS * (D + 8) + (size_t)2 * TC_KEYS * (V + 8) + 3 * 16 * (TC_KEYS + 8)) * sizeof(__nv_bfloat16);
     if (smem > 48 * 1024) cudaFuncSetAttribute(sigmoid_attention_tc_kernel<DK, NBV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    launch_kernel(sigmoid_attention_tc_kernel<DK, NBV>, dim3(n_tiles, H / hpb), 128, smem, st, (const __nv_bfloat16*)q,
-                  (const __nv_bfloat16*)k_pool, (const __nv_bfloat16*)v_pool, (__nv_bfloat16*)out, H, G, D, V, hpb, tiles, bt, max_blocks,
-                  page, num_pages, scale, head_bias, err);
+    // as many blocks as two per SM while a tile can be cut
+    int splits = TC_SPLITS;
+    while (splits > 1 && (long long)n_tiles * (H / hpb) * splits > 296) splits >>= 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(n_tiles, H / hpb, splits);
+    cfg.blockDim = dim3(128);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attrs[2];
+    attrs[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attrs[0].val.programmaticStreamSerializationAllowed = pdl_enabled() ? 1 : 0;
+    attrs[1].id = cudaLaunchAttributeClusterDimension;
+    attrs[1].val.clusterDim.x = 1; attrs[1].val.clusterDim.y = 1; attrs[1].val.clusterDim.z = (unsigned)splits;
+    cfg.attrs = attrs; cfg.numAttrs = splits > 1 ? 2 : 1;
+    cudaLaunchKernelEx(&cfg, sigmoid_attention_tc_kernel<DK, NBV>, (const __nv_bfloat16*)q, (const __nv_bfloat16*)k_pool,
+                       (const __nv_bfloat16*)v_pool, (__nv_bfloat16*)out, H, G, D, V, hpb, tiles, bt, max_blocks, page, num_pages, scale,
+                       head_bias, err);
     return check_launch("sigmoid_attention");
 }
 

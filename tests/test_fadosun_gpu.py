@@ -235,6 +235,35 @@ def test_sigmoid_attention_alone(dtype, heads, kv, dim, vdim, rot, base, hidden)
     assert _rel(_run_mixer(spec, w, x, dtype), want) < MIX_TOL[dtype]
 
 
+@pytest.mark.parametrize("heads,kv,dim,vdim", [(4, 2, 128, 128), (6, 2, 32, 32), (8, 1, 144, 160)])
+@pytest.mark.parametrize("lens", [[1], [63, 64, 65], [513, 1, 448, 2000], [129] * 37])
+def test_sigmoid_attention_key_parts(heads, kv, dim, vdim, lens):
+    """Decoded tokens whose key ranges are cut over a cluster (one, a few and many requests, so eight, fewer and no parts;
+    ranges of fewer tiles than parts, of whole tiles and one key more) against 64-bit values, an empty page in between."""
+    from ember_b200 import ops
+    torch.manual_seed(len(lens) + dim)
+    page, n = 16, len(lens)
+    width = (max(lens) + page - 1) // page
+    pages = 1 + n * width
+    kp, vp = torch.randn(pages, kv, page, dim).bfloat16(), torch.randn(pages, kv, page, vdim).bfloat16()
+    table = (torch.randperm(n * width).view(n, width) + 1).to(torch.int32)
+    q, bias = torch.randn(n, heads, dim).bfloat16(), torch.randn(heads) - 2.0
+    tiles = torch.tensor([[r, r, 1, lens[r] - 1] for r in range(n)], dtype=torch.int32)
+    out = torch.zeros(n, heads * vdim, dtype=torch.bfloat16, device="cuda")
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    ops.sigmoid_attention(q.view(n, -1).cuda(), kp.cuda(), vp.cuda(), out, heads, kv, dim, vdim, tiles.cuda(), n, table.cuda(), page, 0.1,
+                          bias.cuda(), err=err)
+    assert int(err.item()) == 0
+    for r in range(n):
+        k = kp[table[r].long()].double().permute(1, 0, 2, 3).reshape(kv, -1, dim)[:, :lens[r]]
+        v = vp[table[r].long()].double().permute(1, 0, 2, 3).reshape(kv, -1, vdim)[:, :lens[r]]
+        g = heads // kv
+        k, v = k.repeat_interleave(g, 0), v.repeat_interleave(g, 0)
+        w = torch.sigmoid(torch.einsum("hd,hkd->hk", q[r].double(), k) * 0.1 + bias.double()[:, None])
+        want = torch.einsum("hk,hkv->hv", w, v).reshape(-1)
+        assert _rel(out[r].cpu(), want) < 2.0 ** -8                    # (one rounding of the result to bfloat16)
+
+
 def test_a_far_key_that_dominates_is_seen_across_pages_and_portions():
     """Head biases so low that ordinary keys weigh nothing, one early key and two late queries scaled so that their
     scores stand out: the read-out at those queries is that one key's value, in a prompt portion and decoded alone."""
