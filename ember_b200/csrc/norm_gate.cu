@@ -18,6 +18,8 @@
 //   logit_finish      logits <- cap tanh(scale logits / cap)
 // Rows are read from the fp32 residual stream or from fp32 results of a product; a row is reduced by one block
 // (or one warp for the short rows of a head) in an order fixed by the thread layout.
+#include <type_traits>
+
 #include "common.cuh"
 
 EMBER_DEFINE_LAST_ERROR
@@ -152,6 +154,99 @@ norm_add_norm_kernel(const float* __restrict__ y, const float* __restrict__ w, f
 #pragma unroll
         for (int k = 0; k < W; k++) h[k] = h[k] * r2 * g[k];
         row_store<W>(out + base + i, h);
+    }
+}
+
+// The same behind a gate and with either kind of norm on both sides: a
+// step of a few tokens is a chain of such rows, so what counts is one row's latency.  The row stays in registers (PER
+// pieces of four elements a thread), all loads are under way at once, and up to PER = 2 the weights are asked for
+// before the wait for the kernel before.  One row of 2,048 in a step: gate, norm and addition took 7.6 us and the norm
+// behind them 3.4, now 3.7 together; 24 rows 7.1 + 3.4, now 4.4.
+template <typename TO, int PER>
+__global__ void __launch_bounds__(ROW_THREADS)
+gated_norm_add_norm_kernel(const float* __restrict__ y, const float* __restrict__ gate, const float* __restrict__ gate_bias,
+                           const float* __restrict__ w, const float* __restrict__ b, float eps, int centred, float* __restrict__ residual,
+                           const float* __restrict__ w2, const float* __restrict__ b2, float eps2, int centred2, TO* __restrict__ out, int H) {
+    __shared__ float scratch[32];
+    pdl_launch_dependents();
+    constexpr bool EARLY = PER <= 2;
+    const size_t base = (size_t)blockIdx.x * H;
+    auto at = [&](int u) { return (int)(threadIdx.x + u * ROW_THREADS) * 4; };
+    auto piece = [&](const float* p, int i, float (&v)[4]) {
+        if (p && i < H) row_load<4>(p + i, v);
+        else v[0] = v[1] = v[2] = v[3] = 0.0f;
+    };
+    float g1[EARLY ? PER : 1][4], a1[EARLY ? PER : 1][4], g2[EARLY ? PER : 1][4], a2[EARLY ? PER : 1][4], gb[EARLY ? PER : 1][4];
+    if (EARLY) {
+#pragma unroll
+        for (int u = 0; u < PER; u++) {
+            piece(w, at(u), g1[EARLY ? u : 0]);
+            piece(b, at(u), a1[EARLY ? u : 0]);
+            piece(gate ? gate_bias : nullptr, at(u), gb[EARLY ? u : 0]);
+            piece(w2, at(u), g2[EARLY ? u : 0]);
+            piece(b2, at(u), a2[EARLY ? u : 0]);
+        }
+    }
+    pdl_wait();
+    float v[PER][4], h[PER][4], s = 0.0f;
+#pragma unroll
+    for (int u = 0; u < PER; u++) {
+        piece(y + base, at(u), v[u]);
+        piece(residual + base, at(u), h[u]);
+    }
+    if (gate) {
+#pragma unroll
+        for (int u = 0; u < PER; u++) {
+            float z[4], late[4];
+            piece(gate + base, at(u), z);
+            if (!EARLY) piece(gate_bias, at(u), late);
+#pragma unroll
+            for (int k = 0; k < 4; k++) v[u][k] *= sigmoidf_(z[k] + (EARLY ? gb[EARLY ? u : 0][k] : late[k]));
+        }
+    }
+#pragma unroll
+    for (int u = 0; u < PER; u++)
+#pragma unroll
+        for (int k = 0; k < 4; k++) s += v[u][k];
+    const float mean = centred ? block_sum(s, scratch) / (float)H : 0.0f;
+    float ss = 0.0f;
+#pragma unroll
+    for (int u = 0; u < PER; u++)
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            v[u][k] -= mean;
+            if (at(u) < H) ss = fmaf(v[u][k], v[u][k], ss);
+        }
+    const float rstd = 1.0f / sqrtf(block_sum(ss, scratch) / (float)H + eps);
+    s = 0.0f;
+#pragma unroll
+    for (int u = 0; u < PER; u++) {
+        float gl[4], al[4];
+        if (!EARLY) { piece(w, at(u), gl); piece(b, at(u), al); }
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            h[u][k] += v[u][k] * rstd * (EARLY ? g1[EARLY ? u : 0][k] : gl[k]) + (EARLY ? a1[EARLY ? u : 0][k] : al[k]);
+            s += h[u][k];
+        }
+        if (at(u) < H) row_store<4>(residual + base + at(u), h[u]);
+    }
+    const float mean2 = centred2 ? block_sum(s, scratch) / (float)H : 0.0f;
+    ss = 0.0f;
+#pragma unroll
+    for (int u = 0; u < PER; u++)
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            h[u][k] -= mean2;
+            if (at(u) < H) ss = fmaf(h[u][k], h[u][k], ss);
+        }
+    const float rstd2 = 1.0f / sqrtf(block_sum(ss, scratch) / (float)H + eps2);
+#pragma unroll
+    for (int u = 0; u < PER; u++) {
+        float gl[4], al[4];
+        if (!EARLY) { piece(w2, at(u), gl); piece(b2, at(u), al); }
+#pragma unroll
+        for (int k = 0; k < 4; k++) h[u][k] = h[u][k] * rstd2 * (EARLY ? g2[EARLY ? u : 0][k] : gl[k]) + (EARLY ? a2[EARLY ? u : 0][k] : al[k]);
+        if (at(u) < H) row_store<4>(out + base + at(u), h[u]);
     }
 }
 
@@ -504,6 +599,35 @@ EMBER_API int ember_gated_norm_add(const float* y, const float* gate, const floa
     if (centred) launch_kernel(gated_norm_add_kernel<true>, n_rows, ROW_THREADS, smem, st, y, gate, gate_bias, w, b, eps, residual, (__nv_bfloat16*)rounded, H);
     else launch_kernel(gated_norm_add_kernel<false>, n_rows, ROW_THREADS, smem, st, y, gate, gate_bias, w, b, eps, residual, (__nv_bfloat16*)rounded, H);
     return check_launch("gated_norm_add");
+}
+
+// 1 if ember_gated_norm_add_norm takes rows of this width.
+EMBER_API int ember_gated_norm_add_norm_supported(int H) { return H > 0 && H % 4 == 0 && H <= 8 * 4 * ROW_THREADS; }
+
+EMBER_API int ember_gated_norm_add_norm(const float* y, const float* gate, const float* gate_bias, const float* w, const float* b, float eps,
+                                        int centred, float* residual, const float* w2, const float* b2, float eps2, int centred2,
+                                        void* out, int out_dtype, int n_rows, int H, void* stream) {
+    if (n_rows <= 0) return 0;
+    if (!ember_gated_norm_add_norm_supported(H)) return fail("gated_norm_add_norm: width %d is not taken", H);
+    if ((((uintptr_t)y) | ((uintptr_t)gate) | ((uintptr_t)gate_bias) | ((uintptr_t)w) | ((uintptr_t)b) | ((uintptr_t)residual) | ((uintptr_t)w2) |
+         ((uintptr_t)b2) | ((uintptr_t)out)) & 15)
+        return fail("gated_norm_add_norm: operands must be 16-byte aligned");
+    const int pieces = (H + 4 * ROW_THREADS - 1) / (4 * ROW_THREADS);
+    auto run = [&](auto kernel, auto* o) -> int {
+        launch_kernel(kernel, n_rows, ROW_THREADS, 0, (cudaStream_t)stream, y, gate, gate_bias, w, b, eps, centred, residual, w2, b2, eps2,
+                      centred2, o, H);
+        return check_launch("gated_norm_add_norm");
+    };
+    auto pick = [&](auto* o) -> int {
+        using T = std::remove_pointer_t<decltype(o)>;
+        if (pieces <= 1) return run(gated_norm_add_norm_kernel<T, 1>, o);
+        if (pieces <= 2) return run(gated_norm_add_norm_kernel<T, 2>, o);
+        if (pieces <= 4) return run(gated_norm_add_norm_kernel<T, 4>, o);
+        return run(gated_norm_add_norm_kernel<T, 8>, o);
+    };
+    if (out_dtype == EMBER_F32) return pick((float*)out);
+    if (out_dtype == EMBER_BF16) return pick((__nv_bfloat16*)out);
+    return fail("gated_norm_add_norm: unsupported dtype %d", out_dtype);
 }
 
 EMBER_API int ember_norm_add_norm(const float* y, const float* w, float eps, float* residual, const float* w2, float eps2, void* out,

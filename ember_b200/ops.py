@@ -728,6 +728,33 @@ def gated_norm_add(y: torch.Tensor, gate_logits: Optional[torch.Tensor], weight:
           _p(residual), _p(rounded), c_int(n_rows), c_int(H), _stream(stream))
 
 
+def gated_norm_add_norm_usable(width: int) -> bool:
+    """Whether ``gated_norm_add_norm`` takes rows of this width (the rule of ember_gated_norm_add_norm_supported)."""
+    return width % 4 == 0 and 0 < width <= 8192
+
+
+def gated_norm_add_norm(y: torch.Tensor, gate_logits: Optional[torch.Tensor], gate_bias: Optional[torch.Tensor], w: torch.Tensor,
+                        b: Optional[torch.Tensor], eps: float, centred: bool, residual: torch.Tensor, w2: torch.Tensor,
+                        b2: Optional[torch.Tensor], eps2: float, centred2: bool, out: torch.Tensor, n_rows: int,
+                        stream: Optional[int] = None) -> None:
+    """residual[r] += norm(y[r] * sigmoid(gate_logits[r] + gate_bias)) and out[r] = norm2(residual[r]) in one kernel, each norm
+    centred (layer norm) or not (RMS norm)."""
+    H = w.numel()
+    for t, n in ((y, "y"), (gate_logits, "gate_logits"), (gate_bias, "gate_bias"), (w, "w"), (b, "b"), (residual, "residual"), (w2, "w2"), (b2, "b2")):
+        if t is not None:
+            _check(t, n, torch.float32)
+    _check(out, "out")
+    if y.shape[-1] != H or residual.shape[-1] != H or out.shape[-1] != H or w2.numel() != H or \
+            any(t is not None and t.numel() != H for t in (b, b2, gate_bias)) or \
+            (gate_logits is not None and (gate_logits.shape[-1] != H or gate_logits.numel() < n_rows * H)) or \
+            min(y.numel(), residual.numel(), out.numel()) < n_rows * H:
+        raise KernelError(f"gated_norm_add_norm: buffers do not fit {n_rows} rows of {H}")
+    lib = _lib("norm_gate")
+    _call(lib, lib.ember_gated_norm_add_norm, _p(y), _p(gate_logits), _p(gate_bias), _p(w), _p(b), c_float(eps), c_int(1 if centred else 0),
+          _p(residual), _p(w2), _p(b2), c_float(eps2), c_int(1 if centred2 else 0), _p(out), c_int(dtype_code(out.dtype)), c_int(n_rows),
+          c_int(H), _stream(stream))
+
+
 def norm_add_norm(y: torch.Tensor, weight: torch.Tensor, eps: float, residual: torch.Tensor, next_weight: torch.Tensor, next_eps: float,
                   out: torch.Tensor, n_rows: int, stream: Optional[int] = None) -> None:
     """residual[r] += rms_norm(y[r]) and out[r] = rms_norm(residual[r]) of the new rows, each norm with its weight and eps, in

@@ -19,7 +19,7 @@ import torch
 from .. import ops
 from ..config.spec import ConfigError
 from .base import CacheNeed, Runtime, WeightDecl
-from .norm import RMSNorm
+from .norm import RMSNorm, RowNorm
 from .registry import build_part, register_part
 
 
@@ -124,8 +124,8 @@ class GatedSandwichBlock(Arrangement):
     stream rounded once, which the ``gated_add`` before it leaves beside the new residual rows (the first sublayer of
     a step, or one that follows another arrangement, rounds the stream in a kernel of its own).
 
-    Without a gate, and with RMS norms on both sides, the output norm, the addition and the *next* sublayer's input norm
-    are one kernel (``add_then_norm``): the feed-forward's of this layer, and the mixer's of the layer that runs next, which
+    The output norm (with its gate), the addition and the *next* sublayer's input norm are one kernel
+    (``gated_add_norm``, or ``add_then_norm`` for RMS norms without a gate): the feed-forward's of this layer, and the mixer's of the layer that runs next, which
     the model names in ``ctx.memo["block.next_norm"]`` and which finds its normed rows in the blocks' common buffer."""
 
     ROLES = {"mixer_norm": "norm", "mixer": "mixer", "mixer_gate": "gate", "mixer_out_norm": "norm",
@@ -180,6 +180,9 @@ class GatedSandwichBlock(Arrangement):
             gate.forward(ctx, x, logits)
         if gate is None and rounded is None and isinstance(norm_out, RMSNorm) and isinstance(norm_next, RMSNorm):
             norm_out.add_then_norm(ctx, y, h, T, norm_next, normed_x)
+            return True
+        if rounded is None and isinstance(norm_out, RowNorm) and isinstance(norm_next, RowNorm) and ops.gated_norm_add_norm_usable(hidden):
+            norm_out.gated_add_norm(ctx, y, logits, h, T, getattr(gate, "bias", None), norm_next, normed_x)
             return True
         if rounded is not None:
             norm_out.gated_add(ctx, y, logits, h, T, gate_bias=getattr(gate, "bias", None), rounded=rounded)

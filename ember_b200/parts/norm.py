@@ -15,7 +15,20 @@ from .base import Norm, Runtime, WeightDecl
 from .registry import register_part
 
 
-class RMSNorm(Norm):
+class RowNorm(Norm):
+    """RMS and layer norms: what the kernels that join them to a gate, an addition and the norm that comes next need."""
+
+    centred = False
+    bias: Optional[torch.Tensor] = None
+
+    def gated_add_norm(self, ctx, y: torch.Tensor, gate_logits: Optional[torch.Tensor], residual: torch.Tensor, n_rows: int,
+                       gate_bias: Optional[torch.Tensor], after: "RowNorm", out: torch.Tensor) -> None:
+        """residual += norm(y * sigmoid(gate_logits + gate_bias)), and ``out`` = the norm ``after`` of the new rows, in one kernel."""
+        ops.gated_norm_add_norm(y, gate_logits, gate_bias, self.weight, self.bias, self.spec.eps, self.centred, residual, after.weight,
+                                after.bias, after.spec.eps, after.centred, out, n_rows, stream=ctx.stream)
+
+
+class RMSNorm(RowNorm):
     graph_safe = True
 
     def _name(self) -> str:
@@ -60,10 +73,11 @@ class RMSNorm(Norm):
                             stream=ctx.stream)
 
 
-class LayerNorm(Norm):
+class LayerNorm(RowNorm):
     """out = (x - mean) / sqrt(var + eps) * weight + bias, var = mean((x - mean)^2), statistics in fp32."""
 
     graph_safe = True
+    centred = True
 
     def _names(self):
         return self.prefix + self.spec.weight_suffix, self.prefix + self.spec.bias_suffix

@@ -292,6 +292,31 @@ def test_a_far_key_that_dominates_is_seen_across_pages_and_portions():
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("H", [4, 1000, 1024, 1028, 2048, 4100, 8192])
+@pytest.mark.parametrize("centred,centred2,gated", [(True, True, 2), (False, True, 1), (True, False, 0), (False, False, 2)])
+def test_gated_norm_add_norm(dtype, H, centred, centred2, gated):
+    """Gate, norm, addition and the next norm in one kernel: one to eight pieces a thread, whole and ragged."""
+    from ember_b200 import ops
+    g = torch.Generator().manual_seed(H + gated)
+    y, z, h = (torch.randn(6, H, generator=g) for _ in range(3))
+    w, b, w2, b2, zb = (torch.randn(H, generator=g) for _ in range(5))
+    on = lambda t: t.cuda()                                                       # noqa: E731
+    res, out = on(h.clone()), torch.zeros(6, H, device="cuda", dtype=dtype)
+    ops.gated_norm_add_norm(on(y), on(z) if gated else None, on(zb) if gated == 2 else None, on(w), on(b) if centred else None, 1e-5, centred,
+                            res, on(w2), on(b2) if centred2 else None, 1e-6, centred2, out, 5)
+
+    def norm(t, weight, bias, eps, c):
+        t = t - t.mean(-1, keepdim=True) if c else t
+        return t * torch.rsqrt((t * t).mean(-1, keepdim=True) + eps) * weight.double() + (bias.double() if c else 0.0)
+
+    v = y.double() * (torch.sigmoid(z.double() + (zb.double() if gated == 2 else 0.0)) if gated else 1.0)
+    want = h.double() + norm(v, w, b, 1e-5, centred)
+    assert _rel(res[:5].cpu(), want[:5]) < 1e-6 and torch.equal(res[5].cpu(), h[5])
+    assert _rel(out[:5].cpu(), norm(want, w2, b2, 1e-6, centred2)[:5]) < (2.0 ** -8 if dtype == torch.bfloat16 else 2e-6)
+    assert float(out[5].float().abs().max()) == 0.0
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_layer_norm_gate_and_sandwich_kernels(dtype):
     """layer_norm, the fused gate + norm + add, and the per-group norm with both kinds of gate."""
     from ember_b200 import ops
