@@ -53,6 +53,9 @@ class CacheStorage:
         self.dtype = dtype
         self._paged: Dict[int, torch.Tensor] = {}
         self._state: Dict[int, torch.Tensor] = {}
+        # the views of each mixer's cache, made on first use: the tensors they look into live as long as this object, and
+        # cutting them anew for every layer of every step was a tenth of what a short prompt's step takes on the host
+        self._views: Dict[object, Optional[LayerCache]] = {}
         for g in manager.groups:
             if g.paged:
                 n = g.need
@@ -77,6 +80,11 @@ class CacheStorage:
 
     def layer(self, layer) -> Optional[LayerCache]:
         """The cache of one mixer, by cache id (a layer index, or (layer, sub-id)); None if it owns none."""
+        if layer not in self._views:
+            self._views[layer] = self._view(layer)
+        return self._views[layer]
+
+    def _view(self, layer) -> Optional[LayerCache]:
         gi = self.manager.layer_group.get(layer)
         if gi is None:
             return None

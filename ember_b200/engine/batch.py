@@ -259,6 +259,7 @@ class StepContext:
         self.ints = workspace.dynamic("step.ints", max(self._total, 1 << 16), torch.int32)
         self._ng = len(self._table_shapes)
         self._tiles = {}
+        self._tables = {}
         self.memo = {}                # what parts compute once per step and share between layers
         if upload:
             self.upload()
@@ -296,7 +297,10 @@ class StepContext:
         return v
 
     def block_table(self, group: int) -> torch.Tensor:
-        return self._view(7 + group, self._table_shapes[group])
+        t = self._tables.get(group)
+        if t is None:
+            t = self._tables[group] = self._view(7 + group, self._table_shapes[group])
+        return t
 
     def attention_tiles(self, tile_q: int, kind: str = "all"):
         """(device tensor [n, 4] or None, n) for tiles of up to ``tile_q`` queries over the runs of
