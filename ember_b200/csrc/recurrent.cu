@@ -889,9 +889,9 @@ __global__ void __launch_bounds__(32 * RG, CT == 1 ? 3 : 1) scan_chunks_kernel(S
 // every warp stopped between chunks to prepare the next one's tokens, and every token's output waited for its own
 // shuffles.  Here a thread keeps RS rows of C columns, so a read serves C columns and rows go in pairs through the packed
 // fp32 instructions; four warps do nothing but prepare (loads of the chunk after the next, norms, decays, gates of
-// the next); and the outputs of eight tokens are summed over the row groups together.  Every sum is formed in the order
-// of the kernel above.  Delta rule, 16 heads of 128 x 128: one run of 1,500 tokens 735 us there, 392 here; 24 runs of 60
-// 366 there, 256 here (with two computing warps a block, or eight preparing ones, the one run gets no faster).
+// the next); and the outputs of four tokens are summed over the row groups together.  Every sum is formed in the order
+// of the kernel above.  Delta rule, 16 heads of 128 x 128: one run of 1,500 tokens 735 us there, 397 here; 24 runs of 60
+// 366 there, 240 here (256 with the outputs of eight tokens together, which does not fit the registers; with two computing warps a block, or eight preparing ones, the one run gets no faster).
 constexpr int PORTION_WARPS = 4, PORTION_PREPARE = 4;      // computing and preparing warps of a block
 
 __device__ __forceinline__ unsigned long long pair_of(float lo, float hi) {
@@ -929,7 +929,7 @@ __global__ void __launch_bounds__(32 * (PORTION_WARPS + PORTION_PREPARE), 1) sca
     constexpr int VS = RG * (RS + 4);               // a vector in shared memory: row group r starts at r (RS + 4)
     constexpr int TOK = NV * VS + 4 + COLS;         // vectors, four scalars, the block's column values
     constexpr int TPW = CT / NP, EPL = RG * RS / 32;
-    static_assert(CT % NP == 0 && CT % 8 == 0, "whole tokens per preparing warp, whole batches of eight");
+    static_assert(CT % NP == 0 && CT % 4 == 0, "whole tokens per preparing warp, whole batches of four");
     const int s = blockIdx.x, h = blockIdx.y, col0 = blockIdx.z * COLS;
     const int D = p.D, V = p.V, H = p.H, grp = h / (H / p.G);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -1183,16 +1183,17 @@ __global__ void __launch_bounds__(32 * (PORTION_WARPS + PORTION_PREPARE), 1) sca
         PortionRegs<RS / 4, C> X[2];
         fetch(0, X[0]);
         int tt = 0;
-        for (; tt + 8 <= n; tt += 8) {
-            // eight tokens, whose outputs are summed over the row groups together: a lane gives away half of its
-            // tokens at each of the three exchanges and ends with the whole sums of token tt + r
-            float o[8][C], add[8][C], keep[C];
+        for (; tt + 4 <= n; tt += 4) {
+            // four tokens, whose outputs are summed over the row groups together: a lane gives away half of its tokens at
+            // each of two exchanges, adds the other half of the row groups at the third and ends with the whole sums
+            // of token tt + r % 4
+            float o[4][C], add[4][C], keep[C];
             float4 sc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 #pragma unroll
-            for (int u = 0; u < 8; u++) {
+            for (int u = 0; u < 4; u++) {
                 fetch(min(tt + u + 1, CT - 1), X[(u + 1) & 1]);
                 step(X[u & 1], o[u], add[u]);
-                if (r == u) {
+                if ((r & 3) == u) {
                     sc = X[u & 1].sc;
 #pragma unroll
                     for (int c = 0; c < C; c++) keep[c] = add[u][c];
@@ -1200,19 +1201,16 @@ __global__ void __launch_bounds__(32 * (PORTION_WARPS + PORTION_PREPARE), 1) sca
             }
 #pragma unroll
             for (int c = 0; c < C; c++) {
-                float a[4], b[2];
+                float a[2];
 #pragma unroll
-                for (int i = 0; i < 4; i++) {
+                for (int i = 0; i < 2; i++) {
                     const float mine = (r & 1) ? o[2 * i + 1][c] : o[2 * i][c], other = (r & 1) ? o[2 * i][c] : o[2 * i + 1][c];
                     a[i] = mine + __shfl_xor_sync(0xffffffffu, other, 1);
                 }
-#pragma unroll
-                for (int i = 0; i < 2; i++) {
-                    const float mine = (r & 2) ? a[2 * i + 1] : a[2 * i], other = (r & 2) ? a[2 * i] : a[2 * i + 1];
-                    b[i] = mine + __shfl_xor_sync(0xffffffffu, other, 2);
-                }
-                const float mine = (r & 4) ? b[1] : b[0], other = (r & 4) ? b[0] : b[1];
-                store(t0 + tt + r, j + c, finish(sc, mine + __shfl_xor_sync(0xffffffffu, other, 4), keep[c]));
+                const float mine = (r & 2) ? a[1] : a[0], other = (r & 2) ? a[0] : a[1];
+                float sum = mine + __shfl_xor_sync(0xffffffffu, other, 2);
+                sum += __shfl_xor_sync(0xffffffffu, sum, 4);
+                if ((r >> 2) == c) store(t0 + tt + (r & 3), j + c, finish(sc, sum, keep[c]));
             }
         }
         for (; tt < n; tt++) {                      // X[0] holds token tt
