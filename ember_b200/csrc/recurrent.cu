@@ -587,69 +587,23 @@ __global__ void ssm_scan_kernel(SsmArgs p) {
 }
 
 // ------------------------------------------------------------------ the same recurrences, state in registers
-// For up to 256 state rows a block takes 32 value columns: lane = row group r (RG = 8 or 16 of them) + RG x column,
-// and a thread keeps rows r RS .. r RS + RS - 1 of its column in registers.  A dot product over the rows
-// is RS multiply-adds and log2(RG) shuffles; the per-token vectors live in shared memory, one padding word per row
-// group so that the eight groups read eight banks.  The state goes through a shared tile when it is loaded and
-// stored, so that global memory sees whole 128-byte rows.  A prompt portion of one request keeps 8 times the threads
-// of the kernels above busy; those stay for more than 256 rows.
-constexpr int RCOLS = 32;
-
-// RG row groups (8 or 16 lanes of a warp share a column), RS rows a thread, 32 RG threads a block.  The state goes
-// through a shared tile: every thread first fetches RS values of whole 128-byte rows (all loads in flight together).
-template <int RS, int RG>
-__device__ __forceinline__ void regs_load(float (&st)[RS], float* tile, const float* __restrict__ S, int D, int V, int col0,
-                                          const float* __restrict__ extra = nullptr) {
-    const int c = threadIdx.x & 31, w = threadIdx.x >> 5;
-    float tmp[RS];
-#pragma unroll
-    for (int k = 0; k < RS; k++) {
-        const int i = w + RG * k;                      // (RG warps a block: rows w, w + RG, ...)
-        tmp[k] = (i < D && col0 + c < V) ? S[(size_t)i * V + col0 + c]
-                                         : ((extra && i < D && col0 + c == V) ? extra[i] : 0.0f);
-    }
-#pragma unroll
-    for (int k = 0; k < RS; k++) tile[(w + RG * k) * 33 + c] = tmp[k];
-    __syncthreads();
-    const int lane = threadIdx.x & 31, r = lane % RG, cc = w * (32 / RG) + lane / RG;
-#pragma unroll
-    for (int ii = 0; ii < RS; ii++) st[ii] = tile[(r * RS + ii) * 33 + cc];
-}
-template <int RS, int RG>
-__device__ __forceinline__ void regs_store(const float (&st)[RS], float* tile, float* __restrict__ S, int D, int V, int col0,
-                                           float* __restrict__ extra = nullptr) {
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, r = lane % RG, cc = w * (32 / RG) + lane / RG;
-    __syncthreads();
-#pragma unroll
-    for (int ii = 0; ii < RS; ii++) tile[(r * RS + ii) * 33 + cc] = st[ii];
-    __syncthreads();
-    const int c = lane;
-#pragma unroll
-    for (int k = 0; k < RS; k++) {
-        const int i = w + RG * k;
-        if (i < D) {
-            if (col0 + c < V) S[(size_t)i * V + col0 + c] = tile[i * 33 + c];
-            else if (extra && col0 + c == V) extra[i] = tile[i * 33 + c];
-        }
-    }
-}
-template <int RG>
+// For up to 256 state rows a thread keeps RS rows of C neighbouring value columns in registers: lane = row group r (RG = 8
+// of them, rows r RS .. r RS + RS - 1) + RG x column group, so a warp has 4 C columns.  A dot product over the rows is RS
+// multiply-adds and three shuffles; the per-token vectors live in shared memory, one padding word per row group so that
+// the eight groups read eight banks.  The kernels above stay for more than 256 rows.
+constexpr int RG = 8;
 __device__ __forceinline__ float rows_sum(float v) {
 #pragma unroll
     for (int off = 1; off < RG; off <<= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
     return v;
 }
 
-// One kernel for the five recurrences (MODE 0 delta rule, 1 matrix memory, 2 state space, 3 gated linear attention:
-// S <- diag(alpha) S + k v^T, o = S^T q with alpha = sigmoid(z + bias)^(1 / tau) per key channel and q times D^-1/2; 4 time
-// mixing: o = S^T r + (r . (u k)) v read before S <- diag(w) S + k v^T, w = exp(-exp(z + w0)); the bonus's dot product
-// r . (u k) is a warp sum made with the token's vectors).  A run is walked in chunks
-// of CT tokens: while a chunk is computed from shared memory (no block-wide barrier between its tokens), the next
-// chunk's inputs are already on their way into registers; each warp then prepares its tokens of that chunk (unit
-// norms, decays, gates: a token's vector is spread over the warp's lanes, so its sums are warp sums) and stores
-// them into the other buffer.  Per token a thread does RS multiply-adds per dot product and one round of three
-// shuffles: the delta rule's two dot products S^T k and S^T q are both taken of the decayed state (o = q . S_decayed
-// + (k . q) u), so they share the round and the rank-one update is off the critical path.
+// Two kernels -- prompt portions, and decode steps -- for the five recurrences (MODE 0 delta rule, 1 matrix memory, 2 state
+// space, 3 gated linear attention: S <- diag(alpha) S + k v^T, o = S^T q with alpha = sigmoid(z + bias)^(1 / tau) per key
+// channel and q times D^-1/2; 4 time mixing: o = S^T r + (r . (u k)) v read before S <- diag(w) S + k v^T, w = exp(-exp(z +
+// w0)); the bonus's dot product r . (u k) is a sum made with the token's vectors).  The delta rule's two dot products
+// S^T k and S^T q are both taken of the decayed state (o = q . S_decayed + (k . q) u), so that the rank-one update is off
+// the critical path.
 struct ScanArgs {
     float* state; long long state_stride; float* out; const int* query_start; const int* slots;
     int H, G, D, V;                        // D: rows of the state (key channels, or state size)
@@ -664,235 +618,6 @@ struct ScanArgs {
     const float* bonus;                    // time mixing: u [H D] (its w0 is dt_bias)
     int a_head;                            // delta: one decay logit (and bias) per head instead of per head and key channel
 };
-
-template <int N>
-struct TokenRegs {                                  // one token's vectors, scalars and column value, in registers
-    float4 v0[N], v1[N], v2[N], sc;
-    float val;
-};
-
-template <int MODE, int RS, int CT, int RG>
-__global__ void __launch_bounds__(32 * RG, CT == 1 ? 3 : 1) scan_chunks_kernel(ScanArgs p) {
-    constexpr int RTHREADS = 32 * RG, NW = RG;      // warps a block: 32 columns, 32 / RG of them a warp
-    extern __shared__ __align__(16) float smem[];
-    pdl_launch_dependents();
-    pdl_wait();
-    constexpr int NV = (MODE == 0 || MODE == 3 || MODE == 4) ? 3 : 2;
-    constexpr int VS = RG * (RS + 4);               // a vector in shared memory: row group r starts at r (RS + 4)
-    constexpr int TOK = NV * VS + 4 + RCOLS;        // vectors, four scalars, the block's 32 column values
-    constexpr int TPW = (CT + NW - 1) / NW, EPL = RG * RS / 32;   // (CT: 16 or 8 tokens a chunk for prompt portions, 1 for decode steps)
-    const int s = blockIdx.x, h = blockIdx.y, col0 = blockIdx.z * RCOLS;
-    const int D = p.D, V = p.V, H = p.H, grp = h / (H / p.G);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, r = lane % RG;
-    const int cw = warp * (32 / RG) + lane / RG, j = col0 + cw, base = r * (RS + 4);
-    const int n_cols = MODE == 1 ? V + 1 : V;       // (matrix memory: column V is n)
-    const bool live = j < n_cols;
-    float* tile = smem;                             // [RG RS][33], used when the state is loaded and stored
-    float* chunks = smem + RG * RS * 33;            // 2 x CT x TOK
-    float* sbase = p.state + (size_t)p.slots[s] * p.state_stride;
-    float* S = sbase + (size_t)h * D * V;
-    float* extra = MODE == 1 ? sbase + (size_t)H * D * V + (size_t)h * D : nullptr;
-    float st[RS];
-    for (int i = threadIdx.x; i < 2 * CT * TOK; i += RTHREADS) chunks[i] = 0.0f;
-    const int first = p.query_start[s], end = p.query_start[s + 1];
-    const float rate = (MODE == 1 || MODE == 3 || MODE == 4) ? 0.0f : expf(p.A_log[h]);
-    const float qscale = 1.0f / sqrtf((float)D);
-    // where this head's vectors start in a row of x
-    constexpr bool PROJ = MODE == 1 || MODE == 3 || MODE == 4;        // q (or r), k, v at given columns of one projection
-    const int off0 = MODE == 0 ? p.G * D + grp * D : (PROJ ? p.off_k + h * D : H * V + grp * D);               // k | k | B
-    const int off1 = MODE == 0 ? grp * D : (PROJ ? p.off_q + h * D : H * V + p.G * D + grp * D);               // q | q | C
-    const int off_col = MODE == 0 ? 2 * p.G * D + h * V : (PROJ ? p.off_v + h * V : h * V);                    // v | v | x
-
-    float f0[TPW][EPL], f1[TPW][EPL], f2[TPW][EPL], fc[TPW], fs[TPW];
-    auto prefetch = [&](int t0) {
-#pragma unroll
-        for (int w = 0; w < TPW; w++) {
-            const int t = t0 + warp + NW * w;
-            if (warp + NW * w >= CT || t >= end) continue;
-            const float* row = p.x + (size_t)t * p.ld_x;
-#pragma unroll
-            for (int m = 0; m < EPL; m++) {
-                const int i = lane + 32 * m;
-                if (i < D) {
-                    f0[w][m] = row[off0 + i];
-                    f1[w][m] = row[off1 + i];
-                    if (MODE == 0 || MODE == 3 || MODE == 4) f2[w][m] = p.a[(size_t)t * p.ld_a + ((MODE == 0 && p.a_head) ? h : h * D + i)];
-                }
-            }
-            const int c = col0 + lane;
-            fc[w] = c < V ? row[off_col + c] : 1.0f;
-            if (MODE == 0 || MODE == 2) fs[w] = p.b[(size_t)t * p.ld_b + h];
-        }
-    };
-    auto prepare = [&](int t0, float* buf) {
-#pragma unroll
-        for (int w = 0; w < TPW; w++) {
-            const int tt = warp + NW * w, t = t0 + tt;
-            if (tt >= CT || t >= end) continue;
-            float* tok = buf + tt * TOK;
-            float s0 = 0.0f, s1 = 0.0f, s01 = 0.0f;
-#pragma unroll
-            for (int m = 0; m < EPL; m++) {
-                const int i = lane + 32 * m;
-                if (i < D) {
-                    const int vi = i + (i / RS) * 4;
-                    tok[vi] = f0[w][m];
-                    tok[VS + vi] = (MODE == 1 || MODE == 3) ? f1[w][m] * qscale : f1[w][m];
-                    if (MODE == 3)      // alpha = sigmoid(z)^(1 / tau) = exp(logsigmoid(z) / tau)
-                        tok[2 * VS + vi] = expf(logsigmoidf_(f2[w][m] + (p.dt_bias ? p.dt_bias[h * D + i] : 0.0f)) * p.decay_power);
-                    if (MODE == 4) {
-                        tok[2 * VS + vi] = expf(-expf(f2[w][m] + p.dt_bias[h * D + i]));
-                        s0 = fmaf(f1[w][m] * p.bonus[h * D + i], f0[w][m], s0);          // r . (u k)
-                    }
-                    if (MODE == 0) {
-                        tok[2 * VS + vi] = expf(-rate * softplusf_(f2[w][m] + p.dt_bias[p.a_head ? h : h * D + i]));
-                        s0 = fmaf(f0[w][m], f0[w][m], s0); s1 = fmaf(f1[w][m], f1[w][m], s1); s01 = fmaf(f0[w][m], f1[w][m], s01);
-                    }
-                }
-            }
-            tok[NV * VS + 4 + lane] = fc[w];
-            if (MODE == 0) {
-                s0 = warp_sum(s0); s1 = warp_sum(s1); s01 = warp_sum(s01);
-                if (lane == 0) {
-                    tok[NV * VS + 0] = 1.0f / sqrtf(s0 + p.key_eps);            // 1 / |k|
-                    tok[NV * VS + 1] = qscale / sqrtf(s1 + p.key_eps);          // D^-1/2 / |q|
-                    tok[NV * VS + 2] = s01;                                     // k . q, before the norms
-                    tok[NV * VS + 3] = sigmoidf_(fs[w]);
-                }
-            } else if (MODE == 4) {
-                s0 = warp_sum(s0);
-                if (lane == 0) tok[NV * VS + 0] = s0;
-            } else if (MODE == 1) {
-                if (lane == 0) {
-                    const float* g = p.gates + ((size_t)t * H + h) * 4;
-                    tok[NV * VS + 0] = g[0]; tok[NV * VS + 1] = g[1];
-                }
-            } else if (MODE == 2 && lane == 0) {
-                const float dt = softplusf_(fs[w] + p.dt_bias[h]);
-                tok[NV * VS + 0] = expf(-rate * dt); tok[NV * VS + 1] = dt;
-            }
-        }
-    };
-
-    const float skip = MODE == 2 ? p.skip[h] : 0.0f;
-    prefetch(first);                                // (before the state: both trips to global memory overlap)
-    regs_load<RS, RG>(st, tile, S, D, V, col0, extra);
-    prepare(first, chunks);
-    __syncthreads();
-    int cur = 0;
-    for (int t0 = first; t0 < end; t0 += CT, cur ^= 1) {
-        const bool more = t0 + CT < end;
-        if (more) prefetch(t0 + CT);
-        const int n = min(CT, end - t0);
-        const float* buf = chunks + cur * CT * TOK;
-        // a token's operands are fetched into registers while the token before it is computed (two register sets,
-        // the loop unrolled by two), so that no multiply-add waits for shared memory
-        auto fetch = [&](int tt, TokenRegs<RS / 4>& x) {
-            const float* tok = buf + tt * TOK;
-            x.sc = *reinterpret_cast<const float4*>(tok + NV * VS);
-            x.val = tok[NV * VS + 4 + cw];
-#pragma unroll
-            for (int i4 = 0; i4 < RS / 4; i4++) {
-                x.v0[i4] = reinterpret_cast<const float4*>(tok + base)[i4];
-                x.v1[i4] = reinterpret_cast<const float4*>(tok + VS + base)[i4];
-                if (MODE == 0 || MODE == 3 || MODE == 4) x.v2[i4] = reinterpret_cast<const float4*>(tok + 2 * VS + base)[i4];
-            }
-        };
-        auto step = [&](int tt, const TokenRegs<RS / 4>& x) {
-            float o;
-            if (MODE == 0) {
-                float ak[4] = {0.0f, 0.0f, 0.0f, 0.0f}, aq[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-#pragma unroll
-                for (int i4 = 0; i4 < RS / 4; i4++) {
-                    const float4 k = x.v0[i4], q = x.v1[i4], g = x.v2[i4];
-                    st[4 * i4 + 0] *= g.x; st[4 * i4 + 1] *= g.y; st[4 * i4 + 2] *= g.z; st[4 * i4 + 3] *= g.w;
-                    ak[0] = fmaf(st[4 * i4 + 0], k.x, ak[0]); ak[1] = fmaf(st[4 * i4 + 1], k.y, ak[1]);
-                    ak[2] = fmaf(st[4 * i4 + 2], k.z, ak[2]); ak[3] = fmaf(st[4 * i4 + 3], k.w, ak[3]);
-                    aq[0] = fmaf(st[4 * i4 + 0], q.x, aq[0]); aq[1] = fmaf(st[4 * i4 + 1], q.y, aq[1]);
-                    aq[2] = fmaf(st[4 * i4 + 2], q.z, aq[2]); aq[3] = fmaf(st[4 * i4 + 3], q.w, aq[3]);
-                }
-                float sk = (ak[0] + ak[1]) + (ak[2] + ak[3]), sq = (aq[0] + aq[1]) + (aq[2] + aq[3]);
-#pragma unroll
-                for (int off = 1; off < RG; off <<= 1) {
-                    sk += __shfl_xor_sync(0xffffffffu, sk, off);
-                    sq += __shfl_xor_sync(0xffffffffu, sq, off);
-                }
-                const float uk = x.sc.w * (x.val - sk * x.sc.x) * x.sc.x;      // beta (v - S^T k) / |k|
-                o = x.sc.y * fmaf(uk, x.sc.z, sq);
-#pragma unroll
-                for (int i4 = 0; i4 < RS / 4; i4++) {
-                    const float4 k = x.v0[i4];
-                    st[4 * i4 + 0] = fmaf(k.x, uk, st[4 * i4 + 0]); st[4 * i4 + 1] = fmaf(k.y, uk, st[4 * i4 + 1]);
-                    st[4 * i4 + 2] = fmaf(k.z, uk, st[4 * i4 + 2]); st[4 * i4 + 3] = fmaf(k.w, uk, st[4 * i4 + 3]);
-                }
-            } else if (MODE == 4) {
-                float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-#pragma unroll
-                for (int i4 = 0; i4 < RS / 4; i4++) {
-                    const float4 k = x.v0[i4], q = x.v1[i4], g = x.v2[i4];
-                    acc[0] = fmaf(st[4 * i4 + 0], q.x, acc[0]); acc[1] = fmaf(st[4 * i4 + 1], q.y, acc[1]);
-                    acc[2] = fmaf(st[4 * i4 + 2], q.z, acc[2]); acc[3] = fmaf(st[4 * i4 + 3], q.w, acc[3]);
-                    st[4 * i4 + 0] = fmaf(k.x, x.val, g.x * st[4 * i4 + 0]); st[4 * i4 + 1] = fmaf(k.y, x.val, g.y * st[4 * i4 + 1]);
-                    st[4 * i4 + 2] = fmaf(k.z, x.val, g.z * st[4 * i4 + 2]); st[4 * i4 + 3] = fmaf(k.w, x.val, g.w * st[4 * i4 + 3]);
-                }
-                o = fmaf(x.sc.x, x.val, rows_sum<RG>((acc[0] + acc[1]) + (acc[2] + acc[3])));
-            } else if (MODE == 3) {
-                float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-#pragma unroll
-                for (int i4 = 0; i4 < RS / 4; i4++) {
-                    const float4 k = x.v0[i4], q = x.v1[i4], g = x.v2[i4];
-                    st[4 * i4 + 0] = fmaf(k.x, x.val, g.x * st[4 * i4 + 0]); st[4 * i4 + 1] = fmaf(k.y, x.val, g.y * st[4 * i4 + 1]);
-                    st[4 * i4 + 2] = fmaf(k.z, x.val, g.z * st[4 * i4 + 2]); st[4 * i4 + 3] = fmaf(k.w, x.val, g.w * st[4 * i4 + 3]);
-                    acc[0] = fmaf(st[4 * i4 + 0], q.x, acc[0]); acc[1] = fmaf(st[4 * i4 + 1], q.y, acc[1]);
-                    acc[2] = fmaf(st[4 * i4 + 2], q.z, acc[2]); acc[3] = fmaf(st[4 * i4 + 3], q.w, acc[3]);
-                }
-                o = rows_sum<RG>((acc[0] + acc[1]) + (acc[2] + acc[3]));
-            } else {
-                const float keep = x.sc.x, pv = x.sc.y * x.val;                 // put v | dt x
-                float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-#pragma unroll
-                for (int i4 = 0; i4 < RS / 4; i4++) {
-                    const float4 k = x.v0[i4], q = x.v1[i4];
-                    st[4 * i4 + 0] = fmaf(k.x, pv, keep * st[4 * i4 + 0]); st[4 * i4 + 1] = fmaf(k.y, pv, keep * st[4 * i4 + 1]);
-                    st[4 * i4 + 2] = fmaf(k.z, pv, keep * st[4 * i4 + 2]); st[4 * i4 + 3] = fmaf(k.w, pv, keep * st[4 * i4 + 3]);
-                    acc[0] = fmaf(st[4 * i4 + 0], q.x, acc[0]); acc[1] = fmaf(st[4 * i4 + 1], q.y, acc[1]);
-                    acc[2] = fmaf(st[4 * i4 + 2], q.z, acc[2]); acc[3] = fmaf(st[4 * i4 + 3], q.w, acc[3]);
-                }
-                o = rows_sum<RG>((acc[0] + acc[1]) + (acc[2] + acc[3]));
-                if (MODE == 2) o = fmaf(skip, x.val, o);
-            }
-            if (live && r == 0) {
-                const int t = t0 + tt;
-                if (j < V) __stcs(p.out + (size_t)t * H * V + h * V + j, o);
-                else p.gates[((size_t)t * H + h) * 4 + 3] = o;
-            }
-        };
-        TokenRegs<RS / 4> A, B;
-        fetch(0, A);
-        int tt = 0;
-        for (; tt + 1 < n; tt += 2) {
-            fetch(tt + 1, B);
-            step(tt, A);
-            if (tt + 2 < n) fetch(tt + 2, A);
-            step(tt + 1, B);
-        }
-        if (tt < n) step(tt, A);
-        if (more) prepare(t0 + CT, chunks + (cur ^ 1) * CT * TOK);
-        __syncthreads();
-    }
-    regs_store<RS, RG>(st, tile, S, D, V, col0, extra);
-}
-
-// ------------------------------------------------------------------ prompt portions: roles for the warps
-// A portion's tokens follow one another, so what counts is the time of one token.  Three things bounded it in the
-// kernel above: every four columns read all of a token's vectors from shared memory (half the time its bandwidth),
-// every warp stopped between chunks to prepare the next one's tokens, and every token's output waited for its own
-// shuffles.  Here a thread keeps RS rows of C columns, so a read serves C columns and rows go in pairs through the packed
-// fp32 instructions; four warps do nothing but prepare (loads of the chunk after the next, norms, decays, gates of
-// the next); and the outputs of four tokens are summed over the row groups together.  Every sum is formed in the order
-// of the kernel above.  Delta rule, 16 heads of 128 x 128: one run of 1,500 tokens 735 us there, 397 here; 24 runs of 60
-// 366 there, 240 here (256 with the outputs of eight tokens together, which does not fit the registers; with two computing warps a block, or eight preparing ones, the one run gets no faster).
-constexpr int PORTION_WARPS = 4, PORTION_PREPARE = 4;      // computing and preparing warps of a block
 
 __device__ __forceinline__ unsigned long long pair_of(float lo, float hi) {
     unsigned long long r;
@@ -913,15 +638,141 @@ __device__ __forceinline__ unsigned long long pair_fma(unsigned long long a, uns
 }
 
 template <int N, int C>
-struct PortionRegs {                                // one token's vectors (pairs of rows), scalars and C column values
+struct TokenRegs {                                  // one token's vectors (pairs of rows), scalars and C column values
     ulonglong2 v0[N], v1[N], v2[N];
     float4 sc;
     float val[C];
 };
 
+// Where a head's vectors start in a row of x: k | k | B, then q | q | C, then the columns v | v | x.
+template <int MODE>
+__device__ __forceinline__ void scan_offsets(const ScanArgs& p, int h, int grp, int& off0, int& off1, int& off_col) {
+    constexpr bool PROJ = MODE == 1 || MODE == 3 || MODE == 4;        // q (or r), k, v at given columns of one projection
+    const int D = p.D, V = p.V, H = p.H;
+    off0 = MODE == 0 ? p.G * D + grp * D : (PROJ ? p.off_k + h * D : H * V + grp * D);
+    off1 = MODE == 0 ? grp * D : (PROJ ? p.off_q + h * D : H * V + p.G * D + grp * D);
+    off_col = MODE == 0 ? 2 * p.G * D + h * V : (PROJ ? p.off_v + h * V : h * V);
+}
+// A row's decay from its logit (modes 0, 3, 4).
+template <int MODE>
+__device__ __forceinline__ float scan_decay(const ScanArgs& p, float z, float bias, float rate) {
+    if (MODE == 3) return expf(logsigmoidf_(z + bias) * p.decay_power);      // sigmoid(z)^(1 / tau) = exp(logsigmoid(z) / tau)
+    if (MODE == 4) return expf(-expf(z + bias));
+    return expf(-rate * softplusf_(z + bias));
+}
+// A token's scalars: from the sums over its rows (s0, s1, s01) and what is stored per token and head (fs, ft).
+template <int MODE>
+__device__ __forceinline__ float4 scan_scalars(const ScanArgs& p, float s0, float s1, float s01, float fs, float ft, float rate, float qscale,
+                                               float bias_h) {
+    float4 sc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (MODE == 0) {
+        sc.x = 1.0f / sqrtf(s0 + p.key_eps);            // 1 / |k|
+        sc.y = qscale / sqrtf(s1 + p.key_eps);          // D^-1/2 / |q|
+        sc.z = s01;                                     // k . q, before the norms
+        sc.w = sigmoidf_(fs);
+    } else if (MODE == 4) {
+        sc.x = s0;
+    } else if (MODE == 1) {
+        sc.x = fs; sc.y = ft;
+    } else if (MODE == 2) {
+        const float dt = softplusf_(fs + bias_h);
+        sc.x = expf(-rate * dt); sc.y = dt;
+    }
+    return sc;
+}
+// One token: the state moves on; o[c] is this thread's share of the output's dot product, add[c] what scan_finish wants
+// beside its sum over the eight row groups.
+template <int MODE, int RS, int C>
+__device__ __forceinline__ void scan_step(unsigned long long (&st)[C][RS / 2], const TokenRegs<RS / 4, C>& x, float (&o)[C], float (&add)[C]) {
+    constexpr int NV = (MODE == 0 || MODE == 3 || MODE == 4) ? 3 : 2;
+    (void)NV;
+                if (MODE == 0) {
+                    unsigned long long ak[C][2], aq[C][2];
+#pragma unroll
+                    for (int c = 0; c < C; c++) ak[c][0] = ak[c][1] = aq[c][0] = aq[c][1] = 0;
+#pragma unroll
+                    for (int i4 = 0; i4 < RS / 4; i4++)
+#pragma unroll
+                        for (int c = 0; c < C; c++) {
+                            st[c][2 * i4] = pair_mul(st[c][2 * i4], x.v2[i4].x);
+                            st[c][2 * i4 + 1] = pair_mul(st[c][2 * i4 + 1], x.v2[i4].y);
+                            ak[c][0] = pair_fma(st[c][2 * i4], x.v0[i4].x, ak[c][0]);
+                            ak[c][1] = pair_fma(st[c][2 * i4 + 1], x.v0[i4].y, ak[c][1]);
+                        }
+                    float sk[C];
+#pragma unroll
+                    for (int c = 0; c < C; c++) sk[c] = (pair_lo(ak[c][0]) + pair_hi(ak[c][0])) + (pair_lo(ak[c][1]) + pair_hi(ak[c][1]));
+#pragma unroll
+                    for (int off = 1; off < RG; off <<= 1)
+#pragma unroll
+                        for (int c = 0; c < C; c++) sk[c] += __shfl_xor_sync(0xffffffffu, sk[c], off);
+                    // (while the shuffles are under way)
+#pragma unroll
+                    for (int i4 = 0; i4 < RS / 4; i4++)
+#pragma unroll
+                        for (int c = 0; c < C; c++) {
+                            aq[c][0] = pair_fma(st[c][2 * i4], x.v1[i4].x, aq[c][0]);
+                            aq[c][1] = pair_fma(st[c][2 * i4 + 1], x.v1[i4].y, aq[c][1]);
+                        }
+#pragma unroll
+                    for (int c = 0; c < C; c++) {
+                        o[c] = (pair_lo(aq[c][0]) + pair_hi(aq[c][0])) + (pair_lo(aq[c][1]) + pair_hi(aq[c][1]));
+                        const float uk = x.sc.w * (x.val[c] - sk[c] * x.sc.x) * x.sc.x;      // beta (v - S^T k) / |k|
+                        add[c] = uk;
+                        const unsigned long long u2 = pair_of(uk, uk);
+#pragma unroll
+                        for (int i4 = 0; i4 < RS / 4; i4++) {
+                            st[c][2 * i4] = pair_fma(x.v0[i4].x, u2, st[c][2 * i4]);
+                            st[c][2 * i4 + 1] = pair_fma(x.v0[i4].y, u2, st[c][2 * i4 + 1]);
+                        }
+                    }
+                } else {
+                    // S <- keep S + k v^T with a decay per row (3, 4) or per token (1, 2), read before (4) or behind
+#pragma unroll
+                    for (int c = 0; c < C; c++) {
+                        const float put = (MODE == 1 || MODE == 2) ? x.sc.y * x.val[c] : x.val[c];              // put v | dt x
+                        const unsigned long long put2 = pair_of(put, put), keep2 = pair_of(x.sc.x, x.sc.x);
+                        unsigned long long a0 = 0, a1 = 0;
+#pragma unroll
+                        for (int i4 = 0; i4 < RS / 4; i4++) {
+                            const unsigned long long g0 = NV == 3 ? x.v2[i4].x : keep2, g1 = NV == 3 ? x.v2[i4].y : keep2;
+                            if (MODE == 4) {
+                                a0 = pair_fma(st[c][2 * i4], x.v1[i4].x, a0);
+                                a1 = pair_fma(st[c][2 * i4 + 1], x.v1[i4].y, a1);
+                            }
+                            st[c][2 * i4] = pair_fma(x.v0[i4].x, put2, pair_mul(g0, st[c][2 * i4]));
+                            st[c][2 * i4 + 1] = pair_fma(x.v0[i4].y, put2, pair_mul(g1, st[c][2 * i4 + 1]));
+                            if (MODE != 4) {
+                                a0 = pair_fma(st[c][2 * i4], x.v1[i4].x, a0);
+                                a1 = pair_fma(st[c][2 * i4 + 1], x.v1[i4].y, a1);
+                            }
+                        }
+                        o[c] = (pair_lo(a0) + pair_hi(a0)) + (pair_lo(a1) + pair_hi(a1));
+                        add[c] = x.val[c];
+                    }
+                }
+}
+template <int MODE>
+__device__ __forceinline__ float scan_finish(const float4& sc, float skip, float sum, float add) {
+    if (MODE == 0) return sc.y * fmaf(add, sc.z, sum);
+    if (MODE == 4) return fmaf(sc.x, add, sum);
+    if (MODE == 2) return fmaf(skip, add, sum);
+    return sum;
+}
+
+// ------------------------------------------------------------------ prompt portions: roles for the warps
+// A portion's tokens follow one another, so what counts is the time of one token.  Three things bounded it where
+// one column a thread and eight equal warps a block did it: every four columns read all of a token's vectors from shared
+// memory (half the time its bandwidth), every warp stopped between chunks to prepare the next one's tokens, and every
+// token's output waited for its own shuffles.  Here a thread keeps RS rows of C columns, so a read serves C columns and rows go in pairs through the packed
+// fp32 instructions; four warps do nothing but prepare (loads of the chunk after the next, norms, decays, gates of
+// the next); and the outputs of four tokens are summed over the row groups together.  Delta rule, 16 heads of 128 x 128: one run of 1,500 tokens 735 -> 397 us; 24 runs of
+// 60 366 -> 240 (256 with the outputs of eight tokens together, which does not fit the registers; with two computing warps a block, or eight preparing ones, the one run gets no faster).
+constexpr int PORTION_WARPS = 4, PORTION_PREPARE = 4;      // computing and preparing warps of a block
+
 template <int MODE, int RS, int CT, int C>
 __global__ void __launch_bounds__(32 * (PORTION_WARPS + PORTION_PREPARE), 1) scan_portion_kernel(ScanArgs p) {
-    constexpr int RG = 8, NCW = PORTION_WARPS, NP = PORTION_PREPARE, THREADS = 32 * (NCW + NP), COLS = 4 * C * NCW;
+    constexpr int NCW = PORTION_WARPS, NP = PORTION_PREPARE, THREADS = 32 * (NCW + NP), COLS = 4 * C * NCW;
     extern __shared__ __align__(16) float smem[];
     pdl_launch_dependents();
     pdl_wait();
@@ -943,11 +794,8 @@ __global__ void __launch_bounds__(32 * (PORTION_WARPS + PORTION_PREPARE), 1) sca
         const int pw = warp - NCW;
         const float rate = (MODE == 1 || MODE == 3 || MODE == 4) ? 0.0f : expf(p.A_log[h]);
         const float qscale = 1.0f / sqrtf((float)D);
-        // where this head's vectors start in a row of x
-        constexpr bool PROJ = MODE == 1 || MODE == 3 || MODE == 4;        // q (or r), k, v at given columns of one projection
-        const int off0 = MODE == 0 ? p.G * D + grp * D : (PROJ ? p.off_k + h * D : H * V + grp * D);               // k | k | B
-        const int off1 = MODE == 0 ? grp * D : (PROJ ? p.off_q + h * D : H * V + p.G * D + grp * D);               // q | q | C
-        const int off_col = MODE == 0 ? 2 * p.G * D + h * V : (PROJ ? p.off_v + h * V : h * V);                    // v | v | x
+        int off0, off1, off_col;
+        scan_offsets<MODE>(p, h, grp, off0, off1, off_col);
         int row_of[EPL];
         bool row_ok[EPL];
         float bias[EPL], bonus[EPL];
@@ -992,14 +840,9 @@ __global__ void __launch_bounds__(32 * (PORTION_WARPS + PORTION_PREPARE), 1) sca
                 for (int m = 0; m < EPL; m++) {
                     if (!row_ok[m]) f0[w][m] = f1[w][m] = 0.0f;
                     g[w][m] = 0.0f;
-                    if (MODE == 3)      // alpha = sigmoid(z)^(1 / tau) = exp(logsigmoid(z) / tau)
-                        g[w][m] = expf(logsigmoidf_(f2[w][m] + bias[m]) * p.decay_power);
-                    if (MODE == 4) {
-                        g[w][m] = expf(-expf(f2[w][m] + bias[m]));
-                        s0[w] = fmaf(f1[w][m] * bonus[m], f0[w][m], s0[w]);          // r . (u k)
-                    }
+                    if (NV == 3) g[w][m] = scan_decay<MODE>(p, f2[w][m], bias[m], rate);
+                    if (MODE == 4) s0[w] = fmaf(f1[w][m] * bonus[m], f0[w][m], s0[w]);          // r . (u k)
                     if (MODE == 0) {
-                        g[w][m] = expf(-rate * softplusf_(f2[w][m] + bias[m]));
                         s0[w] = fmaf(f0[w][m], f0[w][m], s0[w]);
                         s1[w] = fmaf(f1[w][m], f1[w][m], s1[w]);
                         s01[w] = fmaf(f0[w][m], f1[w][m], s01[w]);
@@ -1030,20 +873,7 @@ __global__ void __launch_bounds__(32 * (PORTION_WARPS + PORTION_PREPARE), 1) sca
                     if (NV == 3) tok[2 * VS + vi] = g[w][m];
                 }
                 if (lane < COLS) tok[NV * VS + 4 + lane] = fc[w];
-                float4 sc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                if (MODE == 0) {
-                    sc.x = 1.0f / sqrtf(s0[w] + p.key_eps);            // 1 / |k|
-                    sc.y = qscale / sqrtf(s1[w] + p.key_eps);          // D^-1/2 / |q|
-                    sc.z = s01[w];                                     // k . q, before the norms
-                    sc.w = sigmoidf_(fs[w]);
-                } else if (MODE == 4) {
-                    sc.x = s0[w];
-                } else if (MODE == 1) {
-                    sc.x = fs[w]; sc.y = ft[w];
-                } else if (MODE == 2) {
-                    const float dt = softplusf_(fs[w] + bias_h);
-                    sc.x = expf(-rate * dt); sc.y = dt;
-                }
+                const float4 sc = scan_scalars<MODE>(p, s0[w], s1[w], s01[w], fs[w], ft[w], rate, qscale, bias_h);
                 if (lane == 0) *reinterpret_cast<float4*>(tok + NV * VS) = sc;
             }
         };
@@ -1089,7 +919,7 @@ __global__ void __launch_bounds__(32 * (PORTION_WARPS + PORTION_PREPARE), 1) sca
         const float* buf = smem + cur * CT * TOK;
         // a token's operands are fetched into registers while the token before it is computed (two register sets),
         // so that no multiply-add waits for shared memory
-        auto fetch = [&](int tt, PortionRegs<RS / 4, C>& x) {
+        auto fetch = [&](int tt, TokenRegs<RS / 4, C>& x) {
             const float* tok = buf + tt * TOK;
             x.sc = *reinterpret_cast<const float4*>(tok + NV * VS);
 #pragma unroll
@@ -1101,86 +931,11 @@ __global__ void __launch_bounds__(32 * (PORTION_WARPS + PORTION_PREPARE), 1) sca
                 if (NV == 3) x.v2[i4] = reinterpret_cast<const ulonglong2*>(tok + 2 * VS + base)[i4];
             }
         };
-        // One token: the state moves on; o[c] is this thread's share of the output's dot product, add[c] what `finish`
-        // wants beside its sum over the eight row groups.
-        auto step = [&](const PortionRegs<RS / 4, C>& x, float (&o)[C], float (&add)[C]) {
-            if (MODE == 0) {
-                unsigned long long ak[C][2], aq[C][2];
-#pragma unroll
-                for (int c = 0; c < C; c++) ak[c][0] = ak[c][1] = aq[c][0] = aq[c][1] = 0;
-#pragma unroll
-                for (int i4 = 0; i4 < RS / 4; i4++)
-#pragma unroll
-                    for (int c = 0; c < C; c++) {
-                        st[c][2 * i4] = pair_mul(st[c][2 * i4], x.v2[i4].x);
-                        st[c][2 * i4 + 1] = pair_mul(st[c][2 * i4 + 1], x.v2[i4].y);
-                        ak[c][0] = pair_fma(st[c][2 * i4], x.v0[i4].x, ak[c][0]);
-                        ak[c][1] = pair_fma(st[c][2 * i4 + 1], x.v0[i4].y, ak[c][1]);
-                    }
-                float sk[C];
-#pragma unroll
-                for (int c = 0; c < C; c++) sk[c] = (pair_lo(ak[c][0]) + pair_hi(ak[c][0])) + (pair_lo(ak[c][1]) + pair_hi(ak[c][1]));
-#pragma unroll
-                for (int off = 1; off < RG; off <<= 1)
-#pragma unroll
-                    for (int c = 0; c < C; c++) sk[c] += __shfl_xor_sync(0xffffffffu, sk[c], off);
-                // (while the shuffles are under way)
-#pragma unroll
-                for (int i4 = 0; i4 < RS / 4; i4++)
-#pragma unroll
-                    for (int c = 0; c < C; c++) {
-                        aq[c][0] = pair_fma(st[c][2 * i4], x.v1[i4].x, aq[c][0]);
-                        aq[c][1] = pair_fma(st[c][2 * i4 + 1], x.v1[i4].y, aq[c][1]);
-                    }
-#pragma unroll
-                for (int c = 0; c < C; c++) {
-                    o[c] = (pair_lo(aq[c][0]) + pair_hi(aq[c][0])) + (pair_lo(aq[c][1]) + pair_hi(aq[c][1]));
-                    const float uk = x.sc.w * (x.val[c] - sk[c] * x.sc.x) * x.sc.x;      // beta (v - S^T k) / |k|
-                    add[c] = uk;
-                    const unsigned long long u2 = pair_of(uk, uk);
-#pragma unroll
-                    for (int i4 = 0; i4 < RS / 4; i4++) {
-                        st[c][2 * i4] = pair_fma(x.v0[i4].x, u2, st[c][2 * i4]);
-                        st[c][2 * i4 + 1] = pair_fma(x.v0[i4].y, u2, st[c][2 * i4 + 1]);
-                    }
-                }
-            } else {
-                // S <- keep S + k v^T with a decay per row (3, 4) or per token (1, 2), read before (4) or behind
-#pragma unroll
-                for (int c = 0; c < C; c++) {
-                    const float put = (MODE == 1 || MODE == 2) ? x.sc.y * x.val[c] : x.val[c];              // put v | dt x
-                    const unsigned long long put2 = pair_of(put, put), keep2 = pair_of(x.sc.x, x.sc.x);
-                    unsigned long long a0 = 0, a1 = 0;
-#pragma unroll
-                    for (int i4 = 0; i4 < RS / 4; i4++) {
-                        const unsigned long long g0 = NV == 3 ? x.v2[i4].x : keep2, g1 = NV == 3 ? x.v2[i4].y : keep2;
-                        if (MODE == 4) {
-                            a0 = pair_fma(st[c][2 * i4], x.v1[i4].x, a0);
-                            a1 = pair_fma(st[c][2 * i4 + 1], x.v1[i4].y, a1);
-                        }
-                        st[c][2 * i4] = pair_fma(x.v0[i4].x, put2, pair_mul(g0, st[c][2 * i4]));
-                        st[c][2 * i4 + 1] = pair_fma(x.v0[i4].y, put2, pair_mul(g1, st[c][2 * i4 + 1]));
-                        if (MODE != 4) {
-                            a0 = pair_fma(st[c][2 * i4], x.v1[i4].x, a0);
-                            a1 = pair_fma(st[c][2 * i4 + 1], x.v1[i4].y, a1);
-                        }
-                    }
-                    o[c] = (pair_lo(a0) + pair_hi(a0)) + (pair_lo(a1) + pair_hi(a1));
-                    add[c] = x.val[c];
-                }
-            }
-        };
-        auto finish = [&](const float4& sc, float sum, float add) {
-            if (MODE == 0) return sc.y * fmaf(add, sc.z, sum);
-            if (MODE == 4) return fmaf(sc.x, add, sum);
-            if (MODE == 2) return fmaf(skip, add, sum);
-            return sum;
-        };
         auto store = [&](int t, int col, float y) {
             if (col < V) __stcs(p.out + (size_t)t * H * V + h * V + col, y);
             else if (col < n_cols) p.gates[((size_t)t * H + h) * 4 + 3] = y;
         };
-        PortionRegs<RS / 4, C> X[2];
+        TokenRegs<RS / 4, C> X[2];
         fetch(0, X[0]);
         int tt = 0;
         for (; tt + 4 <= n; tt += 4) {
@@ -1192,7 +947,7 @@ __global__ void __launch_bounds__(32 * (PORTION_WARPS + PORTION_PREPARE), 1) sca
 #pragma unroll
             for (int u = 0; u < 4; u++) {
                 fetch(min(tt + u + 1, CT - 1), X[(u + 1) & 1]);
-                step(X[u & 1], o[u], add[u]);
+                scan_step<MODE, RS, C>(st, X[u & 1], o[u], add[u]);
                 if ((r & 3) == u) {
                     sc = X[u & 1].sc;
 #pragma unroll
@@ -1210,17 +965,17 @@ __global__ void __launch_bounds__(32 * (PORTION_WARPS + PORTION_PREPARE), 1) sca
                 const float mine = (r & 2) ? a[1] : a[0], other = (r & 2) ? a[0] : a[1];
                 float sum = mine + __shfl_xor_sync(0xffffffffu, other, 2);
                 sum += __shfl_xor_sync(0xffffffffu, sum, 4);
-                if ((r >> 2) == c) store(t0 + tt + (r & 3), j + c, finish(sc, sum, keep[c]));
+                if ((r >> 2) == c) store(t0 + tt + (r & 3), j + c, scan_finish<MODE>(sc, skip, sum, keep[c]));
             }
         }
         for (; tt < n; tt++) {                      // X[0] holds token tt
             float o[C], add[C];
             fetch(min(tt + 1, CT - 1), X[1]);
-            step(X[0], o, add);
+            scan_step<MODE, RS, C>(st, X[0], o, add);
 #pragma unroll
             for (int c = 0; c < C; c++) {
-                const float sum = rows_sum<RG>(o[c]);
-                if (r == c) store(t0 + tt, j + c, finish(X[0].sc, sum, add[c]));
+                const float sum = rows_sum(o[c]);
+                if (r == c) store(t0 + tt, j + c, scan_finish<MODE>(X[0].sc, skip, sum, add[c]));
             }
             X[0] = X[1];
         }
@@ -1237,6 +992,144 @@ __global__ void __launch_bounds__(32 * (PORTION_WARPS + PORTION_PREPARE), 1) sca
         }
 }
 
+// ------------------------------------------------------------------ decode steps
+// One token a run.  A thread asks for its rows of the state first (C neighbouring columns, so that a warp's request is
+// whole 32-byte pieces of eight rows); while they travel the block prepares the token's vectors, an element a thread;
+// then the step, and the columns go back.  The state passes through no shared memory.  24 runs, 16 heads of 128 x 128,
+// delta rule (50 MB in and out): blocks of 256 threads that passed the state through shared memory, one warp of which
+// prepared the token, took 29 us a step, these 20.
+constexpr int SINGLE_WARPS = 4;
+
+template <int MODE, int RS, int C>
+__global__ void __launch_bounds__(32 * SINGLE_WARPS, RS <= 16 ? 4 : 2) scan_single_kernel(ScanArgs p) {
+    constexpr int NV = (MODE == 0 || MODE == 3 || MODE == 4) ? 3 : 2, VS = RG * (RS + 4), THREADS = 32 * SINGLE_WARPS;
+    constexpr int EPT = (RG * RS + THREADS - 1) / THREADS;          // elements of a vector a thread prepares
+    __shared__ __align__(16) float tok[NV * VS];
+    __shared__ float sums[3][SINGLE_WARPS];
+    pdl_launch_dependents();
+    const int s = blockIdx.x, h = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int D = p.D, V = p.V, H = p.H, grp = h / (H / p.G);
+    const int n_cols = MODE == 1 ? V + 1 : V;       // (matrix memory: column V is n)
+    const int r = lane % RG, j = ((int)blockIdx.z * SINGLE_WARPS + warp) * 4 * C + (lane / RG) * C, base = r * (RS + 4);
+    const float rate = (MODE == 1 || MODE == 3 || MODE == 4) ? 0.0f : expf(p.A_log[h]);
+    const float qscale = 1.0f / sqrtf((float)D), skip = MODE == 2 ? p.skip[h] : 0.0f, bias_h = MODE == 2 ? p.dt_bias[h] : 0.0f;
+    int off0, off1, off_col;
+    scan_offsets<MODE>(p, h, grp, off0, off1, off_col);
+    float bias[EPT], bonus[EPT];
+#pragma unroll
+    for (int m = 0; m < EPT; m++) {
+        const int i = min((int)threadIdx.x + THREADS * m, D - 1);
+        bias[m] = 0.0f; bonus[m] = 0.0f;
+        if (MODE == 0) bias[m] = p.dt_bias[p.a_head ? h : h * D + i];
+        if (MODE == 4 || (MODE == 3 && p.dt_bias)) bias[m] = p.dt_bias[h * D + i];
+        if (MODE == 4) bonus[m] = p.bonus[h * D + i];
+    }
+    pdl_wait();
+    const int first = p.query_start[s], end = p.query_start[s + 1];
+    if (first >= end) return;
+    float* sbase = p.state + (size_t)p.slots[s] * p.state_stride;
+    float* S = sbase + (size_t)h * D * V;
+    float* extra = MODE == 1 ? sbase + (size_t)H * D * V + (size_t)h * D : nullptr;
+    // two columns as one 8-byte piece where rows and addresses allow it
+    const bool whole = C == 2 && j + 1 < V && (V & 1) == 0 && (reinterpret_cast<uintptr_t>(S) & 7) == 0;
+    auto place = [&](int i, int c) -> float* {      // row i of column c of this thread, null if there is none
+        if (i >= D || j + c >= n_cols) return nullptr;
+        return MODE == 1 && j + c == V ? extra + i : S + (size_t)i * V + j + c;
+    };
+    unsigned long long st[C][RS / 2];
+    {
+        float v[RS][C];
+        if (whole) {
+            const float* from = S + (size_t)(r * RS) * V + j;
+#pragma unroll
+            for (int ii = 0; ii < RS; ii++) {
+                const float2 f = r * RS + ii < D ? *reinterpret_cast<const float2*>(from + (size_t)ii * V) : make_float2(0.0f, 0.0f);
+                v[ii][0] = f.x; v[ii][C - 1] = f.y;
+            }
+        } else {
+#pragma unroll
+            for (int ii = 0; ii < RS; ii++)
+#pragma unroll
+                for (int c = 0; c < C; c++) {
+                    const float* q = place(r * RS + ii, c);
+                    v[ii][c] = q ? *q : 0.0f;
+                }
+        }
+#pragma unroll
+        for (int ii = 0; ii < RS; ii += 2)
+#pragma unroll
+            for (int c = 0; c < C; c++) st[c][ii / 2] = pair_of(v[ii][c], v[ii + 1][c]);
+    }
+    for (int t = first; t < end; t++) {
+        const float* row = p.x + (size_t)t * p.ld_x;
+        float fs = 0.0f, ft = 0.0f, s0 = 0.0f, s1 = 0.0f, s01 = 0.0f;
+        TokenRegs<RS / 4, C> x;
+#pragma unroll
+        for (int c = 0; c < C; c++) x.val[c] = j + c < V ? row[off_col + j + c] : 1.0f;
+        if (MODE == 0 || MODE == 2) fs = p.b[(size_t)t * p.ld_b + h];
+        if (MODE == 1) { const float* g = p.gates + ((size_t)t * H + h) * 4; fs = g[0]; ft = g[1]; }
+        if (t > first) __syncthreads();             // the token before has been read
+#pragma unroll
+        for (int m = 0; m < EPT; m++) {
+            const int i = (int)threadIdx.x + THREADS * m, vi = i + (i / RS) * 4;
+            if (i >= RG * RS) break;
+            const bool ok = i < D;
+            const float f0 = ok ? row[off0 + i] : 0.0f, f1 = ok ? row[off1 + i] : 0.0f;
+            tok[vi] = f0;
+            tok[VS + vi] = (MODE == 1 || MODE == 3) ? f1 * qscale : f1;
+            if (NV == 3) {
+                const float z = ok ? p.a[(size_t)t * p.ld_a + ((MODE == 0 && p.a_head) ? h : h * D + i)] : 0.0f;
+                tok[2 * VS + vi] = ok ? scan_decay<MODE>(p, z, bias[m], rate) : 0.0f;
+            }
+            if (MODE == 4) s0 = fmaf(f1 * bonus[m], f0, s0);
+            if (MODE == 0) { s0 = fmaf(f0, f0, s0); s1 = fmaf(f1, f1, s1); s01 = fmaf(f0, f1, s01); }
+        }
+        if (MODE == 0 || MODE == 4) {
+            s0 = warp_sum(s0);
+            if (MODE == 0) { s1 = warp_sum(s1); s01 = warp_sum(s01); }
+            if (lane == 0) { sums[0][warp] = s0; sums[1][warp] = s1; sums[2][warp] = s01; }
+        }
+        __syncthreads();
+        if (MODE == 0 || MODE == 4) {
+            s0 = s1 = s01 = 0.0f;
+#pragma unroll
+            for (int w = 0; w < SINGLE_WARPS; w++) { s0 += sums[0][w]; s1 += sums[1][w]; s01 += sums[2][w]; }
+        }
+        x.sc = scan_scalars<MODE>(p, s0, s1, s01, fs, ft, rate, qscale, bias_h);
+#pragma unroll
+        for (int i4 = 0; i4 < RS / 4; i4++) {
+            x.v0[i4] = reinterpret_cast<const ulonglong2*>(tok + base)[i4];
+            x.v1[i4] = reinterpret_cast<const ulonglong2*>(tok + VS + base)[i4];
+            if (NV == 3) x.v2[i4] = reinterpret_cast<const ulonglong2*>(tok + 2 * VS + base)[i4];
+        }
+        float o[C], add[C];
+        scan_step<MODE, RS, C>(st, x, o, add);
+#pragma unroll
+        for (int c = 0; c < C; c++) {
+            const float y = scan_finish<MODE>(x.sc, skip, rows_sum(o[c]), add[c]);
+            if (r == c && j + c < n_cols) {
+                if (j + c < V) __stcs(p.out + (size_t)t * H * V + h * V + j + c, y);
+                else p.gates[((size_t)t * H + h) * 4 + 3] = y;
+            }
+        }
+    }
+    if (whole) {
+        float* to = S + (size_t)(r * RS) * V + j;
+#pragma unroll
+        for (int ii = 0; ii < RS; ii++) {
+            const unsigned long long a = st[0][ii / 2], b = st[C - 1][ii / 2];
+            if (r * RS + ii < D)
+                *reinterpret_cast<float2*>(to + (size_t)ii * V) = (ii & 1) ? make_float2(pair_hi(a), pair_hi(b)) : make_float2(pair_lo(a), pair_lo(b));
+        }
+    } else {
+#pragma unroll
+        for (int ii = 0; ii < RS; ii++)
+#pragma unroll
+            for (int c = 0; c < C; c++)
+                if (float* q = place(r * RS + ii, c)) *q = (ii & 1) ? pair_hi(st[c][ii / 2]) : pair_lo(st[c][ii / 2]);
+    }
+}
+
 inline int rows_per_thread(int D) { return D <= 32 ? 4 : (D <= 64 ? 8 : (D <= 128 ? 16 : (D <= 256 ? 32 : 0))); }
 inline bool regs_kernels_on() {
     static int on = -1;
@@ -1244,15 +1137,10 @@ inline bool regs_kernels_on() {
     return on != 0;
 }
 
-template <int MODE, int RS, int CT, int RG>
-inline int launch_scan_ct(const ScanArgs& p, int S, int n_cols, cudaStream_t st) {
-    constexpr int NV = (MODE == 0 || MODE == 3 || MODE == 4) ? 3 : 2;
-    const size_t smem = ((size_t)RG * RS * 33 + 2 * CT * (NV * RG * (RS + 4) + 4 + RCOLS)) * sizeof(float);
-    if (smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(scan_chunks_kernel<MODE, RS, CT, RG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return fail("scan: %s", cudaGetErrorString(e));
-    }
-    launch_kernel(scan_chunks_kernel<MODE, RS, CT, RG>, dim3(S, p.H, (n_cols + RCOLS - 1) / RCOLS), 32 * RG, smem, st, p);
+template <int MODE, int RS, int C>
+inline int launch_single(const ScanArgs& p, int S, int n_cols, cudaStream_t st) {
+    constexpr int COLS = 4 * C * SINGLE_WARPS;
+    launch_kernel(scan_single_kernel<MODE, RS, C>, dim3(S, p.H, (n_cols + COLS - 1) / COLS), 32 * SINGLE_WARPS, 0, st, p);
     return 0;
 }
 template <int MODE, int RS, int CT, int C>
@@ -1267,15 +1155,14 @@ inline int launch_portion(const ScanArgs& p, int S, int n_cols, cudaStream_t st)
                   smem, st, p);
     return 0;
 }
-// `single`: as many runs as tokens (a decode step): chunks of one token, small blocks, several per SM (the step is
-// bound by the state's bytes).  Anything else goes to the kernel with roles.
+// `single`: as many runs as tokens (a decode step).  Anything else goes to the kernel with roles.
 template <int MODE>
 inline int launch_scan(const ScanArgs& p, int S, int n_cols, bool single, cudaStream_t st) {
     switch (rows_per_thread(p.D)) {
-        case 4: return single ? launch_scan_ct<MODE, 4, 1, 8>(p, S, n_cols, st) : launch_portion<MODE, 4, 16, 2>(p, S, n_cols, st);
-        case 8: return single ? launch_scan_ct<MODE, 8, 1, 8>(p, S, n_cols, st) : launch_portion<MODE, 8, 16, 2>(p, S, n_cols, st);
-        case 16: return single ? launch_scan_ct<MODE, 16, 1, 8>(p, S, n_cols, st) : launch_portion<MODE, 16, 16, 2>(p, S, n_cols, st);
-        default: return single ? launch_scan_ct<MODE, 32, 1, 8>(p, S, n_cols, st) : launch_portion<MODE, 32, 8, 1>(p, S, n_cols, st);
+        case 4: return single ? launch_single<MODE, 4, 2>(p, S, n_cols, st) : launch_portion<MODE, 4, 16, 2>(p, S, n_cols, st);
+        case 8: return single ? launch_single<MODE, 8, 2>(p, S, n_cols, st) : launch_portion<MODE, 8, 16, 2>(p, S, n_cols, st);
+        case 16: return single ? launch_single<MODE, 16, 2>(p, S, n_cols, st) : launch_portion<MODE, 16, 16, 2>(p, S, n_cols, st);
+        default: return single ? launch_single<MODE, 32, 1>(p, S, n_cols, st) : launch_portion<MODE, 32, 8, 1>(p, S, n_cols, st);
     }
 }
 
