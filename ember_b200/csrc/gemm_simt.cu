@@ -158,8 +158,9 @@ __device__ __forceinline__ void finish_pair(float c0, float c1, const float* __r
 // elements of k (a whole 128-byte line of each row), so nothing but the final addition of the parts needs a block
 // barrier and 3 x 4.5 KB a warp are on their way.  Weights that no earlier kernel writes are asked for before the
 // wait for the kernel before.  Rows of 36 floats keep the 16-byte reads of a quarter warp in different banks.
-// Four tokens at the 0.6B widths (hidden 1,024), in a step: o and down 9.1 and 13.8 us, gate/up 4.7, the head's 622 MB 99 us
-// (6.3 TB/s); with the 64 x 64 tiles of the general kernel a whole such step took about 15 ms, now 2.3 ms.
+// Four tokens at the 0.6B widths (hidden 1,024), in a step: o and down 9.0 and 13.8 us, q/k/v and gate/up 5, the head's
+// 622 MB 100 us (6.2 TB/s); with the general kernel everywhere four requests of 75 tokens and four more steps took 143 ms,
+// with this one and the next 23.
 constexpr int FEW_K = 32, FEW_STAGES = 3, FEW_ROW = FEW_K + 4;
 
 template <int MT, int NB>
