@@ -162,6 +162,59 @@ def test_gemm_f32_kernels_share_one_order(N, K, epilogue):
         assert torch.equal(out[:M], first[:M]), M
 
 
+SILU_PROBE = """
+#include "gemm_tc_kernel.cuh"
+#include <cstdio>
+__global__ void compare(unsigned long long* differ) {
+    const unsigned long long stride = (unsigned long long)gridDim.x * blockDim.x;
+    for (unsigned long long i = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; i < (1ull << 32); i += stride) {
+        const float g = __uint_as_float((unsigned)i), want = g / (1.0f + __expf(-g)), got = ember::silu_quotient(g);
+        if (__float_as_uint(got) != __float_as_uint(want) && (got == got || want == want)) atomicAdd(differ, 1ull);
+    }
+}
+int main() {
+    unsigned long long *d, n = 1;
+    if (cudaMalloc(&d, 8) || cudaMemset(d, 0, 8)) return 2;
+    compare<<<1184, 256>>>(d);
+    if (cudaMemcpy(&n, d, 8, cudaMemcpyDeviceToHost)) return 2;
+    std::printf("%llu\\n", n);
+    return 0;
+}
+"""
+
+
+def test_gate_quotient_is_the_division_for_every_float(tmp_path):
+    """All 2^32 gates: the epilogue's quotient has the bits of the division operator."""
+    import subprocess
+
+    from ember_b200.csrc import build
+    src, exe = tmp_path / "silu.cu", tmp_path / "silu"
+    src.write_text(SILU_PROBE)
+    subprocess.run([build.find_nvcc(), *build.ARCH_FLAGS, "-O3", "-std=c++17", "-I", build._HERE, "-o", str(exe), str(src)], check=True)
+    done = subprocess.run([str(exe)], capture_output=True, text=True, timeout=60)
+    assert done.returncode == 0 and int(done.stdout) == 0, done.stdout
+
+
+@pytest.mark.parametrize("M", [4, 40, 200])
+def test_gated_product_of_far_gates(M):
+    """Gates from -95 to 95, the exponential's overflow near -88.7 among them: every quotient above fp32's smallest normal
+    number is there, with the exponential's error (3 + 1.2 |g| units) and one rounding to bfloat16."""
+    from ember_b200 import ops
+    gates = torch.linspace(-95.0, 95.0, 764).bfloat16()
+    w = torch.zeros(2 * 764, 64)
+    w[0::2, 0] = gates.float()                       # row 2i: gate i, row 2i + 1: up = 1
+    w[1::2, 1] = 1.0
+    a = torch.zeros(M, 64)
+    a[:, :2] = 1.0
+    out = torch.full((M, 764), float("nan"), device="cuda", dtype=torch.bfloat16)
+    ops.gemm_tc(a.bfloat16().cuda(), w.bfloat16().cuda(), out, M, ops.EPI_SILU_MUL)
+    g = gates.double()
+    want = g / (1.0 + torch.exp(-g))
+    want = torch.where(g < -88.72, torch.zeros_like(g), want)                       # exp(-g) is infinite in fp32
+    got = out.cpu().double()
+    assert bool(((got - want).abs() <= want.abs() * (2.0 ** -8 + 120 * 2.0 ** -23)).all())
+
+
 @pytest.mark.parametrize("H", [64, 96, 1000, 2048, 5120])
 @pytest.mark.parametrize("odt", [torch.float32, torch.bfloat16])
 def test_rmsnorm(H, odt):
