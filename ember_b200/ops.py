@@ -1189,7 +1189,7 @@ def sigmoid_attention(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tenso
     lib = _lib("sigmoid_attention")
     _call(lib, lib.ember_sigmoid_attention, _p(q), _p(k_pool), _p(v_pool), _p(out), c_int(dtype_code(q.dtype)), c_int(heads),
           c_int(kv_heads), c_int(dim), c_int(vdim), _p(tiles), c_int(n_tiles), _p(block_table), c_int(block_table.shape[-1]),
-          c_int(page), c_int(k_pool.shape[0]), c_float(scale), _p(head_bias), _p(err), _stream(stream))
+          c_int(page), c_int(k_pool.shape[0]), c_float(scale), _p(head_bias), c_int(_sms(q.device)), _p(err), _stream(stream))
 
 
 def gla_scan(proj: torch.Tensor, off_q: int, off_k: int, off_v: int, z: torch.Tensor, z_col: int, z_bias: Optional[torch.Tensor],

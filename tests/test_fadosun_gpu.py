@@ -264,6 +264,33 @@ def test_sigmoid_attention_key_parts(heads, kv, dim, vdim, lens):
         assert _rel(out[r].cpu(), want) < 2.0 ** -8                    # (one rounding of the result to bfloat16)
 
 
+@pytest.mark.parametrize("heads,kv,dim,vdim,page", [(4, 2, 128, 128, 64), (6, 2, 32, 32, 16), (8, 1, 144, 160, 32), (4, 2, 256, 512, 16),
+                                                    (16, 1, 64, 224, 128), (4, 2, 128, 128, 24)])
+def test_sigmoid_attention_does_not_depend_on_the_step(heads, kv, dim, vdim, page):
+    """A decoded token alone (its key range shared out over a cluster), beside one other and among forty: the same bits."""
+    from ember_b200 import ops
+    torch.manual_seed(dim + vdim)
+    lens = [1, 15, 16, 17, 63, 64, 65, 128, 129, 511, 512, 513, 640, 1025, 1500, 2049] + [33] * 24
+    n, width = len(lens), (max(lens) + page - 1) // page
+    kp = torch.randn(n * width, kv, page, dim, device="cuda").bfloat16()
+    vp = torch.randn(n * width, kv, page, vdim, device="cuda").bfloat16()
+    table = torch.randperm(n * width).view(n, width).to(torch.int32).cuda()
+    q, bias = torch.randn(n, heads * dim, device="cuda").bfloat16(), torch.randn(heads, device="cuda") - 2.0
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+
+    def run(rows):
+        out = torch.zeros(n, heads * vdim, dtype=torch.bfloat16, device="cuda")
+        tiles = torch.tensor([[r, r, 1, lens[r] - 1] for r in rows], dtype=torch.int32, device="cuda")
+        ops.sigmoid_attention(q, kp, vp, out, heads, kv, dim, vdim, tiles, len(rows), table, page, 0.1, bias, err=err)
+        return out
+
+    among = run(list(range(n)) * 4)                 # (so many blocks that none is cut, whatever the heads)
+    for rows in [[r] for r in range(16)] + [[14, 9], [15, 13, 12], list(range(12))]:
+        out = run(rows)
+        assert torch.equal(out[rows], among[rows]), rows
+    assert int(err.item()) == 0
+
+
 def test_a_far_key_that_dominates_is_seen_across_pages_and_portions():
     """Head biases so low that ordinary keys weigh nothing, one early key and two late queries scaled so that their
     scores stand out: the read-out at those queries is that one key's value, in a prompt portion and decoded alone."""
