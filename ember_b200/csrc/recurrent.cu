@@ -6,9 +6,11 @@
 // their logarithms, softplus and exponentials, gates, unit norms, the state itself.
 //
 // A step's tokens are S runs (query_start [S + 1]); run s belongs to state slot slots[s].  A recurrence kernel runs
-// one block per (run, head, tile of value columns): the block holds its [keys x columns] tile of the state in shared
-// memory, walks the run's tokens in order and writes the tile back, so a prompt portion and a single decoded token
-// are the same code and the state after a step does not depend on how the tokens were cut into steps.
+// one block per (run, head, tile of value columns): the block holds its [keys x columns] tile of the state (in registers
+// up to 256 keys, else in shared memory), walks the run's tokens in order and writes the tile back.  The kernel of prompt
+// portions and that of decoded tokens add everything in the same order, so outputs and state do not depend, to the
+// bit, on how the tokens were cut into steps (but for the matrix memory's gates, whose running sums are made 32 tokens at a
+// time: there the last bits do).
 #include "common.cuh"
 
 EMBER_DEFINE_LAST_ERROR
@@ -1004,8 +1006,8 @@ template <int MODE, int RS, int C>
 __global__ void __launch_bounds__(32 * SINGLE_WARPS, RS <= 16 ? 4 : 2) scan_single_kernel(ScanArgs p) {
     constexpr int NV = (MODE == 0 || MODE == 3 || MODE == 4) ? 3 : 2, VS = RG * (RS + 4), THREADS = 32 * SINGLE_WARPS;
     constexpr int EPT = (RG * RS + THREADS - 1) / THREADS;          // elements of a vector a thread prepares
+    constexpr int EPL = RG * RS / 32;                               // and of one that a lane of every warp sums
     __shared__ __align__(16) float tok[NV * VS];
-    __shared__ float sums[3][SINGLE_WARPS];
     pdl_launch_dependents();
     const int s = blockIdx.x, h = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int D = p.D, V = p.V, H = p.H, grp = h / (H / p.G);
@@ -1015,15 +1017,16 @@ __global__ void __launch_bounds__(32 * SINGLE_WARPS, RS <= 16 ? 4 : 2) scan_sing
     const float qscale = 1.0f / sqrtf((float)D), skip = MODE == 2 ? p.skip[h] : 0.0f, bias_h = MODE == 2 ? p.dt_bias[h] : 0.0f;
     int off0, off1, off_col;
     scan_offsets<MODE>(p, h, grp, off0, off1, off_col);
-    float bias[EPT], bonus[EPT];
+    float bias[EPT], bonus[EPL];
 #pragma unroll
     for (int m = 0; m < EPT; m++) {
         const int i = min((int)threadIdx.x + THREADS * m, D - 1);
-        bias[m] = 0.0f; bonus[m] = 0.0f;
+        bias[m] = 0.0f;
         if (MODE == 0) bias[m] = p.dt_bias[p.a_head ? h : h * D + i];
         if (MODE == 4 || (MODE == 3 && p.dt_bias)) bias[m] = p.dt_bias[h * D + i];
-        if (MODE == 4) bonus[m] = p.bonus[h * D + i];
     }
+#pragma unroll
+    for (int m = 0; m < EPL; m++) bonus[m] = MODE == 4 ? p.bonus[h * D + min(lane + 32 * m, D - 1)] : 0.0f;
     pdl_wait();
     const int first = p.query_start[s], end = p.query_start[s + 1];
     if (first >= end) return;
@@ -1081,19 +1084,19 @@ __global__ void __launch_bounds__(32 * SINGLE_WARPS, RS <= 16 ? 4 : 2) scan_sing
                 const float z = ok ? p.a[(size_t)t * p.ld_a + ((MODE == 0 && p.a_head) ? h : h * D + i)] : 0.0f;
                 tok[2 * VS + vi] = ok ? scan_decay<MODE>(p, z, bias[m], rate) : 0.0f;
             }
-            if (MODE == 4) s0 = fmaf(f1 * bonus[m], f0, s0);
-            if (MODE == 0) { s0 = fmaf(f0, f0, s0); s1 = fmaf(f1, f1, s1); s01 = fmaf(f0, f1, s01); }
-        }
-        if (MODE == 0 || MODE == 4) {
-            s0 = warp_sum(s0);
-            if (MODE == 0) { s1 = warp_sum(s1); s01 = warp_sum(s01); }
-            if (lane == 0) { sums[0][warp] = s0; sums[1][warp] = s1; sums[2][warp] = s01; }
         }
         __syncthreads();
         if (MODE == 0 || MODE == 4) {
-            s0 = s1 = s01 = 0.0f;
+            // every warp for itself, in the order of the preparing warps above: a token's bits are the same in both kernels
 #pragma unroll
-            for (int w = 0; w < SINGLE_WARPS; w++) { s0 += sums[0][w]; s1 += sums[1][w]; s01 += sums[2][w]; }
+            for (int m = 0; m < EPL; m++) {
+                const int i = lane + 32 * m, vi = i + (i / RS) * 4;
+                const float f0 = tok[vi], f1 = tok[VS + vi];
+                if (MODE == 4) s0 = fmaf(f1 * bonus[m], f0, s0);
+                else { s0 = fmaf(f0, f0, s0); s1 = fmaf(f1, f1, s1); s01 = fmaf(f0, f1, s01); }
+            }
+            s0 = warp_sum(s0);
+            if (MODE == 0) { s1 = warp_sum(s1); s01 = warp_sum(s01); }
         }
         x.sc = scan_scalars<MODE>(p, s0, s1, s01, fs, ft, rate, qscale, bias_h);
 #pragma unroll

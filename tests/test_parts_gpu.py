@@ -531,7 +531,8 @@ def test_attention_refuses_a_group_the_kernels_do_not_take():
 @pytest.mark.parametrize("dim,vdim", [(24, 20), (64, 33), (100, 48), (128, 128), (256, 16)])
 def test_scans_of_portions_equal_single_tokens(mode, dim, vdim):
     """Runs of 0 to 35 tokens (the edges of a chunk of 8 or 16, and of two) in one step against the same tokens one at a
-    time: outputs and states.  Both kernels add in one order, so what is allowed is the rounding of a few operations."""
+    time: outputs and states.  Both kernels add in one order, so they have the same bits; the matrix memory's gates come
+    from a kernel that sums them 32 tokens at a time, whatever the cut: the rounding of a few operations."""
     from ember_b200 import ops
     torch.manual_seed(dim + vdim)
     lens, H = [1, 16, 0, 17, 7, 8, 35, 2], 2
@@ -569,4 +570,4 @@ def test_scans_of_portions_equal_single_tokens(mode, dim, vdim):
             run(1, slice(starts[i] + t, starts[i] + t + 1), [0, 1], [S - i], 1, 1)
     assert torch.isfinite(outs[0]).all()
     for a, b in ((outs[0], outs[1]), (states[0], states[1]), (gate_rows[0], gate_rows[1])):
-        assert float((a - b).norm()) <= 1e-6 * float(b.norm()) + 1e-30
+        assert torch.equal(a, b) if mode != "memory" else float((a - b).norm()) <= 1e-6 * float(b.norm()) + 1e-30
