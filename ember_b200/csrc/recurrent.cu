@@ -766,15 +766,25 @@ __device__ __forceinline__ float scan_finish(const float4& sc, float skip, float
 // A portion's tokens follow one another, so what counts is the time of one token.  Three things bounded it where
 // one column a thread and eight equal warps a block did it: every four columns read all of a token's vectors from shared
 // memory (half the time its bandwidth), every warp stopped between chunks to prepare the next one's tokens, and every
-// token's output waited for its own shuffles.  Here a thread keeps RS rows of C columns, so a read serves C columns and rows go in pairs through the packed
-// fp32 instructions; four warps do nothing but prepare (loads of the chunk after the next, norms, decays, gates of
-// the next); and the outputs of four tokens are summed over the row groups together.  Delta rule, 16 heads of 128 x 128: one run of 1,500 tokens 735 -> 397 us; 24 runs of
-// 60 366 -> 240 (256 with the outputs of eight tokens together, which does not fit the registers; with two computing warps a block, or eight preparing ones, the one run gets no faster).
-constexpr int PORTION_WARPS = 4, PORTION_PREPARE = 4;      // computing and preparing warps of a block
+// token's output waited for its own shuffles.  Here a thread keeps RS rows of C columns, so a read serves C columns and
+// rows go in pairs through the packed fp32 instructions; four warps do nothing but prepare (loads of the chunk after the
+// next, norms, decays, gates of the next); and the outputs of four tokens are summed over the row groups together (eight
+// do not fit the registers; with two computing warps a block, or eight preparing ones, one run gets no faster).
+// us from cold, before -> now, one run of 1,500 tokens | 24 runs of 60:
+//   rows x columns, heads     delta rule               gated linear attention   time mixing
+//    32 x  64, 32          431 -> 248 | 161 ->  99    337 -> 144 | 126 ->  64   329 -> 140 | 130 ->  71
+//   128 x 128, 16          806 -> 431 | 380 -> 255    591 -> 276 | 298 -> 166   565 -> 341 | 285 -> 184
+//   256 x 256,  8         1349 -> 677 | 668 -> 446   1121 -> 523 | 559 -> 470  1052 -> 432 | 521 -> 387
+// Up to 32 rows two blocks share an SM (with one the 24 runs of the delta rule took 142 us).  Beyond 128 rows one block has
+// an SM to itself: four computing warps whose operands come a token ahead while there are no more blocks than SMs, else
+// eight that fetch them as they go and hide one another's waits (24 runs at 256 x 256 with four: delta rule 668,
+// gated linear attention 573; 17 + 7 x 1 tokens 64 | 64, now 47 | 52, once 60 | 53).
+constexpr int PORTION_PREPARE = 4;      // preparing warps of a block, beside NCW computing ones
 
-template <int MODE, int RS, int CT, int C>
-__global__ void __launch_bounds__(32 * (PORTION_WARPS + PORTION_PREPARE), 1) scan_portion_kernel(ScanArgs p) {
-    constexpr int NCW = PORTION_WARPS, NP = PORTION_PREPARE, THREADS = 32 * (NCW + NP), COLS = 4 * C * NCW;
+template <int MODE, int RS, int CT, int C, int NCW>
+__global__ void __launch_bounds__(32 * (NCW + PORTION_PREPARE), RS == 4 ? 2 : 1) scan_portion_kernel(ScanArgs p) {
+    constexpr int NP = PORTION_PREPARE, THREADS = 32 * (NCW + NP), COLS = 4 * C * NCW;
+    constexpr int SETS = NCW > 4 ? 1 : 2;           // register sets for a token's operands
     extern __shared__ __align__(16) float smem[];
     pdl_launch_dependents();
     pdl_wait();
@@ -919,8 +929,8 @@ __global__ void __launch_bounds__(32 * (PORTION_WARPS + PORTION_PREPARE), 1) sca
     for (int t0 = first; t0 < end; t0 += CT, cur ^= 1) {
         const int n = min(CT, end - t0);
         const float* buf = smem + cur * CT * TOK;
-        // a token's operands are fetched into registers while the token before it is computed (two register sets),
-        // so that no multiply-add waits for shared memory
+        // with two register sets a token's operands are fetched while the token before it is computed, so that no
+        // multiply-add waits for shared memory
         auto fetch = [&](int tt, TokenRegs<RS / 4, C>& x) {
             const float* tok = buf + tt * TOK;
             x.sc = *reinterpret_cast<const float4*>(tok + NV * VS);
@@ -937,8 +947,8 @@ __global__ void __launch_bounds__(32 * (PORTION_WARPS + PORTION_PREPARE), 1) sca
             if (col < V) __stcs(p.out + (size_t)t * H * V + h * V + col, y);
             else if (col < n_cols) p.gates[((size_t)t * H + h) * 4 + 3] = y;
         };
-        TokenRegs<RS / 4, C> X[2];
-        fetch(0, X[0]);
+        TokenRegs<RS / 4, C> X[SETS];
+        if (SETS == 2) fetch(0, X[0]);
         int tt = 0;
         for (; tt + 4 <= n; tt += 4) {
             // four tokens, whose outputs are summed over the row groups together: a lane gives away half of its tokens at
@@ -948,10 +958,11 @@ __global__ void __launch_bounds__(32 * (PORTION_WARPS + PORTION_PREPARE), 1) sca
             float4 sc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 #pragma unroll
             for (int u = 0; u < 4; u++) {
-                fetch(min(tt + u + 1, CT - 1), X[(u + 1) & 1]);
-                scan_step<MODE, RS, C>(st, X[u & 1], o[u], add[u]);
+                fetch(SETS == 2 ? min(tt + u + 1, CT - 1) : tt + u, X[SETS == 2 ? (u + 1) & 1 : 0]);
+                const TokenRegs<RS / 4, C>& x = X[SETS == 2 ? u & 1 : 0];
+                scan_step<MODE, RS, C>(st, x, o[u], add[u]);
                 if ((r & 3) == u) {
-                    sc = X[u & 1].sc;
+                    sc = x.sc;
 #pragma unroll
                     for (int c = 0; c < C; c++) keep[c] = add[u][c];
                 }
@@ -970,16 +981,16 @@ __global__ void __launch_bounds__(32 * (PORTION_WARPS + PORTION_PREPARE), 1) sca
                 if ((r >> 2) == c) store(t0 + tt + (r & 3), j + c, scan_finish<MODE>(sc, skip, sum, keep[c]));
             }
         }
-        for (; tt < n; tt++) {                      // X[0] holds token tt
+        for (; tt < n; tt++) {                      // (with two sets X[0] holds token tt)
             float o[C], add[C];
-            fetch(min(tt + 1, CT - 1), X[1]);
+            fetch(SETS == 2 ? min(tt + 1, CT - 1) : tt, X[SETS - 1]);
             scan_step<MODE, RS, C>(st, X[0], o, add);
 #pragma unroll
             for (int c = 0; c < C; c++) {
                 const float sum = rows_sum(o[c]);
                 if (r == c) store(t0 + tt, j + c, scan_finish<MODE>(X[0].sc, skip, sum, add[c]));
             }
-            X[0] = X[1];
+            X[0] = X[SETS - 1];
         }
         asm volatile("bar.sync 1, %0;" ::"n"(THREADS) : "memory");
     }
@@ -1140,21 +1151,26 @@ inline bool regs_kernels_on() {
     return on != 0;
 }
 
+inline int num_sms() {
+    int device = 0, n = 0;
+    return cudaGetDevice(&device) == cudaSuccess && cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, device) == cudaSuccess ? n : 148;
+}
+
 template <int MODE, int RS, int C>
 inline int launch_single(const ScanArgs& p, int S, int n_cols, cudaStream_t st) {
     constexpr int COLS = 4 * C * SINGLE_WARPS;
     launch_kernel(scan_single_kernel<MODE, RS, C>, dim3(S, p.H, (n_cols + COLS - 1) / COLS), 32 * SINGLE_WARPS, 0, st, p);
     return 0;
 }
-template <int MODE, int RS, int CT, int C>
+template <int MODE, int RS, int CT, int C, int NCW = 4>
 inline int launch_portion(const ScanArgs& p, int S, int n_cols, cudaStream_t st) {
-    constexpr int NV = (MODE == 0 || MODE == 3 || MODE == 4) ? 3 : 2, COLS = 4 * C * PORTION_WARPS;
+    constexpr int NV = (MODE == 0 || MODE == 3 || MODE == 4) ? 3 : 2, COLS = 4 * C * NCW;
     constexpr size_t smem = (size_t)2 * CT * (NV * 8 * (RS + 4) + 4 + COLS) * sizeof(float);
     if (smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(scan_portion_kernel<MODE, RS, CT, C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaError_t e = cudaFuncSetAttribute(scan_portion_kernel<MODE, RS, CT, C, NCW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return fail("scan: %s", cudaGetErrorString(e));
     }
-    launch_kernel(scan_portion_kernel<MODE, RS, CT, C>, dim3(S, p.H, (n_cols + COLS - 1) / COLS), 32 * (PORTION_WARPS + PORTION_PREPARE),
+    launch_kernel(scan_portion_kernel<MODE, RS, CT, C, NCW>, dim3(S, p.H, (n_cols + COLS - 1) / COLS), 32 * (NCW + PORTION_PREPARE),
                   smem, st, p);
     return 0;
 }
@@ -1165,7 +1181,10 @@ inline int launch_scan(const ScanArgs& p, int S, int n_cols, bool single, cudaSt
         case 4: return single ? launch_single<MODE, 4, 2>(p, S, n_cols, st) : launch_portion<MODE, 4, 16, 2>(p, S, n_cols, st);
         case 8: return single ? launch_single<MODE, 8, 2>(p, S, n_cols, st) : launch_portion<MODE, 8, 16, 2>(p, S, n_cols, st);
         case 16: return single ? launch_single<MODE, 16, 2>(p, S, n_cols, st) : launch_portion<MODE, 16, 16, 2>(p, S, n_cols, st);
-        default: return single ? launch_single<MODE, 32, 1>(p, S, n_cols, st) : launch_portion<MODE, 32, 8, 1>(p, S, n_cols, st);
+        default:
+            if (single) return launch_single<MODE, 32, 1>(p, S, n_cols, st);
+            if ((long long)S * p.H * ((n_cols + 15) / 16) > num_sms()) return launch_portion<MODE, 32, 8, 1, 8>(p, S, n_cols, st);
+            return launch_portion<MODE, 32, 8, 1>(p, S, n_cols, st);
     }
 }
 

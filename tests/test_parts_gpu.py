@@ -528,7 +528,7 @@ def test_attention_refuses_a_group_the_kernels_do_not_take():
 
 
 @pytest.mark.parametrize("mode", ["delta", "memory", "ssm", "gla", "wkv"])
-@pytest.mark.parametrize("dim,vdim", [(24, 20), (64, 33), (100, 48), (128, 128), (256, 16)])
+@pytest.mark.parametrize("dim,vdim", [(24, 20), (64, 33), (100, 48), (128, 128), (256, 16), (200, 150)])
 def test_scans_of_portions_equal_single_tokens(mode, dim, vdim):
     """Runs of 0 to 35 tokens (the edges of a chunk of 8 or 16, and of two) in one step against the same tokens one at a
     time: outputs and states.  Both kernels add in one order, so they have the same bits; the matrix memory's gates come
