@@ -51,7 +51,7 @@ layer_norm_kernel(const float* __restrict__ x, const int* __restrict__ rows, con
     }
     const float rstd = 1.0f / sqrtf(block_sum(ss, scratch) / (float)H + eps);
     for (int i = threadIdx.x; i < H; i += ROW_THREADS)
-        o[i] = from_float<TO>((in[i] - mean) * rstd * w[i] + (b ? b[i] : 0.0f));
+        o[i] = from_float<TO>(fmaf((in[i] - mean) * rstd, w[i], b ? b[i] : 0.0f));
 }
 
 // ------------------------------------------------------------------------------- gate, norm, add to the stream
@@ -82,7 +82,7 @@ gated_norm_add_kernel(const float* __restrict__ y, const float* __restrict__ gat
     }
     const float rstd = 1.0f / sqrtf(block_sum(ss, scratch) / (float)H + eps);
     for (int i = threadIdx.x; i < H; i += ROW_THREADS) {
-        const float r = residual[base + i] + ((row[i] - mean) * rstd * w[i] + (b ? b[i] : 0.0f));
+        const float r = residual[base + i] + fmaf((row[i] - mean) * rstd, w[i], b ? b[i] : 0.0f);
         residual[base + i] = r;
         if (rounded) rounded[base + i] = __float2bfloat16_rn(r);      // what the next sublayer's products read
     }
@@ -157,38 +157,42 @@ norm_add_norm_kernel(const float* __restrict__ y, const float* __restrict__ w, f
     }
 }
 
-// The same behind a gate and with either kind of norm on both sides: a
-// step of a few tokens is a chain of such rows, so what counts is one row's latency.  The row stays in registers (PER
-// pieces of four elements a thread), all loads are under way at once, and up to PER = 2 the weights are asked for
-// before the wait for the kernel before.  One row of 2,048 in a step: gate, norm and addition took 7.6 us and the norm
-// behind them 3.4, now 3.7 together; 24 rows 7.1 + 3.4, now 4.4.
+// The same behind a gate and with either kind of norm on both sides.  A step of a few tokens is a chain of such rows, so what
+// counts is one row's latency: the row stays in registers (PER pieces of four elements a thread), all loads are under way
+// at once, and up to PER = 2 the weights are asked for before the wait for the kernel before.  The sums are those of the
+// kernels of one norm each, to the bit: gated_norm_add and layer_norm above give a thread the elements thread, thread + 256,
+// .., which it reads from shared memory; an RMS norm behind has the pieces of its own kernel.  Layer norms on both sides and
+// a gate, us with two kernels -> with this: one row of 2,048 6.3 -> 3.4, 24 rows 6.9 -> 3.6, 2,048 rows 20.6 -> 19.8; one
+// row of 8,192 15.7 -> 9.4.  (RMS norms without a gate keep the kernel above: 2,048 rows of 4,096 17.4 us, 19.8 with this.)
 template <typename TO, int PER>
 __global__ void __launch_bounds__(ROW_THREADS)
 gated_norm_add_norm_kernel(const float* __restrict__ y, const float* __restrict__ gate, const float* __restrict__ gate_bias,
                            const float* __restrict__ w, const float* __restrict__ b, float eps, int centred, float* __restrict__ residual,
                            const float* __restrict__ w2, const float* __restrict__ b2, float eps2, int centred2, TO* __restrict__ out, int H) {
+    extern __shared__ __align__(16) float row[];          // H floats: the gated row, then the new row of the stream
     __shared__ float scratch[32];
     pdl_launch_dependents();
     constexpr bool EARLY = PER <= 2;
+    constexpr int E = EARLY ? PER : 1;
     const size_t base = (size_t)blockIdx.x * H;
     auto at = [&](int u) { return (int)(threadIdx.x + u * ROW_THREADS) * 4; };
     auto piece = [&](const float* p, int i, float (&v)[4]) {
         if (p && i < H) row_load<4>(p + i, v);
         else v[0] = v[1] = v[2] = v[3] = 0.0f;
     };
-    float g1[EARLY ? PER : 1][4], a1[EARLY ? PER : 1][4], g2[EARLY ? PER : 1][4], a2[EARLY ? PER : 1][4], gb[EARLY ? PER : 1][4];
+    float g1[E][4], a1[E][4], g2[E][4], a2[E][4], gb[E][4];
     if (EARLY) {
 #pragma unroll
-        for (int u = 0; u < PER; u++) {
-            piece(w, at(u), g1[EARLY ? u : 0]);
-            piece(b, at(u), a1[EARLY ? u : 0]);
-            piece(gate ? gate_bias : nullptr, at(u), gb[EARLY ? u : 0]);
-            piece(w2, at(u), g2[EARLY ? u : 0]);
-            piece(b2, at(u), a2[EARLY ? u : 0]);
+        for (int u = 0; u < E; u++) {
+            piece(w, at(u), g1[u]);
+            piece(b, at(u), a1[u]);
+            piece(gate ? gate_bias : nullptr, at(u), gb[u]);
+            piece(w2, at(u), g2[u]);
+            piece(b2, at(u), a2[u]);
         }
     }
     pdl_wait();
-    float v[PER][4], h[PER][4], s = 0.0f;
+    float v[PER][4], h[PER][4];
 #pragma unroll
     for (int u = 0; u < PER; u++) {
         piece(y + base, at(u), v[u]);
@@ -204,48 +208,62 @@ gated_norm_add_norm_kernel(const float* __restrict__ y, const float* __restrict_
             for (int k = 0; k < 4; k++) v[u][k] *= sigmoidf_(z[k] + (EARLY ? gb[EARLY ? u : 0][k] : late[k]));
         }
     }
+    auto put = [&](const float (&x)[PER][4]) {
 #pragma unroll
-    for (int u = 0; u < PER; u++)
+        for (int u = 0; u < PER; u++)
+            if (at(u) < H) row_store<4>(row + at(u), x[u]);
+        __syncthreads();
+    };
+    // mean and 1 / sqrt(mean square + eps) of the row in shared memory (it may be written again behind)
+    auto statistics = [&](bool about_mean, float e, float& mean) {
+        float s = 0.0f, ss = 0.0f;
+        if (about_mean) {
 #pragma unroll
-        for (int k = 0; k < 4; k++) s += v[u][k];
-    const float mean = centred ? block_sum(s, scratch) / (float)H : 0.0f;
-    float ss = 0.0f;
-#pragma unroll
-    for (int u = 0; u < PER; u++)
-#pragma unroll
-        for (int k = 0; k < 4; k++) {
-            v[u][k] -= mean;
-            if (at(u) < H) ss = fmaf(v[u][k], v[u][k], ss);
+            for (int u = 0; u < 4 * PER; u++)
+                if ((int)threadIdx.x + u * ROW_THREADS < H) s += row[threadIdx.x + u * ROW_THREADS];
         }
-    const float rstd = 1.0f / sqrtf(block_sum(ss, scratch) / (float)H + eps);
-    s = 0.0f;
+        mean = about_mean ? block_sum(s, scratch) / (float)H : 0.0f;
+#pragma unroll
+        for (int u = 0; u < 4 * PER; u++) {
+            if ((int)threadIdx.x + u * ROW_THREADS < H) {
+                const float d = row[threadIdx.x + u * ROW_THREADS] - mean;
+                ss = fmaf(d, d, ss);
+            }
+        }
+        return 1.0f / sqrtf(block_sum(ss, scratch) / (float)H + e);
+    };
+    put(v);
+    float mean;
+    const float rstd = statistics(centred, eps, mean);
 #pragma unroll
     for (int u = 0; u < PER; u++) {
         float gl[4], al[4];
         if (!EARLY) { piece(w, at(u), gl); piece(b, at(u), al); }
 #pragma unroll
-        for (int k = 0; k < 4; k++) {
-            h[u][k] += v[u][k] * rstd * (EARLY ? g1[EARLY ? u : 0][k] : gl[k]) + (EARLY ? a1[EARLY ? u : 0][k] : al[k]);
-            s += h[u][k];
-        }
+        for (int k = 0; k < 4; k++)
+            h[u][k] += fmaf((v[u][k] - mean) * rstd, EARLY ? g1[EARLY ? u : 0][k] : gl[k], EARLY ? a1[EARLY ? u : 0][k] : al[k]);
         if (at(u) < H) row_store<4>(residual + base + at(u), h[u]);
     }
-    const float mean2 = centred2 ? block_sum(s, scratch) / (float)H : 0.0f;
-    ss = 0.0f;
+    float mean2 = 0.0f, rstd2;
+    if (centred2) {
+        put(h);
+        rstd2 = statistics(true, eps2, mean2);
+    } else {
+        float ss = 0.0f;
 #pragma unroll
-    for (int u = 0; u < PER; u++)
-#pragma unroll
-        for (int k = 0; k < 4; k++) {
-            h[u][k] -= mean2;
-            if (at(u) < H) ss = fmaf(h[u][k], h[u][k], ss);
-        }
-    const float rstd2 = 1.0f / sqrtf(block_sum(ss, scratch) / (float)H + eps2);
+        for (int u = 0; u < PER; u++)
+            if (at(u) < H) ss = fmaf(h[u][0], h[u][0], fmaf(h[u][1], h[u][1], fmaf(h[u][2], h[u][2], fmaf(h[u][3], h[u][3], ss))));
+        rstd2 = 1.0f / sqrtf(block_sum(ss, scratch) / (float)H + eps2);
+    }
 #pragma unroll
     for (int u = 0; u < PER; u++) {
         float gl[4], al[4];
         if (!EARLY) { piece(w2, at(u), gl); piece(b2, at(u), al); }
 #pragma unroll
-        for (int k = 0; k < 4; k++) h[u][k] = h[u][k] * rstd2 * (EARLY ? g2[EARLY ? u : 0][k] : gl[k]) + (EARLY ? a2[EARLY ? u : 0][k] : al[k]);
+        for (int k = 0; k < 4; k++) {
+            const float g = EARLY ? g2[EARLY ? u : 0][k] : gl[k];
+            h[u][k] = centred2 ? fmaf((h[u][k] - mean2) * rstd2, g, EARLY ? a2[EARLY ? u : 0][k] : al[k]) : g * (h[u][k] * rstd2);
+        }
         if (at(u) < H) row_store<4>(out + base + at(u), h[u]);
     }
 }
@@ -614,8 +632,8 @@ EMBER_API int ember_gated_norm_add_norm(const float* y, const float* gate, const
         return fail("gated_norm_add_norm: operands must be 16-byte aligned");
     const int pieces = (H + 4 * ROW_THREADS - 1) / (4 * ROW_THREADS);
     auto run = [&](auto kernel, auto* o) -> int {
-        launch_kernel(kernel, n_rows, ROW_THREADS, 0, (cudaStream_t)stream, y, gate, gate_bias, w, b, eps, centred, residual, w2, b2, eps2,
-                      centred2, o, H);
+        launch_kernel(kernel, n_rows, ROW_THREADS, (size_t)H * sizeof(float), (cudaStream_t)stream, y, gate, gate_bias, w, b, eps, centred, residual,
+                      w2, b2, eps2, centred2, o, H);
         return check_launch("gated_norm_add_norm");
     };
     auto pick = [&](auto* o) -> int {

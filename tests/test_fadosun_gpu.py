@@ -344,6 +344,27 @@ def test_gated_norm_add_norm(dtype, H, centred, centred2, gated):
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("H", [4, 252, 1000, 1024, 1028, 2048, 2052, 4096, 4100, 8192])
+@pytest.mark.parametrize("centred,centred2,gated", [(True, True, 2), (False, True, 1), (True, False, 0), (False, False, 2)])
+def test_gated_norm_add_norm_is_its_two_kernels(dtype, H, centred, centred2, gated):
+    """The fused kernel has the bits of the two kernels in turn."""
+    from ember_b200 import ops
+    torch.manual_seed(H + gated)
+    y, z, h = (torch.randn(5, H, device="cuda") for _ in range(3))
+    w, b, w2, b2, zb = (torch.randn(H, device="cuda") for _ in range(5))
+    args = (y, z if gated else None, w, b if centred else None, 1e-5, centred)
+    want_h, want = h.clone(), torch.zeros(5, H, device="cuda", dtype=dtype)
+    ops.gated_norm_add(*args, want_h, 5, gate_bias=zb if gated == 2 else None)
+    if centred2:
+        ops.layer_norm(want_h, w2, b2, 1e-6, want, 5)
+    else:
+        ops.rmsnorm(want_h, w2, 1e-6, want, 5)
+    got = torch.zeros_like(want)
+    ops.gated_norm_add_norm(y, args[1], zb if gated == 2 else None, w, args[3], 1e-5, centred, h, w2, b2 if centred2 else None, 1e-6, centred2, got, 5)
+    assert torch.equal(h, want_h) and torch.equal(got, want)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_layer_norm_gate_and_sandwich_kernels(dtype):
     """layer_norm, the fused gate + norm + add, and the per-group norm with both kinds of gate."""
     from ember_b200 import ops
