@@ -729,9 +729,10 @@ def gated_norm_add(y: torch.Tensor, gate_logits: Optional[torch.Tensor], weight:
           _p(residual), _p(rounded), c_int(n_rows), c_int(H), _stream(stream))
 
 
-def gated_norm_add_norm_usable(width: int) -> bool:
-    """Whether ``gated_norm_add_norm`` takes rows of this width (the rule of ember_gated_norm_add_norm_supported)."""
-    return width % 4 == 0 and 0 < width <= 8192
+def gated_norm_add_norm_usable(width: int, *vectors: Optional[torch.Tensor]) -> bool:
+    """Whether ``gated_norm_add_norm`` takes rows of this width (the rule of ember_gated_norm_add_norm_supported) under these
+    weights and biases, which it reads 16 bytes at a time."""
+    return width % 4 == 0 and 0 < width <= 8192 and all(t is None or t.data_ptr() % 16 == 0 for t in vectors)
 
 
 def gated_norm_add_norm(y: torch.Tensor, gate_logits: Optional[torch.Tensor], gate_bias: Optional[torch.Tensor], w: torch.Tensor,
@@ -739,7 +740,7 @@ def gated_norm_add_norm(y: torch.Tensor, gate_logits: Optional[torch.Tensor], ga
                         b2: Optional[torch.Tensor], eps2: float, centred2: bool, out: torch.Tensor, n_rows: int,
                         stream: Optional[int] = None) -> None:
     """residual[r] += norm(y[r] * sigmoid(gate_logits[r] + gate_bias)) and out[r] = norm2(residual[r]) in one kernel, each norm
-    centred (layer norm) or not (RMS norm)."""
+    centred (layer norm) or not (RMS norm); the bits of ``gated_norm_add`` and ``layer_norm`` or ``rmsnorm`` in turn."""
     H = w.numel()
     for t, n in ((y, "y"), (gate_logits, "gate_logits"), (gate_bias, "gate_bias"), (w, "w"), (b, "b"), (residual, "residual"), (w2, "w2"), (b2, "b2")):
         if t is not None:

@@ -181,15 +181,17 @@ class GatedSandwichBlock(Arrangement):
         if gate is None and rounded is None and isinstance(norm_out, RMSNorm) and isinstance(norm_next, RMSNorm):
             norm_out.add_then_norm(ctx, y, h, T, norm_next, normed_x)
             return True
-        if rounded is None and isinstance(norm_out, RowNorm) and isinstance(norm_next, RowNorm) and ops.gated_norm_add_norm_usable(hidden):
-            norm_out.gated_add_norm(ctx, y, logits, h, T, getattr(gate, "bias", None), norm_next, normed_x)
+        gate_bias = getattr(gate, "bias", None)
+        if (rounded is None and isinstance(norm_out, RowNorm) and isinstance(norm_next, RowNorm) and
+                ops.gated_norm_add_norm_usable(hidden, gate_bias, norm_out.weight, norm_out.bias, norm_next.weight, norm_next.bias)):
+            norm_out.gated_add_norm(ctx, y, logits, h, T, gate_bias, norm_next, normed_x)
             return True
         if rounded is not None:
-            norm_out.gated_add(ctx, y, logits, h, T, gate_bias=getattr(gate, "bias", None), rounded=rounded)
+            norm_out.gated_add(ctx, y, logits, h, T, gate_bias=gate_bias, rounded=rounded)
             ctx.memo["block.stream_rounded.at"] = ctx.memo.get("schedule.index")
             ctx.memo["block.stream_rounded.of"] = h.data_ptr()
         else:
-            norm_out.gated_add(ctx, y, logits, h, T, gate_bias=getattr(gate, "bias", None))
+            norm_out.gated_add(ctx, y, logits, h, T, gate_bias=gate_bias)
         return False
 
     def forward(self, ctx, h: torch.Tensor, caches, owns_cache: bool = True) -> None:

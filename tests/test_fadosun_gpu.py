@@ -364,6 +364,25 @@ def test_gated_norm_add_norm_is_its_two_kernels(dtype, H, centred, centred2, gat
     assert torch.equal(h, want_h) and torch.equal(got, want)
 
 
+def test_norm_weights_at_odd_addresses(dirs):
+    """Norm weights and biases that are views from an odd element of an fp32 tensor: taken, with the same logits."""
+    from ember_b200 import StepEntry
+    from ember_b200.engine.runner import ModelRunner
+    from ember_b200.parts.norm import LayerNorm
+    name, rows = next(iter(FADOSUN)), []
+    for odd in (False, True):
+        runner = ModelRunner.from_dir(dirs[name], dtype="float32", capacity_tokens=64, max_batch_tokens=64, max_requests=2, page_tokens=16)
+        norms = [p for b in runner.model.blocks for p in b.parts.values() if isinstance(p, LayerNorm)]
+        assert len(norms) > 2
+        for p in norms if odd else []:
+            p.weight, p.bias = (torch.cat([t[:1], t])[1:] for t in (p.weight, p.bias))
+            assert p.weight.data_ptr() % 16
+        runner.admit("a"), runner.reserve("a", 20)
+        rows.append(runner.step([StepEntry("a", list(range(1, 21)), tuple(range(20)))]).clone())
+        runner.check_device()
+    assert torch.equal(*rows)
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_layer_norm_gate_and_sandwich_kernels(dtype):
     """layer_norm, the fused gate + norm + add, and the per-group norm with both kinds of gate."""
