@@ -8,13 +8,14 @@ from __future__ import annotations
 
 import ctypes
 from ctypes import c_float, c_longlong, c_void_p
+from operator import index
 from typing import Optional
 
 import torch
 
 from .csrc import build
 
-c_int = int          # a plain int crosses as a C int, and is made in half the time of a ctypes object (fifteen a call)
+c_int = index        # a plain int crosses as a C int, and is made in half the time of a ctypes object (fifteen a call); no floats
 F32, BF16 = 0, 1
 EPI_STORE, EPI_STORE_F32, EPI_ADD_F32, EPI_SILU_MUL = 0, 1, 2, 3
 EPI_SUMS = 5      # tensor-core product of at most 128 tokens: the fp32 sums stay in the split-K scratch

@@ -1,0 +1,19 @@
+"""What crosses to the kernels' C functions as an int."""
+import ctypes
+
+import pytest
+import torch
+
+from ember_b200 import ops
+
+
+@pytest.mark.parametrize("value", [2.0, 2.5, "3", None, torch.tensor(1.5)])
+def test_what_is_no_whole_number_is_refused(value):
+    for convert in (ctypes.c_int, ops.c_int):
+        with pytest.raises(TypeError):
+            convert(value)
+
+
+@pytest.mark.parametrize("value", [0, -3, True, 2 ** 31 - 1, torch.tensor(7)])
+def test_whole_numbers_arrive(value):
+    assert ctypes.c_int(ops.c_int(value)).value == ctypes.c_int(value).value
