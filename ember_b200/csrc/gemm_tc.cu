@@ -20,6 +20,7 @@
 //
 // The reference's products (src/backend/cuda/k_gemm.cu:65-405) are mma.sync kernels for Turing;
 // nothing of them is reused here.
+#include <atomic>
 #include <map>
 #include <mutex>
 #include <tuple>
@@ -155,17 +156,17 @@ static size_t decode_smem(GemmTcParams& p, int num_sms) {
     return (size_t)stages * stage_bytes + 1024 /* alignment slack */ + 256 /* barriers */ + recv;
 }
 
-// The decode-sized kernel may use an SM's whole shared memory (set once per process).
-static bool raise_smem_limit() {
-    static const bool done = [] {
-        cudaError_t e = cudaFuncSetAttribute(gemm_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-        if (e != cudaSuccess) { cudaGetLastError(); return false; }
-        cudaFuncSetAttribute(gemm_tc_kernel<false>, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared);
-        cudaFuncSetAttribute(gemm_tc_kernel<true>, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared);
-        return true;
-    }();
-    return done;
+// The decode-sized kernel may use an SM's whole shared memory (set once; a call that failed is made again).
+static cudaError_t raise_smem_limit() {
+    static std::atomic<bool> done{false};
+    if (done.load(std::memory_order_relaxed)) return cudaSuccess;
+    cudaError_t e = cudaFuncSetAttribute(gemm_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    if (e != cudaSuccess) { cudaGetLastError(); return e; }
+    cudaFuncSetAttribute(gemm_tc_kernel<false>, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared);
+    cudaFuncSetAttribute(gemm_tc_kernel<true>, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared);
+    done.store(true, std::memory_order_relaxed);
+    return cudaSuccess;
 }
 
 // Parts of K, one block of a cluster each, for 17 to 128 tokens; 0: atomics are better.  Up to 64 tokens two blocks fit
@@ -513,7 +514,7 @@ EMBER_API int ember_gemm_tc(const void* A, const void* W, void* out, int ldc, in
         !tensor_map(cols_ptr, cols_extent, K, p.block_cols, &map_cols))
         return fail("gemm_tc: cuTensorMapEncodeTiled failed or is unavailable");
 
-    if (!raise_smem_limit()) return fail("gemm_tc: cannot raise the shared-memory limit");
+    if (const cudaError_t e = raise_smem_limit()) return fail("gemm_tc: cannot raise the shared-memory limit: %s", cudaGetErrorString(e));
     dim3 grid(row_tiles, col_tiles, splits);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
@@ -565,7 +566,7 @@ EMBER_API int ember_gemm_tc_qkv_supported(int M, int N, int K, int n_heads, int 
 // The fused projection of a decode-sized step (at most 128 tokens): 128 weight rows (one head slot) x the tokens per
 // tile, the K range split over a thread-block cluster whose blocks share the tokens out and finish whole heads.
 static int launch_heads_swapped(const void* A, const void* W, GemmTcParams p, int num_sms, cudaStream_t st) {
-    if (!raise_smem_limit()) return fail("gemm_tc: cannot raise the shared-memory limit");
+    if (const cudaError_t e = raise_smem_limit()) return fail("gemm_tc: cannot raise the shared-memory limit: %s", cudaGetErrorString(e));
     p.swapped = 1;
     p.block_cols = (p.M + 15) / 16 * 16;
     const int tiles = p.N / TILE_ROWS;
