@@ -56,6 +56,7 @@ struct AttnTcParams {
     const float* sink;        // [n_heads] or null: exp(sink[h]) joins the denominator once, without key and value
     int n_splits, split_keys;
     int n_tiles;
+    int settled;              // decode: nothing that may still run writes keys or pages before the tile's position
     int cluster_merge;        // the splits of a tile are a thread-block cluster and are merged in its first block's shared memory
     int* err;
 };
@@ -216,12 +217,13 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
             }
         }
     };
-    // A decoded token brings one key; all keys before its position were written by earlier steps, and the copy of a
-    // step's integers that this step's kernels stand behind stands behind those.  So the first tiles without the
-    // new key are asked for now, while the kernel before this one (which makes the queries and that key) still runs: a
-    // layer's attention took 9.9, 25.1 and 43.9 us (one request at 700 keys, 8 at 3,072, 64 at 1,024), now 8.3, 23.4, 39.1.
+    // In a model's step a decoded token brings one key; all keys before its position were written by earlier steps, and the
+    // copy of a step's integers that this step's kernels stand behind stands behind those.  There (`settled`) the first
+    // tiles without the new key are asked for now, while the kernel before this one (which makes the queries and that key)
+    // still runs: a layer's attention took 9.9, 25.1 and 43.9 us (one request at 700 keys, 8 at 3,072, 64 at 1,024), now 8.3,
+    // 23.4, 39.1.
     int early = 0;
-    if (DECODE && warp == 4) {
+    if (DECODE && p.settled && warp == 4) {
         early = min(min(n_kt, NSTAGE), max(0, (pos0 - k_begin) / KT));
         for (int it = 0; it < early; it++) fetch_tile(it, page_row(it));
     }
@@ -650,7 +652,7 @@ EMBER_API int ember_attention_tc(const void* q, const void* k_pool, const void* 
                                  int n_heads, int n_kv, int D, const int* tiles, int n_tiles,
                                  const int* block_table, int max_blocks, int page, int num_pages, int window,
                                  float scale, int n_splits, int split_keys, float* part_o, float* part_ml,
-                                 int* err, float softcap, int chunk, const float* gate, int ld_gate, const float* slopes, const float* sink, void* stream) {
+                                 int* err, float softcap, int chunk, const float* gate, int ld_gate, const float* slopes, const float* sink, int settled, void* stream) {
     if (n_tiles <= 0) return 0;
     if (gate && ld_gate < n_heads * D) return fail("attention_tc: gate rows of %d", ld_gate);
     if (softcap < 0.0f) return fail("attention_tc: a score cap of %g", softcap);
@@ -677,7 +679,7 @@ EMBER_API int ember_attention_tc(const void* q, const void* k_pool, const void* 
     p.cap_log2 = softcap * LOG2E; p.cap_arg = softcap > 0.0f ? 2.0f * LOG2E * scale / softcap : 0.0f;
     p.gate = gate; p.ld_gate = ld_gate; p.slopes = slopes; p.sink = sink;
     p.n_splits = n_splits; p.split_keys = split_keys; p.n_tiles = n_tiles; p.err = err;
-    p.cluster_merge = cluster_merge ? 1 : 0;
+    p.cluster_merge = cluster_merge ? 1 : 0; p.settled = settled ? 1 : 0;
     cudaStream_t st = (cudaStream_t)stream;
     const size_t tile_bytes = (size_t)(D / 64) * KT * 128;
     const size_t q_bytes = ((size_t)(D / 64) * (mode == 1 ? 16 : 64) * 128 + 1023) & ~(size_t)1023;

@@ -51,7 +51,8 @@ inline int check_launch(const char* what) {
 
 // Programmatic dependent launch.  Every kernel is launched with the stream-serialization attribute,
 // so its blocks may start while the kernel before it is still draining; until pdl_wait() returns a
-// kernel touches nothing that an earlier kernel writes (it may set up barriers and prefetch weights).
+// kernel touches nothing that an earlier kernel of the step writes.  It may set up barriers, read the step's uploaded
+// integers and prefetch what its caller says is settled: weights, and the keys of earlier steps.
 // pdl_wait() returns at once when the launch carried no such dependency.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }

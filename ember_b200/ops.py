@@ -433,7 +433,7 @@ def gemm_tc(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, M: int, epilogu
             err: Optional[torch.Tensor] = None, stream: Optional[int] = None, split_mode: int = 0,
             bias: Optional[torch.Tensor] = None) -> None:
     """out (+)= a[:M] @ w.T (+ ``bias``, fp32 [N], in the plain epilogues) on the tcgen05 tensor cores (bf16 in, fp32
-    accumulate).  With ``EPI_SUMS`` (``out`` None,
+    accumulate).  ``w`` is read while the kernel before this one still runs: it is not to be what that kernel writes.  With ``EPI_SUMS`` (``out`` None,
     at most 128 tokens) the fp32 sums are left in the split-K scratch and returned as a view [M, N]: whoever reads
     them sets them back to zero (``qk_norm_rope_store_sums``).
     ``split_mode``: how split-K partial sums are combined (0 automatic, 1 atomics, 2 cluster); 3 runs
@@ -644,14 +644,16 @@ def attention_tc(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, ou
                  part_o: Optional[torch.Tensor] = None, part_ml: Optional[torch.Tensor] = None,
                  err: Optional[torch.Tensor] = None, stream: Optional[int] = None, softcap: float = 0.0, chunk: int = 0,
                  gate: Optional[torch.Tensor] = None, gate_col: int = 0, slopes: Optional[torch.Tensor] = None,
-                 sink: Optional[torch.Tensor] = None) -> None:
+                 sink: Optional[torch.Tensor] = None, keys_settled: bool = False) -> None:
     """bf16 attention over the paged cache on tensor cores (TMA-fed); ``softcap`` > 0 caps the scaled scores by a tanh,
     ``chunk`` > 0 lets position i see j only if floor(i / chunk) == floor(j / chunk), ``gate``, ``slopes`` and
     ``sink`` are those of ``attention_fa``.  Splits are ranges of keys from key 0 on, under a chunk from the 64-key tile that holds the chunk's
     first key.  ``mode`` 0 takes tiles of
     prompt portions, 1 takes single-token tiles and may split their key range: with ``part_o`` / ``part_ml`` the
     splits' partial results go through those buffers and a second kernel merges them; without them (at most 8
-    splits) the splits of a tile are a thread-block cluster and are merged in shared memory."""
+    splits) the splits of a tile are a thread-block cluster and are merged in shared memory.  ``keys_settled`` (mode 1): no
+    kernel that may still run on the stream writes the block table or a key or value before a tile's position, as in a
+    step of decoded tokens; they are then read while the kernel before this one still runs."""
     _check_element_gate(gate, gate_col, n_heads * head_dim)
     _check_slopes(slopes, n_heads)
     _check_slopes(sink, n_heads)
@@ -673,7 +675,7 @@ def attention_tc(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, ou
           c_int(head_dim), _p(tiles), c_int(n_tiles), _p(block_table), c_int(block_table.shape[-1]), c_int(page),
           c_int(k_pool.shape[0]), c_int(window), c_float(scale), c_int(n_splits), c_int(split_keys), _p(part_o),
           _p(part_ml), _p(err), c_float(softcap), c_int(chunk), (_off(gate, gate_col) if gate is not None else c_void_p(0)),
-          c_int(gate.shape[-1] if gate is not None else 0), _p(slopes), _p(sink),
+          c_int(gate.shape[-1] if gate is not None else 0), _p(slopes), _p(sink), c_int(1 if keys_settled else 0),
           c_void_p(stream if stream is not None else current_stream_ptr()))
 
 

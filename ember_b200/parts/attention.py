@@ -245,7 +245,7 @@ class Attention(Mixer):
                     part_o = ctx.buf_dyn("attention.part_o", n * s.num_heads * n_splits * s.head_dim, torch.float32)
                     part_ml = ctx.buf_dyn("attention.part_ml", n * s.num_heads * n_splits * 2, torch.float32)
                 ops.attention_tc(q, cache.k, cache.v, out, 1, *args, tiles, n, table, cache.page_tokens, s.window,
-                                 self.scale, n_splits, split_keys, part_o, part_ml, **kw)
+                                 self.scale, n_splits, split_keys, part_o, part_ml, keys_settled=True, **kw)
             return
         if self.softcap > 0 or self.chunk > 0 or any(t is not None for t in (gate, slopes, sink)):
             raise ops.KernelError("attention: the general kernel has no score cap, chunks, gate, slopes or sink (the tensor-core kernels have)")

@@ -751,3 +751,39 @@ def test_bounded_wait_runs_out_and_returns():
     out = torch.empty(4, 64, device=dev)
     ops.rmsnorm(x, torch.ones(64, device=dev), 1e-6, out, 4)
     assert torch.isfinite(out).all()
+
+
+@pytest.mark.parametrize("heads,kv,dim,page,splits", [(16, 8, 128, 64, 1), (16, 8, 128, 16, 4), (8, 2, 128, 32, 8)])
+def test_single_token_attention_behind_the_kernel_that_writes_the_keys(heads, kv, dim, page, splits):
+    """A portion's keys stored by one kernel and read token by token by the next: without a word of the caller's nothing is read
+    early.  On a cache that is settled the early reads change no bit."""
+    from ember_b200 import ops
+    torch.manual_seed(heads + page)
+    T, N = 400, (heads + 2 * kv) * dim
+    pages = (T + page - 1) // page
+    pos, seq = torch.arange(T, device="cuda").int(), torch.zeros(T, device="cuda").int()
+    table = torch.randperm(pages).int().view(1, pages).cuda()
+    tiles = torch.tensor([[0, t, 1, t] for t in range(T)], dtype=torch.int32, device="cuda")
+    kp = torch.zeros(pages, kv, page, dim, device="cuda", dtype=torch.bfloat16)
+    vp, q = torch.zeros_like(kp), torch.zeros(T, heads * dim, device="cuda", dtype=torch.bfloat16)
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+
+    def attend(out, **kw):
+        ops.attention_tc(q, kp, vp, out, 1, heads, kv, dim, tiles, T, table, page, 0, dim ** -0.5, splits, 128, err=err, **kw)
+
+    for _ in range(5):                                        # every round other keys, so that old ones would show
+        qkv = torch.randn(T, N, device="cuda").bfloat16()
+        got, settled = (torch.zeros(T, heads * dim, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+        torch.cuda.synchronize()
+        ops.qk_norm_rope_store(qkv, T, heads, kv, dim, None, None, 1e-6, None, 0, pos, seq, table, page, kp, vp, q, err=err)
+        attend(got)
+        torch.cuda.synchronize()
+        attend(settled, keys_settled=True)
+        x = qkv.double().view(T, -1, dim)
+        k, v = (x[:, heads + i * kv:heads + (i + 1) * kv].repeat_interleave(heads // kv, 1) for i in range(2))
+        s = torch.einsum("thd,uhd->htu", x[:, :heads], k) * dim ** -0.5
+        s = s.masked_fill(torch.ones(T, T, device="cuda").triu(1).bool(), float("-inf"))
+        want = torch.einsum("htu,uhd->thd", s.softmax(-1), v).reshape(T, -1)
+        assert rel(got, want) < 2.0 ** -7                      # (weights and results rounded to bfloat16)
+        assert torch.equal(got, settled)
+    assert int(err.item()) == 0

@@ -1,5 +1,6 @@
-"""What crosses to the kernels' C functions as an int."""
+"""What crosses to the kernels' C functions as an int, and what they may read early."""
 import ctypes
+import inspect
 
 import pytest
 import torch
@@ -17,3 +18,9 @@ def test_what_is_no_whole_number_is_refused(value):
 @pytest.mark.parametrize("value", [0, -3, True, 2 ** 31 - 1, torch.tensor(7)])
 def test_whole_numbers_arrive(value):
     assert ctypes.c_int(ops.c_int(value)).value == ctypes.c_int(value).value
+
+
+@pytest.mark.parametrize("op,name", [("attention_tc", "keys_settled")])
+def test_early_reads_are_asked_for(op, name):
+    """A kernel reads ahead of the kernel before it only where its caller says that it may."""
+    assert inspect.signature(getattr(ops, op)).parameters[name].default is False
