@@ -156,8 +156,8 @@ __device__ __forceinline__ void finish_pair(float c0, float c1, const float* __r
 // Few tokens (MT of them per block): bound by the weights' way in.  A thread sums one part of K for one weight row
 // and MT tokens; a warp holds NB weight rows x 32 / NB parts and feeds itself through a ring of cp.async stages of 32
 // elements of k (a whole 128-byte line of each row), so nothing but the final addition of the parts needs a block
-// barrier and 3 x 4.5 KB a warp are on their way.  Weights that no earlier kernel writes are asked for before the
-// wait for the kernel before.  Rows of 36 floats keep the 16-byte reads of a quarter warp in different banks.
+// barrier and 3 x 4.5 KB a warp are on their way.  Weights that no kernel still running writes (`settled`) are asked for
+// before the wait for the kernel before.  Rows of 36 floats keep the 16-byte reads of a quarter warp in different banks.
 // Four tokens at the 0.6B widths (hidden 1,024), in a step: o and down 9.0 and 13.8 us, q/k/v and gate/up 5, the head's
 // 622 MB 100 us (6.2 TB/s); with the general kernel everywhere four requests of 75 tokens and four more steps took 143 ms,
 // with this one and the next 23.
@@ -171,7 +171,7 @@ constexpr size_t few_smem() { return (NB * KPARTS / 32) * FEW_STAGES * few_stage
 template <int MT, int NB>
 __global__ void __launch_bounds__(NB * KPARTS)
 gemm_f32_few_kernel(const float* __restrict__ A, int lda, const float* __restrict__ W, int ldw, const float* __restrict__ bias,
-                    float* __restrict__ C, int ldc, int M, int N, int K, int epi) {
+                    float* __restrict__ C, int ldc, int M, int N, int K, int epi, int settled) {
     extern __shared__ __align__(16) float few_shared[];
     constexpr int WP = 32 / NB;                                   // parts of a warp
     pdl_launch_dependents();
@@ -201,13 +201,18 @@ gemm_f32_few_kernel(const float* __restrict__ A, int lda, const float* __restric
             if (r < WP * MT) copy16(dst + r * FEW_K + piece, ok ? A + (size_t)m * lda + k : A, ok);
         }
     };
+    if (settled) {
 #pragma unroll
-    for (int s = 0; s < FEW_STAGES - 1; s++)
-        if (s < steps) fetch_w(s);
+        for (int s = 0; s < FEW_STAGES - 1; s++)
+            if (s < steps) fetch_w(s);
+    }
     pdl_wait();
 #pragma unroll
     for (int s = 0; s < FEW_STAGES - 1; s++) {
-        if (s < steps) fetch_a(s);
+        if (s < steps) {
+            if (!settled) fetch_w(s);
+            fetch_a(s);
+        }
         copies_commit();
     }
 
@@ -271,7 +276,7 @@ static_assert(MANY_SMEM >= (size_t)KPARTS * MANY_M * MANY_OUT * sizeof(float), "
 
 __global__ void __launch_bounds__(KPARTS * 32, 1)
 gemm_f32_many_kernel(const float* __restrict__ A, int lda, const float* __restrict__ W, int ldw, const float* __restrict__ bias,
-                     float* __restrict__ C, int ldc, int M, int N, int K, int epi) {
+                     float* __restrict__ C, int ldc, int M, int N, int K, int epi, int settled) {
     extern __shared__ __align__(16) float many_shared[];
     pdl_launch_dependents();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, tx = lane & 7, ty = lane >> 3;
@@ -300,8 +305,9 @@ gemm_f32_many_kernel(const float* __restrict__ A, int lda, const float* __restri
             copy16(dst + r * MANY_ROW + piece, ok ? A + (size_t)(m0 + r) * lda + k : A, ok);
         }
     };
-    fetch_w(0);
+    if (settled) fetch_w(0);
     pdl_wait();
+    if (!settled) fetch_w(0);
     fetch_a(0);
     copies_commit();
 
@@ -363,12 +369,12 @@ gemm_f32_many_kernel(const float* __restrict__ A, int lda, const float* __restri
 
 template <typename Kernel>
 int launch_f32(Kernel kernel, dim3 grid, int threads, size_t smem, cudaStream_t st, const float* A, int lda, const float* W, int ldw,
-               const float* bias, float* C, int ldc, int M, int N, int K, int epi) {
+               const float* bias, float* C, int ldc, int M, int N, int K, int epi, int settled) {
     if (smem > 48 * 1024) {
         const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return fail("gemm: shared memory %zu: %s", smem, cudaGetErrorString(e));
     }
-    launch_kernel(kernel, grid, threads, smem, st, A, lda, W, ldw, bias, C, ldc, M, N, K, epi);
+    launch_kernel(kernel, grid, threads, smem, st, A, lda, W, ldw, bias, C, ldc, M, N, K, epi, settled);
     return check_launch("gemm_f32");
 }
 
@@ -378,27 +384,27 @@ constexpr int FEW_TOKENS = 32;
 
 template <int MT>
 int launch_few(const float* A, int lda, const float* W, int ldw, const float* bias, float* C, int ldc, int M, int N, int K, int epi,
-               cudaStream_t st) {
+               int settled, cudaStream_t st) {
     const unsigned y = (unsigned)((M + MT - 1) / MT);
     // blocks of 16 weight rows once they fill the SMs twice, else of 8
     if (N >= 16 * 296)
-        return launch_f32(gemm_f32_few_kernel<MT, 16>, dim3((N + 15) / 16, y), 16 * KPARTS, few_smem<MT, 16>(), st, A, lda, W, ldw, bias, C, ldc, M, N, K, epi);
-    return launch_f32(gemm_f32_few_kernel<MT, 8>, dim3((N + 7) / 8, y), 8 * KPARTS, few_smem<MT, 8>(), st, A, lda, W, ldw, bias, C, ldc, M, N, K, epi);
+        return launch_f32(gemm_f32_few_kernel<MT, 16>, dim3((N + 15) / 16, y), 16 * KPARTS, few_smem<MT, 16>(), st, A, lda, W, ldw, bias, C, ldc, M, N, K, epi, settled);
+    return launch_f32(gemm_f32_few_kernel<MT, 8>, dim3((N + 7) / 8, y), 8 * KPARTS, few_smem<MT, 8>(), st, A, lda, W, ldw, bias, C, ldc, M, N, K, epi, settled);
 }
 
 int launch_pieces(const float* A, int lda, const float* W, int ldw, const float* bias, float* C, int ldc, int M, int N, int K, int epi,
-                  cudaStream_t st) {
-    if (M <= 1) return launch_few<1>(A, lda, W, ldw, bias, C, ldc, M, N, K, epi, st);
-    if (M <= 2) return launch_few<2>(A, lda, W, ldw, bias, C, ldc, M, N, K, epi, st);
-    if (M <= 4) return launch_few<4>(A, lda, W, ldw, bias, C, ldc, M, N, K, epi, st);
-    if (M <= 8) return launch_few<8>(A, lda, W, ldw, bias, C, ldc, M, N, K, epi, st);
-    if (M <= FEW_TOKENS) return launch_few<16>(A, lda, W, ldw, bias, C, ldc, M, N, K, epi, st);
+                  int settled, cudaStream_t st) {
+    if (M <= 1) return launch_few<1>(A, lda, W, ldw, bias, C, ldc, M, N, K, epi, settled, st);
+    if (M <= 2) return launch_few<2>(A, lda, W, ldw, bias, C, ldc, M, N, K, epi, settled, st);
+    if (M <= 4) return launch_few<4>(A, lda, W, ldw, bias, C, ldc, M, N, K, epi, settled, st);
+    if (M <= 8) return launch_few<8>(A, lda, W, ldw, bias, C, ldc, M, N, K, epi, settled, st);
+    if (M <= FEW_TOKENS) return launch_few<16>(A, lda, W, ldw, bias, C, ldc, M, N, K, epi, settled, st);
     // a grid has at most 65,535 rows of blocks, half as many tokens here as the 64-row tiles of the general kernel take
     constexpr int ROWS = 65535 * MANY_M;
     for (long long m = 0; m < M; m += ROWS) {
         const int rows = M - m < ROWS ? (int)(M - m) : ROWS;
         const int rc = launch_f32(gemm_f32_many_kernel, dim3((N + MANY_N - 1) / MANY_N, (rows + MANY_M - 1) / MANY_M), KPARTS * 32, MANY_SMEM, st,
-                                  A + (size_t)m * lda, lda, W, ldw, bias, C + (size_t)m * ldc, ldc, rows, N, K, epi);
+                                  A + (size_t)m * lda, lda, W, ldw, bias, C + (size_t)m * ldc, ldc, rows, N, K, epi, settled);
         if (rc) return rc;
     }
     return 0;
@@ -429,7 +435,7 @@ int launch(const void* A, int lda, const void* W, int ldw, const float* bias, vo
 using namespace ember;
 
 EMBER_API int ember_gemm_simt(const void* A, int a_dtype, int lda, const void* W, int w_dtype, int ldw,
-                              const float* bias, void* C, int ldc, int M, int N, int K, int epilogue, void* stream) {
+                              const float* bias, void* C, int ldc, int M, int N, int K, int epilogue, int settled, void* stream) {
     if (M <= 0 || N <= 0) return 0;
     if (K <= 0) return fail("gemm: K=%d", K);
     if (lda < K || ldw < K) return fail("gemm: row strides (%d, %d) smaller than K=%d", lda, ldw, K);
@@ -443,7 +449,7 @@ EMBER_API int ember_gemm_simt(const void* A, int a_dtype, int lda, const void* W
     if (pieces) {
         if (epilogue != 0 && epilogue != 1 && epilogue != 2 && epilogue != 3 && !(epilogue >= 6 && epilogue <= 9))
             return fail("gemm: unknown epilogue %d", epilogue);
-        return launch_pieces((const float*)A, lda, (const float*)W, ldw, bias, (float*)C, ldc, M, N, K, epilogue, st);
+        return launch_pieces((const float*)A, lda, (const float*)W, ldw, bias, (float*)C, ldc, M, N, K, epilogue, settled, st);
     }
     if (a_dtype == EMBER_F32 && w_dtype == EMBER_F32)
         return launch<float, float>(A, lda, W, ldw, bias, C, ldc, M, N, K, epilogue, st);

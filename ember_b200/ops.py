@@ -279,8 +279,9 @@ def silu_mul_interleaved(x: torch.Tensor, out: torch.Tensor, n_out: int, stream:
 
 # ------------------------------------------------------------------------------------ GEMM
 def gemm_simt(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, M: int, epilogue: int = EPI_STORE,
-              bias: Optional[torch.Tensor] = None, stream: Optional[int] = None) -> None:
-    """out (+)= a[:M] @ w.T on the fp32 SIMT pipes (true 32-bit when both are float32)."""
+              bias: Optional[torch.Tensor] = None, stream: Optional[int] = None, weights_settled: bool = False) -> None:
+    """out (+)= a[:M] @ w.T on the fp32 SIMT pipes (true 32-bit when both are float32).  ``weights_settled``: no kernel that may
+    still run on the stream writes ``w``, which is then read while the kernel before this one still runs."""
     _check(a, "a")
     _check(w, "w")
     _check(out, "out")
@@ -300,7 +301,7 @@ def gemm_simt(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, M: int, epilo
     lib = _lib("gemm_simt")
     _call(lib, lib.ember_gemm_simt, _p(a), c_int(dtype_code(a.dtype)), c_int(K), _p(w), c_int(dtype_code(w.dtype)),
           c_int(K), _p(bias), _p(out), c_int(n_out), c_int(M), c_int(N), c_int(K), c_int(epilogue),
-          c_void_p(stream if stream is not None else current_stream_ptr()))
+          c_int(1 if weights_settled else 0), c_void_p(stream if stream is not None else current_stream_ptr()))
 
 
 # ------------------------------------------------------------------------------- attention

@@ -48,4 +48,4 @@ class Linear:
         if ops.gemm_tc_usable(x, self.weight, self.bias, epilogue):
             ops.gemm_tc(x, self.weight, out, m, epilogue, err=ctx.err, stream=ctx.stream, bias=self.bias)
         else:
-            ops.gemm_simt(x, self.weight, out, m, epilogue, bias=self.bias, stream=ctx.stream)
+            ops.gemm_simt(x, self.weight, out, m, epilogue, bias=self.bias, stream=ctx.stream, weights_settled=True)

@@ -787,3 +787,22 @@ def test_single_token_attention_behind_the_kernel_that_writes_the_keys(heads, kv
         assert rel(got, want) < 2.0 ** -7                      # (weights and results rounded to bfloat16)
         assert torch.equal(got, settled)
     assert int(err.item()) == 0
+
+
+@pytest.mark.parametrize("M", [1, 8, 20, 75])
+def test_float32_product_behind_the_kernel_that_writes_its_weights(M):
+    """Without a word of the caller's the weights are read behind the kernel before; settled weights give the same bits."""
+    from ember_b200 import ops
+    torch.manual_seed(M)
+    N, K = 4800, 1024
+    a, w = torch.randn(M, K, device="cuda"), torch.zeros(N, K, device="cuda")
+    got, settled = torch.zeros(M, N, device="cuda"), torch.zeros(M, N, device="cuda")
+    for _ in range(5):                                        # every round other weights, so that old ones would show
+        y, one = torch.randn(N, K, device="cuda"), torch.ones(K, device="cuda")
+        torch.cuda.synchronize()
+        ops.rmsnorm(y, one, 1e-6, w, N)
+        ops.gemm_simt(a, w, got, M, 1)
+        torch.cuda.synchronize()
+        ops.gemm_simt(a, w, settled, M, 1, weights_settled=True)
+        assert torch.equal(got, settled)
+        assert rel(got, a.double() @ w.double().t()) < 2e-6

@@ -20,7 +20,7 @@ def test_whole_numbers_arrive(value):
     assert ctypes.c_int(ops.c_int(value)).value == ctypes.c_int(value).value
 
 
-@pytest.mark.parametrize("op,name", [("attention_tc", "keys_settled")])
+@pytest.mark.parametrize("op,name", [("attention_tc", "keys_settled"), ("gemm_simt", "weights_settled")])
 def test_early_reads_are_asked_for(op, name):
     """A kernel reads ahead of the kernel before it only where its caller says that it may."""
     assert inspect.signature(getattr(ops, op)).parameters[name].default is False
