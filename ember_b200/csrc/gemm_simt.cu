@@ -8,9 +8,9 @@
 //
 //   * float x float with rows of whole 16-byte pieces (every product of the float32 path): K is
 //     cut into KPARTS parts, a part's elements of even k and of odd k are summed apart with k
-//     ascending, and the sums are added in order.  The parts are what lets a product of few tokens keep the whole chip busy; two kernels share
-//     this order, one for few tokens (bound by the weights' way in) and one for many (bound by
-//     the FMA pipes).
+//     ascending, and the sums are added in order.  The parts are what lets a product of few tokens
+//     keep the whole chip busy; two kernels share this order, one for few tokens (bound by the
+//     weights' way in) and one for many (bound by the FMA pipes).
 //   * anything else: k ascending over the whole row, the kernel for all sizes.
 //
 // Epilogues (the reference's are src/backend/cuda/k_gemm.cu:29-53):
@@ -378,9 +378,12 @@ int launch_f32(Kernel kernel, dim3 grid, int threads, size_t smem, cudaStream_t 
     return check_launch("gemm_f32");
 }
 
-// Up to this many tokens the weights' way in is what a product waits for, even when two blocks read them (17 to 32
-// tokens, the second from the L2): a 64-token tile would be more than half padding.
-constexpr int FEW_TOKENS = 32;
+// Up to 16 tokens the kernel for few; 17 to 32, where two of its blocks read the same weights, while the tiles of 64 columns
+// of the other one (of 32 tokens: one row of them) are fewer than half the SMs.  us at 17 and 32 tokens, few / many:
+//   N x K   1,024 x 2,048  19 / 38  17 / 37     1,024 x 3,072  26 / 50  24 / 52     2,048 x 2,048  26 / 35  25 / 36
+//           4,096 x 1,024  29 / 24  28 / 25     6,144 x 1,024  23 / 20  22 / 20    12,288 x 2,048  77 / 68  76 / 70
+//         151,936 x 1,024  432 / 303  426 / 317
+constexpr int FEW_TOKENS = 32, FEW_TOKENS_WIDE = 16, WIDE_COLUMNS = 4096;
 
 template <int MT>
 int launch_few(const float* A, int lda, const float* W, int ldw, const float* bias, float* C, int ldc, int M, int N, int K, int epi,
@@ -398,7 +401,7 @@ int launch_pieces(const float* A, int lda, const float* W, int ldw, const float*
     if (M <= 2) return launch_few<2>(A, lda, W, ldw, bias, C, ldc, M, N, K, epi, settled, st);
     if (M <= 4) return launch_few<4>(A, lda, W, ldw, bias, C, ldc, M, N, K, epi, settled, st);
     if (M <= 8) return launch_few<8>(A, lda, W, ldw, bias, C, ldc, M, N, K, epi, settled, st);
-    if (M <= FEW_TOKENS) return launch_few<16>(A, lda, W, ldw, bias, C, ldc, M, N, K, epi, settled, st);
+    if (M <= (N >= WIDE_COLUMNS ? FEW_TOKENS_WIDE : FEW_TOKENS)) return launch_few<16>(A, lda, W, ldw, bias, C, ldc, M, N, K, epi, settled, st);
     // a grid has at most 65,535 rows of blocks, half as many tokens here as the 64-row tiles of the general kernel take
     constexpr int ROWS = 65535 * MANY_M;
     for (long long m = 0; m < M; m += ROWS) {
