@@ -509,11 +509,21 @@ def gemm_tc_qkv_usable(x: torch.Tensor, w: torch.Tensor, bias, M: int, n_heads: 
 # 74.5 / 51.3 at 4,096 (below, the step is one or two tiles an SM and the longer epilogue has no next tile to
 # hide behind).
 QKV_FUSE_MIN_TOKENS = 512
-# Up to how many tokens the product in the orientation of few tokens does, and up to how many rows of weights it does so
-# beyond 64 tokens (more tiles than a cluster each finds SMs for).  Product + head kernel against the fused product, in a
-# graph, 16/8 heads, K = 2,048: 7.9 / 6.2 us at 8 tokens, 9.9 / 6.7 at 24, 13.1 / 10.3 at 64 (five parts), 17.8 / 16.5 at 128.
-QKV_FUSE_MAX_DECODE_TOKENS = 128
-QKV_FUSE_WIDE_ROWS = 8192
+# Whether the product in the orientation of few tokens does: up to 24 tokens always, beyond while its tiles of 128 rows leave
+# each other the SMs for enough parts of K (four and more; two parts are slower than atomics and a head kernel).  Fused /
+# product + head kernel, us in a graph, rows x K:
+#                4,096 x 2,048  6,144 x 4,096  7,168 x 5,120  8,192 x 4,096  8,192 x 6,144  10,240 x 5,120  10,240 x 8,192
+#     9 tokens     6.6 /  8.5    11.7 / 14.1    15.6 / 17.7    14.7 / 16.9    19.7 / 22.4     21.7 / 23.7     31.0 / 33.5
+#    24 tokens     7.1 / 10.3    12.0 / 15.2    15.8 / 19.6    17.8 / 18.9    24.3 / 24.1     23.6 / 24.9     34.9 / 34.5
+#    64 tokens     9.6 / 13.5    15.2 / 19.3    19.0 / 23.6    25.2 / 22.8    32.7 / 28.2     30.9 / 29.0     42.7 / 38.4
+#    65 tokens    11.1 / 14.2    22.5 / 19.7    25.5 / 24.4    23.6 / 23.5    30.2 / 28.8     39.6 / 29.7     55.7 / 39.3
+#   128 tokens    15.5 / 18.6    32.9 / 25.0    37.2 / 31.2    34.6 / 29.9    42.4 / 35.7     71.2 / 37.3     87.9 / 47.2
+QKV_FUSE_ROWS = ((24, 1 << 30), (64, 7168), (128, 4096))         # (up to so many tokens, up to so many rows)
+
+
+def qkv_fuse_few(M: int, rows: int) -> bool:
+    """Whether a step of ``M`` tokens against ``rows`` rows of weights finishes its heads in the product for few tokens."""
+    return any(M <= m and rows <= n for m, n in QKV_FUSE_ROWS)
 
 
 def rope_table(positions: torch.Tensor, inv_freq: torch.Tensor, T: int, out: torch.Tensor, stream: Optional[int] = None) -> None:

@@ -137,8 +137,7 @@ class Attention(Mixer):
         att = ctx.buf("attention.out", (mt, s.q_dim), rt.dtype)
         table = ctx.block_table(cache.group)
         rotates = self.inv_freq is not None and self.rotary > 0
-        few = T <= (ops.QKV_FUSE_MAX_DECODE_TOKENS if self.qkv.n <= ops.QKV_FUSE_WIDE_ROWS else 64)
-        if (self.FUSE_QKV and (T >= ops.QKV_FUSE_MIN_TOKENS or few) and
+        if (self.FUSE_QKV and (T >= ops.QKV_FUSE_MIN_TOKENS or ops.qkv_fuse_few(T, self.qkv.n)) and
                 ops.gemm_tc_qkv_usable(x, self.qkv.weight, self.qkv.bias, T, s.num_heads, s.num_kv_heads, s.head_dim,
                                        self.rotary if rotates else 0)):
             # norm, rotation and the cache write happen in the product's epilogue: a prompt portion rotates with
@@ -150,9 +149,9 @@ class Attention(Mixer):
                             stream=ctx.stream)
         elif (self.SUMS_TO_HEADS and 16 < T <= 128 and self.qkv.bias is None and ops.gemm_tc_usable(x, self.qkv.weight, self.qkv.bias, ops.EPI_STORE)
               and ops.qk_norm_rope_store_sums_usable(s.head_dim, self.rotary if rotates else 0, self.qkv.n)):
-            # 17 to 128 tokens where the product does not finish the heads (65 and more against more than 8,192 rows): it
-            # cuts K and adds its parts into a zeroed fp32 scratch; the head kernel reads the sums there (and clears
-            # them) instead of a bf16 copy that a pass of its own would have to make
+            # 17 to 128 tokens where the product does not finish the heads (many rows): it cuts K and adds its parts into a
+            # zeroed fp32 scratch; the head kernel reads the sums there (and clears them) instead of a bf16 copy that a
+            # pass of its own would have to make
             sums = ops.gemm_tc(x, self.qkv.weight, None, T, ops.EPI_SUMS, err=ctx.err, stream=ctx.stream)
             ops.qk_norm_rope_store_sums(sums, T, s.num_heads, s.num_kv_heads, self.q_norm_w, self.k_norm_w, s.qk_norm_eps,
                                         self.inv_freq if rotates else None, ctx.positions, ctx.seq_of, table,

@@ -24,3 +24,9 @@ def test_whole_numbers_arrive(value):
 def test_early_reads_are_asked_for(op, name):
     """A kernel reads ahead of the kernel before it only where its caller says that it may."""
     assert inspect.signature(getattr(ops, op)).parameters[name].default is False
+
+
+@pytest.mark.parametrize("tokens,rows,fused", [(1, 14336, True), (24, 14336, True), (25, 7168, True), (25, 7296, False), (64, 7168, True), (65, 7168, False),
+                                               (65, 4096, True), (128, 4096, True), (128, 4224, False), (129, 4096, False)])
+def test_where_the_product_finishes_the_heads(tokens, rows, fused):
+    assert ops.qkv_fuse_few(tokens, rows) is fused
