@@ -131,6 +131,25 @@ static void best_tile_and_parts(int M, int N, int num_k_blocks, int slots, int u
     }
 }
 
+// Whether pairs of SMs are the faster kernel for 512 to 2,047 tokens against a large matrix (40 million weights and more).
+// Pairs read half of the weight tile each but compute rows in pieces of 256, so it is the last row tile and the last wave
+// that decide: the time of a wave is modelled as k_blocks (a cols + b) + c us with a, b and c fitted to 144 measured
+// products (nine matrices from 10,240 x 4,096 to 151,936 x 2,048, 16 numbers of tokens each) for either kernel.  The choice is
+// within 0.4 % of the better kernel on average and at most 3 % off; pairs throughout were up to 24 % off (us, one SM / pairs:
+// 24,576 x 4,096 gated: 560 tokens 109 / 105, 769 tokens 148 / 165, 1,000 tokens 174 / 164; 51,200 x 5,120 gated: 513 tokens 295 / 345,
+// 768 tokens 355 / 319; 4,096 x 12,288 added: 560 tokens 71 / 65, 1,025 tokens 90 / 112).
+static bool pairs_are_faster(int M, int N, int num_k_blocks, bool adds, int num_sms, int max_pairs) {
+    auto us = [&](int slots, int units, double a, double b, double c) {
+        int cols = 0, parts = 1;
+        if (adds) best_tile_and_parts(M, N, num_k_blocks, slots, units, &cols, &parts);
+        else cols = best_block_cols(M, N, slots, units, nullptr);
+        const int rows = TILE_ROWS * units, kb = (num_k_blocks + parts - 1) / parts;
+        const long long n = (long long)((M + rows - 1) / rows) * ((N + cols - 1) / cols) * ((num_k_blocks + kb - 1) / kb);
+        return (double)((n + slots - 1) / slots) * (kb * (a * cols + b) + c);
+    };
+    return us(max_pairs, 2, 0.000875, 0.1874, 2.3) <= us(num_sms, 1, 0.00121, 0.1345, 3.8);
+}
+
 // A cluster's partial sums in shared memory: every block receives its share of the token columns from all of them.
 static size_t cluster_recv_bytes(const GemmTcParams& p) {
     if (p.cluster_splits <= 1 && p.epilogue != 4) return 0;
@@ -393,9 +412,8 @@ EMBER_API int ember_gemm_tc(const void* A, const void* W, void* out, int ldc, in
         // Prefill-sized products: the single-SM persistent kernel or pairs of SMs (tcgen05 cta_group::2),
         // each with the tile width that fills its waves best.  Under the power cap pairs are the more efficient
         // kernel (an SM reads half of the weight tile) and win from about 2,048 tokens on (a 2,048-token prefill
-        // step: 7.55 ms with pairs, 7.9 ms without; at 1,024 tokens the single-SM kernel is 1 % ahead), and from 512 on
-        // for matrices of 40 million weights and more (N 24,576 x K 4,096 gated, us single / pairs: 560 tokens 115 / 113,
-        // 1,024 tokens 164 / 155; N 4,096 x K 12,288 added: 560 tokens 64 / 59; 300 tokens 71 / 80).
+        // step: 7.55 ms with pairs, 7.9 ms without; at 1,024 tokens the single-SM kernel is 1 % ahead); from 512 on
+        // pairs_are_faster says where they do for large matrices (300 tokens, N 4,096 x K 12,288 added: 71 / 80 us).
         // split_mode 4 asks for pairs whenever the device takes them, 5 forbids them, 3 runs one tile per block.
         double cost_single = 0, cost_pair = 0;
         const int bc_single = split_mode == 3 ? (N >= 1024 ? 256 : 128) : best_block_cols(M, N, num_sms, 1, &cost_single);
@@ -404,7 +422,8 @@ EMBER_API int ember_gemm_tc(const void* A, const void* W, void* out, int ldc, in
             if (max_pairs > 0) {
                 const int bc_pair = best_block_cols(M, N, max_pairs, 2, &cost_pair);
                 if (split_mode == 4 || (M >= 2048 && cost_pair <= cost_single * 1.001) ||
-                    (M >= 512 && M < 2048 && (long long)N * K >= 40000000ll)) {
+                    (M >= 512 && M < 2048 && (long long)N * K >= 40000000ll &&
+                     pairs_are_faster(M, N, p.num_k_blocks, epilogue == 2, num_sms, max_pairs))) {
                     p.epilogue = epilogue; p.out = out; p.ldc = ldc; p.err = err;
                     p.accum = nullptr; p.accum_ld = 0; p.stages = 0;
                     return launch_pair(A, W, p, bc_pair, max_pairs, st);
