@@ -223,7 +223,8 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
     // still runs: a layer's attention took 9.9, 25.1 and 43.9 us (one request at 700 keys, 8 at 3,072, 64 at 1,024), now 8.3,
     // 23.4, 39.1.
     int early = 0;
-    if (DECODE && p.settled && warp == 4) {
+    if (DECODE && warp == 4) {
+        if (!p.settled) pdl_wait();
         early = min(min(n_kt, NSTAGE), max(0, (pos0 - k_begin) / KT));
         for (int it = 0; it < early; it++) fetch_tile(it, page_row(it));
     }

@@ -201,18 +201,14 @@ gemm_f32_few_kernel(const float* __restrict__ A, int lda, const float* __restric
             if (r < WP * MT) copy16(dst + r * FEW_K + piece, ok ? A + (size_t)m * lda + k : A, ok);
         }
     };
-    if (settled) {
+    if (!settled) pdl_wait();
 #pragma unroll
-        for (int s = 0; s < FEW_STAGES - 1; s++)
-            if (s < steps) fetch_w(s);
-    }
+    for (int s = 0; s < FEW_STAGES - 1; s++)
+        if (s < steps) fetch_w(s);
     pdl_wait();
 #pragma unroll
     for (int s = 0; s < FEW_STAGES - 1; s++) {
-        if (s < steps) {
-            if (!settled) fetch_w(s);
-            fetch_a(s);
-        }
+        if (s < steps) fetch_a(s);
         copies_commit();
     }
 
@@ -305,9 +301,9 @@ gemm_f32_many_kernel(const float* __restrict__ A, int lda, const float* __restri
             copy16(dst + r * MANY_ROW + piece, ok ? A + (size_t)(m0 + r) * lda + k : A, ok);
         }
     };
-    if (settled) fetch_w(0);
+    if (!settled) pdl_wait();
+    fetch_w(0);
     pdl_wait();
-    if (!settled) fetch_w(0);
     fetch_a(0);
     copies_commit();
 
