@@ -199,16 +199,22 @@ static cudaError_t raise_smem_limit() {
 //   128 tokens        18.4 ->  9.6 [4]      11.5 -> 9.1 [6]      14.6 -> 13.4 [6]     24.7 <- 30.0 [2]      25.4 -> 19.6 [2]
 // (added 4,096 x 12,288 at 128 tokens: 27.7 <- 31.3 [4]; what atomics cost is their traffic, 0.06 us a token at N = 2,048,
 // 1.07 TB/s at the L2.)
-static int cluster_parts(const GemmTcParams& p, int tiles) {
+// Two parts are too few for what is added (5,120 x 5,120 at 65 / 128 tokens: 16.0 / 19.9 <- 20.3 / 26.6), and on tiles that
+// leave no SM a second block, for long K (stored 10,240 x 5,120 at 65 tokens: 31.5 <- 33.2); added sums of very long K stay
+// with atomics (5,120 x 17,408 at 48 tokens: 32.8 <- 34.1).  The numbers of blocks are those of the 148 SMs that they were
+// measured on.
+static int cluster_parts(const GemmTcParams& p, int tiles, int num_sms) {
     static const int choices[] = {8, 6, 5, 4, 2};
+    auto blocks = [&](int n) { return n * num_sms / 148; };
     const bool small = p.block_cols <= 64;
-    if (!small && p.epilogue == 2 && p.num_k_blocks >= 128) return 0;
+    if (p.epilogue == 2 && p.num_k_blocks >= (small ? 256 : 128)) return 0;
     for (int s : choices) {
         const int most = small ? (p.num_k_blocks >= 128 ? 256 : 240) : (s == 8 ? 64 : (s == 5 ? 0 : 128));
         const int per = (p.num_k_blocks + s - 1) / s;
-        if (tiles * s <= most && per >= 2 && (p.num_k_blocks + per - 1) / per == s) return s;
+        if (!small && p.epilogue == 2 && s == 2) return 0;
+        if (tiles * s <= blocks(most) && per >= 2 && (p.num_k_blocks + per - 1) / per == s) return s;
     }
-    if (!small && p.block_cols <= 96 && tiles <= 120 && p.num_k_blocks >= 4) return 2;
+    if (!small && p.block_cols <= 96 && tiles <= blocks(120) && p.num_k_blocks < 64 && p.num_k_blocks >= 4) return 2;
     return small && p.epilogue != 2 ? 1 : 0;
 }
 
@@ -451,7 +457,7 @@ EMBER_API int ember_gemm_tc(const void* A, const void* W, void* out, int ldc, in
     const bool store_epilogue = epilogue != 2;
     p.epilogue = epilogue;
     const bool wide = p.swapped && p.block_cols > 16;
-    const int parts = wide && (split_mode == 0 || split_mode == 2) && !sums ? cluster_parts(p, tiles) : 0;
+    const int parts = wide && (split_mode == 0 || split_mode == 2) && !sums ? cluster_parts(p, tiles, num_sms) : 0;
     const bool use_cluster = p.swapped && (split_mode == 2 || split_mode >= 32 || (split_mode == 0 && (wide ? parts > 0 : store_epilogue)));
     int splits = 1;
     if (p.swapped && use_cluster && split_mode >= 32) {
@@ -591,7 +597,7 @@ static int launch_heads_swapped(const void* A, const void* W, GemmTcParams p, in
     const int tiles = p.N / TILE_ROWS;
     int splits = 1;
     if (p.block_cols > 16) {
-        const int parts = cluster_parts(p, tiles);
+        const int parts = cluster_parts(p, tiles, num_sms);
         splits = parts > 0 ? parts : 1;
     } else if (tiles < num_sms) {
         splits = (num_sms + tiles - 1) / tiles;
