@@ -829,3 +829,35 @@ def test_float32_product_behind_the_kernel_that_writes_its_weights(M):
         ops.gemm_simt(a, w, settled, M, 1, weights_settled=True)
         assert torch.equal(got, settled)
         assert rel(got, a.double() @ w.double().t()) < 2e-6
+
+
+@pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("heads,kv,D", [(4, 2, 4), (6, 1, 36), (16, 8, 128), (4, 4, 132), (5, 1, 144), (2, 1, 192), (32, 1, 252), (2, 1, 256)])
+@pytest.mark.parametrize("window,splits", [(0, 1), (37, 1), (0, 4)])
+def test_attention_general_kernels_have_the_same_bits(dt, heads, kv, D, window, splits):
+    """Whole pieces of four elements at aligned addresses against the kernel for anything (queries that begin one element
+    later): portions that do not fill the warps, single tokens, a page that is not there."""
+    from ember_b200 import ops
+    torch.manual_seed(heads + D + window)
+    page, runs = 16, [(300, 33), (45, 45), (1, 1), (501, 1)]                       # keys after the step, new tokens of it
+    T, width = sum(n for _, n in runs), (501 + page - 1) // page
+    pages = len(runs) * width
+    kp = torch.randn(pages, kv, page, D, device="cuda").to(dt)
+    vp = torch.randn(pages, kv, page, D, device="cuda").to(dt)
+    table = torch.randperm(pages).view(len(runs), width).int()
+    table[3, 20] = pages + 7
+    table = table.cuda()
+    tile_q, tiles, row = ops.attention_tile_queries(heads // kv), [], 0
+    for r, (keys, n) in enumerate(runs):
+        tiles += [[r, row + i, min(tile_q, n - i), keys - n + i] for i in range(0, n, tile_q)]
+        row += n
+    tiles = torch.tensor(tiles, dtype=torch.int32, device="cuda")
+    store = torch.randn(T * heads * D + 1, device="cuda").to(dt)
+    odd = store[1:].view(T, heads * D)
+    outs = []
+    for q in (odd, odd.clone()):
+        out, err = torch.zeros(T, heads * D, device="cuda", dtype=dt), torch.zeros(1, dtype=torch.int32, device="cuda")
+        parts = (torch.zeros(T * heads * splits * D, device="cuda"), torch.zeros(T * heads * splits * 2, device="cuda")) if splits > 1 else (None, None)
+        ops.attention(q, kp, vp, out, T, heads, kv, D, tiles, tiles.shape[0], tile_q, table, page, window, D ** -0.5, splits, 128, *parts, err=err)
+        outs.append((out, int(err.item())))
+    assert odd.data_ptr() % 16 and torch.equal(outs[0][0], outs[1][0]) and outs[0][1] == outs[1][1]

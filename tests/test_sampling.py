@@ -106,3 +106,22 @@ def test_device_sampler_small_top_k(vocab, kind):
     counters = [3 + 7 * r for r in range(rows)]
     got = device.sample(torch.from_numpy(logits).cuda(), params, counters).cpu().tolist()
     assert got == [sample_host(logits[r], params[r], counters[r]) for r in range(rows)]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("vocab", [8192, 8195, 151936])
+@pytest.mark.parametrize("where", ["first", "middle", "last"])
+def test_device_sampler_small_top_k_beside_a_nan(vocab, where):
+    """A NaN sends its row, and no other, from the groups of threads to the selection over the whole row (where a draw means
+    nothing): the call ends, and the rows beside it draw what the host draws."""
+    import torch
+    from ember_b200.sampling import device
+    rng = np.random.default_rng(vocab)
+    rows, at = 6, {"first": 0, "middle": vocab // 2 + 1, "last": vocab - 1}[where]
+    logits = (rng.standard_normal((rows, vocab)) * 3).astype(np.float32)
+    logits[[1, 4], at] = np.nan
+    params = [SamplingParams(temperature=0.7, top_k=[20, 1, 300][r % 3], top_p=[1.0, 0.9][r % 2], seed=5 + r) for r in range(rows)]
+    counters = [9 + r for r in range(rows)]
+    got = device.sample(torch.from_numpy(logits).cuda(), params, counters).cpu().tolist()
+    for r in (0, 2, 3, 5):
+        assert got[r] == sample_host(logits[r], params[r], counters[r])
