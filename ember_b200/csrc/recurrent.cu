@@ -686,73 +686,72 @@ __device__ __forceinline__ float4 scan_scalars(const ScanArgs& p, float s0, floa
 // beside its sum over the eight row groups.
 template <int MODE, int RS, int C>
 __device__ __forceinline__ void scan_step(unsigned long long (&st)[C][RS / 2], const TokenRegs<RS / 4, C>& x, float (&o)[C], float (&add)[C]) {
-    constexpr int NV = (MODE == 0 || MODE == 3 || MODE == 4) ? 3 : 2;
-    (void)NV;
-                if (MODE == 0) {
-                    unsigned long long ak[C][2], aq[C][2];
+    [[maybe_unused]] constexpr int NV = (MODE == 0 || MODE == 3 || MODE == 4) ? 3 : 2;
+    if (MODE == 0) {
+        unsigned long long ak[C][2], aq[C][2];
 #pragma unroll
-                    for (int c = 0; c < C; c++) ak[c][0] = ak[c][1] = aq[c][0] = aq[c][1] = 0;
+        for (int c = 0; c < C; c++) ak[c][0] = ak[c][1] = aq[c][0] = aq[c][1] = 0;
 #pragma unroll
-                    for (int i4 = 0; i4 < RS / 4; i4++)
+        for (int i4 = 0; i4 < RS / 4; i4++)
 #pragma unroll
-                        for (int c = 0; c < C; c++) {
-                            st[c][2 * i4] = pair_mul(st[c][2 * i4], x.v2[i4].x);
-                            st[c][2 * i4 + 1] = pair_mul(st[c][2 * i4 + 1], x.v2[i4].y);
-                            ak[c][0] = pair_fma(st[c][2 * i4], x.v0[i4].x, ak[c][0]);
-                            ak[c][1] = pair_fma(st[c][2 * i4 + 1], x.v0[i4].y, ak[c][1]);
-                        }
-                    float sk[C];
+            for (int c = 0; c < C; c++) {
+                st[c][2 * i4] = pair_mul(st[c][2 * i4], x.v2[i4].x);
+                st[c][2 * i4 + 1] = pair_mul(st[c][2 * i4 + 1], x.v2[i4].y);
+                ak[c][0] = pair_fma(st[c][2 * i4], x.v0[i4].x, ak[c][0]);
+                ak[c][1] = pair_fma(st[c][2 * i4 + 1], x.v0[i4].y, ak[c][1]);
+            }
+        float sk[C];
 #pragma unroll
-                    for (int c = 0; c < C; c++) sk[c] = (pair_lo(ak[c][0]) + pair_hi(ak[c][0])) + (pair_lo(ak[c][1]) + pair_hi(ak[c][1]));
+        for (int c = 0; c < C; c++) sk[c] = (pair_lo(ak[c][0]) + pair_hi(ak[c][0])) + (pair_lo(ak[c][1]) + pair_hi(ak[c][1]));
 #pragma unroll
-                    for (int off = 1; off < RG; off <<= 1)
+        for (int off = 1; off < RG; off <<= 1)
 #pragma unroll
-                        for (int c = 0; c < C; c++) sk[c] += __shfl_xor_sync(0xffffffffu, sk[c], off);
-                    // (while the shuffles are under way)
+            for (int c = 0; c < C; c++) sk[c] += __shfl_xor_sync(0xffffffffu, sk[c], off);
+        // (while the shuffles are under way)
 #pragma unroll
-                    for (int i4 = 0; i4 < RS / 4; i4++)
+        for (int i4 = 0; i4 < RS / 4; i4++)
 #pragma unroll
-                        for (int c = 0; c < C; c++) {
-                            aq[c][0] = pair_fma(st[c][2 * i4], x.v1[i4].x, aq[c][0]);
-                            aq[c][1] = pair_fma(st[c][2 * i4 + 1], x.v1[i4].y, aq[c][1]);
-                        }
+            for (int c = 0; c < C; c++) {
+                aq[c][0] = pair_fma(st[c][2 * i4], x.v1[i4].x, aq[c][0]);
+                aq[c][1] = pair_fma(st[c][2 * i4 + 1], x.v1[i4].y, aq[c][1]);
+            }
 #pragma unroll
-                    for (int c = 0; c < C; c++) {
-                        o[c] = (pair_lo(aq[c][0]) + pair_hi(aq[c][0])) + (pair_lo(aq[c][1]) + pair_hi(aq[c][1]));
-                        const float uk = x.sc.w * (x.val[c] - sk[c] * x.sc.x) * x.sc.x;      // beta (v - S^T k) / |k|
-                        add[c] = uk;
-                        const unsigned long long u2 = pair_of(uk, uk);
+        for (int c = 0; c < C; c++) {
+            o[c] = (pair_lo(aq[c][0]) + pair_hi(aq[c][0])) + (pair_lo(aq[c][1]) + pair_hi(aq[c][1]));
+            const float uk = x.sc.w * (x.val[c] - sk[c] * x.sc.x) * x.sc.x;      // beta (v - S^T k) / |k|
+            add[c] = uk;
+            const unsigned long long u2 = pair_of(uk, uk);
 #pragma unroll
-                        for (int i4 = 0; i4 < RS / 4; i4++) {
-                            st[c][2 * i4] = pair_fma(x.v0[i4].x, u2, st[c][2 * i4]);
-                            st[c][2 * i4 + 1] = pair_fma(x.v0[i4].y, u2, st[c][2 * i4 + 1]);
-                        }
-                    }
-                } else {
-                    // S <- keep S + k v^T with a decay per row (3, 4) or per token (1, 2), read before (4) or behind
+            for (int i4 = 0; i4 < RS / 4; i4++) {
+                st[c][2 * i4] = pair_fma(x.v0[i4].x, u2, st[c][2 * i4]);
+                st[c][2 * i4 + 1] = pair_fma(x.v0[i4].y, u2, st[c][2 * i4 + 1]);
+            }
+        }
+    } else {
+        // S <- keep S + k v^T with a decay per row (3, 4) or per token (1, 2), read before (4) or behind
 #pragma unroll
-                    for (int c = 0; c < C; c++) {
-                        const float put = (MODE == 1 || MODE == 2) ? x.sc.y * x.val[c] : x.val[c];              // put v | dt x
-                        const unsigned long long put2 = pair_of(put, put), keep2 = pair_of(x.sc.x, x.sc.x);
-                        unsigned long long a0 = 0, a1 = 0;
+        for (int c = 0; c < C; c++) {
+            const float put = (MODE == 1 || MODE == 2) ? x.sc.y * x.val[c] : x.val[c];              // put v | dt x
+            const unsigned long long put2 = pair_of(put, put), keep2 = pair_of(x.sc.x, x.sc.x);
+            unsigned long long a0 = 0, a1 = 0;
 #pragma unroll
-                        for (int i4 = 0; i4 < RS / 4; i4++) {
-                            const unsigned long long g0 = NV == 3 ? x.v2[i4].x : keep2, g1 = NV == 3 ? x.v2[i4].y : keep2;
-                            if (MODE == 4) {
-                                a0 = pair_fma(st[c][2 * i4], x.v1[i4].x, a0);
-                                a1 = pair_fma(st[c][2 * i4 + 1], x.v1[i4].y, a1);
-                            }
-                            st[c][2 * i4] = pair_fma(x.v0[i4].x, put2, pair_mul(g0, st[c][2 * i4]));
-                            st[c][2 * i4 + 1] = pair_fma(x.v0[i4].y, put2, pair_mul(g1, st[c][2 * i4 + 1]));
-                            if (MODE != 4) {
-                                a0 = pair_fma(st[c][2 * i4], x.v1[i4].x, a0);
-                                a1 = pair_fma(st[c][2 * i4 + 1], x.v1[i4].y, a1);
-                            }
-                        }
-                        o[c] = (pair_lo(a0) + pair_hi(a0)) + (pair_lo(a1) + pair_hi(a1));
-                        add[c] = x.val[c];
-                    }
+            for (int i4 = 0; i4 < RS / 4; i4++) {
+                const unsigned long long g0 = NV == 3 ? x.v2[i4].x : keep2, g1 = NV == 3 ? x.v2[i4].y : keep2;
+                if (MODE == 4) {
+                    a0 = pair_fma(st[c][2 * i4], x.v1[i4].x, a0);
+                    a1 = pair_fma(st[c][2 * i4 + 1], x.v1[i4].y, a1);
                 }
+                st[c][2 * i4] = pair_fma(x.v0[i4].x, put2, pair_mul(g0, st[c][2 * i4]));
+                st[c][2 * i4 + 1] = pair_fma(x.v0[i4].y, put2, pair_mul(g1, st[c][2 * i4 + 1]));
+                if (MODE != 4) {
+                    a0 = pair_fma(st[c][2 * i4], x.v1[i4].x, a0);
+                    a1 = pair_fma(st[c][2 * i4 + 1], x.v1[i4].y, a1);
+                }
+            }
+            o[c] = (pair_lo(a0) + pair_hi(a0)) + (pair_lo(a1) + pair_hi(a1));
+            add[c] = x.val[c];
+        }
+    }
 }
 template <int MODE>
 __device__ __forceinline__ float scan_finish(const float4& sc, float skip, float sum, float add) {
@@ -1009,8 +1008,12 @@ __global__ void __launch_bounds__(32 * (NCW + PORTION_PREPARE), RS == 4 ? 2 : 1)
 // One token a run.  A thread asks for its rows of the state first (C neighbouring columns, so that a warp's request is
 // whole 32-byte pieces of eight rows); while they travel the block prepares the token's vectors, an element a thread;
 // then the step, and the columns go back.  The state passes through no shared memory.  24 runs, 16 heads of 128 x 128,
-// delta rule (50 MB in and out): blocks of 256 threads that passed the state through shared memory, one warp of which
-// prepared the token, took 29 us a step, these 20.
+// delta rule (50 MB in and out), in a step: blocks of 256 threads that passed the state through shared memory, one warp
+// of which prepared the token, took 29 us, these 20.  From cold, us before -> now, 24 runs:
+//   rows x columns, heads     delta rule      gated linear attention   time mixing
+//    64 x  64, 32           22.5 -> 18.4         20.5 -> 16.5         20.5 -> 17.4
+//   128 x 128, 16           35.8 -> 28.6         30.7 -> 26.5         31.7 -> 24.5
+//   256 x 256,  8           97.2 -> 68.4         74.7 -> 65.5         74.7 -> 61.4
 constexpr int SINGLE_WARPS = 4;
 
 template <int MODE, int RS, int C>
