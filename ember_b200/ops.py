@@ -518,12 +518,9 @@ QKV_FUSE_MIN_TOKENS = 512
 #    64 tokens     9.6 / 13.5    15.2 / 19.3    19.0 / 23.6    25.2 / 22.8    32.7 / 28.2     30.9 / 29.0     42.7 / 38.4
 #    65 tokens    11.1 / 14.2    22.5 / 19.7    25.5 / 24.4    23.6 / 23.5    30.2 / 28.8     39.6 / 29.7     55.7 / 39.3
 #   128 tokens    15.5 / 18.6    32.9 / 25.0    37.2 / 31.2    34.6 / 29.9    42.4 / 35.7     71.2 / 37.3     87.9 / 47.2
-QKV_FUSE_ROWS = ((24, 1 << 30), (64, 7168), (128, 4096))         # (up to so many tokens, up to so many rows)
-
-
 def qkv_fuse_few(M: int, rows: int) -> bool:
     """Whether a step of ``M`` tokens against ``rows`` rows of weights finishes its heads in the product for few tokens."""
-    return any(M <= m and rows <= n for m, n in QKV_FUSE_ROWS)
+    return M <= 24 or (M <= 64 and rows <= 7168) or (M <= 128 and rows <= 4096)
 
 
 def rope_table(positions: torch.Tensor, inv_freq: torch.Tensor, T: int, out: torch.Tensor, stream: Optional[int] = None) -> None:
@@ -746,7 +743,11 @@ def gated_norm_add(y: torch.Tensor, gate_logits: Optional[torch.Tensor], weight:
 def gated_norm_add_norm_usable(width: int, *vectors: Optional[torch.Tensor]) -> bool:
     """Whether ``gated_norm_add_norm`` takes rows of this width (the rule of ember_gated_norm_add_norm_supported) under these
     weights and biases, which it reads 16 bytes at a time."""
-    return width % 4 == 0 and 0 < width <= 8192 and all(t is None or t.data_ptr() % 16 == 0 for t in vectors)
+    addresses = width << 2                           # (a width that is no multiple of four shows in the low bits as well)
+    for t in vectors:
+        if t is not None:
+            addresses |= t.data_ptr()
+    return addresses & 15 == 0 and 0 < width <= 8192
 
 
 def gated_norm_add_norm(y: torch.Tensor, gate_logits: Optional[torch.Tensor], gate_bias: Optional[torch.Tensor], w: torch.Tensor,

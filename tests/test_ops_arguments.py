@@ -30,3 +30,11 @@ def test_early_reads_are_asked_for(op, name):
                                                (65, 4096, True), (128, 4096, True), (128, 4224, False), (129, 4096, False)])
 def test_where_the_product_finishes_the_heads(tokens, rows, fused):
     assert ops.qkv_fuse_few(tokens, rows) is fused
+
+
+def test_where_gate_norm_and_norm_are_one_kernel():
+    whole, odd = torch.zeros(9)[:8], torch.zeros(9)[1:]
+    assert whole.data_ptr() % 16 == 0
+    assert ops.gated_norm_add_norm_usable(8192, None, whole, None, whole)
+    assert not ops.gated_norm_add_norm_usable(2048, whole, odd)
+    assert not any(ops.gated_norm_add_norm_usable(w, whole) for w in (0, 2, 2050, 8196))
