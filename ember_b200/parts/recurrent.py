@@ -9,10 +9,10 @@
 * "mamba1":        selective scan with a diagonal state per channel (a step, a B and a C per token).
 
 All of them project their input with one fused product whose fp32 result the recurrence kernel reads in place (column
-offsets, no copies), run the same kernels for prompt portions and single tokens (a block walks its run's tokens in
-order, so the state after a step does not depend on how the tokens were cut), normalise each head's read-out in
-fp32 and end in an output product that stores into, or adds into, an fp32 [T, hidden] buffer.  A short causal
-convolution's last inputs are part of the state.
+offsets, no copies), add everything in the same order for prompt portions and single tokens (a block walks its run's
+tokens in order, so the state after a step does not depend on how the tokens were cut; the last bits of "mlstm" do,
+whose gates are summed 32 tokens at a time), normalise each head's read-out in fp32 and end in an output product that
+stores into, or adds into, an fp32 [T, hidden] buffer.  A short causal convolution's last inputs are part of the state.
 """
 from __future__ import annotations
 
