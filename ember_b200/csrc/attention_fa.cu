@@ -4,13 +4,8 @@
 //
 // One block handles 128 query rows -- (token, head-of-group) pairs, so the heads of a group share
 // every key tile -- of one key/value head and walks the key tiles of 64 keys up to the causal
-// diagonal:
-//   warp 0      fetches key and value pages by TMA (one box per page and 64-wide half, 128-byte
-//               swizzle) into two rings: a key tile is free once S = Q K^T has read it, its values
-//               only after O += P V, so keys (two stages) run as far ahead as values (three);
-//   warp 1      issues tcgen05.mma: S_j = Q K_j^T (128 x 64, accumulator in tensor memory, two
-//               buffers) and O_j = P_j V_j (128 x 128, V read MN-major straight from the page layout);
-//   warps 2-5   own one query row per thread: they read S_j from tensor memory (tcgen05.ld), keep
+// diagonal, two blocks to an SM:
+//   warps 0-3   own one query row per thread: they read S_j from tensor memory (tcgen05.ld), keep
 //               the reference maximum and the denominator, and write P_j = exp2(S_j - max) as packed
 //               bf16 back into the tensor-memory columns S_j came from; the second product takes P
 //               straight from tensor memory (A operand) and accumulates O in tensor memory.
@@ -18,11 +13,20 @@
 //               more than 8 (a factor 256, harmless in bf16 and fp32); then the row of O is rescaled
 //               in tensor memory (tcgen05.ld / tcgen05.st).  After the first tiles this is rare, so O
 //               stays in tensor memory and the output registers are only filled at the end.
-// S_{j+1} is multiplied while the rows of S_j are being exponentiated.  What bounds a tile is the
-// issuing thread (a tcgen05.mma costs it about 60 cycles, a wait that passes at once 100, twelve
-// instructions and four commits a tile) and the chain S visible -> exponentials -> P ready -> O += P V;
-// measured per 64-key tile: 2,200 cycles, of which the softmax warps work 960.  Every wait is bounded
-// (EMBER_ERR_WAIT_LIMIT) and the tensor memory is freed on every path.
+//   warp 4      fetches key and value pages by TMA (one box per page and 64-wide half, 128-byte
+//               swizzle) into two rings: a key tile is free once S = Q K^T has read it, its values
+//               only after O += P V, so keys (two stages) run as far ahead as values (three);
+//   warp 5      issues S_j = Q K_j^T (128 x 64, two buffers in tensor memory);
+//   warp 6      issues O += P_j V_j (128 x 128, V read MN-major straight from the page layout).
+// S_{j+1} is multiplied while the rows of S_j are being exponentiated.  The two issuing warps go through their loops whole
+// and elect the lane that issues (common.cuh); with one thread, found by its lane number, issuing both products, that thread
+// was what bounded a tile.  Cycles a tile of 64 keys with both blocks of an SM at work, measured on a form with both in one
+// block: one thread a block 1,970, elected 1,560, a warp for each product 1,450, of which a row's thread waits 180, takes the
+// maximum in 290, the exponents in 870 (2 x 64 of them on each of the four special-function units are 1,024) and hands over
+// in 80; the tensor pipe needs 1,280 for the two blocks' tiles.
+// us, before -> now: 61 tokens of 16/8 heads 6.1 -> 5.8, 601 tokens 15.2 -> 11.5, 2,048 tokens 40 -> 33, 2,048 behind 8,192
+// more keys 171 -> 142 (1,090 TFLOP/s), 2,048 tokens of 32/8 heads 62 -> 40.
+// Every wait is bounded (EMBER_ERR_WAIT_LIMIT) and the tensor memory is freed on every path.
 //
 // The reference's prefill attention (src/backend/cuda/k_attention.cu:214-370) is a Turing
 // mma.sync kernel; only the mathematics is shared.
@@ -44,7 +48,9 @@ constexpr int FA_D = 128;             // head size
 constexpr int FA_K_STAGES = 2;        // key tiles in flight or in use (a key tile is free once S = Q K^T has read it,
                                       // two tiles before its values are: two stages look as far ahead as three of values)
 constexpr int FA_V_STAGES = 3;        // value tiles (free once O += P V has read them)
-constexpr int FA_THREADS = 192;
+constexpr int FA_ROW_WARPS = 4;
+constexpr int FA_THREADS = 32 * (FA_ROW_WARPS + 3);
+constexpr size_t FA_SMEM = (size_t)2 * FA_ROWS * 128 + (size_t)(FA_K_STAGES + FA_V_STAGES) * 2 * FA_KT * 128 + 256;
 constexpr float FA_LOG2E = 1.4426950408889634f;
 
 struct FaParams {
@@ -216,6 +222,79 @@ __device__ __forceinline__ void fa_capped_small(const FaParams& p, float& s0, fl
 }
 __device__ __forceinline__ uint32_t fa_swz(int row, int chunk) { return (uint32_t)(row * 128 + ((chunk ^ (row & 7)) << 4)); }
 
+__device__ __forceinline__ float fa_max3(float a, float b, float c) {
+    float d;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+    return d;
+}
+__device__ __forceinline__ unsigned long long fa_add2(unsigned long long a, unsigned long long b) {
+    unsigned long long d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ void fa_unpk2(unsigned long long v, float& lo, float& hi) {
+    uint32_t a, b;
+    asm("mov.b64 {%0, %1}, %2;" : "=r"(a), "=r"(b) : "l"(v));
+    lo = __uint_as_float(a);
+    hi = __uint_as_float(b);
+}
+
+// A warp's 32 rows of O (lanes of tensor memory from ``tmem_o`` on) times their 1 / l, gated, to the output.  The gate's
+// logits and the results are rows of 512 and 256 bytes a (token, head): the rows are turned in shared memory (``turn``) so
+// that the lanes walk along a row.  The logits have been on their way into the L2 since before the first tile.
+__device__ __forceinline__ void fa_store_gated(const FaParams& p, uint32_t tmem_o, float* turn, float inv, bool ok, int quad, int lane,
+                                               int rows, int row0, int kvh, int G) {
+#pragma unroll
+    for (int c = 0; c < FA_D / 32; c++) {
+        uint32_t tu[32];
+        fa_tmem_ld32_nowait(tmem_o + (uint32_t)(c * 32), tu);
+        fa_tmem_wait_ld();
+        if (ok) {
+#pragma unroll
+            for (int e = 0; e < 32; e += 4)
+                *reinterpret_cast<float4*>(turn + lane * (FA_D + 4) + c * 32 + e) =
+                    make_float4(__uint_as_float(tu[e]) * inv, __uint_as_float(tu[e + 1]) * inv, __uint_as_float(tu[e + 2]) * inv,
+                                __uint_as_float(tu[e + 3]) * inv);
+        }
+    }
+    __syncwarp();
+    const int here = ok ? min(32, rows - quad * 32) : 0;
+#pragma unroll 8
+    for (int i = 0; i < here; i++) {
+        const int rr = quad * 32 + i, rq = rr / G, rg = rr - rq * G;
+        const size_t at = (size_t)(kvh * G + rg) * FA_D + 4 * lane;
+        const float4 g = __ldg(reinterpret_cast<const float4*>(p.gate + (size_t)(row0 + rq) * p.ld_gate + at));
+        const float4 v = *reinterpret_cast<const float4*>(turn + i * (FA_D + 4) + 4 * lane);
+        uint2 packed;
+        __nv_bfloat162 a = __floats2bfloat162_rn(v.x * __fdividef(1.0f, 1.0f + __expf(-g.x)), v.y * __fdividef(1.0f, 1.0f + __expf(-g.y)));
+        __nv_bfloat162 b = __floats2bfloat162_rn(v.z * __fdividef(1.0f, 1.0f + __expf(-g.z)), v.w * __fdividef(1.0f, 1.0f + __expf(-g.w)));
+        packed.x = *reinterpret_cast<uint32_t*>(&a);
+        packed.y = *reinterpret_cast<uint32_t*>(&b);
+        *reinterpret_cast<uint2*>(p.out + (size_t)(row0 + rq) * p.n_heads * FA_D + at) = packed;
+    }
+}
+// The same without a gate, a thread its row (``write`` false: nothing is written).
+__device__ __forceinline__ void fa_store_rows(const FaParams& p, uint32_t tmem_o, float inv, bool write, int token, int head) {
+    __nv_bfloat16* dst = p.out + ((size_t)token * p.n_heads + head) * FA_D;
+#pragma unroll
+    for (int c = 0; c < FA_D / 32; c++) {
+        uint32_t tu[32];
+        fa_tmem_ld32_nowait(tmem_o + (uint32_t)(c * 32), tu);
+        fa_tmem_wait_ld();
+        if (write) {
+#pragma unroll
+            for (int q4 = 0; q4 < 4; q4++) {
+                uint4 packed;
+                __nv_bfloat162* h2 = (__nv_bfloat162*)&packed;
+#pragma unroll
+                for (int e = 0; e < 4; e++)
+                    h2[e] = __floats2bfloat162_rn(__uint_as_float(tu[q4 * 8 + 2 * e]) * inv, __uint_as_float(tu[q4 * 8 + 2 * e + 1]) * inv);
+                *reinterpret_cast<uint4*>(dst + c * 32 + q4 * 8) = packed;
+            }
+        }
+    }
+}
+
 // CAP 0: no cap on the scores.  1: a cap of at most FA_PLAIN_CAP (in log2 units): exponents lie between its two ends, so
 // they are taken as they are, without a running maximum: e^cap and its sums stay far inside fp32's (and bf16's) range.
 // 2: a larger cap, with the running maximum.
@@ -229,6 +308,7 @@ attention_fa_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
     constexpr int Q_HALF = FA_ROWS * 128;                // 16 KiB: [128 rows][64 bf16]
     constexpr int KV_HALF = FA_KT * 128;                 // 8 KiB:  [64 keys][64 bf16]
     constexpr int KV_TILE = 2 * KV_HALF;                 // 16 KiB
+    constexpr int KS = FA_K_STAGES, VS = FA_V_STAGES;
     // 1024-byte alignment (needed by the 128-byte swizzle) is asked of the declaration instead of padded for:
     // two blocks have to fit into one SM's shared memory
     extern __shared__ __align__(1024) uint8_t fa_smem_raw[];
@@ -237,24 +317,24 @@ attention_fa_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
         if (threadIdx.x == 0 && p.err) atomicOr(p.err, EMBER_ERR_WAIT_LIMIT);
         return;
     }
-    uint8_t* q_s = smem;                                  // 32 KiB, two halves
-    uint8_t* k_s = q_s + 2 * Q_HALF;                      // FA_K_STAGES x 16 KiB
-    uint8_t* v_s = k_s + FA_K_STAGES * KV_TILE;           // FA_V_STAGES x 16 KiB
-    uint64_t* k_full = (uint64_t*)(v_s + FA_V_STAGES * KV_TILE);
-    uint64_t* k_empty = k_full + FA_K_STAGES;
-    uint64_t* v_full = k_empty + FA_K_STAGES;
-    uint64_t* v_empty = v_full + FA_V_STAGES;
-    uint64_t* s_full = v_empty + FA_V_STAGES;             // [2]
-    uint64_t* q_ready = s_full + 2;
-    uint64_t* p_full = q_ready + 1;                       // [2]: the softmax warps may be a tile ahead of the MMA thread
-    uint64_t* pv_full = p_full + 2;
-    uint64_t* o_done = pv_full + 1;                       // the last O += P V has finished
+    uint8_t* q_s = smem;                                  // 32 KiB, two halves of the head
+    uint8_t* k_s = q_s + 2 * Q_HALF;
+    uint8_t* v_s = k_s + KS * KV_TILE;
+    uint64_t* k_full = (uint64_t*)(v_s + VS * KV_TILE);
+    uint64_t* k_empty = k_full + KS;
+    uint64_t* v_full = k_empty + KS;
+    uint64_t* v_empty = v_full + VS;
+    uint64_t* s_full = v_empty + VS;                      // [score buffer]
+    uint64_t* p_full = s_full + 2;                        // [score buffer]
+    uint64_t* pv_done = p_full + 2;                       // [score buffer]: O has this buffer's tile
+    uint64_t* q_ready = pv_done + 2;
+    uint64_t* o_done = q_ready + 1;                       // the last O += P V has finished
     uint32_t* tmem_slot = (uint32_t*)(o_done + 1);
     volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int tile = p.n_tiles - 1 - (int)blockIdx.x;     // later tiles have more keys: start them first
-    const int kvh = blockIdx.y;
+    const int warp = warp_number(), lane = threadIdx.x & 31;
+    const int tile = p.n_tiles - 1 - (int)blockIdx.x / p.n_kv;      // later tiles have more keys: start them first, of all heads
+    const int kvh = (int)blockIdx.x % p.n_kv;
     const int seq = p.tiles[tile * 4 + 0], row0 = p.tiles[tile * 4 + 1], nq = p.tiles[tile * 4 + 2],
               pos0 = p.tiles[tile * 4 + 3];
     const int G = p.n_heads / p.n_kv;
@@ -265,27 +345,26 @@ attention_fa_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
     const int n_kt = hi > k_begin ? (hi - k_begin + FA_KT - 1) / FA_KT : 0;
 
     if (threadIdx.x == 0) {
-        for (int i = 0; i < FA_K_STAGES; i++) {
+        for (int i = 0; i < KS; i++) {
             fa_mbar_init(&k_full[i], 1);
             fa_mbar_init(&k_empty[i], 1);
         }
-        for (int i = 0; i < FA_V_STAGES; i++) {
+        for (int i = 0; i < VS; i++) {
             fa_mbar_init(&v_full[i], 1);
             fa_mbar_init(&v_empty[i], 1);
         }
         for (int i = 0; i < 2; i++) {
             fa_mbar_init(&s_full[i], 1);
+            fa_mbar_init(&p_full[i], FA_ROW_WARPS);
+            fa_mbar_init(&pv_done[i], 1);
         }
-        fa_mbar_init(q_ready, 4);
-        fa_mbar_init(&p_full[0], 4);
-        fa_mbar_init(&p_full[1], 4);
-        fa_mbar_init(pv_full, 1);
+        fa_mbar_init(q_ready, FA_ROW_WARPS);
         fa_mbar_init(o_done, 1);
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
-    if (warp == 1) {
+    if (warp == FA_ROW_WARPS) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(fa_s32(tmem_slot)), "r"(256) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
@@ -293,26 +372,24 @@ attention_fa_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = *tmem_slot;
-    const uint32_t tmem_s0 = tmem, tmem_o = tmem + 128;   // S buffers at columns 0 and 64, O tile at 128
+    const uint32_t tmem_s0 = tmem, tmem_o0 = tmem + 128;  // S buffers at columns 0 and 64, O at 128
 
     pdl_launch_dependents();
     pdl_wait();
 
-    if (warp == 0) {
+    if (warp == FA_ROW_WARPS) {
         // ---------------------------------------------------------------- page fetcher
         const int* bt = p.block_table + (size_t)seq * p.max_blocks;
         const int boxes = FA_KT / p.page;
+        const int last_page = min((hi - 1) / p.page, p.max_blocks - 1);      // (keys beyond the last are this run's own pages again)
         auto page_row = [&](int it) {
             int blk = 0;
             if (lane < boxes && it < n_kt) {
-                blk = bt[min((k_begin + it * FA_KT + lane * p.page) / p.page, p.max_blocks - 1)];
+                blk = bt[min((k_begin + it * FA_KT) / p.page + lane, last_page)];
                 if (blk < 0 || blk >= p.num_pages) blk = 0;
             }
             return (blk * p.n_kv + kvh) * p.page;
         };
-        // Keys and values travel in rings of their own: a key tile is free as soon as S = Q K^T has read it,
-        // long before the value tile of the same keys, so key tiles are requested three tiles ahead and the
-        // latency of a fetch (16 small boxes a tile with 16-token pages) stays off the critical path.
         // (the tensor maps are named directly: the copy instruction wants the address of the kernel parameter)
         auto fetch_k = [&](uint8_t* dst, uint64_t* bar, int y) {
             if (lane == 0) fa_expect_tx(bar, (uint32_t)KV_TILE);
@@ -331,95 +408,84 @@ attention_fa_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
             }
         };
         bool ok = true;
-        // order of need: K_0 .. K_{ks-1}, then V_i before K_{i + ks}
-        int yk = page_row(0);
-        for (int it = 0; it < min(n_kt, FA_K_STAGES); it++) {
+        int y = page_row(0);
+        for (int it = 0; it < n_kt; it++) {
+            const int bk = it % KS, bv = it % VS;
             const int y_next = page_row(it + 1);
-            fetch_k(k_s + it * KV_TILE, &k_full[it], yk);
-            yk = y_next;
-        }
-        int yv = page_row(0);
-        for (int it = 0; it < n_kt && ok; it++) {
-            const int bv = it % FA_V_STAGES;
-            const int yv_next = page_row(it + 1);
-            if (it >= FA_V_STAGES) ok = fa_wait(&v_empty[bv], (uint32_t)(it / FA_V_STAGES - 1) & 1u, abort_flag);
-            ok = __all_sync(0xffffffffu, ok);
+            if (it >= KS) ok = __all_sync(0xffffffffu, fa_wait(&k_empty[bk], (uint32_t)(it / KS - 1) & 1u, abort_flag));
             if (!ok) break;
-            fetch_v(v_s + bv * KV_TILE, &v_full[bv], yv);
-            yv = yv_next;
-            const int ik = it + FA_K_STAGES;
-            if (ik < n_kt) {
-                const int bk = ik % FA_K_STAGES;
-                const int yk_next = page_row(ik + 1);
-                ok = fa_wait(&k_empty[bk], (uint32_t)(ik / FA_K_STAGES - 1) & 1u, abort_flag);
-                ok = __all_sync(0xffffffffu, ok);
-                if (!ok) break;
-                fetch_k(k_s + bk * KV_TILE, &k_full[bk], yk);
-                yk = yk_next;
-            }
+            fetch_k(k_s + bk * KV_TILE, &k_full[bk], y);
+            if (it >= VS) ok = __all_sync(0xffffffffu, fa_wait(&v_empty[bv], (uint32_t)(it / VS - 1) & 1u, abort_flag));
+            if (!ok) break;
+            fetch_v(v_s + bv * KV_TILE, &v_full[bv], y);
+            y = y_next;
         }
-    } else if (warp == 1) {
-        // ------------------------------------------------------------------ MMA issuer
-        if (lane == 0 && n_kt > 0) {
-            const uint32_t idesc_s = fa_idesc(FA_KT, 0), idesc_o = fa_idesc(FA_D, 1);
-            bool ok = fa_wait(q_ready, 0, abort_flag);
-            // operand descriptors are made once: the issuing thread is the critical path of a tile (every
-            // instruction it spends between two waits is time the softmax warps wait for S)
-            uint64_t dq[FA_D / 16];
-#pragma unroll
-            for (int kk = 0; kk < FA_D / 16; kk++) dq[kk] = fa_desc_k(q_s + (kk >> 2) * Q_HALF) + (uint64_t)(2 * (kk & 3));
-            const uint64_t dk0 = fa_desc_k(k_s), dv0 = fa_desc_mn(v_s, KV_HALF);      // stage b: + b * KV_TILE / 16
-            auto issue_s = [&](int j) {
-                const int b = j % FA_K_STAGES;
-                const uint32_t d = tmem_s0 + (uint32_t)((j & 1) * FA_KT);
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-#pragma unroll
-                for (int kk = 0; kk < FA_D / 16; kk++) {
-                    // second half of the head: KV_HALF bytes further; 16 elements: 32 bytes inside the swizzled row
-                    const uint64_t db = dk0 + (uint64_t)((b * KV_TILE + (kk >> 2) * KV_HALF) >> 4) + (uint64_t)(2 * (kk & 3));
-                    fa_mma(d, dq[kk], db, idesc_s, kk > 0 ? 1u : 0u);
-                }
-                fa_commit(&s_full[j & 1]);
-                fa_commit(&k_empty[b]);          // the keys of tile j are no longer read
-            };
-            if (ok) ok = fa_wait(&k_full[0], 0, abort_flag);
-            if (ok) issue_s(0);
+    } else if (warp > FA_ROW_WARPS) {
+        // ------------------------------------------------------------------ MMA issuers
+        bool ok = true;
+        auto wait = [&](uint64_t* bar, int phase) { ok = __all_sync(0xffffffffu, ok && fa_wait(bar, (uint32_t)phase & 1u, abort_flag)); };
+        if (warp == FA_ROW_WARPS + 1) {
+            // keys -> scores
+            const uint32_t idesc = fa_idesc(FA_KT, 0);
+            const uint64_t dq0 = fa_desc_k(q_s), dk0 = fa_desc_k(k_s);        // stage b: + b * KV_TILE / 16
+            if (n_kt > 0) wait(q_ready, 0);
+            int b = 0, phase = 0;
             for (int j = 0; j < n_kt && ok; j++) {
-                if (j + 1 < n_kt) {
-                    ok = fa_wait(&k_full[(j + 1) % FA_K_STAGES], (uint32_t)((j + 1) / FA_K_STAGES) & 1u, abort_flag);
-                    // S_{j+1} reuses the columns of S_{j-1} / P_{j-1}: the second product of tile j - 1 was
-                    // issued before and the tensor core runs in order, and p_full(j - 1) said S_{j-1} was read
-                    if (!ok) break;
-                    issue_s(j + 1);
-                }
-                const int b = j % FA_V_STAGES;
-                // (one barrier per S buffer: the softmax warps finish tile j + 1 without this thread, so a single
-                // barrier could complete twice before it is looked at here)
-                ok = fa_wait(&p_full[j & 1], (uint32_t)(j >> 1) & 1u, abort_flag);
-                if (ok) ok = fa_wait(&v_full[b], (uint32_t)(j / FA_V_STAGES) & 1u, abort_flag);
+                // S_j takes the columns of S_{j-2} / P_{j-2}
+                if (j >= 2) wait(&pv_done[j & 1], (j >> 1) - 1);
+                if (ok) wait(&k_full[b], phase);
                 if (!ok) break;
+                const uint32_t d = tmem_s0 + (uint32_t)((j & 1) * FA_KT);
+                const uint64_t dk = dk0 + (uint64_t)((b * KV_TILE) >> 4);
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                if (elect_one()) {
 #pragma unroll
-                for (int kk = 0; kk < FA_KT / 16; kk++) {
-                    // P_j: 64 keys = 32 packed columns in the S buffer of tile j; 16 keys = 8 columns per step
-                    const uint32_t pa = tmem_s0 + (uint32_t)((j & 1) * FA_KT + kk * 8);
-                    const uint64_t db = dv0 + (uint64_t)((b * KV_TILE + kk * 16 * 128) >> 4);
-                    fa_mma_ts(tmem_o, pa, db, idesc_o, (j > 0 || kk > 0) ? 1u : 0u);
+                    for (int kk = 0; kk < FA_D / 16; kk++)
+                        // second half of the head: a half further; 16 elements: 32 bytes inside the swizzled row
+                        fa_mma(d, dq0 + (uint64_t)(((kk >> 2) * Q_HALF) >> 4) + (uint64_t)(2 * (kk & 3)),
+                               dk + (uint64_t)(((kk >> 2) * KV_HALF) >> 4) + (uint64_t)(2 * (kk & 3)), idesc, kk > 0 ? 1u : 0u);
+                    fa_commit(&s_full[j & 1]);
+                    fa_commit(&k_empty[b]);          // the keys of tile j are no longer read
                 }
-                fa_commit(&v_empty[b]);         // the values of tile j are no longer read
-                fa_commit(pv_full);             // O_j is complete, P may be overwritten
-                if (j == n_kt - 1) fa_commit(o_done);
+                __syncwarp();
+                if (++b == KS) { b = 0; phase++; }
+            }
+            // a tile's scores say that O has the tile before the last one, too; behind the last tile that is said alone
+            if (ok && n_kt >= 2) wait(&pv_done[n_kt & 1], (n_kt >> 1) - 1);
+            if (ok && n_kt > 0 && elect_one()) fa_arrive(&s_full[n_kt & 1]);
+        } else {
+            // probabilities and values -> O
+            const uint32_t idesc = fa_idesc(FA_D, 1);
+            const uint64_t dv0 = fa_desc_mn(v_s, KV_HALF);
+            int b = 0, phase = 0;
+            for (int j = 0; j < n_kt && ok; j++) {
+                wait(&v_full[b], phase);
+                if (ok) wait(&p_full[j & 1], j >> 1);
+                if (!ok) break;
+                // P_j: 64 keys = 32 packed columns in the S buffer of tile j; 16 keys = 8 columns per step
+                const uint32_t pa = tmem_s0 + (uint32_t)((j & 1) * FA_KT);
+                const uint64_t dv = dv0 + (uint64_t)((b * KV_TILE) >> 4);
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                if (elect_one()) {
+#pragma unroll
+                    for (int kk = 0; kk < FA_KT / 16; kk++)
+                        fa_mma_ts(tmem_o0, pa + (uint32_t)(kk * 8), dv + (uint64_t)((kk * 16 * 128) >> 4), idesc, (j > 0 || kk > 0) ? 1u : 0u);
+                    fa_commit(&pv_done[j & 1]);
+                    fa_commit(&v_empty[b]);          // the values of tile j are no longer read
+                    if (j == n_kt - 1) fa_commit(o_done);
+                }
+                __syncwarp();
+                if (++b == VS) { b = 0; phase++; }
             }
         }
     } else {
         // ------------------------------------------------- softmax / accumulation: one row per thread
-        const int quad = warp & 3;
+        const int quad = warp;
         const int r = quad * 32 + lane;
-        const int qi = min(r, rows - 1) / G;
-        const int qpos = pos0 + qi;
+        const int qpos = pos0 + min(r, rows - 1) / G;
+        const int rq = r / G, rg = r - rq * G;
         // query rows -> shared memory (zero beyond `rows`)
         {
-            const int rq = r / G, rg = r - rq * G;
             const __nv_bfloat16* src = p.q + ((size_t)(row0 + rq) * p.n_heads + kvh * G + rg) * FA_D;
 #pragma unroll
             for (int c = 0; c < 16; c++) {
@@ -432,28 +498,32 @@ attention_fa_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
             if (lane == 0) fa_arrive(q_ready);
         }
         if (p.gate && r < rows) {
-            const int rq = r / G, rg = r - rq * G;
             const float* g = p.gate + (size_t)(row0 + rq) * p.ld_gate + (kvh * G + rg) * FA_D;
 #pragma unroll
             for (int c = 0; c < FA_D; c += 32) asm volatile("prefetch.global.L2 [%0];" ::"l"(g + c));
         }
         float m_ref = -INFINITY, l_run = 0.0f;      // reference maximum (exponent base) and denominator
         const uint32_t lane_base = (uint32_t)(quad * 32) << 16;
+        const uint32_t tmem_s = tmem_s0 + lane_base, tmem_o = tmem_o0 + lane_base;
         bool ok = true;
         // the first key this row sees, and the first that every row of the tile sees
-        const int last_q = pos0 + (rows - 1) / G;
-        int row_lo = lo, all_lo = lo;
+        const int last_q = pos0 + nq - 1;
+        int row_lo = 0, all_lo = 0;
         if (p.window > 0) { row_lo = max(row_lo, qpos - p.window + 1); all_lo = max(all_lo, last_q - p.window + 1); }
         if (p.chunk > 0) { row_lo = max(row_lo, qpos - qpos % p.chunk); all_lo = max(all_lo, last_q - last_q % p.chunk); }
-        const int head = kvh * G + min(r, rows - 1) % G;
+        const int head = kvh * G + rg;
         const float slope = BIAS && p.slopes ? p.slopes[head] * p.raw_per_slope : 0.0f;
+        // the maximum is taken over the raw scores; the scale (> 0) is folded into the exponent below (capped scores
+        // are scaled already)
+        const float to_log2 = CAP ? 1.0f : p.scale_log2;
         for (int j = 0; j < n_kt; j++) {
             const int k0 = k_begin + j * FA_KT;
+            const uint32_t scores = tmem_s + (uint32_t)((j & 1) * FA_KT);
             if (ok) ok = fa_wait(&s_full[j & 1], (uint32_t)(j >> 1) & 1u, abort_flag);
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             uint32_t su[FA_KT];
-            fa_tmem_ld32_nowait(tmem_s0 + lane_base + (uint32_t)((j & 1) * FA_KT), su);
-            fa_tmem_ld32_nowait(tmem_s0 + lane_base + (uint32_t)((j & 1) * FA_KT + 32), su + 32);
+#pragma unroll
+            for (int c = 0; c < FA_KT; c += 32) fa_tmem_ld32_nowait(scores + (uint32_t)c, su + c);
             fa_tmem_wait_ld();
             float* s = reinterpret_cast<float*>(su);
             if (CAP) {
@@ -474,16 +544,12 @@ attention_fa_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
                     for (int i = 0; i < FA_KT; i++) s[i] = fa_capped(p, s[i]);
                 }
             }
-
             if (BIAS) {
 #pragma unroll
                 for (int i = 0; i < FA_KT; i++) s[i] = fmaf(slope, (float)i, s[i]);
             }
-            const bool interior = k0 >= all_lo && k0 + FA_KT <= hi && k0 + FA_KT - 1 <= pos0;
-            // the maximum is taken over the raw scores; the scale (> 0) is folded into the exponent below (capped scores
-            // are scaled already)
-            const float to_log2 = CAP ? 1.0f : p.scale_log2;
-            float tmax;
+            // (the first row sees up to pos0)
+            const bool interior = k0 >= all_lo && k0 + FA_KT - 1 <= pos0;
             if (!interior) {
 #pragma unroll
                 for (int i = 0; i < FA_KT; i++) {
@@ -491,134 +557,86 @@ attention_fa_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
                     s[i] = key >= row_lo && key <= qpos ? s[i] : -INFINITY;
                 }
             }
-            if (CAP != 1) {   // four independent chains instead of one of 64 dependent maxima
-                float t0 = s[0], t1 = s[1], t2 = s[2], t3 = s[3];
+            float tmax = -INFINITY;
+            if (CAP != 1) {   // four independent chains, two scores a step
+                float t0 = fmaxf(s[0], s[1]), t1 = fmaxf(s[2], s[3]), t2 = fmaxf(s[4], s[5]), t3 = fmaxf(s[6], s[7]);
 #pragma unroll
-                for (int i = 4; i < FA_KT; i += 4) {
-                    t0 = fmaxf(t0, s[i]);
-                    t1 = fmaxf(t1, s[i + 1]);
-                    t2 = fmaxf(t2, s[i + 2]);
-                    t3 = fmaxf(t3, s[i + 3]);
+                for (int i = 8; i < FA_KT; i += 8) {
+                    t0 = fa_max3(t0, s[i], s[i + 1]);
+                    t1 = fa_max3(t1, s[i + 2], s[i + 3]);
+                    t2 = fa_max3(t2, s[i + 4], s[i + 5]);
+                    t3 = fa_max3(t3, s[i + 6], s[i + 7]);
                 }
                 tmax = fmaxf(fmaxf(t0, t1), fmaxf(t2, t3));
-            } else {
-                tmax = -INFINITY;
             }
             const float tile_bias = BIAS ? slope * (float)(k0 - qpos) * to_log2 : 0.0f;
             tmax = BIAS ? fmaf(tmax, to_log2, tile_bias) : tmax * to_log2;
             // raise the reference maximum only when the true one has outgrown it by more than 2^8
             const bool raise = CAP != 1 && (tmax > m_ref + 8.0f || (m_ref == -INFINITY && tmax > -INFINITY));
-            const bool warp_raise = CAP != 1 && __any_sync(0xffffffffu, raise);
-            if (warp_raise && j > 0) {
-                // O is complete up to tile j - 1 once the previous second product has finished
-                if (ok) ok = fa_wait(pv_full, (uint32_t)(j - 1) & 1u, abort_flag);
+            if (CAP != 1 && __any_sync(0xffffffffu, raise)) {
                 const float factor = raise ? (m_ref == -INFINITY ? 0.0f : exp2f(m_ref - tmax)) : 1.0f;
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                if (j > 0) {
+                    // O is complete up to the tile before: the next tile's scores waited for that
+                    if (ok) ok = fa_wait(&s_full[(j + 1) & 1], (uint32_t)((j + 1) >> 1) & 1u, abort_flag);
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
-                for (int c = 0; c < FA_D / 16; c++) {
-                    float t[16];
-                    fa_tmem_ld16(tmem_o + lane_base + (uint32_t)(c * 16), t);
+                    for (int c = 0; c < FA_D / 16; c++) {
+                        float o[16];
+                        fa_tmem_ld16(tmem_o + (uint32_t)(c * 16), o);
 #pragma unroll
-                    for (int i = 0; i < 16; i++) t[i] *= factor;
-                    fa_tmem_st16(tmem_o + lane_base + (uint32_t)(c * 16), t);
+                        for (int i = 0; i < 16; i++) o[i] *= factor;
+                        fa_tmem_st16(tmem_o + (uint32_t)(c * 16), o);
+                    }
+                    fa_tmem_wait_st();
                 }
-                fa_tmem_wait_st();
-                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-            }
-            if (raise) {
-                l_run *= m_ref == -INFINITY ? 0.0f : exp2f(m_ref - tmax);
-                m_ref = tmax;
+                l_run *= factor;
+                if (raise) m_ref = tmax;
             }
             const float neg_base = (m_ref == -INFINITY ? 0.0f : -m_ref) + tile_bias;
-            float sum0 = 0.0f, sum1 = 0.0f, sum2 = 0.0f, sum3 = 0.0f;
+            const unsigned long long scale2 = fa_pk2(to_log2, to_log2), base2 = fa_pk2(neg_base, neg_base);
+            unsigned long long sum0 = 0, sum1 = 0;
             uint32_t packed[FA_KT / 2];
 #pragma unroll
             for (int i = 0; i < FA_KT / 2; i += 2) {
-                const float p0 = fa_ex2(CAP == 1 ? s[2 * i] : fmaf(s[2 * i], to_log2, neg_base));
-                const float p1 = fa_ex2(CAP == 1 ? s[2 * i + 1] : fmaf(s[2 * i + 1], to_log2, neg_base));
-                const float p2 = fa_ex2(CAP == 1 ? s[2 * i + 2] : fmaf(s[2 * i + 2], to_log2, neg_base));
-                const float p3 = fa_ex2(CAP == 1 ? s[2 * i + 3] : fmaf(s[2 * i + 3], to_log2, neg_base));
-                sum0 += p0; sum1 += p1; sum2 += p2; sum3 += p3;
+                unsigned long long x0 = fa_pk2(s[2 * i], s[2 * i + 1]), x1 = fa_pk2(s[2 * i + 2], s[2 * i + 3]);
+                if (CAP != 1) { x0 = fa_fma2(x0, scale2, base2); x1 = fa_fma2(x1, scale2, base2); }
+                float p0, p1, p2, p3;
+                fa_unpk2(x0, p0, p1);
+                fa_unpk2(x1, p2, p3);
+                p0 = fa_ex2(p0); p1 = fa_ex2(p1); p2 = fa_ex2(p2); p3 = fa_ex2(p3);
+                sum0 = fa_add2(sum0, fa_pk2(p0, p1));
+                sum1 = fa_add2(sum1, fa_pk2(p2, p3));
                 __nv_bfloat162 h2 = __floats2bfloat162_rn(p0, p1), h3 = __floats2bfloat162_rn(p2, p3);
                 packed[i] = *reinterpret_cast<uint32_t*>(&h2);
                 packed[i + 1] = *reinterpret_cast<uint32_t*>(&h3);
             }
-            const float sum = (sum0 + sum1) + (sum2 + sum3);
             // P_j replaces S_j in tensor memory (its first 32 columns)
-            fa_tmem_st32(tmem_s0 + lane_base + (uint32_t)((j & 1) * FA_KT), packed);
+            fa_tmem_st32(scores, packed);
             fa_tmem_wait_st();
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-            l_run += sum;
             __syncwarp();
             if (lane == 0) fa_arrive(&p_full[j & 1]);
+            float a, b, c, d;
+            fa_unpk2(sum0, a, b);
+            fa_unpk2(sum1, c, d);
+            l_run += (a + b) + (c + d);
         }
-        // (a barrier of its own: the rows of the last tile can be done while O += P V of the tile before the last
-        // still waits for its values, two phases of pv_full behind, and a parity cannot tell two phases apart;
-        // the wait in the loop above is safe, S_j being complete only after O += P V of tile j - 2)
         if (n_kt > 0 && ok) ok = fa_wait(o_done, 0, abort_flag);
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         if (BIAS && p.sink) l_run += fa_ex2(fmaf(p.sink[head], FA_LOG2E, m_ref == -INFINITY ? 0.0f : -m_ref));
         const float inv = l_run > 0.0f ? 1.0f / l_run : 0.0f;
         if (n_kt > 0 && p.gate) {
-            // The gate's logits and the results are rows of 512 and 256 bytes a (token, head): a warp turns its 32 rows in
-            // shared memory (queries, keys and values have all been read) so that its lanes walk along a row.
-            // Its logits have been on their way into the L2 since before the first tile.
+            // queries, keys and values have all been read: the rows are turned in their place
             ok = __all_sync(0xffffffffu, ok);
-            float* turn = reinterpret_cast<float*>(smem) + quad * 32 * (FA_D + 4);
-#pragma unroll
-            for (int c = 0; c < FA_D / 32; c++) {
-                uint32_t tu[32];
-                fa_tmem_ld32_nowait(tmem_o + lane_base + (uint32_t)(c * 32), tu);
-                fa_tmem_wait_ld();
-                if (ok) {
-#pragma unroll
-                    for (int e = 0; e < 32; e += 4)
-                        *reinterpret_cast<float4*>(turn + lane * (FA_D + 4) + c * 32 + e) =
-                            make_float4(__uint_as_float(tu[e]) * inv, __uint_as_float(tu[e + 1]) * inv, __uint_as_float(tu[e + 2]) * inv,
-                                        __uint_as_float(tu[e + 3]) * inv);
-                }
-            }
-            __syncwarp();
-            const int here = ok ? min(32, rows - quad * 32) : 0;
-#pragma unroll 8
-            for (int i = 0; i < here; i++) {
-                const int rr = quad * 32 + i, rq = rr / G, rg = rr - rq * G;
-                const size_t at = (size_t)(kvh * G + rg) * FA_D + 4 * lane;
-                const float4 g = __ldg(reinterpret_cast<const float4*>(p.gate + (size_t)(row0 + rq) * p.ld_gate + at));
-                const float4 v = *reinterpret_cast<const float4*>(turn + i * (FA_D + 4) + 4 * lane);
-                uint2 packed;
-                __nv_bfloat162 a = __floats2bfloat162_rn(v.x * __fdividef(1.0f, 1.0f + __expf(-g.x)), v.y * __fdividef(1.0f, 1.0f + __expf(-g.y)));
-                __nv_bfloat162 b = __floats2bfloat162_rn(v.z * __fdividef(1.0f, 1.0f + __expf(-g.z)), v.w * __fdividef(1.0f, 1.0f + __expf(-g.w)));
-                packed.x = *reinterpret_cast<uint32_t*>(&a);
-                packed.y = *reinterpret_cast<uint32_t*>(&b);
-                *reinterpret_cast<uint2*>(p.out + (size_t)(row0 + rq) * p.n_heads * FA_D + at) = packed;
-            }
+            fa_store_gated(p, tmem_o, reinterpret_cast<float*>(smem) + quad * 32 * (FA_D + 4), inv, ok, quad, lane, rows, row0, kvh, G);
         } else if (n_kt > 0) {
-            const int rq = r / G, rg = r - rq * G;
-            __nv_bfloat16* dst = p.out + ((size_t)(row0 + rq) * p.n_heads + kvh * G + rg) * FA_D;
-#pragma unroll
-            for (int c = 0; c < FA_D / 32; c++) {
-                uint32_t tu[32];
-                fa_tmem_ld32_nowait(tmem_o + lane_base + (uint32_t)(c * 32), tu);
-                fa_tmem_wait_ld();
-                if (ok && r < rows) {
-#pragma unroll
-                    for (int q4 = 0; q4 < 4; q4++) {
-                        uint4 packed;
-                        __nv_bfloat162* h2 = (__nv_bfloat162*)&packed;
-#pragma unroll
-                        for (int e = 0; e < 4; e++)
-                            h2[e] = __floats2bfloat162_rn(__uint_as_float(tu[q4 * 8 + 2 * e]) * inv, __uint_as_float(tu[q4 * 8 + 2 * e + 1]) * inv);
-                        *reinterpret_cast<uint4*>(dst + c * 32 + q4 * 8) = packed;
-                    }
-                }
-            }
+            fa_store_rows(p, tmem_o, inv, ok && r < rows, row0 + rq, kvh * G + rg);
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (threadIdx.x == 0 && *abort_flag && p.err) atomicOr(p.err, EMBER_ERR_WAIT_LIMIT);
-    if (warp == 1) {
+    if (warp == FA_ROW_WARPS) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(256) : "memory");
     }
@@ -691,7 +709,7 @@ EMBER_API int ember_attention_fa(const void* q, const void* k_pool, const void* 
     if (n_heads <= 0 || n_kv <= 0 || n_heads % n_kv) return fail("attention_fa: bad head counts %d/%d", n_heads, n_kv);
     if (!ember_attention_fa_supported(D, n_heads / n_kv, page))
         return fail("attention_fa: head size %d, group %d, page %d are not taken", D, n_heads / n_kv, page);
-    if (n_kv > 65535) return fail("attention_fa: grid too large");
+    if (n_kv > 65535 || (long long)n_kv * n_tiles > 0x7fffffffll) return fail("attention_fa: grid too large");
     CUtensorMap mk, mv;
     const long long total_rows = (long long)num_pages * n_kv * page;
     if (!fa_pool_map(k_pool, total_rows, page, &mk) || !fa_pool_map(v_pool, total_rows, page, &mv))
@@ -705,15 +723,14 @@ EMBER_API int ember_attention_fa(const void* q, const void* k_pool, const void* 
     p.cap_z = softcap > 0.0f ? scale / softcap : 0.0f;
     p.cap_arg = softcap > 0.0f ? 2.0f * FA_LOG2E * scale / softcap : 0.0f; p.gate = gate; p.ld_gate = ld_gate; p.n_tiles = n_tiles; p.err = err;
     p.slopes = slopes; p.sink = sink; p.raw_per_slope = softcap > 0.0f ? FA_LOG2E : 1.0f / scale;
-    const size_t smem = (size_t)2 * FA_ROWS * 128 + (size_t)(FA_K_STAGES + FA_V_STAGES) * 2 * FA_KT * 128 + 256;
     auto run = [&](auto kernel, bool& ready) -> int {
         if (!ready) {
-            cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            if (e != cudaSuccess) return fail("attention_fa: shared memory %zu: %s", smem, cudaGetErrorString(e));
+            cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FA_SMEM);
+            if (e != cudaSuccess) return fail("attention_fa: shared memory %zu: %s", FA_SMEM, cudaGetErrorString(e));
             cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared);
             ready = true;
         }
-        launch_kernel(kernel, dim3(n_tiles, n_kv), dim3(FA_THREADS), smem, (cudaStream_t)stream, mk, mv, p);
+        launch_kernel(kernel, dim3((unsigned)(n_kv * n_tiles)), dim3(FA_THREADS), FA_SMEM, (cudaStream_t)stream, mk, mv, p);
         return check_launch("attention_fa");
     };
     static bool ready[5] = {false, false, false, false, false};

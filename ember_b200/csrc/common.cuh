@@ -132,6 +132,18 @@ __device__ __forceinline__ bool mbarrier_wait_bounded(uint32_t bar_shared, uint3
     return false;
 }
 
+// One lane of a warp whose lanes are all here, the same one each time.  What issues tensor instructions and TMA copies goes
+// through its loops as a whole warp and elects the lane that issues: the control flow then is uniform, and so are the registers
+// that these instructions take their operands from.  A lane singled out by its number pays for moving each operand there
+// (attention: 77 cycles an MMA of 128 x 64 x 16 against 56).
+__device__ __forceinline__ bool elect_one() {
+    uint32_t one;
+    asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}" : "=r"(one));
+    return one != 0;
+}
+// The warp's number, known to be the same in all its lanes.
+__device__ __forceinline__ int warp_number() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
+
 __device__ __forceinline__ float to_float(float x) { return x; }
 __device__ __forceinline__ float to_float(__nv_bfloat16 x) { return __bfloat162float(x); }
 

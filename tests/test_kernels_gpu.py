@@ -570,6 +570,54 @@ def test_attention_fa_many_blocks(heads, kv, page, window):
         assert rel(out.float().view(T, heads, D), want) < 6e-3
 
 
+@pytest.mark.parametrize("page", [16, 64])
+@pytest.mark.parametrize("heads,kv", [(4, 4), (4, 2), (16, 2)])
+@pytest.mark.parametrize("held", [0, 1, 63, 64, 65])
+def test_attention_fa_edges(heads, kv, page, held):
+    """The tcgen05 kernel at the edges of its tiles (128 rows, 64 keys): every count of queries around them behind no, one and
+    about a tile of cached keys.  What lies beyond a run's last key in its key tile must not be read from elsewhere: the
+    block table ends in -1 and the pool's first page, which no run holds, is NaN."""
+    from ember_b200 import ops
+    from ember_b200.engine.batch import StepBatch, attention_tiles
+    D, dt, dev = 128, torch.bfloat16, "cuda"
+    rows = 128 // (heads // kv)
+    new = sorted({2, rows - 1, rows, rows + 1, 63, 64, 65})
+    torch.manual_seed(heads * page + held)
+    ctx_lens, S = [held + n for n in new], len(new)
+    nblk = max((c + page - 1) // page for c in ctx_lens) + 4
+    perm = (torch.randperm(S * nblk) + 1).reshape(S, nblk).int()
+    kp = torch.zeros(S * nblk + 1, kv, page, D, dtype=dt)
+    vp = torch.zeros_like(kp)
+    kp[0], vp[0] = float("nan"), float("nan")
+    ks, vs, qs = [], [], []
+    for s in range(S):
+        k, v, q = torch.randn(ctx_lens[s], kv, D).to(dt), torch.randn(ctx_lens[s], kv, D).to(dt), torch.randn(new[s], heads, D).to(dt)
+        ks.append(k.float()), vs.append(v.float()), qs.append(q.float())
+        used = (ctx_lens[s] + page - 1) // page
+        perm[s, used:] = -1
+        for b in range(used):
+            lo, hi = b * page, min((b + 1) * page, ctx_lens[s])
+            kp[perm[s, b], :, :hi - lo], vp[perm[s, b], :, :hi - lo] = k[lo:hi].transpose(0, 1), v[lo:hi].transpose(0, 1)
+    T = sum(new)
+    positions = np.concatenate([np.arange(c - n, c) for c, n in zip(ctx_lens, new)]).astype(np.int32)
+    batch = StepBatch(requests=list(range(S)), tokens=np.zeros(T, np.int32), positions=positions,
+                      seq_of=np.repeat(np.arange(S), new).astype(np.int32), query_start=np.cumsum([0] + new).astype(np.int32),
+                      context_len=np.asarray(ctx_lens, np.int32), block_tables=[perm.numpy()],
+                      state_slots=np.zeros(S, np.int32), logit_rows=np.zeros(0, np.int32))
+    scale = 1.0 / math.sqrt(D)
+    want = torch.cat([attention_ref(qs[s].to(dev), ks[s].to(dev), vs[s].to(dev), scale, 0) for s in range(S)])
+    tiles = torch.from_numpy(attention_tiles(batch, ops.attention_fa_tile_queries(heads // kv), "multi")).to(dev)
+    err = torch.zeros(1, dtype=torch.int32, device=dev)
+    out = torch.full((T, heads * D), float("nan"), device=dev, dtype=dt)
+    ops.attention_fa(torch.cat(qs).to(dt).to(dev).view(T, -1), kp.to(dev), vp.to(dev), out, heads, kv, D, tiles, tiles.shape[0],
+                     perm.to(dev), page, 0, scale, err=err)
+    assert int(err.item()) == 0
+    got = out.float().view(T, heads, D)
+    # a probability and a result are rounded to bf16, 2^-9 of themselves at most: 7.8e-3 of a row's norm if all erred alike
+    assert float(((got - want).norm(dim=-1) / want.norm(dim=-1)).max()) < 8e-3
+    assert rel(got, want) < 6e-3
+
+
 @pytest.mark.parametrize("heads,kv,page,M", [(4, 2, 16, 300), (3, 1, 64, 200), (6, 2, 32, 2100), (5, 1, 16, 2304),
                                              (16, 8, 16, 8), (4, 2, 64, 1), (3, 1, 32, 16), (40, 8, 16, 5)])
 @pytest.mark.parametrize("norm,rotate", [(True, True), (False, True), (True, False)])
