@@ -75,7 +75,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_c
     uint32_t* tmem_base_slot = (uint32_t*)(tmem_empty_bar + 2);
     volatile int* abort_flag = (volatile int*)(tmem_base_slot + 1);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_number(), lane = threadIdx.x & 31;
     const uint32_t rank = cluster_ctarank();                // 0: leader, 1: peer
     const int pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
     const int n_kb = p.num_k_blocks;
@@ -111,31 +111,32 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_c
     pdl_wait();
 
     if (warp == 0) {
-        if (lane == 0) {
-            int s = 0;
-            uint32_t phase = 0;
-            bool ok = true, wrapped = false;
-            uint8_t* st = smem;
-            for (int u = pair; u < units && ok; u += n_pairs) {
-                const int t = u / k_splits, kb0 = (u - t * k_splits) * p.k_blocks_per_split;
-                const int kb1 = min(n_kb, kb0 + p.k_blocks_per_split);
-                const int col_tile = t / p.row_tiles, row_tile = t - col_tile * p.row_tiles;
-                const int row0 = row_tile * 2 * TILE_ROWS + (int)rank * TILE_ROWS;
-                const int col0 = col_tile * p.block_cols + (int)rank * half_cols;
-                for (int i = kb0; i < kb1; i++) {
-                    if (wrapped) ok = mbar_wait(&empty_bar[s], phase ^ 1u, abort_flag);
-                    if (!ok) break;
+        int s = 0;
+        uint32_t phase = 0;
+        bool ok = true, wrapped = false;
+        uint8_t* st = smem;
+        for (int u = pair; u < units && ok; u += n_pairs) {
+            const int t = u / k_splits, kb0 = (u - t * k_splits) * p.k_blocks_per_split;
+            const int kb1 = min(n_kb, kb0 + p.k_blocks_per_split);
+            const int col_tile = t / p.row_tiles, row_tile = t - col_tile * p.row_tiles;
+            const int row0 = row_tile * 2 * TILE_ROWS + (int)rank * TILE_ROWS;
+            const int col0 = col_tile * p.block_cols + (int)rank * half_cols;
+            for (int i = kb0; i < kb1; i++) {
+                if (wrapped) ok = __all_sync(0xffffffffu, mbar_wait(&empty_bar[s], phase ^ 1u, abort_flag));
+                if (!ok) break;
+                if (elect_one()) {
                     const uint32_t bar = map_to_rank(smem_u32(&full_bar[s]), 0);
                     if (rank == 0) mbar_expect_tx(&full_bar[s], (uint32_t)(2 * (a_bytes + b_bytes)));
                     tma_load_2d_pair(st, &map_rows, bar, i * TILE_K, row0);
                     tma_load_2d_pair(st + a_bytes, &map_cols, bar, i * TILE_K, col0);
-                    st += stage_bytes;
-                    if (++s == p.stages) { s = 0; st = smem; phase ^= 1u; wrapped = true; }
                 }
+                __syncwarp();
+                st += stage_bytes;
+                if (++s == p.stages) { s = 0; st = smem; phase ^= 1u; wrapped = true; }
             }
         }
     } else if (warp == 1) {
-        if (lane == 0 && rank == 0) {
+        if (rank == 0) {
             const uint32_t idesc = umma_idesc_pair(p.block_cols);
             int li = 0, s = 0;
             uint32_t phase = 0;
@@ -146,22 +147,25 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_c
             for (int u = pair; u < units && ok; u += n_pairs, li++) {
                 const int kb0 = (u % k_splits) * p.k_blocks_per_split, kb1 = min(n_kb, kb0 + p.k_blocks_per_split);
                 const int acc = li & 1;
-                if (li >= 2) ok = mbar_wait(&tmem_empty_bar[acc], ((uint32_t)(li >> 1) & 1u) ^ 1u, abort_flag);
+                if (li >= 2) ok = __all_sync(0xffffffffu, mbar_wait(&tmem_empty_bar[acc], ((uint32_t)(li >> 1) & 1u) ^ 1u, abort_flag));
                 if (!ok) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint32_t d = tmem_d + (uint32_t)(acc * p.block_cols);
                 for (int i = kb0; i < kb1; i++) {
-                    ok = mbar_wait(&full_bar[s], phase, abort_flag);
+                    ok = __all_sync(0xffffffffu, mbar_wait(&full_bar[s], phase, abort_flag));
                     if (!ok) break;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    if (elect_one()) {
 #pragma unroll
-                    for (int k = 0; k < TILE_K / UMMA_K; k++)
-                        tcgen05_mma_bf16_pair(d, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), idesc, (i > kb0 || k > 0) ? 1u : 0u);
-                    tcgen05_commit_pair(&empty_bar[s]);
+                        for (int k = 0; k < TILE_K / UMMA_K; k++)
+                            tcgen05_mma_bf16_pair(d, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), idesc, (i > kb0 || k > 0) ? 1u : 0u);
+                        tcgen05_commit_pair(&empty_bar[s]);
+                    }
+                    __syncwarp();
                     da += dstep; db += dstep;
                     if (++s == p.stages) { s = 0; phase ^= 1u; da = da0; db = db0; }
                 }
-                if (ok) tcgen05_commit_pair(&tmem_full_bar[acc]);
+                if (ok && elect_one()) tcgen05_commit_pair(&tmem_full_bar[acc]);
             }
         }
     } else {
