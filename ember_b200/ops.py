@@ -360,6 +360,17 @@ def sample(logits: torch.Tensor, params: torch.Tensor, out: torch.Tensor, rows: 
           c_void_p(stream if stream is not None else current_stream_ptr()))
 
 
+def sample_host(logits: torch.Tensor, params: bytes, out: torch.Tensor, rows: int, stream: Optional[int] = None) -> None:
+    """The same with the parameter rows on the host (``bytes``, read before this returns): they travel with the launch."""
+    _check(logits, "logits", torch.float32)
+    _check(out, "out", torch.int32)
+    if logits.dim() != 2 or logits.shape[0] < rows or len(params) < rows * 32 or out.numel() < rows:
+        raise KernelError("sample: buffers do not fit the rows")
+    lib = _lib("sampling")
+    _call(lib, lib.ember_sample_host, _p(logits), c_int(rows), c_int(logits.shape[1]), params, _p(out),
+          c_void_p(stream if stream is not None else current_stream_ptr()))
+
+
 def argmax(logits: torch.Tensor, out: torch.Tensor, rows: int, part_v: torch.Tensor, part_i: torch.Tensor,
            stream: Optional[int] = None) -> None:
     """out[r] = index of the largest logit of row r, lowest index on ties (greedy sampling)."""

@@ -1,24 +1,39 @@
 """Device sampler: one kernel launch for all rows of a step."""
 from __future__ import annotations
 
+import functools
 import struct
+from operator import attrgetter
 from typing import Optional, Sequence
 
-import numpy as np
 import torch
 
-from .. import ops, transfers
+from .. import ops
 from .params import SamplingParams
 
-_ROW = struct.Struct("<fiffQQ")   # temperature, top_k, top_p, min_p, seed, counter: 32 bytes
+_U64 = (1 << 64) - 1
 
 
-def pack_params(params: Sequence[SamplingParams], counters: Sequence[int]) -> np.ndarray:
-    buf = bytearray(_ROW.size * len(params))
-    for i, (p, c) in enumerate(zip(params, counters)):
-        _ROW.pack_into(buf, i * _ROW.size, float(p.temperature), int(p.top_k), float(p.top_p), float(p.min_p),
-                       int(p.seed) & ((1 << 64) - 1), int(c) & ((1 << 64) - 1))
-    return np.frombuffer(buf, dtype=np.uint8)          # a view of the bytearray: writable
+@functools.lru_cache(maxsize=64)
+def _rows_struct(rows: int) -> struct.Struct:
+    return struct.Struct("<" + "fiffQQ" * rows)     # temperature, top_k, top_p, min_p, seed, counter: 32 bytes a row
+
+
+_fields = attrgetter("temperature", "top_k", "top_p", "min_p", "seed")
+
+
+def pack_params(params: Sequence[SamplingParams], counters: Sequence[int]) -> bytes:
+    values = []
+    for p, c in zip(params, counters):
+        values += _fields(p)
+        values.append(c)
+    try:
+        return _rows_struct(len(params)).pack(*values)
+    except struct.error:                            # numbers of other types, seeds and counters outside 64 bits
+        for i in range(0, len(values), 6):
+            t, k, top, low, seed, c = values[i:i + 6]
+            values[i:i + 6] = float(t), int(k), float(top), float(low), int(seed) & _U64, int(c) & _U64
+        return _rows_struct(len(params)).pack(*values)
 
 
 _scratch = {}
@@ -31,27 +46,6 @@ def _argmax_scratch(device, rows: int):
         got = (torch.empty(n, dtype=torch.float32, device=device), torch.empty(n, dtype=torch.int32, device=device))
         _scratch[device] = got
     return got
-
-
-_staging = {}
-
-
-def _param_staging(device, nbytes: int):
-    """Pinned and device buffers for the parameter rows, from a ring of four (pinning memory per call costs more
-    than the kernel); a slot is taken again only after the copy out of it has run."""
-    ring = _staging.setdefault(device, {"at": 0, "slots": []})
-    if len(ring["slots"]) < 4:
-        n = max(nbytes, 64 * _ROW.size)
-        ring["slots"].append([torch.empty(n, dtype=torch.uint8, pin_memory=True),
-                              torch.empty(n, dtype=torch.uint8, device=device), torch.cuda.Event()])
-        return ring["slots"][-1]
-    ring["at"] = (ring["at"] + 1) % 4
-    slot = ring["slots"][ring["at"]]
-    slot[2].synchronize()
-    if slot[0].numel() < nbytes:
-        slot[0] = torch.empty(nbytes, dtype=torch.uint8, pin_memory=True)
-        slot[1] = torch.empty(nbytes, dtype=torch.uint8, device=device)
-    return slot
 
 
 def sample(logits: torch.Tensor, params: Sequence[SamplingParams], counters: Sequence[int],
@@ -67,10 +61,5 @@ def sample(logits: torch.Tensor, params: Sequence[SamplingParams], counters: Seq
         part_v, part_i = _argmax_scratch(logits.device, rows)
         ops.argmax(logits, out, rows, part_v, part_i)
         return out
-    host, dev, event = _param_staging(logits.device, rows * _ROW.size)
-    host[:rows * _ROW.size].copy_(torch.from_numpy(pack_params(params, counters)))
-    dev[:rows * _ROW.size].copy_(host[:rows * _ROW.size], non_blocking=True)
-    event.record()
-    transfers.add_h2d(rows * _ROW.size)
-    ops.sample(logits, dev, out, rows)
+    ops.sample_host(logits, pack_params(params, counters), out, rows)
     return out

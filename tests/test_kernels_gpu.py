@@ -618,6 +618,25 @@ def test_attention_fa_edges(heads, kv, page, held):
     assert rel(got, want) < 6e-3
 
 
+@pytest.mark.parametrize("rows", [1, 63, 64, 65, 130])
+@pytest.mark.parametrize("V", [1000, 20000])
+def test_sample_parameters_from_the_host(rows, V):
+    """Parameter rows that travel with the launch (64 of them) give the ids that rows in device memory give."""
+    from ember_b200 import SamplingParams, ops
+    from ember_b200.sampling import device
+    torch.manual_seed(rows)
+    logits = torch.randn(rows, V, device="cuda") * 3
+    params = [SamplingParams(temperature=(0.0, 0.7, 1.3)[i % 3], top_k=(0, 5, 40)[i % 3], top_p=(1.0, 0.9)[i % 2], min_p=(0.0, 0.05)[i % 2],
+                             seed=(1 << 63) + i if i % 2 else -i) for i in range(rows)]
+    packed = device.pack_params(params, [7 * i for i in range(rows)])
+    want, got = (torch.full((rows,), -1, dtype=torch.int32, device="cuda") for _ in range(2))
+    ops.sample(logits, torch.frombuffer(bytearray(packed), dtype=torch.uint8).cuda(), want, rows)
+    ops.sample_host(logits, packed, got, rows)
+    assert torch.equal(got, want) and bool((want >= 0).all())
+    with pytest.raises(ops.KernelError):
+        ops.sample_host(logits, packed[:-1], got, rows)
+
+
 @pytest.mark.parametrize("heads,kv,page,M", [(4, 2, 16, 300), (3, 1, 64, 200), (6, 2, 32, 2100), (5, 1, 16, 2304),
                                              (16, 8, 16, 8), (4, 2, 64, 1), (3, 1, 32, 16), (40, 8, 16, 5)])
 @pytest.mark.parametrize("norm,rotate", [(True, True), (False, True), (True, False)])
