@@ -632,12 +632,13 @@ def attention_fa(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, ou
                  n_kv: int, head_dim: int, tiles: torch.Tensor, n_tiles: int, block_table: torch.Tensor, page: int,
                  window: int, scale: float, err: Optional[torch.Tensor] = None, stream: Optional[int] = None,
                  softcap: float = 0.0, chunk: int = 0, gate: Optional[torch.Tensor] = None, gate_col: int = 0,
-                 slopes: Optional[torch.Tensor] = None, sink: Optional[torch.Tensor] = None) -> None:
+                 slopes: Optional[torch.Tensor] = None, sink: Optional[torch.Tensor] = None, release_late: bool = False) -> None:
     """bf16 causal attention of prompt portions on tcgen05 tensor cores (S and O in tensor memory).  ``softcap`` > 0: the
     scaled score becomes softcap * tanh(score / softcap); ``chunk`` > 0: position i sees j only if
     floor(i / chunk) == floor(j / chunk); ``gate`` (fp32 [T, ..]): element i of a token's result is multiplied by
     sigmoid(gate[t, gate_col + i]); ``slopes`` (fp32 [n_heads]): slopes[h] * (i - j) is taken off the score after the cap;
-    ``sink`` (fp32 [n_heads]): exp(sink[h]) joins the softmax's denominator."""
+    ``sink`` (fp32 [n_heads]): exp(sink[h]) joins the softmax's denominator.  ``release_late``: an ``attention_tc`` with
+    ``beside`` follows."""
     _check_element_gate(gate, gate_col, n_heads * head_dim)
     _check_slopes(slopes, n_heads)
     _check_slopes(sink, n_heads)
@@ -654,7 +655,7 @@ def attention_fa(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, ou
           _p(tiles), c_int(n_tiles), _p(block_table), c_int(block_table.shape[-1]), c_int(page), c_int(k_pool.shape[0]),
           c_int(window), c_float(scale), _p(err), c_float(softcap), c_int(chunk),
           (_off(gate, gate_col) if gate is not None else c_void_p(0)), c_int(gate.shape[-1] if gate is not None else 0),
-          _p(slopes), _p(sink), c_void_p(stream if stream is not None else current_stream_ptr()))
+          _p(slopes), _p(sink), c_int(1 if release_late else 0), c_void_p(stream if stream is not None else current_stream_ptr()))
 
 
 def attention_tc(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, out: torch.Tensor, mode: int,
@@ -663,7 +664,7 @@ def attention_tc(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, ou
                  part_o: Optional[torch.Tensor] = None, part_ml: Optional[torch.Tensor] = None,
                  err: Optional[torch.Tensor] = None, stream: Optional[int] = None, softcap: float = 0.0, chunk: int = 0,
                  gate: Optional[torch.Tensor] = None, gate_col: int = 0, slopes: Optional[torch.Tensor] = None,
-                 sink: Optional[torch.Tensor] = None, keys_settled: bool = False) -> None:
+                 sink: Optional[torch.Tensor] = None, keys_settled: bool = False, beside: bool = False) -> None:
     """bf16 attention over the paged cache on tensor cores (TMA-fed); ``softcap`` > 0 caps the scaled scores by a tanh,
     ``chunk`` > 0 lets position i see j only if floor(i / chunk) == floor(j / chunk), ``gate``, ``slopes`` and
     ``sink`` are those of ``attention_fa``.  Splits are ranges of keys from key 0 on, under a chunk from the 64-key tile that holds the chunk's
@@ -672,7 +673,9 @@ def attention_tc(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, ou
     splits' partial results go through those buffers and a second kernel merges them; without them (at most 8
     splits) the splits of a tile are a thread-block cluster and are merged in shared memory.  ``keys_settled`` (mode 1): no
     kernel that may still run on the stream writes the block table or a key or value before a tile's position, as in a
-    step of decoded tokens; they are then read while the kernel before this one still runs."""
+    step of decoded tokens; they are then read while the kernel before this one still runs.  ``beside`` (mode 1): the kernel
+    launched on the stream directly before this one is the ``attention_fa`` of the same step's prompt portions with
+    ``release_late``; the two run at the same time."""
     _check_element_gate(gate, gate_col, n_heads * head_dim)
     _check_slopes(slopes, n_heads)
     _check_slopes(sink, n_heads)
@@ -694,7 +697,7 @@ def attention_tc(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, ou
           c_int(head_dim), _p(tiles), c_int(n_tiles), _p(block_table), c_int(block_table.shape[-1]), c_int(page),
           c_int(k_pool.shape[0]), c_int(window), c_float(scale), c_int(n_splits), c_int(split_keys), _p(part_o),
           _p(part_ml), _p(err), c_float(softcap), c_int(chunk), (_off(gate, gate_col) if gate is not None else c_void_p(0)),
-          c_int(gate.shape[-1] if gate is not None else 0), _p(slopes), _p(sink), c_int(1 if keys_settled else 0),
+          c_int(gate.shape[-1] if gate is not None else 0), _p(slopes), _p(sink), c_int(1 if keys_settled else 0), c_int(1 if beside else 0),
           c_void_p(stream if stream is not None else current_stream_ptr()))
 
 

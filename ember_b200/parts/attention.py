@@ -213,11 +213,13 @@ class Attention(Mixer):
                 ops.attention_tc(q, cache.k, cache.v, out, 0, *args, tiles, n, table, cache.page_tokens, s.window,
                                  self.scale, **kw)
                 return
+            beside = False                      # decoded tokens beside prompt portions: their attention runs beside the portions'
             if self._fa():
                 tiles, n = ctx.attention_tiles(ops.attention_fa_tile_queries(s.group), "multi")
                 if n:
+                    beside = ctx.attention_tiles(1, "single")[1] > 0
                     ops.attention_fa(q, cache.k, cache.v, out, *args, tiles, n, table, cache.page_tokens, s.window,
-                                     self.scale, **kw)
+                                     self.scale, release_late=beside, **kw)
             else:
                 tiles, n = ctx.attention_tiles(tq, "multi")
                 if n:
@@ -244,7 +246,7 @@ class Attention(Mixer):
                     part_o = ctx.buf_dyn("attention.part_o", n * s.num_heads * n_splits * s.head_dim, torch.float32)
                     part_ml = ctx.buf_dyn("attention.part_ml", n * s.num_heads * n_splits * 2, torch.float32)
                 ops.attention_tc(q, cache.k, cache.v, out, 1, *args, tiles, n, table, cache.page_tokens, s.window,
-                                 self.scale, n_splits, split_keys, part_o, part_ml, keys_settled=True, **kw)
+                                 self.scale, n_splits, split_keys, part_o, part_ml, keys_settled=True, beside=beside, **kw)
             return
         if self.softcap > 0 or self.chunk > 0 or any(t is not None for t in (gate, slopes, sink)):
             raise ops.KernelError("attention: the general kernel has no score cap, chunks, gate, slopes or sink (the tensor-core kernels have)")
