@@ -131,23 +131,28 @@ static void best_tile_and_parts(int M, int N, int num_k_blocks, int slots, int u
     }
 }
 
-// Whether pairs of SMs are the faster kernel for 512 to 2,047 tokens against a large matrix (40 million weights and more).
-// Pairs read half of the weight tile each but compute rows in pieces of 256, so it is the last row tile and the last wave
-// that decide: the time of a wave is modelled as k_blocks (a cols + b) + c us with a, b and c fitted to 144 measured
-// products (nine matrices from 10,240 x 4,096 to 151,936 x 2,048, 16 numbers of tokens each) for either kernel.  The choice is
-// within 0.4 % of the better kernel on average and at most 3 % off; pairs throughout were up to 24 % off (us, one SM / pairs:
-// 24,576 x 4,096 gated: 560 tokens 109 / 105, 769 tokens 148 / 165, 1,000 tokens 174 / 164; 51,200 x 5,120 gated: 513 tokens 295 / 345,
-// 768 tokens 355 / 319; 4,096 x 12,288 added: 560 tokens 71 / 65, 1,025 tokens 90 / 112).
+// Whether pairs of SMs are the faster kernel for 256 to 2,047 tokens.  Pairs read half of the weight tile each but compute rows
+// in pieces of 256, so it is the last row tile and the last wave that decide: the time is modelled as waves (k_blocks a cols +
+// b) + c us with a, b and c fitted to 329 measured products for either kernel (fifteen matrices of 1,024 x 3,072 to
+// 151,936 x 2,048, 23 numbers of tokens each; least absolute errors).  The choice is within 0.6 % of the better kernel on average
+// and at most 5 % off; the model of before, of kernels whose issuing threads bounded them, and for large matrices from 512
+// tokens only, was 3.4 % off and at most 21 % (us, one SM / pairs: 12,288 x 2,048 gated 1,280 tokens 54 / 48, 4,096 x 4,096 added 560
+// tokens 27 / 23, 6,144 x 4,096 1,700 tokens 75 / 63, 24,576 x 4,096 gated 440 tokens 89 / 74; 4,096 x 2,048 384 tokens 12.9 / 13.3).
+static double modelled_us(bool pairs, int M, int N, int num_k_blocks, int cols, int parts, int slots) {
+    const int rows = TILE_ROWS * (pairs ? 2 : 1), kb = (num_k_blocks + parts - 1) / parts;
+    const long long n = (long long)((M + rows - 1) / rows) * ((N + cols - 1) / cols) * ((num_k_blocks + kb - 1) / kb);
+    const double waves = (double)((n + slots - 1) / slots);
+    return pairs ? waves * (kb * 0.001412 * cols + 1.316) + 4.81 : waves * (kb * 0.001712 * cols + 0.716) + 3.79;
+}
 static bool pairs_are_faster(int M, int N, int num_k_blocks, bool adds, int num_sms, int max_pairs) {
-    auto us = [&](int slots, int units, double a, double b, double c) {
+    auto us = [&](bool pairs) {
+        const int slots = pairs ? max_pairs : num_sms, units = pairs ? 2 : 1;
         int cols = 0, parts = 1;
         if (adds) best_tile_and_parts(M, N, num_k_blocks, slots, units, &cols, &parts);
         else cols = best_block_cols(M, N, slots, units, nullptr);
-        const int rows = TILE_ROWS * units, kb = (num_k_blocks + parts - 1) / parts;
-        const long long n = (long long)((M + rows - 1) / rows) * ((N + cols - 1) / cols) * ((num_k_blocks + kb - 1) / kb);
-        return (double)((n + slots - 1) / slots) * (kb * (a * cols + b) + c);
+        return modelled_us(pairs, M, N, num_k_blocks, cols, parts, slots);
     };
-    return us(max_pairs, 2, 0.000875, 0.1874, 2.3) <= us(num_sms, 1, 0.00121, 0.1345, 3.8);
+    return us(true) <= us(false);
 }
 
 // A cluster's partial sums in shared memory: every block receives its share of the token columns from all of them.
@@ -416,10 +421,9 @@ EMBER_API int ember_gemm_tc(const void* A, const void* W, void* out, int ldc, in
         col_tiles = 1;
     } else {
         // Prefill-sized products: the single-SM persistent kernel or pairs of SMs (tcgen05 cta_group::2),
-        // each with the tile width that fills its waves best.  Under the power cap pairs are the more efficient
-        // kernel (an SM reads half of the weight tile) and win from about 2,048 tokens on (a 2,048-token prefill
-        // step: 7.55 ms with pairs, 7.9 ms without; at 1,024 tokens the single-SM kernel is 1 % ahead); from 512 on
-        // pairs_are_faster says where they do for large matrices (300 tokens, N 4,096 x K 12,288 added: 71 / 80 us).
+        // each with the tile width that fills its waves best.  Pairs are the more efficient kernel (an SM reads half of
+        // the weight tile) and win from 2,048 tokens on; from 256 on, where fewer rows fill their tiles of 256,
+        // pairs_are_faster says where they do (for the matrices that it was measured on and larger ones).
         // split_mode 4 asks for pairs whenever the device takes them, 5 forbids them, 3 runs one tile per block.
         double cost_single = 0, cost_pair = 0;
         const int bc_single = split_mode == 3 ? (N >= 1024 ? 256 : 128) : best_block_cols(M, N, num_sms, 1, &cost_single);
@@ -428,7 +432,7 @@ EMBER_API int ember_gemm_tc(const void* A, const void* W, void* out, int ldc, in
             if (max_pairs > 0) {
                 const int bc_pair = best_block_cols(M, N, max_pairs, 2, &cost_pair);
                 if (split_mode == 4 || (M >= 2048 && cost_pair <= cost_single * 1.001) ||
-                    (M >= 512 && M < 2048 && (long long)N * K >= 40000000ll &&
+                    (M >= 256 && M < 2048 && N >= 1024 && K >= 1024 &&
                      pairs_are_faster(M, N, p.num_k_blocks, epilogue == 2, num_sms, max_pairs))) {
                     p.epilogue = epilogue; p.out = out; p.ldc = ldc; p.err = err;
                     p.accum = nullptr; p.accum_ld = 0; p.stages = 0;
@@ -667,7 +671,11 @@ EMBER_API int ember_gemm_tc_qkv(const void* A, const void* W, int M, int N, int 
     const int block_cols = (N % 256 == 0) ? 256 : 128;          // whole heads in a tile
     if (split_mode != 5) {
         const int max_pairs = pair_capacity(num_sms);
-        if (max_pairs > 0 && (split_mode == 4 || M >= 2048)) return launch_pair(A, W, p, block_cols, max_pairs, st);
+        // whole heads leave no choice of the width; the model has to see 5 % in pairs (us, one SM / pairs: 4,096 x 2,048 601 tokens
+        // 18.4 / 18.8, 1,280 tokens 28.2 / 25.5; 6,144 x 4,096 512 tokens 31.0 / 29.0, 1,024 tokens 52.1 / 45.9)
+        auto us = [&](bool pairs) { return modelled_us(pairs, M, N, p.num_k_blocks, block_cols, 1, pairs ? max_pairs : num_sms); };
+        if (max_pairs > 0 && (split_mode == 4 || M >= 2048 || (M >= 512 && us(true) <= 0.95 * us(false))))
+            return launch_pair(A, W, p, block_cols, max_pairs, st);
     }
     return launch_persistent(A, W, p, block_cols, num_sms, st);
 }

@@ -162,6 +162,30 @@ def test_gemm_f32_kernels_share_one_order(N, K, epilogue):
         assert torch.equal(out[:M], first[:M]), M
 
 
+@pytest.mark.parametrize("M", [255, 256, 257, 384, 500, 640, 1100, 2047])
+@pytest.mark.parametrize("N,K,epilogue", [(1024, 1024, 0), (1040, 1032, 2), (4096, 2048, 1), (2048, 3072, 2), (6144, 1024, 3), (1023, 1024, 0)])
+def test_gemm_tc_pairs_from_256_tokens(M, N, K, epilogue):
+    """Both sides of the rule for pairs of SMs (256 and 2,048 tokens, 1,024 rows and columns), odd sizes: the same outputs as
+    one SM a tile."""
+    from ember_b200 import ops
+    torch.manual_seed(M + N)
+    a, w = torch.randn(M, K, device="cuda").bfloat16(), (torch.randn(N, K, device="cuda") * 0.02).bfloat16()
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    prev = torch.randn(M + 1, N, device="cuda")
+    outs = []
+    for mode in (0, 4, 5):
+        out = prev.clone() if epilogue in (1, 2) else torch.zeros(M + 1, N // 2 if epilogue == 3 else N, device="cuda", dtype=torch.bfloat16)
+        ops.gemm_tc(a, w, out, M, epilogue, err=err, split_mode=mode)
+        outs.append(out)
+    want = ref_epilogue(a.float() @ w.float().t(), epilogue, prev[:M])
+    for out in outs:
+        assert int(err.item()) == 0 and torch.equal(out[M], outs[2][M])
+        if epilogue == 2:
+            assert rel(out[:M], want) < 1e-5                  # (parts of K added in any order)
+        else:
+            assert torch.equal(out, outs[2]) and rel(out[:M].float(), want) < (1e-5 if epilogue == 1 else 5e-3)
+
+
 @pytest.mark.parametrize("M", [511, 512, 560, 769, 1025, 2047, 2048])
 @pytest.mark.parametrize("N,K,epilogue", [(10240, 4096, 0), (24576, 1640, 3), (4096, 9768, 2), (4096, 9760, 2)])
 def test_gemm_tc_pairs_for_large_matrices(M, N, K, epilogue):
