@@ -9,8 +9,8 @@
 //   * float x float with rows of whole 16-byte pieces (every product of the float32 path): K is
 //     cut into KPARTS parts, a part's elements of even k and of odd k are summed apart with k
 //     ascending, and the sums are added in order.  The parts are what lets a product of few tokens
-//     keep the whole chip busy; two kernels share this order, one for few tokens (bound by the
-//     weights' way in) and one for many (bound by the FMA pipes).
+//     keep the whole chip busy; three kernels share this order, one for few tokens (bound by the
+//     weights' way in), one for many (bound by the FMA pipes) and one for many and few columns.
 //   * anything else: k ascending over the whole row, the kernel for all sizes.
 //
 // Epilogues (the reference's are src/backend/cuda/k_gemm.cu:29-53):
@@ -19,6 +19,8 @@
 //   6 relu(c[2j]) * c[2j+1] likewise     7 gelu(c[2j]) * c[2j+1], gelu in its tanh form
 //   8 gelu(c) in its exact form (erf), stored in the activation dtype     9 max(c, 0)^2 likewise
 // An optional fp32 bias[N] is added before the epilogue.
+#include <type_traits>
+
 #include "common.cuh"
 
 EMBER_DEFINE_LAST_ERROR
@@ -161,14 +163,14 @@ __device__ __forceinline__ void finish_pair(float c0, float c1, const float* __r
 // Four tokens at the 0.6B widths (hidden 1,024), in a step: o and down 9.0 and 13.8 us, q/k/v and gate/up 5, the head's
 // 622 MB 100 us (6.2 TB/s); with the general kernel everywhere four requests of 75 tokens and four more steps took 143 ms,
 // with this one and the next 23.
-constexpr int FEW_K = 32, FEW_STAGES = 3, FEW_ROW = FEW_K + 4;
+constexpr int FEW_K = 32, FEW_ROW = FEW_K + 4;
 
 template <int MT, int NB>
 constexpr size_t few_stage_floats() { return 32 * FEW_ROW + (32 / NB) * MT * FEW_K; }
-template <int MT, int NB>
+template <int MT, int NB, int FEW_STAGES>
 constexpr size_t few_smem() { return (NB * KPARTS / 32) * FEW_STAGES * few_stage_floats<MT, NB>() * sizeof(float); }
 
-template <int MT, int NB>
+template <int MT, int NB, int FEW_STAGES>
 __global__ void __launch_bounds__(NB * KPARTS)
 gemm_f32_few_kernel(const float* __restrict__ A, int lda, const float* __restrict__ W, int ldw, const float* __restrict__ bias,
                     float* __restrict__ C, int ldc, int M, int N, int K, int epi, int settled) {
@@ -363,6 +365,160 @@ gemm_f32_many_kernel(const float* __restrict__ A, int lda, const float* __restri
     }
 }
 
+// Many tokens and few columns: with one block a tile the tiles above are one to three waves of blocks, the last of them mostly
+// empty.  Here a cluster of four blocks makes a tile of 64 tokens x 64 columns, two to an SM: two parts of K a block, a warp
+// for the even and one for the odd elements of k of each part.  A thread keeps 16 tokens x 8 columns of that sum, paired along
+// the tokens; operands lie k-major, brought by 4-byte copies whose 8 k x 4 rows fall into 32 banks into a ring of three
+// stages that the two warps of a part share.  The parts of a tile meet in distributed shared memory, every block finishes
+// a quarter of its tokens.  The sums are those of the kernel above, in its order.
+// us, kernel above -> this, at (N, K) = (1,024, 2,048), (1,024, 3,072), (2,048, 2,048): 64 tokens 37 -> 31, 53 -> 44, 38 -> 34; 128
+// tokens 37 -> 34, 54 -> 47, 38 -> 35; 300 tokens 68 -> 50, 98 -> 71, 103 -> 80; 2,048 tokens 247 -> 234, 358 -> 330, 488 -> 449.
+// From 4,096 columns on it is ahead where rows of 64 are full (300 tokens x 4,096 x 1,024: 93 -> 88) and behind where they are not
+// (65 tokens x 6,144 x 1,024: 37 -> 53), so those stay with the kernel above.  Neither gets beyond 34 TFLOP/s: the same sums by
+// plain multiply-adds take 119 us where these take 88, and operands loaded 16 bytes at a time into registers and stored
+// turned 104.
+constexpr int NARROW_T = 64, NARROW_N = 64, NARROW_K = 16, NARROW_STAGES = 3, NARROW_CLUSTER = 4, NARROW_PARTS = KPARTS / NARROW_CLUSTER;
+constexpr int NARROW_ROW = NARROW_N + 4;                          // floats of a k in a stage's operand, and of a row of sums
+constexpr int NARROW_STAGE = 2 * NARROW_K * NARROW_ROW;           // floats
+constexpr size_t NARROW_SMEM = (size_t)NARROW_PARTS * NARROW_STAGES * NARROW_STAGE * sizeof(float);
+static_assert(NARROW_T == NARROW_N && NARROW_SMEM >= (size_t)NARROW_PARTS * NARROW_T * NARROW_ROW * sizeof(float), "the parts' tiles take the stages' place");
+
+// 4 bytes from global to shared memory; zero when !valid.
+__device__ __forceinline__ void copy4(float* dst, const float* src, bool valid) {
+    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(d), "l"(src), "r"(valid ? 4 : 0) : "memory");
+}
+__device__ __forceinline__ unsigned long long pack_pair(float lo, float hi) {
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(__float_as_uint(lo)), "r"(__float_as_uint(hi)));
+    return r;
+}
+
+__global__ void __cluster_dims__(NARROW_CLUSTER, 1, 1) __launch_bounds__(NARROW_PARTS * 64, 2)
+gemm_f32_narrow_kernel(const float* __restrict__ A, int lda, const float* __restrict__ W, int ldw, const float* __restrict__ bias,
+                       float* __restrict__ C, int ldc, int M, int N, int K, int epi, int settled) {
+    extern __shared__ __align__(16) float narrow_shared[];
+    pdl_launch_dependents();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, tx = lane & 7, ty = lane >> 3;
+    const int local = warp >> 1, odd = warp & 1, rank = blockIdx.x % NARROW_CLUSTER;
+    const int n0 = (int)(blockIdx.x / NARROW_CLUSTER) * NARROW_N, m0 = blockIdx.y * NARROW_T;
+    const int len = part_length(K), steps = len / NARROW_K, k_first = (rank * NARROW_PARTS + local) * len;
+    float* stages = narrow_shared + local * NARROW_STAGES * NARROW_STAGE;
+    const int ck = odd * 8 + tx;                                  // a warp copies 8 of a stage's 16 elements of k
+
+    auto fetch = [&](float* dst, const float* X, int ldx, int first, int count, int step) {
+        const int k = k_first + step * NARROW_K + ck;
+        const float* src = X + (size_t)(first + ty) * ldx + k;
+#pragma unroll
+        for (int r = 0; r < 64; r += 4) {
+            const bool ok = first + r + ty < count && k < K;
+            copy4(dst + ck * NARROW_ROW + ty + r, ok ? src + (size_t)r * ldx : X, ok);
+        }
+    };
+    auto fetch_w = [&](int step) { fetch(stages + (step % NARROW_STAGES) * NARROW_STAGE + NARROW_K * NARROW_ROW, W, ldw, n0, N, step); };
+    auto fetch_a = [&](int step) { fetch(stages + (step % NARROW_STAGES) * NARROW_STAGE, A, lda, m0, M, step); };
+    auto pair_sync = [&] { asm volatile("bar.sync %0, 64;" ::"r"(local + 1) : "memory"); };
+    if (!settled) pdl_wait();
+#pragma unroll
+    for (int s = 0; s < NARROW_STAGES - 1; s++)
+        if (s < steps) fetch_w(s);
+    pdl_wait();
+#pragma unroll
+    for (int s = 0; s < NARROW_STAGES - 1; s++) {
+        if (s < steps) fetch_a(s);
+        copies_commit();
+    }
+
+    // tokens 16 g + 4 ty + 0..3 (pairs), columns 32 h + 4 tx + 0..3
+    unsigned long long acc[8][8];
+#pragma unroll
+    for (int i = 0; i < 8; i++)
+#pragma unroll
+        for (int j = 0; j < 8; j++) acc[i][j] = 0;
+    for (int step = 0; step < steps; step++) {
+        copies_wait<NARROW_STAGES - 2>();
+        pair_sync();                                              // both warps' copies of this stage are there, the one before is read
+        if (step + NARROW_STAGES - 1 < steps) {
+            fetch_w(step + NARROW_STAGES - 1);
+            fetch_a(step + NARROW_STAGES - 1);
+        }
+        copies_commit();
+        const float* as = stages + (step % NARROW_STAGES) * NARROW_STAGE + odd * NARROW_ROW + ty * 4;
+        const float* ws = stages + (step % NARROW_STAGES) * NARROW_STAGE + (NARROW_K + odd) * NARROW_ROW + tx * 4;
+#pragma unroll
+        for (int k = 0; k < NARROW_K; k += 2) {
+            ulonglong2 a[4];
+            float4 w[2];
+#pragma unroll
+            for (int g = 0; g < 4; g++) a[g] = *(const ulonglong2*)(as + k * NARROW_ROW + g * 16);
+#pragma unroll
+            for (int h = 0; h < 2; h++) w[h] = *(const float4*)(ws + k * NARROW_ROW + h * 32);
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                const unsigned long long w2[4] = {pack_pair(w[h].x, w[h].x), pack_pair(w[h].y, w[h].y), pack_pair(w[h].z, w[h].z), pack_pair(w[h].w, w[h].w)};
+#pragma unroll
+                for (int j = 0; j < 4; j++)
+#pragma unroll
+                    for (int g = 0; g < 4; g++) {
+                        acc[2 * g][h * 4 + j] = fma_pair(a[g].x, w2[j], acc[2 * g][h * 4 + j]);
+                        acc[2 * g + 1][h * 4 + j] = fma_pair(a[g].y, w2[j], acc[2 * g + 1][h * 4 + j]);
+                    }
+            }
+        }
+    }
+    copies_wait<0>();
+    __syncthreads();
+
+    // a part: the sums of even k, then those of odd k added
+    float* part = narrow_shared + local * NARROW_T * NARROW_ROW;  // [tokens][NARROW_ROW]
+#pragma unroll
+    for (int who = 0; who < 2; who++) {
+        if (odd == who) {
+#pragma unroll
+            for (int i = 0; i < 8; i++)
+#pragma unroll
+                for (int half = 0; half < 2; half++) {
+                    const int m = (i >> 1) * 16 + ty * 4 + (i & 1) * 2 + half;
+#pragma unroll
+                    for (int h = 0; h < 2; h++) {
+                        float* dst = part + m * NARROW_ROW + h * 32 + tx * 4;
+                        float v[4];
+#pragma unroll
+                        for (int j = 0; j < 4; j++) v[j] = __uint_as_float((unsigned)(acc[i][h * 4 + j] >> (32 * half)));
+                        if (who == 1) {
+                            const float4 even = *(const float4*)dst;
+                            v[0] = even.x + v[0]; v[1] = even.y + v[1]; v[2] = even.z + v[2]; v[3] = even.w + v[3];
+                        }
+                        *(float4*)dst = make_float4(v[0], v[1], v[2], v[3]);
+                    }
+                }
+        }
+        pair_sync();
+    }
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    // this block's quarter of the tokens, the parts in order
+    uint32_t base[KPARTS];
+#pragma unroll
+    for (int q = 0; q < KPARTS; q++) {
+        const uint32_t mine = (uint32_t)__cvta_generic_to_shared(narrow_shared + (q % NARROW_PARTS) * NARROW_T * NARROW_ROW);
+        asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(base[q]) : "r"(mine), "r"(q / NARROW_PARTS));
+    }
+    constexpr int SHARE = NARROW_T / NARROW_CLUSTER;
+    for (int i = threadIdx.x; i < SHARE * NARROW_N / 2; i += NARROW_PARTS * 64) {
+        const int m = rank * SHARE + i / (NARROW_N / 2), n = (i % (NARROW_N / 2)) * 2;
+        if (m0 + m >= M || n0 + n >= N) continue;
+        float2 d[KPARTS];
+#pragma unroll
+        for (int q = 0; q < KPARTS; q++)
+            asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(d[q].x), "=f"(d[q].y) : "r"(base[q] + (uint32_t)((m * NARROW_ROW + n) * 4)));
+        float2 c = d[0];
+#pragma unroll
+        for (int q = 1; q < KPARTS; q++) { c.x += d[q].x; c.y += d[q].y; }
+        finish_pair(c.x, c.y, bias, C, ldc, m0 + m, n0 + n, N, epi);
+    }
+    asm volatile("barrier.cluster.arrive.aligned;\nbarrier.cluster.wait.aligned;" ::: "memory");      // (nobody leaves while its parts are read)
+}
+
 template <typename Kernel>
 int launch_f32(Kernel kernel, dim3 grid, int threads, size_t smem, cudaStream_t st, const float* A, int lda, const float* W, int ldw,
                const float* bias, float* C, int ldc, int M, int N, int K, int epi, int settled) {
@@ -380,15 +536,25 @@ int launch_f32(Kernel kernel, dim3 grid, int threads, size_t smem, cudaStream_t 
 //           4,096 x 1,024  29 / 24  28 / 25     6,144 x 1,024  23 / 20  22 / 20    12,288 x 2,048  77 / 68  76 / 70
 //         151,936 x 1,024  432 / 303  426 / 317
 constexpr int FEW_TOKENS = 32, FEW_TOKENS_WIDE = 16, WIDE_COLUMNS = 4096;
+// More than 32 tokens: the kernel of clusters up to this many columns (its comment has both sides).
+constexpr int NARROW_COLUMNS = 2048;
 
 template <int MT>
 int launch_few(const float* A, int lda, const float* W, int ldw, const float* bias, float* C, int ldc, int M, int N, int K, int epi,
                int settled, cudaStream_t st) {
     const unsigned y = (unsigned)((M + MT - 1) / MT);
-    // blocks of 16 weight rows once they fill the SMs twice, else of 8
-    if (N >= 16 * 296)
-        return launch_f32(gemm_f32_few_kernel<MT, 16>, dim3((N + 15) / 16, y), 16 * KPARTS, few_smem<MT, 16>(), st, A, lda, W, ldw, bias, C, ldc, M, N, K, epi, settled);
-    return launch_f32(gemm_f32_few_kernel<MT, 8>, dim3((N + 7) / 8, y), 8 * KPARTS, few_smem<MT, 8>(), st, A, lda, W, ldw, bias, C, ldc, M, N, K, epi, settled);
+    auto run = [&](auto nb, auto depth) {
+        constexpr int NB = decltype(nb)::value, ST = decltype(depth)::value;
+        return launch_f32(gemm_f32_few_kernel<MT, NB, ST>, dim3((N + NB - 1) / NB, y), NB * KPARTS, few_smem<MT, NB, ST>(), st, A, lda, W, ldw, bias, C, ldc, M, N, K, epi, settled);
+    };
+    using std::integral_constant;
+    // blocks of 16 weight rows once they fill the SMs twice, else of 8; where there is no more than one of those for an SM, the
+    // two warps of a block are all that fetches there, and look eight stages ahead instead of three (1,024 rows of K 2,048 /
+    // 3,072, 4 tokens 8.1 / 11.1 -> 6.0 / 8.2 us, 16 tokens 16.4 / 23.4 -> 11.5 / 15.3; 4,096 rows of K 1,024 would lose, 4 tokens 7.1
+    // -> 8.0, 16 tokens 14.3 -> 23.8)
+    if (N >= 16 * 296) return run(integral_constant<int, 16>(), integral_constant<int, 3>());
+    if (MT >= 4 && (unsigned)(N + 7) / 8 * y <= 148) return run(integral_constant<int, 8>(), integral_constant<int, 8>());
+    return run(integral_constant<int, 8>(), integral_constant<int, 3>());
 }
 
 int launch_pieces(const float* A, int lda, const float* W, int ldw, const float* bias, float* C, int ldc, int M, int N, int K, int epi,
@@ -399,11 +565,16 @@ int launch_pieces(const float* A, int lda, const float* W, int ldw, const float*
     if (M <= 8) return launch_few<8>(A, lda, W, ldw, bias, C, ldc, M, N, K, epi, settled, st);
     if (M <= (N >= WIDE_COLUMNS ? FEW_TOKENS_WIDE : FEW_TOKENS)) return launch_few<16>(A, lda, W, ldw, bias, C, ldc, M, N, K, epi, settled, st);
     // a grid has at most 65,535 rows of blocks, half as many tokens here as the 64-row tiles of the general kernel take
+    const bool narrow = M > 32 && N <= NARROW_COLUMNS;
     constexpr int ROWS = 65535 * MANY_M;
     for (long long m = 0; m < M; m += ROWS) {
         const int rows = M - m < ROWS ? (int)(M - m) : ROWS;
-        const int rc = launch_f32(gemm_f32_many_kernel, dim3((N + MANY_N - 1) / MANY_N, (rows + MANY_M - 1) / MANY_M), KPARTS * 32, MANY_SMEM, st,
-                                  A + (size_t)m * lda, lda, W, ldw, bias, C + (size_t)m * ldc, ldc, rows, N, K, epi, settled);
+        const float* a = A + (size_t)m * lda;
+        float* c = C + (size_t)m * ldc;
+        const int rc = narrow ? launch_f32(gemm_f32_narrow_kernel, dim3((N + NARROW_N - 1) / NARROW_N * NARROW_CLUSTER, (rows + NARROW_T - 1) / NARROW_T), NARROW_PARTS * 64,
+                                           NARROW_SMEM, st, a, lda, W, ldw, bias, c, ldc, rows, N, K, epi, settled)
+                              : launch_f32(gemm_f32_many_kernel, dim3((N + MANY_N - 1) / MANY_N, (rows + MANY_M - 1) / MANY_M), KPARTS * 32, MANY_SMEM, st, a, lda, W, ldw,
+                                           bias, c, ldc, rows, N, K, epi, settled);
         if (rc) return rc;
     }
     return 0;

@@ -162,6 +162,30 @@ def test_gemm_f32_kernels_share_one_order(N, K, epilogue):
         assert torch.equal(out[:M], first[:M]), M
 
 
+@pytest.mark.parametrize("M", [33, 63, 64, 65, 128, 129, 300])
+@pytest.mark.parametrize("N,K", [(2, 4), (62, 260), (64, 1024), (1024, 1000), (2046, 132), (2048, 2048), (2050, 132)])
+@pytest.mark.parametrize("epilogue", [0, 2, 3])
+def test_gemm_f32_narrow(M, N, K, epilogue):
+    """float32 products of more than 32 tokens on both sides of the line between the two kernels (2,048 columns) and at the
+    edges of their tiles: the bits that single tokens get."""
+    from ember_b200 import ops
+    torch.manual_seed(N + K + M)
+    a, w, bias = torch.randn(M, K, device="cuda"), torch.randn(N, K, device="cuda"), torch.randn(N, device="cuda")
+    n_out = N // 2 if epilogue == 3 else N
+    prev = torch.randn(M + 1, n_out, device="cuda")
+    out = prev.clone()
+    ops.gemm_simt(a, w, out, M, epilogue, bias=bias)
+    assert torch.equal(out[M], prev[M])
+    rows = [0, M // 2, M - 1]
+    for r in rows:
+        one = prev[r:r + 1].clone()
+        ops.gemm_simt(a[r:r + 1].contiguous(), w, one, 1, epilogue, bias=bias)
+        assert torch.equal(one[0], out[r])
+    c = a.double() @ w.double().t() + bias.double()
+    want = c[:, 0::2] * torch.sigmoid(c[:, 0::2]) * c[:, 1::2] if epilogue == 3 else c + (prev[:M].double() if epilogue == 2 else 0.0)
+    assert rel(out[:M].double(), want) < 2e-6
+
+
 @pytest.mark.parametrize("M", [255, 256, 257, 384, 500, 640, 1100, 2047])
 @pytest.mark.parametrize("N,K,epilogue", [(1024, 1024, 0), (1040, 1032, 2), (4096, 2048, 1), (2048, 3072, 2), (6144, 1024, 3), (1023, 1024, 0)])
 def test_gemm_tc_pairs_from_256_tokens(M, N, K, epilogue):
