@@ -25,6 +25,7 @@ EPI_GELU = 8      # gelu(c + bias) in its exact form, 0.5 z (1 + erf(z / sqrt 2)
 EPI_SQUARE_RELU = 9      # max(c + bias, 0)^2, stored like EPI_STORE
 PLAIN_EPILOGUES = (EPI_STORE, EPI_STORE_F32, EPI_ADD_F32, EPI_GELU, EPI_SQUARE_RELU)      # those that take a bias in both products
 GATED_EPILOGUES = (EPI_SILU_MUL, EPI_RELU_MUL, EPI_GELU_MUL)
+BF16_EPILOGUES = (EPI_STORE, EPI_GELU, EPI_SQUARE_RELU) + GATED_EPILOGUES      # what the tensor-core product stores in bfloat16
 GATED_EPILOGUE_OF = {"silu": EPI_SILU_MUL, "relu": EPI_RELU_MUL, "gelu_tanh": EPI_GELU_MUL}
 
 
@@ -412,7 +413,8 @@ def reserve_scratch(device, floats: int) -> torch.Tensor:
     """Makes the split-K scratch at least ``floats`` long.  A ``Linear`` reserves 128 x its output width when it
     is built, so that a loaded model never grows the scratch inside a step."""
     global _scratch_version
-    device = torch.device(device)
+    if not isinstance(device, torch.device):
+        device = torch.device(device)
     t = _tc_scratch.get(device)
     if t is None or t.numel() < floats:
         t = torch.zeros(max(int(floats), 1 << 20), dtype=torch.float32, device=device)
@@ -467,7 +469,7 @@ def gemm_tc(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, M: int, epilogu
         return scratch[:M * N].view(M, N)
     _check(out, "out")
     n_out = N // 2 if epilogue in GATED_EPILOGUES else N
-    want = torch.bfloat16 if epilogue in (EPI_STORE, EPI_GELU, EPI_SQUARE_RELU) + GATED_EPILOGUES else torch.float32
+    want = torch.bfloat16 if epilogue in BF16_EPILOGUES else torch.float32
     if out.dtype != want:
         raise KernelError(f"gemm: epilogue {epilogue} writes {want}, the output is {out.dtype}")
     if out.shape[-1] != n_out or out.numel() < M * n_out or a.numel() < M * K:
@@ -476,10 +478,11 @@ def gemm_tc(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, M: int, epilogu
         _check(bias, "bias", torch.float32)
         if bias.numel() != N or epilogue not in PLAIN_EPILOGUES:
             raise KernelError(f"gemm: a bias of {bias.numel()} for N={N} under epilogue {epilogue}")
-    scratch = _scratch(a.device, min(M, 128) * N) if M <= 128 else None
+    device = a.device
+    scratch = reserve_scratch(device, M * N) if M <= 128 else None
     lib = _lib("gemm_tc")
     _call(lib, lib.ember_gemm_tc, _p(a), _p(w), _p(out), c_int(n_out), c_int(M), c_int(N), c_int(K), c_int(epilogue), _p(bias),
-          _p(scratch), c_longlong(scratch.numel() if scratch is not None else 0), c_int(_sms(a.device)), c_int(split_mode),
+          _p(scratch), c_longlong(scratch.numel() if scratch is not None else 0), c_int(_sms(device)), c_int(split_mode),
           _p(err),
           c_void_p(stream if stream is not None else current_stream_ptr()))
 

@@ -180,11 +180,11 @@ class Attention(Mixer):
         return (ops.attention_tc_supported(s.head_dim, s.group, rt.page_tokens, 0),
                 ops.attention_tc_supported(s.head_dim, s.group, rt.page_tokens, 1))
 
-    def _fa(self) -> bool:
-        """Whether prompt portions go to the tcgen05 kernel (needs the single-token kernel beside it)."""
+    def _fa(self, single: Optional[bool] = None) -> bool:
+        """Whether prompt portions go to the tcgen05 kernel (needs the single-token kernel beside it: ``single``, if known)."""
         s, rt = self.spec, self.rt
         return (rt.dtype == torch.bfloat16 and ops.attention_fa_supported(s.head_dim, s.group, rt.page_tokens)
-                and self._tc_modes()[1])
+                and (self._tc_modes()[1] if single is None else single))
 
     def tile_requests(self):
         s = self.spec
@@ -214,7 +214,7 @@ class Attention(Mixer):
                                  self.scale, **kw)
                 return
             beside = False                      # decoded tokens beside prompt portions: their attention runs beside the portions'
-            if self._fa():
+            if self._fa(single):
                 tiles, n = ctx.attention_tiles(ops.attention_fa_tile_queries(s.group), "multi")
                 if n:
                     beside = ctx.attention_tiles(1, "single")[1] > 0
