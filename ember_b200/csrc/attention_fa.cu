@@ -70,7 +70,8 @@ struct FaParams {
     const float* sink;        // [n_heads] or null: exp(sink[h]) joins the denominator, without key and value
     float raw_per_slope;      // what a slope of 1 is in the units of the scores as they come: 1 / scale, or log2(e) behind a cap
     int n_tiles;
-    int release_late;         // the next kernel may start (and read what this one reads) once this one's inputs are there
+    unsigned long long* released;      // where the kernel behind this one finds `ticket` once this one's inputs are there, or null
+    unsigned long long ticket;         // (a number of its own for each launch)
     int* err;
 };
 
@@ -375,9 +376,13 @@ attention_fa_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
     const uint32_t tmem = *tmem_slot;
     const uint32_t tmem_s0 = tmem, tmem_o0 = tmem + 128;  // S buffers at columns 0 and 64, O at 128
 
-    if (!p.release_late) pdl_launch_dependents();
+    if (!p.released) pdl_launch_dependents();
     pdl_wait();
-    if (p.release_late) pdl_launch_dependents();
+    if (p.released && threadIdx.x == 0) {
+        // (what this thread has waited for, whoever acquires the ticket sees)
+        if (blockIdx.x == 0) release_ticket(p.released, p.ticket);
+        pdl_launch_dependents();
+    }
 
     if (warp == FA_ROW_WARPS) {
         // ---------------------------------------------------------------- page fetcher
@@ -705,7 +710,7 @@ EMBER_API int ember_attention_fa_tile_queries(int group) { return group >= 1 && 
 EMBER_API int ember_attention_fa(const void* q, const void* k_pool, const void* v_pool, void* out, int n_heads, int n_kv,
                                  int D, const int* tiles, int n_tiles, const int* block_table, int max_blocks, int page,
                                  int num_pages, int window, float scale, int* err, float softcap, int chunk, const float* gate, int ld_gate,
-                                 const float* slopes, const float* sink, int release_late, void* stream) {
+                                 const float* slopes, const float* sink, unsigned long long* released, unsigned long long ticket, void* stream) {
     if (n_tiles <= 0) return 0;
     if (gate && ((((uintptr_t)gate) & 15) || ld_gate < n_heads * FA_D || (ld_gate & 3))) return fail("attention_fa: gate rows of %d", ld_gate);
     if (n_heads <= 0 || n_kv <= 0 || n_heads % n_kv) return fail("attention_fa: bad head counts %d/%d", n_heads, n_kv);
@@ -723,7 +728,8 @@ EMBER_API int ember_attention_fa(const void* q, const void* k_pool, const void* 
     if (scale <= 0.0f) return fail("attention_fa: a score scale of %g (it must be positive)", scale);
     p.cap_log2 = softcap * FA_LOG2E;
     p.cap_z = softcap > 0.0f ? scale / softcap : 0.0f;
-    p.cap_arg = softcap > 0.0f ? 2.0f * FA_LOG2E * scale / softcap : 0.0f; p.gate = gate; p.ld_gate = ld_gate; p.n_tiles = n_tiles; p.release_late = release_late ? 1 : 0; p.err = err;
+    p.cap_arg = softcap > 0.0f ? 2.0f * FA_LOG2E * scale / softcap : 0.0f; p.gate = gate; p.ld_gate = ld_gate; p.n_tiles = n_tiles; p.err = err;
+    p.released = released && !is_capturing((cudaStream_t)stream) ? released : nullptr; p.ticket = ticket;
     p.slopes = slopes; p.sink = sink; p.raw_per_slope = softcap > 0.0f ? FA_LOG2E : 1.0f / scale;
     auto run = [&](auto kernel, bool& ready) -> int {
         if (!ready) {

@@ -56,7 +56,8 @@ struct AttnTcParams {
     const float* sink;        // [n_heads] or null: exp(sink[h]) joins the denominator once, without key and value
     int n_splits, split_keys;
     int n_tiles;
-    int beside;               // decode: the kernel before this one reads what this one reads and let it go once that was there
+    const unsigned long long* released;      // decode: where attention_fa, launched directly before, leaves `ticket` once what both read is there, or null
+    unsigned long long ticket;
     int settled;              // decode: nothing that may still run writes keys or pages before the tile's position
     int cluster_merge;        // the splits of a tile are a thread-block cluster and are merged in its first block's shared memory
     int* err;
@@ -224,16 +225,21 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
     // still runs: a layer's attention took 9.9, 25.1 and 43.9 us (one request at 700 keys, 8 at 3,072, 64 at 1,024), now 8.3,
     // 23.4, 39.1.
     int early = 0;
-    if (DECODE && warp == 4) {
-        if (!p.settled && !p.beside) pdl_wait();
+    if (DECODE && warp == 4 && (p.settled || !p.released)) {
+        if (!p.settled) pdl_wait();
         early = min(min(n_kt, NSTAGE), max(0, (pos0 - k_begin) / KT));
         for (int it = 0; it < early; it++) fetch_tile(it, page_row(it));
     }
-    // Queries and the newest keys are written by the kernel before this one; `beside` the step's prompt portions, whose
-    // attention released this kernel behind its own wait for them, they are there already, and the two kernels run at the
-    // same time: one streams the cache, the other computes (eight layers of 32/8 heads, 512 tokens behind 512 keys beside 48
-    // requests of 600 to 1,200: 2,834 us a step one after the other, 2,749 side by side).
-    if (!DECODE || !p.beside) pdl_wait();
+    // Queries and the newest keys are written by the kernel before this one.  Beside the step's prompt portions it is the
+    // kernel before theirs: behind the ticket that theirs leaves (common.cuh) both are there, and the two kernels run at the same
+    // time: one streams the cache, the other computes (eight layers of 32/8 heads, 512 tokens behind 512 keys beside 48
+    // requests of 600 to 1,200: 2,834 us a step one after the other, 2,709 to 2,749 side by side).
+    bool there = false;
+    if (DECODE && p.released) {
+        there = __syncthreads_or(threadIdx.x == 0 && acquire_ticket(p.released) == p.ticket);
+        if (there) asm volatile("fence.proxy.async.global;" ::: "memory");      // (the newest key's page is fetched by TMA)
+    }
+    if (!there) pdl_wait();
 
     // ---- query rows -> shared memory (row r = token r / G, head kvh * G + r % G), zero beyond `rows`
     for (int idx = threadIdx.x; idx < QROWS * (D / 8); idx += ATC_THREADS) {
@@ -521,7 +527,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
                 __float2bfloat16_rn(gated(gate_row, r * D + d, acc * with_sink(BIAS ? p.sink : nullptr, kvh * G + r, M, L)));
         }
     }
-    if (p.beside) pdl_wait();      // (so that who waits for this kernel waits for the one beside it, too)
+    if (there) pdl_wait();      // (so that who waits for this kernel waits for the one beside it, too)
 }
 
 // Merges split partials in ascending order (same arithmetic as attention.cu's combine).  The maxima and
@@ -659,7 +665,8 @@ EMBER_API int ember_attention_tc(const void* q, const void* k_pool, const void* 
                                  int n_heads, int n_kv, int D, const int* tiles, int n_tiles,
                                  const int* block_table, int max_blocks, int page, int num_pages, int window,
                                  float scale, int n_splits, int split_keys, float* part_o, float* part_ml,
-                                 int* err, float softcap, int chunk, const float* gate, int ld_gate, const float* slopes, const float* sink, int settled, int beside, void* stream) {
+                                 int* err, float softcap, int chunk, const float* gate, int ld_gate, const float* slopes, const float* sink, int settled,
+                                 const unsigned long long* released, unsigned long long ticket, void* stream) {
     if (n_tiles <= 0) return 0;
     if (gate && ld_gate < n_heads * D) return fail("attention_tc: gate rows of %d", ld_gate);
     if (softcap < 0.0f) return fail("attention_tc: a score cap of %g", softcap);
@@ -686,7 +693,8 @@ EMBER_API int ember_attention_tc(const void* q, const void* k_pool, const void* 
     p.cap_log2 = softcap * LOG2E; p.cap_arg = softcap > 0.0f ? 2.0f * LOG2E * scale / softcap : 0.0f;
     p.gate = gate; p.ld_gate = ld_gate; p.slopes = slopes; p.sink = sink;
     p.n_splits = n_splits; p.split_keys = split_keys; p.n_tiles = n_tiles; p.err = err;
-    p.cluster_merge = cluster_merge ? 1 : 0; p.settled = settled ? 1 : 0; p.beside = mode == 1 && beside ? 1 : 0;
+    p.cluster_merge = cluster_merge ? 1 : 0; p.settled = settled ? 1 : 0;
+    p.released = mode == 1 && released && !is_capturing((cudaStream_t)stream) ? released : nullptr; p.ticket = ticket;
     cudaStream_t st = (cudaStream_t)stream;
     const size_t tile_bytes = (size_t)(D / 64) * KT * 128;
     const size_t q_bytes = ((size_t)(D / 64) * (mode == 1 ? 16 : 64) * 128 + 1023) & ~(size_t)1023;

@@ -52,10 +52,31 @@ inline int check_launch(const char* what) {
 // Programmatic dependent launch.  Every kernel is launched with the stream-serialization attribute,
 // so its blocks may start while the kernel before it is still draining; until pdl_wait() returns a
 // kernel touches nothing that an earlier kernel of the step writes.  It may set up barriers, read the step's uploaded
-// integers and prefetch what its caller says is settled: weights, and the keys of earlier steps.
+// integers and prefetch what its caller says is settled: weights, and the keys of earlier steps.  The one exception acquires a
+// ticket instead (below).
 // pdl_wait() returns at once when the launch carried no such dependency.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// A kernel that is to run beside the one in front of it (attention_tc.cu beside attention_fa.cu) cannot wait for that one,
+// and launch_dependents orders no memory.  So the one in front, behind its own pdl_wait(), stores a ticket with release
+// semantics, and the other reads it with acquire semantics: all that the first had waited for happens before what the second
+// does then (other threads of its block: behind a block barrier).  Each launch has a ticket of its own, and who does not
+// find it waits with pdl_wait(): this decides, it never spins.
+__device__ __forceinline__ void release_ticket(unsigned long long* at, unsigned long long ticket) {
+    asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(at), "l"(ticket) : "memory");
+}
+__device__ __forceinline__ unsigned long long acquire_ticket(const unsigned long long* at) {
+    unsigned long long v;
+    asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(at) : "memory");
+    return v;
+}
+// A captured launch would find the ticket of the replay before: none there.
+inline bool is_capturing(cudaStream_t stream) {
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream, &status) != cudaSuccess) { cudaGetLastError(); return true; }
+    return status != cudaStreamCaptureStatusNone;
+}
 
 inline bool pdl_enabled() {
     static int on = -1;

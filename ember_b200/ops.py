@@ -7,7 +7,8 @@ sizes.  Tensors are torch tensors used as typed device buffers.
 from __future__ import annotations
 
 import ctypes
-from ctypes import c_float, c_longlong, c_void_p
+import itertools
+from ctypes import c_float, c_longlong, c_ulonglong, c_void_p
 from operator import index
 from typing import Optional
 
@@ -631,6 +632,26 @@ def _check_element_gate(gate, col: int, n: int) -> None:
             raise KernelError(f"attention: a gate of {tuple(gate.shape)} from column {col} for {n} elements a token")
 
 
+_TICKET_SLOTS = 64
+_tickets = itertools.count(1)
+_ticket_slots = {}          # a device's words that its tickets are left in, taken in turn
+_released = None            # (stream, launches up to it, word, ticket) of the last ``attention_fa`` with ``release_late``
+
+
+def _new_ticket(device):
+    slots = _ticket_slots.get(device)
+    if slots is None:
+        slots = _ticket_slots.setdefault(device, torch.zeros(_TICKET_SLOTS, dtype=torch.int64, device=device))
+    ticket = next(_tickets)
+    return slots.data_ptr() + 8 * (ticket % _TICKET_SLOTS), ticket
+
+
+def _ticket_before(stream: int):
+    """The ticket of an ``attention_fa`` on ``stream`` behind which no kernel of this library has been launched, else none."""
+    last = _released
+    return last[2:] if last is not None and last[:2] == (stream, _launches) else (0, 0)
+
+
 def attention_fa(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, out: torch.Tensor, n_heads: int,
                  n_kv: int, head_dim: int, tiles: torch.Tensor, n_tiles: int, block_table: torch.Tensor, page: int,
                  window: int, scale: float, err: Optional[torch.Tensor] = None, stream: Optional[int] = None,
@@ -642,6 +663,7 @@ def attention_fa(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, ou
     sigmoid(gate[t, gate_col + i]); ``slopes`` (fp32 [n_heads]): slopes[h] * (i - j) is taken off the score after the cap;
     ``sink`` (fp32 [n_heads]): exp(sink[h]) joins the softmax's denominator.  ``release_late``: an ``attention_tc`` with
     ``beside`` follows."""
+    global _released
     _check_element_gate(gate, gate_col, n_heads * head_dim)
     _check_slopes(slopes, n_heads)
     _check_slopes(sink, n_heads)
@@ -654,11 +676,16 @@ def attention_fa(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, ou
     if k_pool.dim() != 4 or tuple(k_pool.shape[1:]) != (n_kv, page, head_dim) or v_pool.shape != k_pool.shape:
         raise KernelError(f"attention: pools {tuple(k_pool.shape)} are not [pages, {n_kv}, {page}, {head_dim}]")
     lib = _lib("attention_fa")
+    if stream is None:
+        stream = current_stream_ptr()
+    word, ticket = _new_ticket(q.device) if release_late else (0, 0)
     _call(lib, lib.ember_attention_fa, _p(q), _p(k_pool), _p(v_pool), _p(out), c_int(n_heads), c_int(n_kv), c_int(head_dim),
           _p(tiles), c_int(n_tiles), _p(block_table), c_int(block_table.shape[-1]), c_int(page), c_int(k_pool.shape[0]),
           c_int(window), c_float(scale), _p(err), c_float(softcap), c_int(chunk),
           (_off(gate, gate_col) if gate is not None else c_void_p(0)), c_int(gate.shape[-1] if gate is not None else 0),
-          _p(slopes), _p(sink), c_int(1 if release_late else 0), c_void_p(stream if stream is not None else current_stream_ptr()))
+          _p(slopes), _p(sink), c_void_p(word), c_ulonglong(ticket), c_void_p(stream))
+    if release_late:
+        _released = (stream, _launches, word, ticket)
 
 
 def attention_tc(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, out: torch.Tensor, mode: int,
@@ -678,7 +705,8 @@ def attention_tc(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, ou
     kernel that may still run on the stream writes the block table or a key or value before a tile's position, as in a
     step of decoded tokens; they are then read while the kernel before this one still runs.  ``beside`` (mode 1): the kernel
     launched on the stream directly before this one is the ``attention_fa`` of the same step's prompt portions with
-    ``release_late``; the two run at the same time."""
+    ``release_late``; the two run at the same time.  Behind any other launch of this library, and while the stream is
+    captured, it has no effect."""
     _check_element_gate(gate, gate_col, n_heads * head_dim)
     _check_slopes(slopes, n_heads)
     _check_slopes(sink, n_heads)
@@ -696,12 +724,15 @@ def attention_tc(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, ou
         if part_o.numel() < n_tiles * n_heads * n_splits * head_dim or part_ml.numel() < n_tiles * n_heads * n_splits * 2:
             raise KernelError("attention: split buffers too small")
     lib = _lib("attention_tc")
+    if stream is None:
+        stream = current_stream_ptr()
+    word, ticket = _ticket_before(stream) if beside else (0, 0)
     _call(lib, lib.ember_attention_tc, _p(q), _p(k_pool), _p(v_pool), _p(out), c_int(mode), c_int(n_heads), c_int(n_kv),
           c_int(head_dim), _p(tiles), c_int(n_tiles), _p(block_table), c_int(block_table.shape[-1]), c_int(page),
           c_int(k_pool.shape[0]), c_int(window), c_float(scale), c_int(n_splits), c_int(split_keys), _p(part_o),
           _p(part_ml), _p(err), c_float(softcap), c_int(chunk), (_off(gate, gate_col) if gate is not None else c_void_p(0)),
-          c_int(gate.shape[-1] if gate is not None else 0), _p(slopes), _p(sink), c_int(1 if keys_settled else 0), c_int(1 if beside else 0),
-          c_void_p(stream if stream is not None else current_stream_ptr()))
+          c_int(gate.shape[-1] if gate is not None else 0), _p(slopes), _p(sink), c_int(1 if keys_settled else 0), c_void_p(word), c_ulonglong(ticket),
+          c_void_p(stream))
 
 
 # ------------------------------------------------ norms and gates around a sublayer (csrc/norm_gate.cu)

@@ -668,40 +668,51 @@ def test_attention_fa_edges(heads, kv, page, held):
 
 @pytest.mark.parametrize("window", [0, 90])
 @pytest.mark.parametrize("heads,kv,page", [(16, 8, 64), (8, 1, 16)])
-def test_attention_of_decoded_tokens_beside_portions(heads, kv, page, window):
-    """A step's two attention kernels side by side give the bits they give one after the other, and what is launched behind
-    them sees both (the copy below), with the key ranges whole, merged in a cluster and merged through buffers."""
+@pytest.mark.parametrize("n_splits,split_keys,buffers", [(1, 0, False), (3, 512, False), (3, 512, True)])
+def test_attention_of_decoded_tokens_beside_portions(heads, kv, page, window, n_splits, split_keys, buffers):
+    """Four layers on the same buffers, each a product that writes the layer's queries, keys and values (and lets its follower
+    start early, like all that follows), the step's two attention kernels and a product that reads their output: with the
+    two side by side a layer has the bits that it has with one after the other.  A decode kernel that read too early would
+    see the layer before, and so would the last product if it did not wait for both."""
     from ember_b200 import ops
     from ember_b200.engine.batch import StepBatch, attention_tiles
-    D, dt, dev = 128, torch.bfloat16, "cuda"
+    D, dt, dev, K = 128, torch.bfloat16, "cuda", 256
     torch.manual_seed(heads + page)
-    ctx_lens, new = [1500, 640] + [700 + 37 * i for i in range(20)], [900, 300] + [1] * 20
-    S, T = len(ctx_lens), sum(new)
+    ctx_lens, new = [3000, 640] + [700 + 37 * i for i in range(20)], [1500, 300] + [1] * 20
+    S, T, N = len(ctx_lens), sum(new), (heads + 2 * kv) * D
     nblk = max((c + page - 1) // page for c in ctx_lens)
-    perm = torch.randperm(S * nblk).reshape(S, nblk).int()
-    kp, vp = (torch.randn(S * nblk, kv, page, D, device=dev).to(dt) for _ in range(2))
-    q = torch.randn(T, heads * D, device=dev).to(dt)
+    table = torch.randperm(S * nblk).reshape(S, nblk).int()
     positions = np.concatenate([np.arange(c - n, c) for c, n in zip(ctx_lens, new)]).astype(np.int32)
     batch = StepBatch(requests=list(range(S)), tokens=np.zeros(T, np.int32), positions=positions,
                       seq_of=np.repeat(np.arange(S), new).astype(np.int32), query_start=np.cumsum([0] + new).astype(np.int32),
-                      context_len=np.asarray(ctx_lens, np.int32), block_tables=[perm.numpy()],
+                      context_len=np.asarray(ctx_lens, np.int32), block_tables=[table.numpy()],
                       state_slots=np.zeros(S, np.int32), logit_rows=np.zeros(0, np.int32))
     multi, single = (torch.from_numpy(attention_tiles(batch, n, k)).to(dev) for n, k in ((ops.attention_fa_tile_queries(heads // kv), "multi"), (1, "single")))
-    table, err, n = perm.to(dev), torch.zeros(1, dtype=torch.int32, device=dev), single.shape[0]
-    for n_splits, split_keys, buffers in ((1, 0, False), (3, 512, False), (3, 512, True)):
-        po = torch.empty(n * heads * n_splits * D, device=dev) if buffers else None
-        pml = torch.empty(n * heads * n_splits * 2, device=dev) if buffers else None
-        got = []
-        for beside in (False, True, True, True):
-            out = torch.zeros(T, heads * D, device=dev, dtype=dt)
+    pos, seq, table, n = torch.from_numpy(positions).to(dev), torch.from_numpy(batch.seq_of).to(dev), table.to(dev), single.shape[0]
+    held_k, held_v = (torch.randn(S * nblk, kv, page, D, device=dev).to(dt) for _ in range(2))
+    xs = [torch.randn(T, K, device=dev).to(dt) for _ in range(4)]
+    w = (torch.randn(N, K, device=dev) * 0.1).to(dt)
+    w_o = (torch.randn(256, heads * D, device=dev) * 0.1).to(dt)
+    err = torch.zeros(1, dtype=torch.int32, device=dev)
+    po = torch.empty(n * heads * n_splits * D, device=dev) if buffers else None
+    pml = torch.empty(n * heads * n_splits * 2, device=dev) if buffers else None
+    got = []
+    for beside in (False, True, True, True):
+        kp, vp = held_k.clone(), held_v.clone()
+        q, out = torch.zeros(T, heads * D, device=dev, dtype=dt), torch.zeros(T, heads * D, device=dev, dtype=dt)
+        after = [torch.zeros(T, 256, device=dev) for _ in xs]
+        for x, o in zip(xs, after):
+            ops.gemm_tc_qkv(x, w, T, heads, kv, None, None, 1e-6, None, None, pos, seq, table, page, kp, vp, q, err=err)
             ops.attention_fa(q, kp, vp, out, heads, kv, D, multi, multi.shape[0], table, page, window, 0.09, err=err, release_late=beside)
             ops.attention_tc(q, kp, vp, out, 1, heads, kv, D, single, n, table, page, window, 0.09, n_splits, split_keys, po, pml, err=err,
                              keys_settled=beside, beside=beside)
-            copy = torch.empty(T, heads * D, device=dev, dtype=torch.float32)
-            copy.copy_(out)
-            got.append(copy)
-        assert int(err.item()) == 0
-        assert bool(got[0].abs().sum(dim=1).min() > 0) and all(torch.equal(g, got[0]) for g in got[1:])
+            ops.gemm_tc(out, w_o, o, T, ops.EPI_STORE_F32, err=err)
+        got.append(after)
+    assert int(err.item()) == 0
+    assert all(bool(o.abs().sum(dim=1).min() > 0) for o in got[0])
+    assert all(not torch.equal(x, y) for x, y in zip(got[0], got[0][1:]))
+    for run in got[1:]:
+        assert all(torch.equal(x, y) for x, y in zip(run, got[0]))
 
 
 @pytest.mark.parametrize("rows", [1, 63, 64, 65, 130])
