@@ -133,16 +133,21 @@ static void best_tile_and_parts(int M, int N, int num_k_blocks, int slots, int u
 
 // Whether pairs of SMs are the faster kernel for 256 to 2,047 tokens.  Pairs read half of the weight tile each but compute rows
 // in pieces of 256, so it is the last row tile and the last wave that decide: the time is modelled as waves (k_blocks a cols +
-// b) + c us with a, b and c fitted to 329 measured products for either kernel (fifteen matrices of 1,024 x 3,072 to
-// 151,936 x 2,048, 23 numbers of tokens each; least absolute errors).  The choice is within 0.6 % of the better kernel on average
-// and at most 5 % off; the model of before, of kernels whose issuing threads bounded them, and for large matrices from 512
-// tokens only, was 3.4 % off and at most 21 % (us, one SM / pairs: 12,288 x 2,048 gated 1,280 tokens 54 / 48, 4,096 x 4,096 added 560
-// tokens 27 / 23, 6,144 x 4,096 1,700 tokens 75 / 63, 24,576 x 4,096 gated 440 tokens 89 / 74; 4,096 x 2,048 384 tokens 12.9 / 13.3).
-static double modelled_us(bool pairs, int M, int N, int num_k_blocks, int cols, int parts, int slots) {
+// b) + c us, and d us for each million sums that K's parts add at the L2 (more than their tiles take where there are many: 256
+// tokens x 2,048 x 6,144 in nine parts 15 us, of which the first terms see 9).  a to d are fitted to 537 measured products
+// for either kernel (21 matrices of 1,024 x 3,072 to 151,936 x 2,048, 26 numbers of tokens each, 17 for the largest), the
+// choice weighing more than the times.  Held against the same products measured anew (two runs, which differ by 4 %): within
+// 0.2 % of the better kernel on average, at most 5.6 % off (3,072 x 2,304, 280 tokens: 17.3 where one SM takes 16.4), the next
+// 4.0 % (12,288 x 2,048 gated, 560 tokens: 30.2 where pairs take 29.1).  Without d it was 0.5 % off and at most 18 %; one SM
+// wherever the rule before the present kernels said so (for large matrices from 512 tokens only) 3.4 % off and at most 20 %.
+// us, one SM / pairs: 12,288 x 2,048 gated 1,280 tokens 54 / 48, 4,096 x 4,096 added 560 tokens 26 / 23, 6,144 x 4,096 1,700 tokens
+// 75 / 63, 24,576 x 4,096 gated 440 tokens 89 / 74; 4,096 x 2,048 384 tokens 12.9 / 13.3, 4,096 x 12,288 added 1,100 tokens 87 / 93.
+static double modelled_us(bool pairs, int M, int N, int num_k_blocks, int cols, int parts, bool adds, int slots) {
     const int rows = TILE_ROWS * (pairs ? 2 : 1), kb = (num_k_blocks + parts - 1) / parts;
-    const long long n = (long long)((M + rows - 1) / rows) * ((N + cols - 1) / cols) * ((num_k_blocks + kb - 1) / kb);
-    const double waves = (double)((n + slots - 1) / slots);
-    return pairs ? waves * (kb * 0.001412 * cols + 1.316) + 4.81 : waves * (kb * 0.001712 * cols + 0.716) + 3.79;
+    parts = (num_k_blocks + kb - 1) / kb;
+    const double waves = (double)(((long long)((M + rows - 1) / rows) * ((N + cols - 1) / cols) * parts + slots - 1) / slots);
+    const double added = adds ? 1e-6 * M * N * parts : 0.0;
+    return pairs ? waves * (kb * 0.001371 * cols + 1.438) + 4.226 + 0.7323 * added : waves * (kb * 0.001656 * cols + 0.9706) + 3.413 + 0.7537 * added;
 }
 static bool pairs_are_faster(int M, int N, int num_k_blocks, bool adds, int num_sms, int max_pairs) {
     auto us = [&](bool pairs) {
@@ -150,9 +155,14 @@ static bool pairs_are_faster(int M, int N, int num_k_blocks, bool adds, int num_
         int cols = 0, parts = 1;
         if (adds) best_tile_and_parts(M, N, num_k_blocks, slots, units, &cols, &parts);
         else cols = best_block_cols(M, N, slots, units, nullptr);
-        return modelled_us(pairs, M, N, num_k_blocks, cols, parts, slots);
+        return modelled_us(pairs, M, N, num_k_blocks, cols, parts, adds, slots);
     };
     return us(true) <= us(false);
+}
+
+// ... for what it was measured on and larger matrices.
+static bool pairs_from_256(int M, int N, int K, int epilogue, int num_sms, int max_pairs) {
+    return M >= 256 && N >= 1024 && K >= 1024 && pairs_are_faster(M, N, (K + TILE_K - 1) / TILE_K, epilogue == 2, num_sms, max_pairs);
 }
 
 // A cluster's partial sums in shared memory: every block receives its share of the token columns from all of them.
@@ -386,6 +396,11 @@ EMBER_API long long ember_gemm_tc_scratch_floats(int max_tokens_swapped, int N) 
     return (long long)max_tokens_swapped * N;
 }
 
+// What ember_gemm_tc chooses for 256 to 2,047 tokens on a device of so many SMs that runs so many pairs at once (host only).
+EMBER_API int ember_gemm_tc_on_pairs(int M, int N, int K, int epilogue, int num_sms, int max_pairs) {
+    return pairs_from_256(M, N, K, epilogue, num_sms, max_pairs) ? 1 : 0;
+}
+
 // C = A . W^T with the fused epilogue.  `scratch` is a zero-filled fp32 buffer of at least
 // min(M, 128) * N floats (used only when the K range is split; it is left zeroed).
 // Epilogue 8 stores gelu(sum + bias) in bf16 (the exact form, by erf), epilogue 9 max(sum + bias, 0)^2.  `bias` (fp32 [N] or null) joins the sums of
@@ -432,8 +447,7 @@ EMBER_API int ember_gemm_tc(const void* A, const void* W, void* out, int ldc, in
             if (max_pairs > 0) {
                 const int bc_pair = best_block_cols(M, N, max_pairs, 2, &cost_pair);
                 if (split_mode == 4 || (M >= 2048 && cost_pair <= cost_single * 1.001) ||
-                    (M >= 256 && M < 2048 && N >= 1024 && K >= 1024 &&
-                     pairs_are_faster(M, N, p.num_k_blocks, epilogue == 2, num_sms, max_pairs))) {
+                    (M < 2048 && pairs_from_256(M, N, K, epilogue, num_sms, max_pairs))) {
                     p.epilogue = epilogue; p.out = out; p.ldc = ldc; p.err = err;
                     p.accum = nullptr; p.accum_ld = 0; p.stages = 0;
                     return launch_pair(A, W, p, bc_pair, max_pairs, st);
@@ -671,10 +685,11 @@ EMBER_API int ember_gemm_tc_qkv(const void* A, const void* W, int M, int N, int 
     const int block_cols = (N % 256 == 0) ? 256 : 128;          // whole heads in a tile
     if (split_mode != 5) {
         const int max_pairs = pair_capacity(num_sms);
-        // whole heads leave no choice of the width; the model has to see 5 % in pairs (us, one SM / pairs: 4,096 x 2,048 601 tokens
-        // 18.4 / 18.8, 1,280 tokens 28.2 / 25.5; 6,144 x 4,096 512 tokens 31.0 / 29.0, 1,024 tokens 52.1 / 45.9)
-        auto us = [&](bool pairs) { return modelled_us(pairs, M, N, p.num_k_blocks, block_cols, 1, pairs ? max_pairs : num_sms); };
-        if (max_pairs > 0 && (split_mode == 4 || M >= 2048 || (M >= 512 && us(true) <= 0.95 * us(false))))
+        // whole heads leave no choice of the width; the model has to see 8 % in pairs, whose heads take longer than plain tiles
+        // (us, one SM / pairs: 4,096 x 2,048 601 tokens 19.1 / 19.4, 1,152 tokens 19.2 / 25.8, 1,280 tokens 28.3 / 25.9; 6,144 x
+        // 4,096 512 tokens 31.4 / 29.7, 1,024 tokens 52.9 / 47.2; 7,168 x 5,120 512 tokens 39.1 / 35.3, 560 tokens 41.2 / 53.6)
+        auto us = [&](bool pairs) { return modelled_us(pairs, M, N, p.num_k_blocks, block_cols, 1, false, pairs ? max_pairs : num_sms); };
+        if (max_pairs > 0 && (split_mode == 4 || M >= 2048 || (M >= 512 && us(true) <= 0.92 * us(false))))
             return launch_pair(A, W, p, block_cols, max_pairs, st);
     }
     return launch_persistent(A, W, p, block_cols, num_sms, st);

@@ -1,0 +1,41 @@
+"""Which kernel a product goes to, where that is decided by a model of its time: the choice against measured times."""
+import pytest
+
+from ember_b200.csrc import build
+
+# (rows, columns of the matrix, epilogue: 0 stored, 1 stored in fp32, 2 added, 3 gated), {tokens: (us on single SMs, us on pairs)}, B200,
+# 148 SMs, 74 pairs at once
+PRODUCTS = [
+    ((4096, 4096, 2), {560: (26.1, 22.7), 601: (26.5, 22.7), 640: (26.8, 22.7), 1400: (45.3, 40.4)}),
+    ((2048, 6144, 2), {256: (15.8, 16.4), 560: (20.3, 19.5), 640: (20.8, 19.4), 1600: (32.8, 33.9)}),
+    ((4096, 12288, 2), {830: (77.7, 72.3), 1100: (87.0, 92.8), 1152: (87.4, 93.2), 1600: (137.8, 126.4)}),
+    ((12288, 2048, 3), {560: (30.2, 29.1), 640: (30.6, 29.5), 1280: (54.9, 47.5)}),
+    ((24576, 4096, 3), {440: (84.5, 73.1), 560: (105.7, 99.6), 768: (115.4, 104.9), 1024: (157.2, 136.3)}),
+    ((6144, 1024, 3), {1536: (18.8, 19.5), 1600: (20.3, 23.3), 1920: (23.9, 25.9), 2047: (25.4, 26.0)}),
+    ((6144, 4096, 0), {601: (30.1, 29.0), 1700: (73.5, 62.9)}),
+    ((4096, 2048, 0), {384: (13.0, 13.4), 1280: (22.5, 20.5)}),
+    ((4096, 1024, 0), {1280: (14.7, 13.6), 1400: (14.9, 14.0)}),
+    ((10240, 5120, 0), {256: (36.4, 34.7), 300: (43.1, 51.6)}),
+]
+
+
+@pytest.fixture(scope="module")
+def on_pairs():
+    try:
+        lib = build.load("gemm_tc")
+    except (build.BuildError, OSError) as e:
+        pytest.skip(f"the product's library cannot be built or loaded here: {e}")
+    return lib.ember_gemm_tc_on_pairs
+
+
+@pytest.mark.parametrize("matrix,times", PRODUCTS, ids=lambda v: "x".join(map(str, v)) if isinstance(v, tuple) else "")
+def test_pairs_or_single_sms(on_pairs, matrix, times):
+    """The kernel chosen is at most 5 % slower than the other one (the measurements repeat within 4 %)."""
+    n, k, epilogue = matrix
+    for tokens, us in times.items():
+        assert us[on_pairs(tokens, n, k, epilogue, 148, 74)] <= 1.05 * min(us), (matrix, tokens)
+
+
+@pytest.mark.parametrize("tokens,n,k", [(255, 4096, 4096), (1024, 1023, 4096), (1024, 4096, 1016)])
+def test_single_sms_below_what_was_measured(on_pairs, tokens, n, k):
+    assert not on_pairs(tokens, n, k, 2, 148, 74)
