@@ -165,6 +165,16 @@ static bool pairs_from_256(int M, int N, int K, int epilogue, int num_sms, int m
     return M >= 256 && N >= 1024 && K >= 1024 && pairs_are_faster(M, N, (K + TILE_K - 1) / TILE_K, epilogue == 2, num_sms, max_pairs);
 }
 
+// The same for the product that finishes its heads.  Whole heads leave no choice of the width; the model has to see 8 % in
+// pairs, whose heads take longer than plain tiles (us, one SM / pairs: 4,096 x 2,048 601 tokens 19.1 / 19.4, 1,152 tokens 19.2 /
+// 25.8, 1,280 tokens 28.3 / 25.9; 6,144 x 4,096 512 tokens 31.4 / 29.7, 1,024 tokens 52.9 / 47.2; 7,168 x 5,120 512 tokens 39.1 /
+// 35.3, 560 tokens 41.2 / 53.6; 1,536 x 1,024 512 to 2,047 tokens 12.5 to 13.6 / 13.1 to 14.4).
+static int qkv_block_cols(int N) { return (N % 256 == 0) ? 256 : 128; }          // whole heads in a tile
+static bool qkv_pairs_from_512(int M, int N, int K, int block_cols, int num_sms, int max_pairs) {
+    auto us = [&](bool pairs) { return modelled_us(pairs, M, N, (K + TILE_K - 1) / TILE_K, block_cols, 1, false, pairs ? max_pairs : num_sms); };
+    return M >= 512 && N >= 1024 && K >= 1024 && us(true) <= 0.92 * us(false);
+}
+
 // A cluster's partial sums in shared memory: every block receives its share of the token columns from all of them.
 static size_t cluster_recv_bytes(const GemmTcParams& p) {
     if (p.cluster_splits <= 1 && p.epilogue != 4) return 0;
@@ -399,6 +409,11 @@ EMBER_API long long ember_gemm_tc_scratch_floats(int max_tokens_swapped, int N) 
 // What ember_gemm_tc chooses for 256 to 2,047 tokens on a device of so many SMs that runs so many pairs at once (host only).
 EMBER_API int ember_gemm_tc_on_pairs(int M, int N, int K, int epilogue, int num_sms, int max_pairs) {
     return pairs_from_256(M, N, K, epilogue, num_sms, max_pairs) ? 1 : 0;
+}
+
+// ... and ember_gemm_tc_qkv for 512 to 2,047.
+EMBER_API int ember_gemm_tc_qkv_on_pairs(int M, int N, int K, int num_sms, int max_pairs) {
+    return qkv_pairs_from_512(M, N, K, qkv_block_cols(N), num_sms, max_pairs) ? 1 : 0;
 }
 
 // C = A . W^T with the fused epilogue.  `scratch` is a zero-filled fp32 buffer of at least
@@ -682,14 +697,10 @@ EMBER_API int ember_gemm_tc_qkv(const void* A, const void* W, int M, int N, int 
     p.qkv.q_out = (__nv_bfloat16*)q_out; p.qkv.k_pool = (__nv_bfloat16*)k_pool; p.qkv.v_pool = (__nv_bfloat16*)v_pool;
     p.qkv.write_kv = write_kv;
     if (M <= 128) return launch_heads_swapped(A, W, p, num_sms, st);
-    const int block_cols = (N % 256 == 0) ? 256 : 128;          // whole heads in a tile
+    const int block_cols = qkv_block_cols(N);
     if (split_mode != 5) {
         const int max_pairs = pair_capacity(num_sms);
-        // whole heads leave no choice of the width; the model has to see 8 % in pairs, whose heads take longer than plain tiles
-        // (us, one SM / pairs: 4,096 x 2,048 601 tokens 19.1 / 19.4, 1,152 tokens 19.2 / 25.8, 1,280 tokens 28.3 / 25.9; 6,144 x
-        // 4,096 512 tokens 31.4 / 29.7, 1,024 tokens 52.9 / 47.2; 7,168 x 5,120 512 tokens 39.1 / 35.3, 560 tokens 41.2 / 53.6)
-        auto us = [&](bool pairs) { return modelled_us(pairs, M, N, p.num_k_blocks, block_cols, 1, false, pairs ? max_pairs : num_sms); };
-        if (max_pairs > 0 && (split_mode == 4 || M >= 2048 || (M >= 512 && us(true) <= 0.92 * us(false))))
+        if (max_pairs > 0 && (split_mode == 4 || M >= 2048 || qkv_pairs_from_512(M, N, K, block_cols, num_sms, max_pairs)))
             return launch_pair(A, W, p, block_cols, max_pairs, st);
     }
     return launch_persistent(A, W, p, block_cols, num_sms, st);

@@ -809,6 +809,33 @@ def test_gemm_tc_qkv(heads, kv, page, M, norm, rotate):
     assert int(err.item()) == 2
 
 
+@pytest.mark.parametrize("M", [511, 512, 513, 1281, 2047])
+@pytest.mark.parametrize("heads,kv,page,K", [(16, 8, 64, 2048), (32, 8, 16, 4096), (6, 2, 32, 328)])
+def test_gemm_tc_qkv_pairs_from_512_tokens(M, heads, kv, page, K):
+    """Both sides of the rule for pairs of SMs (512 and 2,048 tokens): the queries and cache pages that one SM a tile gives."""
+    from ember_b200 import ops
+    torch.manual_seed(M + K)
+    dev, D, N = "cuda", 128, (heads + 2 * kv) * 128
+    a, w = (torch.randn(M, K, device=dev) * 0.5).bfloat16(), (torch.randn(N, K, device=dev) * 0.1).bfloat16()
+    qw, kw = 1 + 0.1 * torch.randn(D, device=dev), 1 + 0.1 * torch.randn(D, device=dev)
+    pos, seq = torch.arange(70, 70 + M, device=dev).int(), torch.zeros(M, device=dev).int()
+    pages = (70 + M + page - 1) // page
+    table = torch.randperm(pages, device=dev).int().view(1, -1)
+    cs = torch.empty(D // 4, M, 4, device=dev)
+    ops.rope_table(pos, 1.0 / (10000.0 ** (torch.arange(D // 2, device=dev).float() * 2 / D)), M, cs)
+    err, got = torch.zeros(1, dtype=torch.int32, device=dev), []
+    for mode in (5, 4, 0):
+        kp, vp = (torch.zeros(pages, kv, page, D, device=dev, dtype=torch.bfloat16) for _ in range(2))
+        q = torch.zeros(M + 1, heads * D, device=dev, dtype=torch.bfloat16)
+        ops.gemm_tc_qkv(a, w, M, heads, kv, qw, kw, 1e-5, cs, None, pos, seq, table, page, kp, vp, q, err=err, split_mode=mode)
+        got.append((q, kp, vp))
+    assert int(err.item()) == 0 and float(got[0][0][M].abs().max()) == 0.0
+    for one in got[1:]:
+        assert all(torch.equal(x, y) for x, y in zip(one, got[0]))
+    v = (a.float() @ w[(heads + kv) * D:].float().t()).view(M, kv, D)
+    assert rel(got[0][2][table[0, (pos // page).long()].long(), :, (pos % page).long()].float(), v) < 5e-3
+
+
 @pytest.mark.parametrize("heads,kv,M,K", [(16, 8, 17, 2048), (16, 8, 64, 2048), (3, 1, 65, 136), (4, 2, 100, 328), (16, 8, 128, 2048),
                                           (40, 8, 33, 4096), (1, 1, 48, 64)])
 @pytest.mark.parametrize("norm,rotate", [(True, True), (False, True), (True, False)])

@@ -17,14 +17,25 @@ PRODUCTS = [
     ((4096, 1024, 0), {1280: (14.7, 13.6), 1400: (14.9, 14.0)}),
     ((10240, 5120, 0), {256: (36.4, 34.7), 300: (43.1, 51.6)}),
 ]
+# ... of the products that finish their heads
+HEAD_PRODUCTS = [
+    ((1536, 1024), {512: (13.4, 14.4), 1152: (12.8, 13.3), 2047: (13.1, 13.6)}),
+    ((4096, 2048), {512: (19.6, 19.4), 601: (19.1, 19.4), 1152: (19.2, 25.8), 1280: (28.3, 25.9), 2047: (31.6, 29.0)}),
+    ((6144, 4096), {601: (31.4, 29.7), 768: (33.0, 30.8), 1024: (52.9, 47.2), 1792: (79.0, 68.8)}),
+    ((7168, 5120), {512: (39.1, 35.3), 560: (41.2, 53.6), 768: (62.5, 54.3), 1280: (74.0, 68.1), 1920: (105.3, 123.4)}),
+]
 
 
 @pytest.fixture(scope="module")
-def on_pairs():
+def lib():
     try:
-        lib = build.load("gemm_tc")
+        return build.load("gemm_tc")
     except (build.BuildError, OSError) as e:
         pytest.skip(f"the product's library cannot be built or loaded here: {e}")
+
+
+@pytest.fixture(scope="module")
+def on_pairs(lib):
     return lib.ember_gemm_tc_on_pairs
 
 
@@ -39,3 +50,14 @@ def test_pairs_or_single_sms(on_pairs, matrix, times):
 @pytest.mark.parametrize("tokens,n,k", [(255, 4096, 4096), (1024, 1023, 4096), (1024, 4096, 1016)])
 def test_single_sms_below_what_was_measured(on_pairs, tokens, n, k):
     assert not on_pairs(tokens, n, k, 2, 148, 74)
+
+
+@pytest.mark.parametrize("matrix,times", HEAD_PRODUCTS, ids=lambda v: "x".join(map(str, v)) if isinstance(v, tuple) else "")
+def test_pairs_or_single_sms_for_heads(lib, matrix, times):
+    for tokens, us in times.items():
+        assert us[lib.ember_gemm_tc_qkv_on_pairs(tokens, *matrix, 148, 74)] <= 1.05 * min(us), (matrix, tokens)
+
+
+@pytest.mark.parametrize("tokens,n,k", [(511, 6144, 4096), (1024, 6144, 1016), (1024, 896, 4096)])
+def test_single_sms_for_heads_below_what_was_measured(lib, tokens, n, k):
+    assert not lib.ember_gemm_tc_qkv_on_pairs(tokens, n, k, 148, 74)
