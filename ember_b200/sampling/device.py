@@ -8,7 +8,7 @@ from typing import Optional, Sequence
 
 import torch
 
-from .. import ops
+from .. import ops, transfers
 from .params import SamplingParams
 
 _U64 = (1 << 64) - 1
@@ -61,5 +61,7 @@ def sample(logits: torch.Tensor, params: Sequence[SamplingParams], counters: Seq
         part_v, part_i = _argmax_scratch(logits.device, rows)
         ops.argmax(logits, out, rows, part_v, part_i)
         return out
-    ops.sample_host(logits, pack_params(params, counters), out, rows)
+    packed = pack_params(params, counters)
+    ops.sample_host(logits, packed, out, rows)
+    transfers.add_h2d(len(packed))
     return out

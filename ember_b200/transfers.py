@@ -1,8 +1,8 @@
 """Counts of the bytes that cross between host and device on the serving path.
 
-Every host-to-device and device-to-host copy a step makes goes through three places: the step's one packed
-upload (``engine.batch.StepContext.upload``), the sampler's parameter rows (``sampling.device.sample``) and the
-read-back of the sampled ids with the error word (``engine.engine.Engine``).  Each adds what it copied here, so a
+What a step moves goes through three places: the step's one packed upload (``engine.batch.StepContext.upload``), the
+sampler's parameter rows (``sampling.device.sample``; arguments of its launch, not a copy, but bytes that cross) and the
+read-back of the sampled ids with the error word (``engine.engine.Engine``).  Each adds what it moved here, so a
 benchmark can report the bytes a step really moved instead of a formula.
 """
 from __future__ import annotations

@@ -29,6 +29,16 @@ def test_host_noise_is_stateless():
     assert abs(g.mean() - 0.5772) < 0.06                                      # Gumbel(0, 1) mean
 
 
+@pytest.mark.parametrize("rows", [1, 3, 70])
+def test_parameter_rows_are_counted_as_moved(rows, monkeypatch):
+    from ember_b200 import ops, transfers
+    from ember_b200.sampling import device
+    monkeypatch.setattr(ops, "sample_host", lambda logits, packed, out, rows: None)
+    before = transfers.snapshot()
+    device.sample(torch.zeros(rows, 8), [SamplingParams(temperature=1.0)] * rows, list(range(rows)))
+    assert transfers.snapshot() == (before[0] + 32 * rows, before[1])
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("vocab", [1000, 4099, 151936])
 def test_device_equals_host(vocab):
