@@ -399,8 +399,7 @@ __device__ __forceinline__ void scan_part(const float* __restrict__ logits, int 
 }
 
 // A small top-k in two scans of the raw logits instead of seven of the scaled ones (which spend their time on the
-// division and on the cluster's barriers, not on memory: 32 rows of 151,936 with top-k 20 took 102 us, now 44 with the
-// parameters' copy).
+// division and on the cluster's barriers, not on memory: 32 rows of 151,936 with top-k 20 took 102 us, now 21).
 //
 // Every group of four threads has the largest logit it saw; the k-th largest L of the cluster's 2,048 group maxima
 // cannot lie above the k-th largest logit, so the kept set is among the elements whose scaled value reaches L / T.
@@ -488,8 +487,10 @@ __device__ bool gather_candidates(const float* __restrict__ logits, int V, const
     return true;
 }
 
+// Two blocks to an SM: left to itself the compiler takes 54 registers a thread where 32 do without a spill, and 32 rows are two waves
+// of one block an SM then (vocabulary 151,936, top-k 20: a pass 33 us, 21 with two; 64 rows 52 and 38).
 template <int CL>
-__global__ void __launch_bounds__(SAMPLE_THREADS)
+__global__ void __launch_bounds__(SAMPLE_THREADS, 2)
 sample_kernel(const float* __restrict__ logits_all, int V, const SampleParams* __restrict__ params,
               int* __restrict__ out, const __grid_constant__ SampleRows given) {
     __shared__ Shared sh;
@@ -749,7 +750,7 @@ EMBER_API int ember_sample(const float* logits, int rows, int V, const void* par
 }
 
 // params: host memory, read before this returns; 64 rows travel with a launch.  A pass over 32 rows of 151,936: 43.5 us with the
-// rows in a ring of pinned buffers, copied to device memory ahead of the launch, 33.2 with this; the kernel takes 18.8.
+// rows in a ring of pinned buffers, copied to device memory ahead of the launch, 21 with this; the kernel takes 19.
 EMBER_API int ember_sample_host(const float* logits, int rows, int V, const void* params, int* out, void* stream) {
     if (rows <= 0) return 0;
     if (V <= 0) return fail("sample: vocabulary %d", V);
