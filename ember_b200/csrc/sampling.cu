@@ -40,9 +40,13 @@ struct SampleParams {  // 32 bytes per row, mirrored by the Python side
 };
 
 // The rows of a launch as a kernel argument: the host hands them over with the launch itself, without a buffer, a copy and
-// what it takes to keep that buffer alive.
-constexpr int SAMPLE_ROWS = 64;
-struct SampleRows { SampleParams row[SAMPLE_ROWS]; };
+// what it takes to keep that buffer alive.  A launch with room for more rows carries more bytes, so there are three (us at a
+// vocabulary of 2,000, with room for 256 / for 1,000: 65 rows 22 / 24, 192 rows 40 / 42; more than a thousand rows, whose
+// arguments would not fit (32,764 bytes), are several launches, as more than 64 were before: 128, 256 and 512 rows of 151,936 took
+// 104, 224 and 450 us, 89, 183 and 348 in one launch, and 62, 118 and 219 with two blocks an SM).
+constexpr int FEW_ROWS = 64, SOME_ROWS = 256, MANY_ROWS = 1000;
+template <int ROWS>
+struct SampleRows { SampleParams row[ROWS]; };
 
 __host__ __device__ __forceinline__ unsigned long long rng_mix(unsigned long long z) {
     z += 0x9E3779B97F4A7C15ull;
@@ -489,10 +493,10 @@ __device__ bool gather_candidates(const float* __restrict__ logits, int V, const
 
 // Two blocks to an SM: left to itself the compiler takes 54 registers a thread where 32 do without a spill, and 32 rows are two waves
 // of one block an SM then (vocabulary 151,936, top-k 20: a pass 33 us, 21 with two; 64 rows 52 and 38).
-template <int CL>
+template <int CL, int ROWS>
 __global__ void __launch_bounds__(SAMPLE_THREADS, 2)
 sample_kernel(const float* __restrict__ logits_all, int V, const SampleParams* __restrict__ params,
-              int* __restrict__ out, const __grid_constant__ SampleRows given) {
+              int* __restrict__ out, const __grid_constant__ SampleRows<ROWS> given) {
     __shared__ Shared sh;
     const int row = blockIdx.x / CL;
     const unsigned rank = CL > 1 ? cl_rank() : 0;
@@ -717,7 +721,8 @@ EMBER_API int ember_argmax(const float* logits, int rows, int V, float* part_v, 
 }
 
 namespace ember {
-static int launch_sample(const float* logits, int rows, int V, const SampleParams* params, int* out, const SampleRows& given, cudaStream_t stream) {
+template <int ROWS>
+int launch_sample(const float* logits, int rows, int V, const SampleParams* params, int* out, const SampleRows<ROWS>& given, cudaStream_t stream) {
     // A row is shared by a cluster of 8 blocks (one block alone spends 0.2-2 ms on a vocabulary of 150,000: its
     // passes are instruction-bound on one SM); small vocabularies stay with one block.
     constexpr int CL = 8;
@@ -730,12 +735,25 @@ static int launch_sample(const float* logits, int rows, int V, const SampleParam
         attr[0].id = cudaLaunchAttributeClusterDimension;
         attr[0].val.clusterDim.x = CL; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
         cfg.attrs = attr; cfg.numAttrs = 1;
-        if (cudaLaunchKernelEx(&cfg, sample_kernel<CL>, logits, V, params, out, given) == cudaSuccess)
+        if (cudaLaunchKernelEx(&cfg, sample_kernel<CL, ROWS>, logits, V, params, out, given) == cudaSuccess)
             return check_launch("sample");
         cudaGetLastError();                     // clusters of 8 not available: one block per row
     }
-    sample_kernel<1><<<rows, SAMPLE_THREADS, 0, stream>>>(logits, V, params, out, given);
+    sample_kernel<1, ROWS><<<rows, SAMPLE_THREADS, 0, stream>>>(logits, V, params, out, given);
     return check_launch("sample");
+}
+
+// ROWS a launch, one launch after the other.
+template <int ROWS>
+int launch_given(const float* logits, int rows, int V, const SampleParams* params, int* out, cudaStream_t stream) {
+    SampleRows<ROWS> given;
+    for (int r = 0; r < rows; r += ROWS) {
+        const int n = rows - r < ROWS ? rows - r : ROWS;
+        memcpy(given.row, params + r, (size_t)n * sizeof(SampleParams));       // (what lies behind them is not read)
+        const int rc = launch_sample<ROWS>(logits + (size_t)r * V, n, V, nullptr, out + r, given, stream);
+        if (rc) return rc;
+    }
+    return 0;
 }
 }  // namespace ember
 
@@ -745,21 +763,19 @@ EMBER_API int ember_sample(const float* logits, int rows, int V, const void* par
     if (V <= 0) return fail("sample: vocabulary %d", V);
     if (!params) return fail("sample: no parameters");
     static_assert(sizeof(SampleParams) == 32, "parameter rows are 32 bytes");
-    static const SampleRows none = {};
-    return launch_sample(logits, rows, V, (const SampleParams*)params, out, none, (cudaStream_t)stream);
+    static const SampleRows<1> none = {};
+    return launch_sample<1>(logits, rows, V, (const SampleParams*)params, out, none, (cudaStream_t)stream);
 }
 
-// params: host memory, read before this returns; 64 rows travel with a launch.  A pass over 32 rows of 151,936: 43.5 us with the
-// rows in a ring of pinned buffers, copied to device memory ahead of the launch, 21 with this; the kernel takes 19.
+// params: host memory, read before this returns.  They travel with the launch: a pass over 32 rows of 151,936 took 43.5 us with
+// the rows in a ring of pinned buffers, copied to device memory ahead of the launch, and takes 21 like this (the kernel 19).
 EMBER_API int ember_sample_host(const float* logits, int rows, int V, const void* params, int* out, void* stream) {
     if (rows <= 0) return 0;
     if (V <= 0) return fail("sample: vocabulary %d", V);
-    for (int r = 0; r < rows; r += SAMPLE_ROWS) {
-        const int n = rows - r < SAMPLE_ROWS ? rows - r : SAMPLE_ROWS;
-        SampleRows given = {};
-        memcpy(given.row, (const SampleParams*)params + r, (size_t)n * sizeof(SampleParams));
-        const int rc = launch_sample(logits + (size_t)r * V, n, V, nullptr, out + r, given, (cudaStream_t)stream);
-        if (rc) return rc;
-    }
-    return 0;
+    if (!params) return fail("sample: no parameters");
+    const SampleParams* p = (const SampleParams*)params;
+    cudaStream_t st = (cudaStream_t)stream;
+    if (rows <= FEW_ROWS) return launch_given<FEW_ROWS>(logits, rows, V, p, out, st);
+    if (rows <= SOME_ROWS) return launch_given<SOME_ROWS>(logits, rows, V, p, out, st);
+    return launch_given<MANY_ROWS>(logits, rows, V, p, out, st);
 }

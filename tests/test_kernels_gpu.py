@@ -715,10 +715,10 @@ def test_attention_of_decoded_tokens_beside_portions(heads, kv, page, window, n_
         assert all(torch.equal(x, y) for x, y in zip(run, got[0]))
 
 
-@pytest.mark.parametrize("rows", [1, 63, 64, 65, 130])
+@pytest.mark.parametrize("rows", [1, 63, 64, 65, 130, 256, 257, 1000, 1001])
 @pytest.mark.parametrize("V", [1000, 20000])
 def test_sample_parameters_from_the_host(rows, V):
-    """Parameter rows that travel with the launch (64 of them) give the ids that rows in device memory give."""
+    """Parameter rows that travel with the launch (64, 256 or 1,000 of them) give the ids that rows in device memory give."""
     from ember_b200 import SamplingParams, ops
     from ember_b200.sampling import device
     torch.manual_seed(rows)
