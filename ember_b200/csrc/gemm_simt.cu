@@ -539,6 +539,22 @@ constexpr int FEW_TOKENS = 32, FEW_TOKENS_WIDE = 16, WIDE_COLUMNS = 4096;
 // More than 32 tokens: the kernel of clusters up to this many columns (its comment has both sides).
 constexpr int NARROW_COLUMNS = 2048;
 
+// Whether the kernel for few looks eight stages ahead instead of three, with blocks of 8 weight rows.  Where an SM has no more than one
+// block, its two warps are all that fetches there (the rings of 16 tokens also leave no room for a second one; three stages
+// do, and a grid that does not fill the chip evenly gets some SMs two).  us, three / eight stages, K 2,048:
+//   blocks          16            32            56            74            128           146           148           192
+//   3, 4 tokens     5.7 / 4.7     6.1 / 4.9     6.5 / 5.6     6.1 / 4.9     9.0 / 5.9     9.1 / 6.1     6.3 / 5.4     9.3 / 6.8
+//   5 to 8          7.5 / 7.8     7.8 / 7.7     9.0 / 7.9     7.8 / 7.9    12.8 / 8.2    12.4 / 8.1     7.9 / 8.1    12.5 / 14.5
+//   9 to 16         9.8 / 11.1    9.9 / 10.9   12.5 / 11.2    9.7 / 11.2   16.8 / 11.5   16.7 / 11.6    9.8 / 11.6   17.0 / 20.4
+// and alike at K 64 to 6,144.  Up to 8 tokens it does for 148 blocks and fewer (up to 5 % behind where blocks are few), beyond them not
+// (3,072 rows of K 1,024, 4 tokens 6.3 / 7.6); 9 to 16 tokens from 52 blocks on (44 and 48: 10 % ahead to 10 % behind), but not
+// where a grid of 74 or 148 blocks is even by itself.  One and two tokens are up to 36 % ahead from 88 blocks on and up to 12 %
+// behind below; they have not been given it yet.
+constexpr unsigned EVEN_BLOCKS = 148;          // a block an SM
+static bool few_looks_far(int MT, unsigned blocks) {
+    return MT >= 4 && blocks <= EVEN_BLOCKS && (MT < 16 || (blocks >= 52 && blocks != EVEN_BLOCKS / 2 && blocks != EVEN_BLOCKS));
+}
+
 template <int MT>
 int launch_few(const float* A, int lda, const float* W, int ldw, const float* bias, float* C, int ldc, int M, int N, int K, int epi,
                int settled, cudaStream_t st) {
@@ -548,12 +564,9 @@ int launch_few(const float* A, int lda, const float* W, int ldw, const float* bi
         return launch_f32(gemm_f32_few_kernel<MT, NB, ST>, dim3((N + NB - 1) / NB, y), NB * KPARTS, few_smem<MT, NB, ST>(), st, A, lda, W, ldw, bias, C, ldc, M, N, K, epi, settled);
     };
     using std::integral_constant;
-    // blocks of 16 weight rows once they fill the SMs twice, else of 8; where there is no more than one of those for an SM, the
-    // two warps of a block are all that fetches there, and look eight stages ahead instead of three (1,024 rows of K 2,048 /
-    // 3,072, 4 tokens 8.1 / 11.1 -> 6.0 / 8.2 us, 16 tokens 16.4 / 23.4 -> 11.5 / 15.3; 4,096 rows of K 1,024 would lose, 4 tokens 7.1
-    // -> 8.0, 16 tokens 14.3 -> 23.8)
+    // blocks of 16 weight rows once they fill the SMs twice, else of 8
     if (N >= 16 * 296) return run(integral_constant<int, 16>(), integral_constant<int, 3>());
-    if (MT >= 4 && (unsigned)(N + 7) / 8 * y <= 148) return run(integral_constant<int, 8>(), integral_constant<int, 8>());
+    if (few_looks_far(MT, (unsigned)(N + 7) / 8 * y)) return run(integral_constant<int, 8>(), integral_constant<int, 8>());
     return run(integral_constant<int, 8>(), integral_constant<int, 3>());
 }
 
@@ -603,6 +616,9 @@ int launch(const void* A, int lda, const void* W, int ldw, const float* bias, vo
 }  // namespace ember
 
 using namespace ember;
+
+// Whether a float32 product of few tokens, `mt` of them a block, looks eight stages ahead (host only).
+EMBER_API int ember_gemm_f32_few_looks_far(int mt, int blocks) { return few_looks_far(mt, (unsigned)blocks) ? 1 : 0; }
 
 EMBER_API int ember_gemm_simt(const void* A, int a_dtype, int lda, const void* W, int w_dtype, int ldw,
                               const float* bias, void* C, int ldc, int M, int N, int K, int epilogue, int settled, void* stream) {

@@ -61,3 +61,23 @@ def test_pairs_or_single_sms_for_heads(lib, matrix, times):
 @pytest.mark.parametrize("tokens,n,k", [(511, 6144, 4096), (1024, 6144, 1016), (1024, 896, 4096)])
 def test_single_sms_for_heads_below_what_was_measured(lib, tokens, n, k):
     assert not lib.ember_gemm_tc_qkv_on_pairs(tokens, n, k, 148, 74)
+
+
+# float32 products of few tokens: tokens a block, columns: {blocks: (us with three stages, us with eight)}
+FEW = [
+    (4, 2048, {16: (5.7, 4.7), 56: (6.5, 5.6), 74: (6.1, 4.9), 128: (9.0, 5.9), 148: (6.3, 5.4)}),
+    (8, 2048, {56: (9.0, 7.9), 128: (12.8, 8.2), 146: (12.4, 8.1), 192: (12.5, 14.5)}),
+    (16, 1024, {8: (5.7, 6.4), 37: (5.6, 6.5), 64: (7.7, 6.6), 74: (5.6, 6.6), 128: (9.3, 7.0), 148: (5.7, 6.8), 192: (9.4, 11.9)}),
+    (16, 2048, {8: (9.7, 10.9), 32: (9.9, 10.9), 64: (13.7, 11.1), 74: (9.7, 11.2), 147: (16.8, 11.6), 148: (9.8, 11.6), 149: (16.6, 18.9)}),
+    (16, 3072, {16: (13.8, 14.9), 64: (19.7, 14.9), 148: (13.9, 15.4)}),
+]
+
+
+@pytest.mark.parametrize("tokens,columns,times", FEW, ids=lambda v: str(v) if isinstance(v, int) else "")
+def test_how_far_products_of_few_tokens_look_ahead(tokens, columns, times):
+    try:
+        far = build.load("gemm_simt").ember_gemm_f32_few_looks_far
+    except (build.BuildError, OSError) as e:
+        pytest.skip(f"the product's library cannot be built or loaded here: {e}")
+    for blocks, us in times.items():
+        assert us[far(tokens, blocks)] <= 1.05 * min(us), (tokens, columns, blocks)
