@@ -371,12 +371,9 @@ gemm_f32_many_kernel(const float* __restrict__ A, int lda, const float* __restri
 // the tokens; operands lie k-major, brought by 4-byte copies whose 8 k x 4 rows fall into 32 banks into a ring of three
 // stages that the two warps of a part share.  The parts of a tile meet in distributed shared memory, every block finishes
 // a quarter of its tokens.  The sums are those of the kernel above, in its order.
-// us, kernel above -> this, at (N, K) = (1,024, 2,048), (1,024, 3,072), (2,048, 2,048): 64 tokens 37 -> 31, 53 -> 44, 38 -> 34; 128
-// tokens 37 -> 34, 54 -> 47, 38 -> 35; 300 tokens 68 -> 50, 98 -> 71, 103 -> 80; 2,048 tokens 247 -> 234, 358 -> 330, 488 -> 449.
-// From 4,096 columns on it is ahead where rows of 64 are full (300 tokens x 4,096 x 1,024: 93 -> 88) and behind where they are not
-// (65 tokens x 6,144 x 1,024: 37 -> 53), so those stay with the kernel above.  Neither gets beyond 34 TFLOP/s: the same sums by
-// plain multiply-adds take 119 us where these take 88, and operands loaded 16 bytes at a time into registers and stored
-// turned 104.
+// Where it is ahead and where not: clusters_are_faster.  It reaches 39 TFLOP/s (2,048 tokens x 1,024 x 3,072), the kernel above 36:
+// neither gets to the FMA pipes' 74.  The same sums by plain multiply-adds take 119 us where these take 88 (300 tokens x 4,096 x
+// 1,024), and operands loaded 16 bytes at a time into registers and stored turned 104.
 constexpr int NARROW_T = 64, NARROW_N = 64, NARROW_K = 16, NARROW_STAGES = 3, NARROW_CLUSTER = 4, NARROW_PARTS = KPARTS / NARROW_CLUSTER;
 constexpr int NARROW_ROW = NARROW_N + 4;                          // floats of a k in a stage's operand, and of a row of sums
 constexpr int NARROW_STAGE = 2 * NARROW_K * NARROW_ROW;           // floats
@@ -536,8 +533,6 @@ int launch_f32(Kernel kernel, dim3 grid, int threads, size_t smem, cudaStream_t 
 //           4,096 x 1,024  29 / 24  28 / 25     6,144 x 1,024  23 / 20  22 / 20    12,288 x 2,048  77 / 68  76 / 70
 //         151,936 x 1,024  432 / 303  426 / 317
 constexpr int FEW_TOKENS = 32, FEW_TOKENS_WIDE = 16, WIDE_COLUMNS = 4096;
-// More than 32 tokens: the kernel of clusters up to this many columns (its comment has both sides).
-constexpr int NARROW_COLUMNS = 2048;
 
 // Whether the kernel for few looks eight stages ahead instead of three, with blocks of 8 weight rows.  Where an SM has no more than one
 // block, its two warps are all that fetches there (the rings of 16 tokens also leave no room for a second one; three stages
@@ -570,6 +565,29 @@ int launch_few(const float* A, int lda, const float* W, int ldw, const float* bi
     return run(integral_constant<int, 8>(), integral_constant<int, 3>());
 }
 
+// More than 32 tokens: whether clusters are the faster kernel.  The chip takes 148 tiles of the kernel for many at a time (32 tokens x 64
+// columns) and 70 clusters (64 x 64; 71 and 72 are seen to leave some for a second turn), so they lose where the 64 tokens
+// put them into one more turn than their halves.  us, many / clusters, K 1,024:
+//   columns      512           1,024         1,280         1,536         2,048         2,304
+//   65 tokens    20.0 / 18.9   19.9 / 19.4   19.9 / 19.7                 20.2 / 19.7   20.1 / 25.8
+//   200          19.9 / 19.5   20.0 / 20.0   20.0 / 27.9   37.1 / 28.9   38.6 / 38.1   38.9 / 43.6
+//   280          19.9 / 20.0   20.0 / 29.1   38.3 / 29.6   38.6 / 38.9   38.9 / 45.9
+//   300          20.2 / 20.0   37.1 / 29.3   38.6 / 30.1                 55.8 / 46.2   56.9 / 53.7
+//   520          20.0 / 27.2   39.0 / 43.7   56.8 / 52.5   57.5 / 60.7   75.9 / 78.2
+//   1,024        39.1 / 39.7   76.2 / 70.9   94.5 / 87.4                 133 / 131     151 / 147
+// (K 3,072: 53.9 / 48.3 for 1,024 columns and 200 tokens, 53.8 / 70.2 for 280.)  From 2,304 columns on they are ahead for 300 tokens and
+// more (up to 17 %) and far behind for 65 to 200.  Over 592 products of 64 to 2,048 columns, K 1,024 to 3,072, the choice is
+// within 0.1 % of the better kernel on average and at most 4.1 % off; clusters throughout were 2.5 % off, at most 47 %.
+// Short K does not pay for the cluster's barriers: at K 64 to 256 they are 3 to 127 % slower (39 % on average), at 512 up to 72 %
+// except for a few of them (8 clusters and fewer: 3 to 19 % faster).
+constexpr int NARROW_COLUMNS = 2048, NARROW_AT_ONCE = 70;
+static bool clusters_are_faster(int M, int N, int K) {
+    if (N > NARROW_COLUMNS || K < 512) return false;
+    const long long cols = (N + NARROW_N - 1) / NARROW_N, tiles = cols * ((M + MANY_M - 1) / MANY_M), clusters = cols * ((M + NARROW_T - 1) / NARROW_T);
+    if (K < 1024) return clusters <= 8;
+    return tiles > 3 * EVEN_BLOCKS || clusters <= NARROW_AT_ONCE * ((tiles + EVEN_BLOCKS - 1) / EVEN_BLOCKS);
+}
+
 int launch_pieces(const float* A, int lda, const float* W, int ldw, const float* bias, float* C, int ldc, int M, int N, int K, int epi,
                   int settled, cudaStream_t st) {
     if (M <= 1) return launch_few<1>(A, lda, W, ldw, bias, C, ldc, M, N, K, epi, settled, st);
@@ -578,7 +596,7 @@ int launch_pieces(const float* A, int lda, const float* W, int ldw, const float*
     if (M <= 8) return launch_few<8>(A, lda, W, ldw, bias, C, ldc, M, N, K, epi, settled, st);
     if (M <= (N >= WIDE_COLUMNS ? FEW_TOKENS_WIDE : FEW_TOKENS)) return launch_few<16>(A, lda, W, ldw, bias, C, ldc, M, N, K, epi, settled, st);
     // a grid has at most 65,535 rows of blocks, half as many tokens here as the 64-row tiles of the general kernel take
-    const bool narrow = M > 32 && N <= NARROW_COLUMNS;
+    const bool narrow = clusters_are_faster(M, N, K);
     constexpr int ROWS = 65535 * MANY_M;
     for (long long m = 0; m < M; m += ROWS) {
         const int rows = M - m < ROWS ? (int)(M - m) : ROWS;
@@ -619,6 +637,9 @@ using namespace ember;
 
 // Whether a float32 product of few tokens, `mt` of them a block, looks eight stages ahead (host only).
 EMBER_API int ember_gemm_f32_few_looks_far(int mt, int blocks) { return few_looks_far(mt, (unsigned)blocks) ? 1 : 0; }
+
+// ... and whether one of more tokens goes to clusters.
+EMBER_API int ember_gemm_f32_clusters(int M, int N, int K) { return clusters_are_faster(M, N, K) ? 1 : 0; }
 
 EMBER_API int ember_gemm_simt(const void* A, int a_dtype, int lda, const void* W, int w_dtype, int ldw,
                               const float* bias, void* C, int ldc, int M, int N, int K, int epilogue, int settled, void* stream) {

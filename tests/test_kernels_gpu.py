@@ -163,11 +163,12 @@ def test_gemm_f32_kernels_share_one_order(N, K, epilogue):
 
 
 @pytest.mark.parametrize("M", [33, 63, 64, 65, 128, 129, 300])
-@pytest.mark.parametrize("N,K", [(2, 4), (62, 260), (64, 1024), (1024, 1000), (2046, 132), (2048, 2048), (2050, 132)])
+@pytest.mark.parametrize("N,K", [(2, 4), (62, 260), (64, 1024), (1024, 1000), (2046, 132), (2048, 2048), (2050, 132),
+                                 (2, 1028), (60, 516), (62, 1100), (1022, 1036), (1278, 1504), (2046, 1032), (2050, 1032)])
 @pytest.mark.parametrize("epilogue", [0, 2, 3])
 def test_gemm_f32_narrow(M, N, K, epilogue):
-    """float32 products of more than 32 tokens on both sides of the line between the two kernels (2,048 columns) and at the
-    edges of their tiles: the bits that single tokens get."""
+    """float32 products of more than 32 tokens on both sides of the lines between the two kernels (2,048 columns, K of 512 and
+    1,024, full turns) and at the edges of their tiles: the bits that single tokens get."""
     from ember_b200 import ops
     torch.manual_seed(N + K + M)
     a, w, bias = torch.randn(M, K, device="cuda"), torch.randn(N, K, device="cuda"), torch.randn(N, device="cuda")

@@ -81,3 +81,30 @@ def test_how_far_products_of_few_tokens_look_ahead(tokens, columns, times):
         pytest.skip(f"the product's library cannot be built or loaded here: {e}")
     for blocks, us in times.items():
         assert us[far(tokens, blocks)] <= 1.05 * min(us), (tokens, columns, blocks)
+
+
+# float32 products of more tokens: (rows, columns of the matrix): {tokens: (us on tiles, us on clusters)}
+MANY = [
+    ((512, 1024), {65: (20.0, 18.9), 280: (19.9, 20.0), 520: (20.0, 27.2), 600: (37.2, 29.0), 1100: (39.1, 44.1)}),
+    ((768, 1024), {340: (20.0, 27.5), 410: (37.8, 29.2), 720: (39.1, 44.6), 2048: (112.7, 98.1)}),
+    ((1024, 1024), {200: (20.0, 20.0), 280: (20.0, 29.1), 300: (37.1, 29.3), 520: (39.0, 43.7), 640: (57.1, 46.2)}),
+    ((1280, 1024), {200: (20.0, 27.9), 300: (38.6, 30.1), 1024: (94.5, 87.4)}),
+    ((1536, 1024), {160: (20.0, 27.8), 200: (37.1, 28.9), 340: (38.9, 44.6)}),
+    ((2048, 1024), {150: (37.3, 29.5), 280: (38.9, 45.9), 300: (55.8, 46.2), 1024: (133.0, 131.3)}),
+    ((1280, 3072), {200: (54.0, 69.1), 300: (103.2, 71.8), 2048: (456.4, 413.4)}),
+    ((64, 1024), {33: (19.4, 12.7), 640: (19.9, 14.3)}),
+    ((2304, 1024), {65: (20.1, 25.8), 200: (38.9, 43.6)}),
+]
+
+
+@pytest.mark.parametrize("matrix,times", MANY, ids=lambda v: "x".join(map(str, v)) if isinstance(v, tuple) else "")
+def test_tiles_or_clusters(matrix, times):
+    try:
+        clusters = build.load("gemm_simt").ember_gemm_f32_clusters
+    except (build.BuildError, OSError) as e:
+        pytest.skip(f"the product's library cannot be built or loaded here: {e}")
+    for tokens, us in times.items():
+        assert us[clusters(tokens, *matrix)] <= 1.05 * min(us), (matrix, tokens)
+    n = matrix[0]
+    assert not any(clusters(m, n, k) for m in (33, 64, 300, 2048) for k in (64, 256, 508))
+    assert clusters(33, 64, 512) and not clusters(280, 1024, 512)
