@@ -70,8 +70,8 @@ struct FaParams {
     const float* sink;        // [n_heads] or null: exp(sink[h]) joins the denominator, without key and value
     float raw_per_slope;      // what a slope of 1 is in the units of the scores as they come: 1 / scale, or log2(e) behind a cap
     int n_tiles;
-    unsigned long long* released;      // where the kernel behind this one finds `ticket` once this one's inputs are there, or null
-    unsigned long long ticket;         // (a number of its own for each launch)
+    int* released;            // where the kernel behind this one finds `ticket` once this one's inputs are there, or null
+    int ticket;               // (a number of its own for each launch)
     int* err;
 };
 
@@ -710,7 +710,7 @@ EMBER_API int ember_attention_fa_tile_queries(int group) { return group >= 1 && 
 EMBER_API int ember_attention_fa(const void* q, const void* k_pool, const void* v_pool, void* out, int n_heads, int n_kv,
                                  int D, const int* tiles, int n_tiles, const int* block_table, int max_blocks, int page,
                                  int num_pages, int window, float scale, int* err, float softcap, int chunk, const float* gate, int ld_gate,
-                                 const float* slopes, const float* sink, unsigned long long* released, unsigned long long ticket, void* stream) {
+                                 const float* slopes, const float* sink, int* released, int ticket, void* stream) {
     if (n_tiles <= 0) return 0;
     if (gate && ((((uintptr_t)gate) & 15) || ld_gate < n_heads * FA_D || (ld_gate & 3))) return fail("attention_fa: gate rows of %d", ld_gate);
     if (n_heads <= 0 || n_kv <= 0 || n_heads % n_kv) return fail("attention_fa: bad head counts %d/%d", n_heads, n_kv);
@@ -729,7 +729,7 @@ EMBER_API int ember_attention_fa(const void* q, const void* k_pool, const void* 
     p.cap_log2 = softcap * FA_LOG2E;
     p.cap_z = softcap > 0.0f ? scale / softcap : 0.0f;
     p.cap_arg = softcap > 0.0f ? 2.0f * FA_LOG2E * scale / softcap : 0.0f; p.gate = gate; p.ld_gate = ld_gate; p.n_tiles = n_tiles; p.err = err;
-    p.released = released && !is_capturing((cudaStream_t)stream) ? released : nullptr; p.ticket = ticket;
+    p.released = released; p.ticket = ticket;
     p.slopes = slopes; p.sink = sink; p.raw_per_slope = softcap > 0.0f ? FA_LOG2E : 1.0f / scale;
     auto run = [&](auto kernel, bool& ready) -> int {
         if (!ready) {

@@ -56,8 +56,8 @@ struct AttnTcParams {
     const float* sink;        // [n_heads] or null: exp(sink[h]) joins the denominator once, without key and value
     int n_splits, split_keys;
     int n_tiles;
-    const unsigned long long* released;      // decode: where attention_fa, launched directly before, leaves `ticket` once what both read is there, or null
-    unsigned long long ticket;
+    const int* released;      // decode: where attention_fa, launched directly before, leaves `ticket` once what both read is there, or null
+    int ticket;
     int settled;              // decode: nothing that may still run writes keys or pages before the tile's position
     int cluster_merge;        // the splits of a tile are a thread-block cluster and are merged in its first block's shared memory
     int* err;
@@ -666,7 +666,7 @@ EMBER_API int ember_attention_tc(const void* q, const void* k_pool, const void* 
                                  const int* block_table, int max_blocks, int page, int num_pages, int window,
                                  float scale, int n_splits, int split_keys, float* part_o, float* part_ml,
                                  int* err, float softcap, int chunk, const float* gate, int ld_gate, const float* slopes, const float* sink, int settled,
-                                 const unsigned long long* released, unsigned long long ticket, void* stream) {
+                                 const int* released, int ticket, void* stream) {
     if (n_tiles <= 0) return 0;
     if (gate && ld_gate < n_heads * D) return fail("attention_tc: gate rows of %d", ld_gate);
     if (softcap < 0.0f) return fail("attention_tc: a score cap of %g", softcap);

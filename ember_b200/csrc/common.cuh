@@ -63,15 +63,15 @@ __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepc
 // semantics, and the other reads it with acquire semantics: all that the first had waited for happens before what the second
 // does then (other threads of its block: behind a block barrier).  Each launch has a ticket of its own, and who does not
 // find it waits with pdl_wait(): this decides, it never spins.
-__device__ __forceinline__ void release_ticket(unsigned long long* at, unsigned long long ticket) {
-    asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(at), "l"(ticket) : "memory");
+__device__ __forceinline__ void release_ticket(int* at, int ticket) {
+    asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(at), "r"(ticket) : "memory");
 }
-__device__ __forceinline__ unsigned long long acquire_ticket(const unsigned long long* at) {
-    unsigned long long v;
-    asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(at) : "memory");
+__device__ __forceinline__ int acquire_ticket(const int* at) {
+    int v;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(at) : "memory");
     return v;
 }
-// A captured launch would find the ticket of the replay before: none there.
+// A captured launch that looks for a ticket would find the one of the replay before: it is given none.
 inline bool is_capturing(cudaStream_t stream) {
     cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(stream, &status) != cudaSuccess) { cudaGetLastError(); return true; }

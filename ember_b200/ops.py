@@ -8,7 +8,7 @@ from __future__ import annotations
 
 import ctypes
 import itertools
-from ctypes import c_float, c_longlong, c_ulonglong, c_void_p
+from ctypes import c_float, c_longlong, c_void_p
 from operator import index
 from typing import Optional
 
@@ -632,24 +632,16 @@ def _check_element_gate(gate, col: int, n: int) -> None:
             raise KernelError(f"attention: a gate of {tuple(gate.shape)} from column {col} for {n} elements a token")
 
 
-_TICKET_SLOTS = 64
+_TICKET_WORDS = 64
 _tickets = itertools.count(1)
-_ticket_slots = {}          # a device's words that its tickets are left in, taken in turn
-_released = None            # (stream, launches up to it, word, ticket) of the last ``attention_fa`` with ``release_late``
+_ticket_words = {}          # a device's words that its tickets are left in, taken in turn: (the tensor, their addresses)
+_released = (None, 0, None, 0)            # stream, launches up to it, word and ticket of the last ``attention_fa`` with ``release_late``
+_NO_WORD = c_void_p(0)
 
 
-def _new_ticket(device):
-    slots = _ticket_slots.get(device)
-    if slots is None:
-        slots = _ticket_slots.setdefault(device, torch.zeros(_TICKET_SLOTS, dtype=torch.int64, device=device))
-    ticket = next(_tickets)
-    return slots.data_ptr() + 8 * (ticket % _TICKET_SLOTS), ticket
-
-
-def _ticket_before(stream: int):
-    """The ticket of an ``attention_fa`` on ``stream`` behind which no kernel of this library has been launched, else none."""
-    last = _released
-    return last[2:] if last is not None and last[:2] == (stream, _launches) else (0, 0)
+def _ticket_words_of(device: int):
+    t = torch.zeros(_TICKET_WORDS, dtype=torch.int32, device=device if device >= 0 else "cpu")
+    return _ticket_words.setdefault(device, (t, [c_void_p(t.data_ptr() + 4 * i) for i in range(_TICKET_WORDS)]))
 
 
 def attention_fa(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, out: torch.Tensor, n_heads: int,
@@ -678,12 +670,15 @@ def attention_fa(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, ou
     lib = _lib("attention_fa")
     if stream is None:
         stream = current_stream_ptr()
-    word, ticket = _new_ticket(q.device) if release_late else (0, 0)
+    word, ticket = _NO_WORD, 0
+    if release_late:
+        ticket = next(_tickets) & 0x3fffffff       # (a word is overwritten many times before a number comes again)
+        word = (_ticket_words.get(q.get_device()) or _ticket_words_of(q.get_device()))[1][ticket % _TICKET_WORDS]
     _call(lib, lib.ember_attention_fa, _p(q), _p(k_pool), _p(v_pool), _p(out), c_int(n_heads), c_int(n_kv), c_int(head_dim),
           _p(tiles), c_int(n_tiles), _p(block_table), c_int(block_table.shape[-1]), c_int(page), c_int(k_pool.shape[0]),
           c_int(window), c_float(scale), _p(err), c_float(softcap), c_int(chunk),
           (_off(gate, gate_col) if gate is not None else c_void_p(0)), c_int(gate.shape[-1] if gate is not None else 0),
-          _p(slopes), _p(sink), c_void_p(word), c_ulonglong(ticket), c_void_p(stream))
+          _p(slopes), _p(sink), word, ticket, c_void_p(stream))
     if release_late:
         _released = (stream, _launches, word, ticket)
 
@@ -726,12 +721,16 @@ def attention_tc(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, ou
     lib = _lib("attention_tc")
     if stream is None:
         stream = current_stream_ptr()
-    word, ticket = _ticket_before(stream) if beside else (0, 0)
+    word, ticket = _NO_WORD, 0
+    if beside:
+        last = _released
+        if last[1] == _launches and last[0] == stream:      # (no kernel of this library has been launched since)
+            word, ticket = last[2], last[3]
     _call(lib, lib.ember_attention_tc, _p(q), _p(k_pool), _p(v_pool), _p(out), c_int(mode), c_int(n_heads), c_int(n_kv),
           c_int(head_dim), _p(tiles), c_int(n_tiles), _p(block_table), c_int(block_table.shape[-1]), c_int(page),
           c_int(k_pool.shape[0]), c_int(window), c_float(scale), c_int(n_splits), c_int(split_keys), _p(part_o),
           _p(part_ml), _p(err), c_float(softcap), c_int(chunk), (_off(gate, gate_col) if gate is not None else c_void_p(0)),
-          c_int(gate.shape[-1] if gate is not None else 0), _p(slopes), _p(sink), c_int(1 if keys_settled else 0), c_void_p(word), c_ulonglong(ticket),
+          c_int(gate.shape[-1] if gate is not None else 0), _p(slopes), _p(sink), c_int(1 if keys_settled else 0), word, ticket,
           c_void_p(stream))
 
 
