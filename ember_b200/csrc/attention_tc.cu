@@ -134,7 +134,9 @@ __device__ __forceinline__ uint32_t swz(int row, int chunk) { return (uint32_t)(
 
 // HALVES = head_dim / 64.  DECODE: warps split the keys of a tile; else warps split the rows.  BIAS: slopes and a sink may
 // be there.
-template <int HALVES, bool DECODE, bool BIAS>
+// BESIDE: beside the step's prompt portions, see below; an instance of its own, so that other decode steps do without its branches.
+// (The wait at the end stands in all of them: without it, never taken, a decode step of 28 layers takes 1,191 us instead of 1,188.)
+template <int HALVES, bool DECODE, bool BIAS, bool BESIDE = false>
 __global__ void __launch_bounds__(ATC_THREADS)
 attention_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
                     const AttnTcParams p) {
@@ -225,7 +227,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
     // still runs: a layer's attention took 9.9, 25.1 and 43.9 us (one request at 700 keys, 8 at 3,072, 64 at 1,024), now 8.3,
     // 23.4, 39.1.
     int early = 0;
-    if (DECODE && warp == 4 && (p.settled || !p.released)) {
+    if (DECODE && warp == 4 && (!BESIDE || p.settled)) {
         if (!p.settled) pdl_wait();
         early = min(min(n_kt, NSTAGE), max(0, (pos0 - k_begin) / KT));
         for (int it = 0; it < early; it++) fetch_tile(it, page_row(it));
@@ -235,7 +237,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
     // time: one streams the cache, the other computes (eight layers of 32/8 heads, 512 tokens behind 512 keys beside 48
     // requests of 600 to 1,200: 2,834 us a step one after the other, 2,709 to 2,749 side by side).
     bool there = false;
-    if (DECODE && p.released) {
+    if (BESIDE) {
         there = __syncthreads_or(threadIdx.x == 0 && acquire_ticket(p.released) == p.ticket);
         if (there) asm volatile("fence.proxy.async.global;" ::: "memory");      // (the newest key's page is fetched by TMA)
     }
@@ -527,7 +529,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
                 __float2bfloat16_rn(gated(gate_row, r * D + d, acc * with_sink(BIAS ? p.sink : nullptr, kvh * G + r, M, L)));
         }
     }
-    if (there) pdl_wait();      // (so that who waits for this kernel waits for the one beside it, too)
+    if (p.released) pdl_wait();      // (so that who waits for this kernel waits for the one beside it, too)
 }
 
 // Merges split partials in ascending order (same arithmetic as attention.cu's combine).  The maxima and
@@ -726,9 +728,11 @@ EMBER_API int ember_attention_tc(const void* q, const void* k_pool, const void* 
     };
     int rc;
     if (slopes || sink) {
-        if (D == 128) rc = mode == 1 ? run(attention_tc_kernel<2, true, true>) : run(attention_tc_kernel<2, false, true>);
+        if (D == 128 && p.released) rc = run(attention_tc_kernel<2, true, true, true>);
+        else if (D == 128) rc = mode == 1 ? run(attention_tc_kernel<2, true, true>) : run(attention_tc_kernel<2, false, true>);
         else rc = mode == 1 ? run(attention_tc_kernel<1, true, true>) : run(attention_tc_kernel<1, false, true>);
-    } else if (D == 128) rc = mode == 1 ? run(attention_tc_kernel<2, true, false>) : run(attention_tc_kernel<2, false, false>);
+    } else if (D == 128 && p.released) rc = run(attention_tc_kernel<2, true, false, true>);
+    else if (D == 128) rc = mode == 1 ? run(attention_tc_kernel<2, true, false>) : run(attention_tc_kernel<2, false, false>);
     else rc = mode == 1 ? run(attention_tc_kernel<1, true, false>) : run(attention_tc_kernel<1, false, false>);
     if (rc) return rc;
     if (n_splits > 1 && !cluster_merge) {

@@ -351,7 +351,8 @@ def attention(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, out: 
 # -------------------------------------------------------------------------------- sampling
 def sample(logits: torch.Tensor, params: torch.Tensor, out: torch.Tensor, rows: int,
            stream: Optional[int] = None) -> None:
-    """out[r] = token drawn from logits[r] under the packed 32-byte parameter row r."""
+    """out[r] = token drawn from logits[r] under the packed 32-byte parameter row r, which is read on the device when the kernel
+    runs: in a captured graph, whose rows are to change between replays, this is the form."""
     _check(logits, "logits", torch.float32)
     _check(params, "params", torch.uint8)
     _check(out, "out", torch.int32)
@@ -363,7 +364,8 @@ def sample(logits: torch.Tensor, params: torch.Tensor, out: torch.Tensor, rows: 
 
 
 def sample_host(logits: torch.Tensor, params: bytes, out: torch.Tensor, rows: int, stream: Optional[int] = None) -> None:
-    """The same with the parameter rows on the host (``bytes``, read before this returns): they travel with the launch."""
+    """The same with the parameter rows on the host (``bytes``, read before this returns): they travel with the launch, and a
+    captured launch keeps them."""
     _check(logits, "logits", torch.float32)
     _check(out, "out", torch.int32)
     if logits.dim() != 2 or logits.shape[0] < rows or len(params) < rows * 32 or out.numel() < rows:
