@@ -543,7 +543,7 @@ constexpr int FEW_TOKENS = 32, FEW_TOKENS_WIDE = 16, WIDE_COLUMNS = 4096;
 //   9 to 16         9.8 / 11.1    9.9 / 10.9   12.5 / 11.2    9.7 / 11.2   16.8 / 11.5   16.7 / 11.6    9.8 / 11.6   17.0 / 20.4
 // and alike at K 64 to 6,144.  Up to 8 tokens it does for 148 blocks and fewer (up to 5 % behind where blocks are few), beyond them not
 // (3,072 rows of K 1,024, 4 tokens 6.3 / 7.6); 9 to 16 tokens from 52 blocks on (44 and 48: 10 % ahead to 10 % behind), but not
-// where a grid of 74 or 148 blocks is even by itself.  One and two tokens are up to 36 % ahead from 88 blocks on and up to 12 %
+// where a grid of 74 or 148 blocks is even by itself.  One and two tokens are up to 36 % ahead from 96 blocks on and up to 12 %
 // behind below; they have not been given it yet.
 constexpr unsigned EVEN_BLOCKS = 148;          // a block an SM
 static bool few_looks_far(int MT, unsigned blocks) {
